@@ -21,25 +21,23 @@
 //   split into BF16 hi + lo (lo = bf16(v - hi)); the signal planes are stored
 //   as consecutive 128-byte blocks of 64 samples in the 128-byte-swizzle
 //   K-major layout, whose 8-row atoms have a 128-byte row pitch, so with the
-//   descriptor starting at block kb row a reads block a + kb.  B rows 0..63
-//   hold g_hi by phase, rows 64..127 g_lo:
-//     MMA 1: D[:, 0:128] += A_hi x B        (x_hi*g_hi | x_hi*g_lo)
-//     MMA 2: D[:, 0:128] += A_lo x B        (x_lo*g_hi | x_lo*g_lo)
-//     y[j0 + 64a + b] = D[a][b] + D[a][64 + b]
+//   descriptor starting at block kb row a reads block a + kb.  B's 128 rows hold
+//   g_hi and g_lo by phase in alternate groups of eight (bfBand):
+//     MMA 1: D += A_hi x B        (x_hi*g_hi | x_hi*g_lo)
+//     MMA 2: D += A_lo x B        (x_lo*g_hi | x_lo*g_lo)
+//     y[j0 + 64a + b] = D[a][column of g_hi, b] + D[a][column of g_lo, b]
 //   The three products hi*hi, hi*lo, lo*hi leave the lo*lo term (2^-16 of each
 //   product) out, 1.25e-5 of the peak output on the 256-tap FIR workload; the
 //   fourth rides in the same MMA (N = 128 instead of 64 for the lo plane) at no
 //   measurable cost here (the tile loop is not MMA-bound) and brings it to 8.7e-6.
 //
-// Each CTA owns consecutive tiles of one channel: the taps are staged into
-// shared memory once and the band built from there; the next tile's signal is
-// staged into the second buffer while the tensor core works on the current
-// one.  The integer kernel is persistent: one wave of CTAs strides over the
-// (channel, tile range) work items, keeps a band of shared taps for all of them
-// and fetches each item's first segment during the previous item's last tile.
+// All kernels are persistent: one wave of CTAs strides over runs of consecutive tiles of one
+// channel.  The integer kernel keeps a band of shared taps for all of a CTA's runs
+// and fetches each run's first segment during the previous run's last tile.
 // All waits on the tensor core are bounded; on expiry the kernel sets the error word it
 // was given (the calling handle's or plan's), frees its TMEM and exits.
 #include <algorithm>
+#include <climits>
 #include <cstdio>
 
 #include <cuda_bf16.h>
@@ -501,24 +499,14 @@ constexpr int kBfTile = kRows * kBfPhases;
 constexpr int kBfMaxTaps = kFirBfMaxTaps;
 static_assert(kBfTile == kFirBfTile, "ragged run tiles and kernel tiles must agree");
 constexpr int kBfThreads = 512;
-constexpr int kBfPadLeft = 64; // zero taps ahead of the reversed taps (phase offsets)
 
 __host__ __device__ constexpr int bfK(int T) { return ((63 + T + 15) / 16) * 16; }
 __host__ __device__ constexpr int bfBlocks(int T) { return kRows + (bfK(T) + 63) / 64; }
 // 16-byte plane chunks staged per thread by bfStage
 constexpr int kBfChunksPerThread = (bfBlocks(kBfMaxTaps) * 8 + kBfThreads - 1) / kBfThreads;
-__host__ __device__ constexpr int bfTapSlots(int T) { return kBfPadLeft + bfK(T) + 8; }
 
-__device__ __forceinline__ void splitBf16(float v, uint16_t &hi, uint16_t &lo)
-{
-   const __nv_bfloat16 h = __float2bfloat16_rn(v);
-   const __nv_bfloat16 l = __float2bfloat16_rn(v - __bfloat162float(h));
-   hi = __bfloat16_as_ushort(h);
-   lo = __bfloat16_as_ushort(l);
-}
-
-// The same for two values at once, packed (a in the low half): one paired conversion
-// per plane, rounding each value exactly as splitBf16 does.
+// Two values as BF16 hi + lo (lo = bf16(v - hi)), packed (a in the low half): one paired
+// conversion per plane.
 __device__ __forceinline__ void splitBf16x2(float a, float b, uint32_t &hi, uint32_t &lo)
 {
    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
@@ -579,36 +567,6 @@ __device__ __forceinline__ void bfStage(const float *x, long long q0, long long 
    }
 }
 
-// Raw FP32 tiles (nb blocks of 64 samples) are bulk-copied by the TMA engine
-// when the whole tile lies inside the input and is 16-byte aligned, then split
-// in shared memory; other tiles (row edges, unaligned rows) are staged by the
-// threads straight into the planes (bfStage).
-// Split a raw tile into the signal planes: sample i (64 per 128-byte block
-// k = i / 64) goes to block k, 16-byte chunk c = (i % 64) / 8 stored at
-// k*128 + ((c ^ (k & 7)) * 16), as hi and lo BF16.  Sample i is raw[mis + i]
-// (mis < 4: the bulk copy started at the 16-byte boundary below the tile).  A
-// thread takes 4 samples (consecutive lanes, consecutive addresses) and writes
-// half a chunk of each plane.
-__device__ __forceinline__ void bfSplit(const float *raw, int mis, int nb, unsigned char *Ahi, unsigned char *Alo,
-                                        int tid)
-{
-   for (int f = tid; f < nb * 16; f += kBfThreads) {
-      float4 v;
-      if (mis == 0) v = ((const float4 *) raw)[f];
-      else {
-         const float *p = raw + mis + 4 * f;
-         v = make_float4(p[0], p[1], p[2], p[3]);
-      }
-      const int k = f >> 4, c = (f >> 1) & 7, half = f & 1;
-      uint2 hv, lv;
-      splitBf16x2(v.x, v.y, hv.x, lv.x);
-      splitBf16x2(v.z, v.w, hv.y, lv.y);
-      const int off = k * 128 + ((c ^ (k & 7)) << 4) + half * 8;
-      *(uint2 *) (Ahi + off) = hv;
-      *(uint2 *) (Alo + off) = lv;
-   }
-}
-
 // A run of consecutive output tiles [t0, t1) of one channel:
 //     y[j] = sum_{c<T} x[inShift + j + c] * g(c),  x zero outside [0, inLen),
 //     g(c) = h[T-1-c] (reverse = 1: DSPLIB_fir correlation order) or h[c] (reverse = 0).
@@ -618,424 +576,464 @@ struct BfRun {
    float *y;
    long long inShift, inLen;
    int outLen, T, reverse, t0, t1;
-   int *err; // error word for an expired bounded wait
 };
 
-// Shared memory for taps up to Tmax: two sets of hi/lo signal planes (tile t is
-// split into set t % 2 while the tensor core reads the other; a drained tile's set
-// also stages its output), a ring of raw FP32 tiles fetched by the TMA engine ahead
-// of their split (up to two when they fit beside the band, none for the longest
-// taps: those tiles are staged by the threads straight from global memory), the
-// taps band and the split taps.  Two accumulators of 128 TMEM columns each.
-//
-// Warp roles: warps 0-15 (the workers) build the band, split tiles into the planes
-// and drain the accumulators; warp 16 issues the MMAs.  The issuing thread may stall
-// in tcgen05.mma while the tensor core is busy, so it has a warp of its own.
-// Handshakes: planesFull[b] (a worker arrives once plane set b holds a tile and
-// accumulator b is free) and mmaDone[b] (tcgen05.commit once the MMAs reading set b
-// and writing accumulator b completed); the workers synchronise among themselves on
-// named barrier 1.
-constexpr size_t kBfSmemLimit = 227 * 1024;
-constexpr uint32_t kBfTmemCols = 256;
-constexpr int kBfWorkers = kBfThreads;         // worker threads (16 warps)
-constexpr int kBfBlock = kBfWorkers + 32;      // + the MMA warp
-constexpr uint32_t kBfBar = 1;                 // the workers' named barrier
-// Layout for taps up to T (the batched kernels lay out shared memory per run, for that
-// run's taps, in an allocation of kBfSmemLimit): the barriers and the TMEM slot in the
-// first 1024 bytes, then the plane sets, the raw ring, the band and the split taps.
-__host__ __device__ constexpr size_t bfPlaneBytes(int T) { return (size_t) ((bfBlocks(T) * 128 + 1023) & ~1023); }
-// a raw tile and the up to 3 samples before it (copies start on a 16-byte boundary),
-// padded to 128 bytes so that the band behind the ring keeps its 128-byte alignment
-__host__ __device__ constexpr size_t bfRawBytes(int T) { return (size_t) bfBlocks(T) * 256 + 128; }
-__host__ __device__ constexpr size_t bfSmemBytesFor(int T, int stages)
-{
-   return 2048 + 4 * bfPlaneBytes(T) + stages * bfRawBytes(T) + (size_t) bfK(T) * 256 + 4 * (size_t) bfTapSlots(T);
-}
-__host__ __device__ inline int bfStages(int T)
-{
-   return bfSmemBytesFor(T, 2) <= kBfSmemLimit ? 2 : (bfSmemBytesFor(T, 1) <= kBfSmemLimit ? 1 : 0);
-}
-__host__ __device__ inline size_t bfSmemBytes(int T) { return bfSmemBytesFor(T, bfStages(T)); }
-static_assert(bfSmemBytesFor(kBfMaxTaps, 0) <= kBfSmemLimit, "two plane sets and the longest band fit");
+// Pipeline of the split-BF16x3 FIR.  One persistent CTA per SM; the warps of a role
+// walk the CTA's tiles in the same order and meet only on mbarriers, so the fetch of a tile,
+// the split of the one before, its predecessor's MMAs and the drain of the one before that
+// run at the same time:
+//   warp 17      (fetch) bulk-copies raw FP32 tiles into a ring of two slots;
+//   warps 0-7    (split) write raw tile n as hi/lo planes into set b = n % 2 once tile n - 2's
+//                MMAs have read it, and with a run's first tile its taps band;
+//   warp 16      (MMA)   one thread issues tile n's MMAs into accumulator b once the planes
+//                are full and the accumulator is drained;
+//   warps 8-15   (drain) read accumulator b, free it, add the hi and lo taps' columns
+//                and store them by whole lines through shared memory.
+// What bounds it: the SM's shared-memory data path.  The MMAs read 8 KB each (two N = 128
+// MMAs per 16 taps, 64 clocks each at 128 bytes a clock: 2560 clocks a tile of 8192 outputs
+// with 256 taps), and raw tile, planes, staged outputs and stores pass the same path, about
+// 1800 clocks more.  Measured on 1024 channels x 65536 samples x 256 taps: 143 us in a short
+// run (175 us in a long one, under the power cap) against 240 us for the earlier form, where
+// 16 warps split and drained in lock step behind five barriers a tile, an expanded band
+// (256 bytes a tap) was built for every run and the issuing thread gave an MMA every 100 clocks.
+constexpr int kBfSplitWarps = 8, kBfSplitThreads = 32 * kBfSplitWarps;
+constexpr int kBfDrainWarps = 8;
+constexpr int kBfMmaWarp = kBfSplitWarps + kBfDrainWarps;
+constexpr int kBfFetchWarp = kBfMmaWarp + 1;
+constexpr int kBfCta = 32 * (kBfFetchWarp + 1);
+constexpr uint32_t kBfSplitBar = 1;   // the split threads' named barrier
+constexpr uint32_t kBfTmemCols = 256; // two accumulators of 128 columns
+constexpr int kBfMaxBlocks = bfBlocks(kBfMaxTaps);
+constexpr int kBfQuads = (kBfMaxBlocks * 16 + kBfSplitThreads - 1) / kBfSplitThreads; // 4-sample groups per split thread
+
+// Shared memory: barriers and the TMEM slot (1024 bytes), two sets of hi/lo planes, an
+// output tile, two raw tiles (with up to 3 samples before and 8 behind), two taps bands (runs alternate, so the next run's band is built while this one's is read).
+constexpr size_t kBfRawFloats = (size_t) kBfMaxBlocks * 64 + 32;
+constexpr size_t kBfPlane = (size_t) ((kBfMaxBlocks * 128 + 1023) & ~1023);
+__host__ __device__ constexpr size_t bfBandBytes(int T) { return (size_t) (bfK(T) / 8 + 8) * 256; }
+__host__ __device__ constexpr size_t bfSmemBytes(int Tmax) { return 2048 + 4 * kBfPlane + kBfTile * 4 + 8 * kBfRawFloats + 2 * bfBandBytes(Tmax); }
+static_assert(bfSmemBytes(kBfMaxTaps) <= 227 * 1024, "two plane sets and two of the longest bands fit");
 
 struct BfSmem {
-   unsigned char *sets; // plane set b: hi at sets + 2 b planeBytes, lo planeBytes further (1024-byte aligned)
-   size_t planeBytes;
-   float *raw;          // stages x rawFloats
-   int rawFloats, stages;
-   unsigned char *Bt;
-   uint16_t *gHi, *gLo;
-   uint64_t *mbar, *planesFull, *full; // MMA completion and plane-set readiness per accumulator; raw tiles
+   uint64_t *mmaDone, *planesFull, *accFree; // one per plane set / accumulator
+   uint64_t *rawFull, *rawFree;              // one per raw slot
    uint32_t *tslot;
-   __device__ float *slot(int k) const { return raw + (size_t) k * rawFloats; }
-   __device__ unsigned char *hi(int b) const { return sets + (size_t) (2 * b) * planeBytes; }
-   __device__ unsigned char *lo(int b) const { return sets + (size_t) (2 * b + 1) * planeBytes; }
+   unsigned char *sets, *bands;
+   float *stage; // one output tile, 1024 floats per drain warp
+   float *raw;
+   size_t bandBytes;
+   __device__ float *slot(int k) const { return raw + (size_t) k * kBfRawFloats; }
+   __device__ unsigned char *hi(int b) const { return sets + (size_t) (2 * b) * kBfPlane; }
+   __device__ unsigned char *lo(int b) const { return sets + (size_t) (2 * b + 1) * kBfPlane; }
+   __device__ unsigned char *band(int k) const { return bands + (size_t) (k & 1) * bandBytes; }
 };
 
-__device__ __forceinline__ BfSmem bfSmemLayout(unsigned char *smraw, int T)
+__device__ __forceinline__ BfSmem bfSmemLayout(unsigned char *smraw, int Tmax)
 {
    BfSmem L;
    unsigned char *sm = (unsigned char *) (((uintptr_t) smraw + 1023) & ~(uintptr_t) 1023);
-   L.mbar = (uint64_t *) sm;
-   L.planesFull = L.mbar + 2;
-   L.full = L.planesFull + 2;
-   L.tslot = (uint32_t *) (L.full + 2);
-   const size_t pb = bfPlaneBytes(T);
-   L.stages = bfStages(T);
-   L.planeBytes = pb;
+   L.mmaDone = (uint64_t *) sm;
+   L.planesFull = L.mmaDone + 2;
+   L.accFree = L.planesFull + 2;
+   L.rawFull = L.accFree + 2;
+   L.rawFree = L.rawFull + 2;
+   L.tslot = (uint32_t *) (L.rawFree + 2);
    L.sets = sm + 1024;
-   L.raw = (float *) (L.sets + 4 * pb);
-   L.rawFloats = (int) (bfRawBytes(T) / 4);
-   L.Bt = (unsigned char *) L.raw + (size_t) L.stages * bfRawBytes(T);
-   L.gHi = (uint16_t *) (L.Bt + (size_t) bfK(T) * 256); // split taps with zero padding
-   L.gLo = L.gHi + bfTapSlots(T);
+   L.stage = (float *) (L.sets + 4 * kBfPlane);
+   L.raw = L.stage + kBfTile;
+   L.bands = (unsigned char *) (L.raw + 2 * kBfRawFloats);
+   L.bandBytes = bfBandBytes(Tmax);
    return L;
 }
 
-// The workers' barrier phases and copies in flight, carried across the runs of one CTA.
-struct BfPipe {
-   uint32_t tiles = 0;   // tiles split so far: tile n uses plane set and accumulator n % 2
-   uint32_t mmaPar = 0;  // mmaDone phase, one bit per accumulator
-   uint32_t par = 0;     // raw-tile barrier phase, one bit per stage
-   uint32_t pending = 0; // stages with a bulk copy issued and not yet waited for
-};
-
-// The MMA thread's state.
-struct BfIssuer {
-   uint32_t tiles = 0;
-   uint32_t pfPar = 0;          // planesFull phase, one bit per accumulator
-   uint32_t commits0 = 0, commits1 = 0; // commits per accumulator
-};
-
-// Workers: wait for the MMAs of accumulator b (bounded; thread 0 waits, the barrier
-// releases the rest).
-__device__ __forceinline__ bool bfWaitMma(const BfSmem &L, BfPipe &pp, int b, int *err, int tid)
+// Blocks of tile t that its valid output rows read (a short last tile needs fewer; the rows
+// beyond are computed from stale planes and never stored).
+__device__ __forceinline__ int bfTileBlocks(const BfRun &r, int t)
 {
-   const bool done = tid == 0 ? tc::mbarWait(L.mbar + b, (pp.mmaPar >> b) & 1) : true;
-   pp.mmaPar ^= 1u << b;
-   if (!done && tid == 0) raiseError(err);
-   return !tc::namedSyncOr(kBfBar, kBfWorkers, !done);
+   const int outs = (int) min((long long) kBfTile, (long long) r.outLen - (long long) t * kBfTile);
+   return (outs + kBfPhases - 1) / kBfPhases + (bfK(r.T) + 63) / 64;
 }
 
-// Workers: drain accumulator b (output tile t of run r, its MMAs complete) through
-// plane set b into y.
-__device__ __forceinline__ void bfDrain(const BfRun &r, const BfSmem &L, uint32_t tmem, int b, int t, int tid)
+// Samples between the 16-byte boundary at or below a tile's first input and that input:
+// the same for every tile of a channel (a tile is 8192 samples).
+__device__ __forceinline__ int bfMis(const BfRun &r)
 {
-   const int warp = tid >> 5, lane = tid & 31;
-   tc::fenceAfterSync();
-   const long long j0 = (long long) t * kBfTile;
-   unsigned char *stage = L.hi(b); // the set spans both planes: 2 * planeBytes >= 32 KB
-   {
-      // Warp w drains TMEM lane quadrant w % 4 (rows a) and output quarter qt = w / 4
-      // (16 phases): y[j0 + 64a + 16*qt + b] = D[a][16*qt + b] + D[a][64 + 16*qt + b].
-      const int quad = warp & 3, qt = warp >> 2, half = qt >> 1;
-      const uint32_t acc = tmem + (uint32_t) b * 128 + ((uint32_t) (quad * 32) << 16);
-      const int row = quad * 32 + lane;
-      // 16-byte chunk v4 of row half (row, half) rotated to slot (v4 + row) & 7 so that
-      // eight consecutive rows store to distinct banks.  Two passes of 8 columns keep
-      // the register footprint small.
-      float *os = (float *) stage + row * kBfPhases + half * 32;
+   return (int) ((((long long) ((uintptr_t) r.x >> 2)) + r.inShift) & 3);
+}
+
+// The raw window of tile t: `len` samples from input index w0 on, w0 on a 16-byte boundary.
+// The bulk copy takes its part inside the input, [lo, hi), both ends on 16-byte boundaries;
+// the split threads write the rest (up to 3 samples beside each end, and the zeros outside
+// the input).
+struct BfWindow {
+   long long w0, lo, hi;
+   int len;
+};
+__device__ __forceinline__ BfWindow bfWindow(const BfRun &r, int t, int mis, int blocks)
+{
+   BfWindow w;
+   w.w0 = r.inShift + (long long) t * kBfTile - mis;
+   w.len = blocks * kBfPhases + (mis ? 4 : 0);
+   w.lo = w.w0 >= 0 ? w.w0 : w.w0 + ((-w.w0 + 3) & ~3LL);
+   w.hi = w.w0 + ((min(w.w0 + w.len, r.inLen) - w.w0) & ~3LL);
+   if (w.hi < w.lo) w.hi = w.lo;
+   return w;
+}
+
+__device__ __forceinline__ void bfFixEdges(const BfRun &r, const BfWindow &w, float *raw, int tid)
+{
+   for (int i = tid; i < (int) (w.lo - w.w0); i += kBfSplitThreads) {
+      const long long q = w.w0 + i;
+      raw[i] = (q >= 0 && q < r.inLen) ? r.x[q] : 0.0f;
+   }
+   for (int i = (int) (w.hi - w.w0) + tid; i < w.len; i += kBfSplitThreads) {
+      const long long q = w.w0 + i;
+      raw[i] = (q >= 0 && q < r.inLen) ? r.x[q] : 0.0f;
+   }
+}
+
+// Split a raw tile into the planes: sample i (64 per 128-byte block k = i / 64) goes to
+// block k, 16-byte chunk c = (i % 64) / 8 stored at k * 128 + ((c ^ (k & 7)) * 16), as hi and lo
+// BF16.  Sample i is raw[MIS + i].  A thread takes 4 samples (consecutive lanes, consecutive
+// addresses) and writes half a chunk of each plane; its groups are 16 blocks apart, so they
+// share c and k & 7.  A full tile has at least 8 groups a thread (FULL: no test on those).
+template <int MIS, bool FULL>
+__device__ __forceinline__ void bfSplitMis(const float *raw, int nQuad, unsigned char *hi, unsigned char *lo, int tid)
+{
+   static_assert(8 * kBfSplitThreads <= kRows * 16 && kBfQuads == 9, "groups of a full tile");
+   const int k = tid >> 4, off = k * 128 + ((((tid >> 1) & 7) ^ (k & 7)) << 4) + (tid & 1) * 8;
+   const float4 *src = (const float4 *) raw + tid;
+   hi += off;
+   lo += off;
 #pragma unroll
-      for (int h8 = 0; h8 < 2; h8++) {
-         uint32_t a[8], c[8];
-         tc::tmemLoad8(acc + qt * 16 + h8 * 8, a);
-         tc::tmemLoad8(acc + 64 + qt * 16 + h8 * 8, c);
-         tc::tmemWaitLoad();
+   for (int u0 = 0; u0 < kBfQuads; u0 += 3) {
+      float f[3][8];
+#pragma unroll
+      for (int u = 0; u < 3; u++)
+         if ((FULL && u0 + u < 8) || tid + (u0 + u) * kBfSplitThreads < nQuad) {
+            *(float4 *) &f[u][0] = src[(u0 + u) * kBfSplitThreads];
+            if (MIS) *(float4 *) &f[u][4] = src[(u0 + u) * kBfSplitThreads + 1];
+         }
+#pragma unroll
+      for (int u = 0; u < 3; u++)
+         if ((FULL && u0 + u < 8) || tid + (u0 + u) * kBfSplitThreads < nQuad) {
+            uint2 hv, lv;
+            splitBf16x2(f[u][MIS + 0], f[u][MIS + 1], hv.x, lv.x);
+            splitBf16x2(f[u][MIS + 2], f[u][MIS + 3], hv.y, lv.y);
+            *(uint2 *) (hi + (u0 + u) * (kBfSplitThreads * 8)) = hv;
+            *(uint2 *) (lo + (u0 + u) * (kBfSplitThreads * 8)) = lv;
+         }
+   }
+}
+
+__device__ __forceinline__ void bfSplit(const float *raw, int mis, int nQuad, unsigned char *hi, unsigned char *lo,
+                                        int tid)
+{
+   if (nQuad >= kRows * 16) {
+      switch (mis) { // uniform over the run
+      case 0: bfSplitMis<0, true>(raw, nQuad, hi, lo, tid); break;
+      case 1: bfSplitMis<1, true>(raw, nQuad, hi, lo, tid); break;
+      case 2: bfSplitMis<2, true>(raw, nQuad, hi, lo, tid); break;
+      default: bfSplitMis<3, true>(raw, nQuad, hi, lo, tid); break;
+      }
+   }
+   else {
+      switch (mis) {
+      case 0: bfSplitMis<0, false>(raw, nQuad, hi, lo, tid); break;
+      case 1: bfSplitMis<1, false>(raw, nQuad, hi, lo, tid); break;
+      case 2: bfSplitMis<2, false>(raw, nQuad, hi, lo, tid); break;
+      default: bfSplitMis<3, false>(raw, nQuad, hi, lo, tid); break;
+      }
+   }
+}
+
+// Taps band of a run.  Column n = 16 u + 8 v + i of the accumulator (u < 8, v = 0: hi taps,
+// 1: lo taps, i < 8) is phase b = 63 - (8 u + i); its operand row holds g[m - b], so the
+// 16-byte chunk q (taps m = 8 q .. 8 q + 7) of that row is G[8 (q + u) + i ..], G[k] = g[k - 63]:
+// it depends on q + u only.  With the phases in this order the K-major descriptor of the
+// band therefore reads one copy of each chunk, at (q + u) * 256 + v * 128 + i * 16 (256 bytes
+// between K chunks, 128 between groups of 8 columns), K / 8 + 8 rows of 256 bytes in all
+// instead of 256 bytes a tap.
+__device__ __forceinline__ void bfBand(const BfRun &r, unsigned char *band, int tid)
+{
+   const int T = r.T, n = bfK(T) + 64;
+   for (int c = tid; c < n; c += kBfSplitThreads) { // c = 8 (q + u) + i
+      uint32_t hv[4], lv[4];
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+         const int k0 = c + 2 * e - 63, k1 = k0 + 1;
+         const float g0 = (k0 >= 0 && k0 < T) ? r.h[r.reverse ? T - 1 - k0 : k0] : 0.0f;
+         const float g1 = (k1 >= 0 && k1 < T) ? r.h[r.reverse ? T - 1 - k1 : k1] : 0.0f;
+         splitBf16x2(g0, g1, hv[e], lv[e]);
+      }
+      unsigned char *d = band + (c >> 3) * 256 + (c & 7) * 16;
+      *(uint4 *) d = make_uint4(hv[0], hv[1], hv[2], hv[3]);
+      *(uint4 *) (d + 128) = make_uint4(lv[0], lv[1], lv[2], lv[3]);
+   }
+}
+
+// Drain one accumulator: warp (quad, half) takes 32 rows of 32 phases each, outputs
+// 64 (32 quad + lane) + 32 (1 - half) .. + 32 of tile t, one row a lane.  The sums go to the
+// warp's own 4 KB of shared memory, the 16-byte units of a row permuted by the row (eight
+// rows store to distinct banks), and leave as whole coalesced lines.  (Stored from
+// registers, a warp's store covers 32 rows, and the kernel is bound by its partial lines:
+// 207 us on 1024 x 65536 x 256 taps; with four drain warps instead of eight 195 us, their
+// chain of loads, sums and stores then being the longest of the pipeline.)
+__device__ __forceinline__ void bfDrain(const BfRun &r, const BfSmem &L, uint32_t acc, int b, int t, int dw, int lane)
+{
+   const int quad = dw & 3, half = dw >> 2;
+   const int o0 = quad * (32 * kBfPhases) + 32 * (1 - half); // first output of the warp's first row
+   const long long j0 = (long long) t * kBfTile + o0;
+   float *stage = L.stage + dw * (32 * 32);
+   __syncwarp(); // the previous tile has left the staging rows
+#pragma unroll
+   for (int p = 0; p < 2; p++) {
+      uint32_t d[32];
+      tc::tmemLoad32(acc + ((uint32_t) (quad * 32) << 16) + half * 64 + p * 32, d);
+      tc::tmemWaitLoad();
+      if (p == 1) { // the warp's part is in registers
+         tc::fenceBeforeSync();
+         __syncwarp();
+         if (lane == 0) tc::mbarArrive(L.accFree + b);
+      }
+      // columns 16 u + i (hi taps) and 16 u + 8 + i: phase 63 - 8 (4 half + 2 p + u) - i
+#pragma unroll
+      for (int u = 0; u < 2; u++)
 #pragma unroll
          for (int v = 0; v < 2; v++) {
-            const int v4 = (qt & 1) * 4 + h8 * 2 + v;
-            float4 o;
-            o.x = __uint_as_float(a[4 * v + 0]) + __uint_as_float(c[4 * v + 0]);
-            o.y = __uint_as_float(a[4 * v + 1]) + __uint_as_float(c[4 * v + 1]);
-            o.z = __uint_as_float(a[4 * v + 2]) + __uint_as_float(c[4 * v + 2]);
-            o.w = __uint_as_float(a[4 * v + 3]) + __uint_as_float(c[4 * v + 3]);
-            *(float4 *) (os + (((v4 + row) & 7) << 2)) = o;
+            auto sum = [&](int i) { return __uint_as_float(d[16 * u + i]) + __uint_as_float(d[16 * u + 8 + i]); };
+            const int unit = 7 - 2 * (2 * p + u) - v;
+            *(float4 *) (stage + lane * 32 + ((unit ^ (lane & 7)) << 2)) =
+                make_float4(sum(4 * v + 3), sum(4 * v + 2), sum(4 * v + 1), sum(4 * v));
          }
+   }
+   __syncwarp();
+   float *y = r.y + j0;
+   const long long left = (long long) r.outLen - j0; // valid outputs from the warp's first one on
+   if (((uintptr_t) y & 15) == 0 && left >= 31 * kBfPhases + 32) {
+#pragma unroll
+      for (int i = 0; i < 8; i++) { // unit lane % 8 of row 4 i + lane / 8
+         const int row = 4 * i + (lane >> 3);
+         *(float4 *) (y + row * kBfPhases + (lane & 7) * 4) =
+             *(const float4 *) (stage + row * 32 + (((lane & 7) ^ (row & 7)) << 2));
       }
    }
-   tc::fenceBeforeSync();
-   tc::namedSync(kBfBar, kBfWorkers); // the output tile is complete in shared memory; the accumulator is free
-   storeTile<float>(r.y + j0, (int) min((long long) kBfTile, (long long) r.outLen - j0), (const unsigned char *) stage,
-                    [](int ci) {
-                       const int row = ci >> 4, half = (ci >> 3) & 1, v4 = ci & 7;
-                       return (row * kBfPhases + half * 32 + (((v4 + row) & 7) << 2)) * 4;
-                    },
-                    tid, kBfWorkers);
-   tc::namedSync(kBfBar, kBfWorkers); // the staged output has left plane set b: it may be split into again
+   else {
+#pragma unroll
+      for (int row = 0; row < 32; row++) {
+         const float v = stage[row * 32 + (((lane >> 2) ^ (row & 7)) << 2) + (lane & 3)];
+         if (row * kBfPhases + lane < left) y[row * kBfPhases + lane] = v;
+      }
+   }
 }
 
-// Workers: build the taps band of run r, then split its tiles into alternate plane
-// sets (handing each to the MMA warp) and drain tile t - 1 while tile t's MMAs run.
-// Returns false when a bounded wait gave up.
-__device__ __forceinline__ bool bfWork(const BfRun &r, const BfSmem &L, uint32_t tmem, BfPipe &pp, int tid)
+// MMA thread: the Toeplitz contraction of one tile into accumulator d, committed to done.
+__device__ __forceinline__ void bfIssue(int K, uint32_t ahi, uint32_t alo, uint32_t bt, uint32_t d, uint64_t *done)
 {
-   const int T_ = r.T;
-   const int Kt = bfK(T_);
-   const int nb = bfBlocks(T_);
-   const int slots = bfTapSlots(T_);
-   const int S = L.stages;
-   auto q0 = [&](int t) { return r.inShift + (long long) t * kBfTile; };
-   // Blocks of tile t the MMAs read for its valid output rows (a short last tile needs
-   // fewer; the rows beyond are computed from stale planes and never stored).
-   auto blocksOf = [&](int t) {
-      const int outs = (int) min((long long) kBfTile, (long long) r.outLen - (long long) t * kBfTile);
-      return min(nb, (outs + kBfPhases - 1) / kBfPhases + (Kt + 63) / 64);
-   };
-   // samples between the 16-byte boundary at or below the tile's first input and that input
-   auto misOf = [&](int t) { return (int) ((((long long) ((uintptr_t) r.x >> 2)) + q0(t)) & 3); };
-   auto bytesOf = [&](int t) { return (uint32_t) blocksOf(t) * 256u + (misOf(t) ? 16u : 0u); };
-   // The raw window of tile t is [w0, w0 + bytes / 4), w0 = q - mis on a 16-byte boundary.
-   // The bulk copy takes its part inside the input, [lo, hi), both ends on 16-byte
-   // boundaries (window offsets multiples of 4 samples); the threads write the rest:
-   // the up to 3 samples beside each end and the zeros outside the input.
-   auto bulkLo = [&](int t) {
-      const long long w0 = q0(t) - misOf(t);
-      return w0 >= 0 ? w0 : w0 + ((-w0 + 3) & ~3LL);
-   };
-   auto bulkHi = [&](int t) {
-      const long long w0 = q0(t) - misOf(t), end = min(w0 + (long long) (bytesOf(t) / 4), r.inLen);
-      return w0 + ((end - w0) & ~3LL);
-   };
-   auto bulkOk = [&](int t) { return S > 0 && bulkHi(t) > bulkLo(t); };
-   auto fetch = [&](int t, int k) {
-      const long long w0 = q0(t) - misOf(t), lo = bulkLo(t), hi = bulkHi(t);
-      tc::mbarExpectTx(L.full + k, (uint32_t) (hi - lo) * 4u);
-      tc::bulkLoad(L.slot(k) + (lo - w0), r.x + lo, (uint32_t) (hi - lo) * 4u, L.full + k);
-   };
-   // the window's samples outside the bulk range: input values or zeros beyond it
-   auto fixEdges = [&](int t, int k) {
-      const long long w0 = q0(t) - misOf(t), lo = bulkLo(t), hi = bulkHi(t);
-      const int W = (int) (bytesOf(t) / 4);
-      float *raw = L.slot(k);
-      for (int i = tid; i < (int) (lo - w0); i += kBfWorkers) {
-         const long long q = w0 + i;
-         raw[i] = (q >= 0 && q < r.inLen) ? r.x[q] : 0.0f;
-      }
-      for (int i = (int) (hi - w0) + tid; i < W; i += kBfWorkers) {
-         const long long q = w0 + i;
-         raw[i] = (q >= 0 && q < r.inLen) ? r.x[q] : 0.0f;
-      }
-   };
-   // The first raw tiles are fetched while the taps band is built.  (Every MMA of the
-   // previous run completed: its last tile was drained.)
-   if (tid == 0)
-      for (int k = 0; k < S && r.t0 + k < r.t1; k++)
-         if (bulkOk(r.t0 + k)) fetch(r.t0 + k, k);
-   for (int k = 0; k < S && r.t0 + k < r.t1; k++)
-      if (bulkOk(r.t0 + k)) pp.pending |= 1u << k;
-   // g[c] split into hi/lo, stored at slot c + kBfPadLeft; zero elsewhere.
-   for (int sl = tid; sl < slots; sl += kBfWorkers) {
-      const int c = sl - kBfPadLeft;
-      uint16_t hi = 0, lo = 0;
-      if (c >= 0 && c < T_) splitBf16(r.reverse ? r.h[T_ - 1 - c] : r.h[c], hi, lo);
-      L.gHi[sl] = hi;
-      L.gLo[sl] = lo;
-   }
-   tc::namedSync(kBfBar, kBfWorkers);
-   // Taps band, K-major no swizzle: 16-byte chunk (q, n) at q*2048 + (n/8)*128 + (n%8)*16 holds
-   // B[8q .. 8q+7][n]; rows n < 64: g_hi[m - n], rows n >= 64: g_lo[m - (n - 64)].
-   // Each chunk is 8 consecutive split taps from an arbitrary element offset o: the two
-   // aligned 16-byte vectors around it, shifted into place (funnel shifts by 16 bits for
-   // odd offsets), instead of 8 scalar reads.
-   for (int cidx = tid; cidx < (Kt / 8) * 128; cidx += kBfWorkers) {
-      const int q = cidx >> 7, n = cidx & 127;
-      const int o = kBfPadLeft + 8 * q - (n & 63);
-      const uint4 *base = (const uint4 *) (n < 64 ? L.gHi : L.gLo) + (o >> 3);
-      const uint4 lo4 = base[0], hi4 = base[1];
-      const int rr = o & 7, h = rr >> 1;
-      // words h .. h + 4 of the 8 (selects, not an indexed array: it stays in registers)
-      const uint32_t w0 = h == 0 ? lo4.x : h == 1 ? lo4.y : h == 2 ? lo4.z : lo4.w;
-      const uint32_t w1 = h == 0 ? lo4.y : h == 1 ? lo4.z : h == 2 ? lo4.w : hi4.x;
-      const uint32_t w2 = h == 0 ? lo4.z : h == 1 ? lo4.w : h == 2 ? hi4.x : hi4.y;
-      const uint32_t w3 = h == 0 ? lo4.w : h == 1 ? hi4.x : h == 2 ? hi4.y : hi4.z;
-      const uint32_t w4 = h == 0 ? hi4.x : h == 1 ? hi4.y : h == 2 ? hi4.z : hi4.w;
-      uint4 v;
-      if (rr & 1) {
-         v.x = __funnelshift_r(w0, w1, 16);
-         v.y = __funnelshift_r(w1, w2, 16);
-         v.z = __funnelshift_r(w2, w3, 16);
-         v.w = __funnelshift_r(w3, w4, 16);
-      }
-      else {
-         v.x = w0;
-         v.y = w1;
-         v.z = w2;
-         v.w = w3;
-      }
-      *(uint4 *) (L.Bt + q * 2048 + (n >> 3) * 128 + (n & 7) * 16) = v;
-   }
-   for (int t = r.t0; t <= r.t1; t++) {
-      const int cur = (int) (pp.tiles & 1), prev = cur ^ 1;
-      if (t < r.t1) {
-         // plane set and accumulator cur are free: tile t - 2 was drained
-         const int k = S > 0 ? (t - r.t0) % S : 0;
-         bool ok = true;
-         const bool viaBulk = bulkOk(t);
-         if (viaBulk) {
-            ok = tid == 0 ? tc::mbarWait(L.full + k, (pp.par >> k) & 1) : true; // the barrier below releases the rest
-            pp.par ^= 1u << k;
-            pp.pending &= ~(1u << k);
-         }
-         if (!ok && tid == 0) raiseError(r.err);
-         if (viaBulk) fixEdges(t, k);
-         if (tc::namedSyncOr(kBfBar, kBfWorkers, !ok)) return false; // the raw tile landed (and the band is built)
-         if (viaBulk) bfSplit(L.slot(k), misOf(t), blocksOf(t), L.hi(cur), L.lo(cur), tid);
-         else bfStage(r.x, q0(t), r.inLen, blocksOf(t), L.hi(cur), L.lo(cur), tid); // straight from global memory
-         tc::fenceProxyAsync();
-         tc::fenceBeforeSync();
-         tc::namedSync(kBfBar, kBfWorkers); // planes (and band) written; the raw stage is free again
-         if (tid == 0) tc::mbarArrive(L.planesFull + cur);
-         if (t + S < r.t1 && bulkOk(t + S)) {
-            if (tid == 0) fetch(t + S, k);
-            pp.pending |= 1u << k;
-         }
-         pp.tiles++;
-      }
-      if (t > r.t0) {
-         // tile t - 1 (accumulator and plane set prev) while tile t's MMAs run
-         if (!bfWaitMma(L, pp, prev, r.err, tid)) return false;
-         bfDrain(r, L, tmem, prev, t - 1, tid);
-      }
-   }
-   return true;
-}
-
-// MMA thread: for each tile of run r, once its plane set is full, the Toeplitz
-// contraction into the tile's accumulator and a commit to its mmaDone barrier.
-__device__ __forceinline__ bool bfIssue(const BfRun &r, const BfSmem &L, uint32_t tmem, BfIssuer &mi)
-{
-   const int Kt = bfK(r.T);
-   const uint32_t bt = tc::smemAddr(L.Bt);
    const uint32_t id128 = tc::idesc(1, 1, 1, kRows, 128);
-   for (int t = r.t0; t < r.t1; t++) {
-      const int b = (int) (mi.tiles & 1);
-      if (!tc::mbarWait(L.planesFull + b, (mi.pfPar >> b) & 1)) {
-         raiseError(r.err);
-         return false;
+   // The swizzle is applied on absolute shared-memory address bits, so a start
+   // that is not atom-aligned (block k16 / 4 of the plane) keeps base offset 0.
+   uint64_t dHi = tc::descSw128(ahi, 1024, 0), dLo = tc::descSw128(alo, 1024, 0), dB = tc::descNoSwizzle(bt, 256, 128);
+   int k16 = 0;
+   // descriptor addresses count 16 bytes: 16 taps are 32 bytes of a plane, two rows (512 bytes) of the band
+   for (; k16 + 4 <= K / 16; k16 += 4, dHi += 8, dLo += 8, dB += 128) {
+#pragma unroll
+      for (int sub = 0; sub < 4; sub++) {
+         tc::mmaF16(d, dHi + 2 * sub, dB + 32 * sub, id128, k16 + sub > 0);
+         tc::mmaF16(d, dLo + 2 * sub, dB + 32 * sub, id128, true);
       }
-      mi.pfPar ^= 1u << b;
-      tc::fenceAfterSync();
-      const uint32_t ahi = tc::smemAddr(L.hi(b)), alo = tc::smemAddr(L.lo(b));
-      const uint32_t d = tmem + (uint32_t) b * 128;
-      for (int k16 = 0; k16 < Kt / 16; k16++) {
-         const int blk = k16 >> 2, sub = k16 & 3;
-         // The swizzle is applied on absolute shared-memory address bits, so a start
-         // that is not atom-aligned (block blk of the plane) keeps base offset 0.
-         const uint64_t dHi = tc::descSw128(ahi + blk * 128 + sub * 32, 1024, 0);
-         const uint64_t dLo = tc::descSw128(alo + blk * 128 + sub * 32, 1024, 0);
-         const uint64_t dB = tc::descNoSwizzle(bt + k16 * 4096, 2048, 128);
-         tc::mmaF16(d, dHi, dB, id128, k16 > 0);
-         tc::mmaF16(d, dLo, dB, id128, true);
-      }
-      tc::commit(L.mbar + b);
-      if (b) mi.commits1++;
-      else mi.commits0++;
-      mi.tiles++;
    }
-   return true;
+   for (; k16 < K / 16; k16++, dHi += 2, dLo += 2, dB += 32) {
+      tc::mmaF16(d, dHi, dB, id128, k16 > 0);
+      tc::mmaF16(d, dLo, dB, id128, true);
+   }
+   tc::commit(done);
 }
 
-// Set-up and tear-down shared by the bf16x3 kernels.
-__device__ __forceinline__ uint32_t bfBegin(const BfSmem &L, int tid)
+// The kernel body: `get(i)` describes run i (i < nRuns); runs are taken in turn by the
+// CTAs of the grid.  Every wait is bounded: a role whose wait gives up raises the error word
+// and leaves, and the others follow as theirs give up.
+template <typename Get>
+__device__ __forceinline__ void bfPipeline(const BfSmem &L, int nRuns, int *err, Get get)
 {
-   if ((tid >> 5) == 0) tc::tmemAlloc(L.tslot, kBfTmemCols);
+   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+   if (warp == 0) tc::tmemAlloc(L.tslot, kBfTmemCols);
    if (tid == 0) {
-      for (int k = 0; k < 2; k++) tc::mbarInit(L.mbar + k, 1);
-      for (int k = 0; k < 2; k++) tc::mbarInit(L.planesFull + k, 1);
-      for (int k = 0; k < 2; k++) tc::mbarInit(L.full + k, 1);
+      for (int k = 0; k < 2; k++) {
+         tc::mbarInit(L.mmaDone + k, 1);
+         tc::mbarInit(L.planesFull + k, kBfSplitWarps);
+         tc::mbarInit(L.accFree + k, kBfDrainWarps);
+         tc::mbarInit(L.rawFull + k, 1);
+         tc::mbarInit(L.rawFree + k, kBfSplitWarps);
+      }
       tc::fenceMbarInit();
    }
    tc::fenceBeforeSync();
    __syncthreads();
    tc::fenceAfterSync();
-   return *L.tslot;
-}
-
-// After the roles' loops (also after a failure): the MMA thread waits (bounded) for its
-// last commit on each accumulator, worker 0 for the bulk copies still in flight; then
-// the accumulators are released.
-__device__ __forceinline__ void bfEnd(const BfSmem &L, const BfPipe &pp, const BfIssuer &mi, uint32_t tmem, int tid)
-{
-   if (tid == kBfWorkers) {
-      if (mi.commits0) (void) tc::mbarWait(L.mbar, (mi.commits0 - 1) & 1);
-      if (mi.commits1) (void) tc::mbarWait(L.mbar + 1, (mi.commits1 - 1) & 1);
+   const uint32_t tmem = *L.tslot;
+   uint32_t n = 0; // tile n of this CTA uses plane set and accumulator n % 2, phase (n / 2) % 2
+   if (warp < kBfSplitWarps) {
+      bool ok = true;
+      int runs = 0, before = 0; // runs so far, tiles of the previous one
+      for (int i = blockIdx.x; ok && i < nRuns; i += gridDim.x, runs++) {
+         const BfRun r = get(i);
+         const int mis = bfMis(r);
+         // The band's buffer was last read by the run before the previous one: its MMAs are
+         // known to be complete (tile n - 3 or earlier) if the previous run had two tiles or
+         // more, else once tile n - 2's are.
+         if (before >= 2 || n < 2) bfBand(r, L.band(runs), tid);
+         for (int t = r.t0; t < r.t1; t++, n++) {
+            const int b = (int) (n & 1), blocks = bfTileBlocks(r, t);
+            // the MMAs of tile n - 2 have read set b, and the raw tile has landed
+            ok = n < 2 || tc::mbarWait(L.mmaDone + b, ((n >> 1) - 1) & 1);
+            if (t == r.t0 && before < 2 && n >= 2) bfBand(r, L.band(runs), tid);
+            ok = ok && tc::mbarWait(L.rawFull + b, (n >> 1) & 1);
+            const long long w0 = r.inShift - mis + (long long) t * kBfTile;
+            if (w0 < 0 || w0 + blocks * kBfPhases + 4 > r.inLen) { // the same for every split thread
+               if (ok) bfFixEdges(r, bfWindow(r, t, mis, blocks), L.slot(b), tid);
+               tc::namedSync(kBfSplitBar, kBfSplitThreads);
+            }
+            if (!ok) {
+               raiseError(err);
+               break;
+            }
+            bfSplit(L.slot(b), mis, blocks * 16, L.hi(b), L.lo(b), tid);
+            tc::fenceProxyAsync();
+            __syncwarp();
+            if (lane == 0) {
+               tc::mbarArrive(L.planesFull + b);
+               tc::mbarArrive(L.rawFree + b);
+            }
+         }
+         before = r.t1 - r.t0;
+      }
    }
-   if (tid == 0)
-      for (int k = 0; k < 2; k++)
-         if ((pp.pending >> k) & 1) (void) tc::mbarWait(L.full + k, (pp.par >> k) & 1);
+   else if (warp < kBfMmaWarp) {
+      bool ok = true;
+      for (int i = blockIdx.x; ok && i < nRuns; i += gridDim.x) {
+         const BfRun r = get(i);
+         for (int t = r.t0; t < r.t1; t++, n++) {
+            const int b = (int) (n & 1);
+            if (!tc::mbarWait(L.mmaDone + b, (n >> 1) & 1)) {
+               raiseError(err);
+               ok = false;
+               break;
+            }
+            tc::fenceAfterSync();
+            bfDrain(r, L, tmem + (uint32_t) b * 128, b, t, warp - kBfSplitWarps, lane);
+         }
+      }
+   }
+   else if (warp == kBfMmaWarp && tc::electOne()) {
+      bool ok = true;
+      int runs = 0;
+      for (int i = blockIdx.x; ok && i < nRuns; i += gridDim.x, runs++) {
+         const BfRun r = get(i);
+         const int K = bfK(r.T);
+         const uint32_t bt = tc::smemAddr(L.band(runs));
+         for (int t = r.t0; t < r.t1; t++, n++) {
+            const int b = (int) (n & 1);
+            if (!tc::mbarWait(L.planesFull + b, (n >> 1) & 1) ||
+                (n >= 2 && !tc::mbarWait(L.accFree + b, ((n >> 1) - 1) & 1))) {
+               raiseError(err);
+               ok = false;
+               break;
+            }
+            tc::fenceAfterSync();
+            bfIssue(K, tc::smemAddr(L.hi(b)), tc::smemAddr(L.lo(b)), bt, tmem + (uint32_t) b * 128, L.mmaDone + b);
+         }
+      }
+      // n MMA groups were committed: wait (bounded) for the last two before TMEM is released
+      for (uint32_t k = n >= 2 ? n - 2 : 0; k < n; k++) (void) tc::mbarWait(L.mmaDone + (k & 1), (k >> 1) & 1);
+   }
+   else if (warp == kBfFetchWarp && tc::electOne()) {
+      bool ok = true;
+      uint32_t issued = 0;
+      for (int i = blockIdx.x; ok && i < nRuns; i += gridDim.x) {
+         const BfRun r = get(i);
+         const int mis = bfMis(r);
+         for (int t = r.t0; t < r.t1; t++, n++) {
+            const int b = (int) (n & 1);
+            if (n >= 2 && !tc::mbarWait(L.rawFree + b, ((n >> 1) - 1) & 1)) {
+               raiseError(err);
+               ok = false;
+               break;
+            }
+            const BfWindow w = bfWindow(r, t, mis, bfTileBlocks(r, t));
+            const uint32_t bytes = (uint32_t) (w.hi - w.lo) * 4u;
+            if (bytes) {
+               tc::mbarExpectTx(L.rawFull + b, bytes);
+               tc::bulkLoad(L.slot(b) + (w.lo - w.w0), r.x + w.lo, bytes, L.rawFull + b);
+            }
+            else tc::mbarArrive(L.rawFull + b);
+            issued = n + 1;
+         }
+      }
+      // copies still in flight land (bounded) before shared memory is given up
+      for (uint32_t k = issued >= 2 ? issued - 2 : 0; k < issued; k++)
+         (void) tc::mbarWait(L.rawFull + (k & 1), (k >> 1) & 1);
+   }
    tc::fenceBeforeSync();
    __syncthreads();
    tc::fenceAfterSync();
-   if ((tid >> 5) == 0) tc::tmemFree(tmem, kBfTmemCols);
+   if (warp == 0) tc::tmemFree(tmem, kBfTmemCols);
 }
 
-__global__ void __launch_bounds__(kBfBlock, 1) fir_bf16x3_tc_kernel(FirLaunch a, int tilesPerCta)
+// Dense batch: run i = tiles [part * tilesPerRun, ...) of channel i / parts.
+__global__ void __launch_bounds__(kBfCta, 1) fir_bf16x3_tc_kernel(FirLaunch a, int tilesPerRun)
 {
    extern __shared__ __align__(16) unsigned char smraw[];
-   const BfSmem L = bfSmemLayout(smraw, a.T);
-   const int tid = threadIdx.x;
-   const uint32_t tmem = bfBegin(L, tid);
    const int nt = (a.outSize + kBfTile - 1) / kBfTile;
-   BfPipe pp;
-   BfIssuer mi;
-   if (tid < kBfWorkers || tid == kBfWorkers)
-      for (int l = blockIdx.y; l < a.batch; l += gridDim.y) {
-         BfRun r;
-         r.x = (const float *) a.x + (long long) l * a.inPitch;
-         r.h = (const float *) a.h + (long long) l * a.filtPitch;
-         r.y = (float *) a.y + (long long) l * a.outPitch;
-         r.inShift = 0;
-         r.inLen = (long long) a.outSize + a.T - 1;
-         r.outLen = a.outSize;
-         r.T = a.T;
-         r.reverse = 1;
-         r.t0 = blockIdx.x * tilesPerCta;
-         r.t1 = min(nt, r.t0 + tilesPerCta);
-         r.err = a.err;
-         if (!(tid < kBfWorkers ? bfWork(r, L, tmem, pp, tid) : bfIssue(r, L, tmem, mi))) break;
-      }
-   bfEnd(L, pp, mi, tmem, tid);
+   const int parts = (nt + tilesPerRun - 1) / tilesPerRun;
+   bfPipeline(bfSmemLayout(smraw, a.T), a.batch * parts, a.err, [&](int i) {
+      const int l = i / parts, part = i - l * parts;
+      BfRun r;
+      r.x = (const float *) a.x + (long long) l * a.inPitch;
+      r.h = (const float *) a.h + (long long) l * a.filtPitch;
+      r.y = (float *) a.y + (long long) l * a.outPitch;
+      r.inShift = 0;
+      r.inLen = (long long) a.outSize + a.T - 1;
+      r.outLen = a.outSize;
+      r.T = a.T;
+      r.reverse = 1;
+      r.t0 = part * tilesPerRun;
+      r.t1 = min(nt, r.t0 + tilesPerRun);
+      return r;
+   });
 }
 
-// Work lists of the batched filter bank: runs of up to kFirBfRunTiles tiles of one
-// channel, longest first, taken in turn by one persistent CTA per SM.  DX = false:
-// forward, y = valid correlation of x with the taps (DSPLIB_fir order); DX = true:
-// input gradient, the full convolution of the output gradient with the taps.
-__global__ void __launch_bounds__(kBfBlock, 1)
+// Work lists of the batched filter bank: runs of consecutive tiles of one channel, longest
+// first.  dx = 0: forward, y = valid correlation of x with the taps (DSPLIB_fir order);
+// dx = 1: input gradient, the full convolution of the output gradient with the taps.
+__global__ void __launch_bounds__(kBfCta, 1)
     fir_bf16x3_ragged_kernel(const RaggedChan *chans, const int4 *runs, int nRuns, const float *in,
                              const float *taps, float *out, int dx, int Tmax, int *err)
 {
    extern __shared__ __align__(16) unsigned char smraw[];
-   // barriers and the TMEM slot sit at fixed offsets; the rest is laid out per run
-   const BfSmem L = bfSmemLayout(smraw, Tmax);
-   const int tid = threadIdx.x;
-   const uint32_t tmem = bfBegin(L, tid);
-   BfPipe pp;
-   BfIssuer mi;
-   if (tid < kBfWorkers || tid == kBfWorkers)
-      for (int i = blockIdx.x; i < nRuns; i += gridDim.x) {
-         const int4 it = runs[i];
-         const RaggedChan c = chans[it.x];
-         const BfSmem Lr = bfSmemLayout(smraw, c.T);
-         BfRun r;
-         r.x = in + c.xOff;
-         r.h = taps + c.hOff;
-         r.y = out + (dx ? c.xOff : c.pOff); // forward: plane 0 of the work buffer
-         r.T = c.T;
-         r.inShift = dx ? -(long long) (c.T - 1) : 0;
-         r.inLen = dx ? c.L - c.T + 1 : c.L;
-         r.outLen = dx ? c.L : c.L - c.T + 1;
-         r.reverse = dx ? 0 : 1;
-         r.t0 = it.y;
-         r.t1 = it.y + it.z;
-         r.err = err;
-         if (!(tid < kBfWorkers ? bfWork(r, Lr, tmem, pp, tid) : bfIssue(r, Lr, tmem, mi))) break;
-      }
-   bfEnd(L, pp, mi, tmem, tid);
+   bfPipeline(bfSmemLayout(smraw, Tmax), nRuns, err, [&](int i) {
+      const int4 it = runs[i];
+      const RaggedChan c = chans[it.x];
+      BfRun r;
+      r.x = in + c.xOff;
+      r.h = taps + c.hOff;
+      r.y = out + (dx ? c.xOff : c.pOff); // forward: plane 0 of the work buffer
+      r.T = c.T;
+      r.inShift = dx ? -(long long) (c.T - 1) : 0;
+      r.inLen = dx ? c.L - c.T + 1 : c.L;
+      r.outLen = dx ? c.L : c.L - c.T + 1;
+      r.reverse = dx ? 0 : 1;
+      r.t0 = it.y;
+      r.t1 = it.y + it.z;
+      return r;
+   });
 }
 
-
 // ------------------------------------------------------------------ taps gradient (split-BF16x3)
+
+constexpr int kBfWorkers = kBfThreads;         // worker threads (16 warps)
+constexpr int kBfBlock = kBfWorkers + 32;      // + the MMA warp
+constexpr uint32_t kBfBar = 1;                 // the workers' named barrier
 
 // Taps gradient of the filter bank, dh_lag[c] = sum_j gu[j] x[j + c] (c < T), on the
 // tensor cores.  With j = 64 r + s (row r, phase s) and t' = c + s:
@@ -1226,6 +1224,17 @@ cudaError_t launchFirIntTc(const FirLaunch &a, bool qmode, cudaStream_t s)
 
 bool firBf16x3Supported(const FirLaunch &a) { return a.dtype == DSPLIB_FLOAT32 && a.T >= 1 && a.T <= kBfMaxTaps; }
 
+// Tiles per run (the built-in rule, when the autotuner has no entry): long runs build
+// fewer bands, short ones spread evenly over the SMs; at least 8 runs an SM keep the last
+// wave's idle share below an eighth.
+static int bfTilesPerRun(int nt, int batch)
+{
+   const long long sms = deviceSms() > 0 ? deviceSms() : 148;
+   int tpr = nt;
+   while (tpr > 1 && (long long) ((nt + tpr - 1) / tpr) * batch < sms * 8) tpr = (tpr + 1) / 2;
+   return tpr;
+}
+
 cudaError_t launchFirBf16x3(const FirLaunch &a, cudaStream_t s)
 {
    if (!firBf16x3Supported(a)) return cudaErrorNotSupported;
@@ -1234,9 +1243,11 @@ cudaError_t launchFirBf16x3(const FirLaunch &a, cudaStream_t s)
        cudaFuncSetAttribute(fir_bf16x3_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
    if (e != cudaSuccess) return e;
    const int nt = (a.outSize + kBfTile - 1) / kBfTile;
-   const int tpc = a.tuneTpc > 0 ? (a.tuneTpc < nt ? a.tuneTpc : nt) : tilesPerCtaFor(nt, a.batch, 1);
-   dim3 grid((nt + tpc - 1) / tpc, a.batch < 65535 ? a.batch : 65535);
-   fir_bf16x3_tc_kernel<<<grid, kBfBlock, smem, s>>>(a, tpc);
+   const int tpr = a.tuneTpc > 0 ? (a.tuneTpc < nt ? a.tuneTpc : nt) : bfTilesPerRun(nt, a.batch);
+   const long long runs = (long long) a.batch * ((nt + tpr - 1) / tpr);
+   if (runs > INT_MAX) return cudaErrorInvalidValue;
+   const int sms = deviceSms() > 0 ? deviceSms() : 148;
+   fir_bf16x3_tc_kernel<<<(int) std::min<long long>(runs, sms), kBfCta, smem, s>>>(a, tpr);
    countLaunch();
    return cudaGetLastError();
 }
@@ -1246,14 +1257,14 @@ cudaError_t launchFirBf16x3Ragged(const RaggedChan *chans, const int4 *runs, int
 {
    if (Tmax < 1 || Tmax > kBfMaxTaps) return cudaErrorNotSupported;
    if (nRuns <= 0) return cudaSuccess;
-   const size_t smem = kBfSmemLimit; // every run's layout (for its own taps) fits
+   const size_t smem = bfSmemBytes(Tmax);
    cudaError_t e =
        cudaFuncSetAttribute(fir_bf16x3_ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
    if (e != cudaSuccess) return e;
    int sms = 148, dev = 0;
    if (cudaGetDevice(&dev) == cudaSuccess) (void) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
    const int grid = nRuns < sms ? nRuns : sms;
-   fir_bf16x3_ragged_kernel<<<grid, kBfBlock, smem, s>>>(chans, runs, nRuns, in, taps, out, dx ? 1 : 0, Tmax, err);
+   fir_bf16x3_ragged_kernel<<<grid, kBfCta, smem, s>>>(chans, runs, nRuns, in, taps, out, dx ? 1 : 0, Tmax, err);
    countLaunch();
    return cudaGetLastError();
 }
@@ -1291,7 +1302,7 @@ std::vector<int> firTuneCandidates(const FirLaunch &a, FirKernelKind kind)
    };
    if (kind == FIR_F32_BF16X3) {
       const int nt = (a.outSize + kBfTile - 1) / kBfTile;
-      c = tileCounts(nt, tilesPerCtaFor(nt, a.batch, 1));
+      c = tileCounts(nt, bfTilesPerRun(nt, a.batch));
    }
    else {
       const int nt = (a.outSize + kTile - 1) / kTile;

@@ -52,6 +52,19 @@ __host__ __device__ constexpr uint32_t idesc(uint32_t dfmt, uint32_t afmt, uint3
    return (dfmt << 4) | (afmt << 7) | (bfmt << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
+// One lane of a converged warp.  MMAs are issued from a branch on this predicate: the compiler
+// then keeps their descriptors in uniform registers (M = 128, N = 128, K = 16 every 64 clocks;
+// 100 clocks from a branch on the lane number).
+__device__ __forceinline__ bool electOne()
+{
+   uint32_t r;
+   asm volatile("{\n\t.reg .pred e;\n\t"
+                "elect.sync _|e, 0xffffffff;\n\t"
+                "selp.u32 %0, 1, 0, e;\n\t}\n"
+                : "=r"(r));
+   return r != 0;
+}
+
 __device__ __forceinline__ void mmaI8(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t id, bool accum)
 {
    asm volatile("{\n\t.reg .pred p;\n\t"

@@ -238,6 +238,33 @@ def test_bf16x3_unaligned_rows():
     assert np.max(_relerr(host(od)[:, : N - T + 1], y64)) <= 1e-5
 
 
+@pytest.mark.parametrize("T", [1, 2, 17, 449, 512])
+@pytest.mark.parametrize("out", [1, 63, 65, 8191, 8192, 8193, 24577])
+def test_bf16x3_tile_edges(out, T):
+    """Last tiles of every length around a 64-output row and an 8192-output tile, taps at the
+    ends of their range and of a 16-tap step, every alignment of the rows on both sides, runs
+    of one and of several tiles; nothing is written between the rows.  Bar: 1e-5 of each
+    channel's peak, as above (the peak of a one-output channel is that output's operands)."""
+    rng = np.random.default_rng(out * 1000 + T)
+    B, N = 5, out + T - 1
+    x = np.zeros((B, N + 1), np.float32)
+    x[:, :N] = rng.standard_normal((B, N))
+    hh = (rng.standard_normal((B, T)) / np.sqrt(T)).astype(np.float32)
+    args, pin, pfilt, pout = D.fir_setup(D.FLOAT32, B, N, T, nch=1, in_pitch=N + 1, out_pitch=out + 3)
+    pout.dim_x = out
+    got = np.full((B, out + 3), 7.5, np.float32)
+    h = D.FirHandle()
+    assert h.init(args, pin, pfilt, pout) == D.SUCCESS
+    h.set_precision(D.FIR_BF16X3)
+    xd, hd, od = dev(x), dev(hh), dev(got)
+    assert h.exec(xd, hd, od) == D.SUCCESS, h.last_error()
+    got = host(od)
+    y64 = oracle.fir_f64(np.ascontiguousarray(x[:, :N]), hh, T, nch=1)
+    peak = np.maximum(np.abs(y64).max(axis=1), np.abs(x).max(axis=1) * np.abs(hh).max(axis=1))
+    assert (np.abs(got[:, :out] - y64).max(axis=1) <= 1e-5 * peak).all()
+    assert (got[:, out:] == 7.5).all()
+
+
 def _golden_cases():
     import os
 
