@@ -681,7 +681,7 @@ struct AdjArgs {
    const float *gy;      // output gradient (packed)
    const float2 *ckptF;  // forward checkpoints
    const float2 *ckptA;  // adjoint checkpoints (processing order)
-   float *g;             // gradient w.r.t. the FIR output (packed)
+   float *g;             // gradient w.r.t. the FIR output (the scratch's plane)
    float *part;          // 5 coefficient-gradient sums per unit and stage
    int first;            // this launch's first unit (a bucket of one stage count)
 };
@@ -779,7 +779,7 @@ __global__ void __launch_bounds__(32) bank_adjoint_kernel(AdjArgs a)
       if ((lane & 3) == 0 && k < 5) a.part[(base + s) * 5 + k] = r;
    }
    __syncwarp(); // every lane's last read of the stage sequences precedes the staging writes
-   storePacked(g, a.g + c.xOff, t0, Lu, sStage, lane);
+   storePacked(g, a.g + c.gOff, t0, Lu, sStage, lane);
 }
 
 // Coefficient gradients of one channel (one CTA, coefficients spread over its warps): per

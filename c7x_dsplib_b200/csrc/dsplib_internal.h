@@ -300,6 +300,7 @@ void firApplyChoice(FirLaunch &a, FirKernelKind kind, int choice);
 struct RaggedChan {
    long long xOff, hOff, cOff, pOff;
    int L, T, S, Lu;
+   long long gOff;   // its slice of the gradient plane of the scratch (gradient at the FIR output)
    long long ckOff;  // first unit state (float2) of the channel: one per 512-sample unit and stage
    long long phiOff; // first double of the channel's unit transitions
    long long grpOff; // first float of the channel's chain group states (2S per 32 units)

@@ -498,12 +498,9 @@ constexpr int kBfPhases = 64;
 constexpr int kBfTile = kRows * kBfPhases;
 constexpr int kBfMaxTaps = kFirBfMaxTaps;
 static_assert(kBfTile == kFirBfTile, "ragged run tiles and kernel tiles must agree");
-constexpr int kBfThreads = 512;
 
 __host__ __device__ constexpr int bfK(int T) { return ((63 + T + 15) / 16) * 16; }
 __host__ __device__ constexpr int bfBlocks(int T) { return kRows + (bfK(T) + 63) / 64; }
-// 16-byte plane chunks staged per thread by bfStage
-constexpr int kBfChunksPerThread = (bfBlocks(kBfMaxTaps) * 8 + kBfThreads - 1) / kBfThreads;
 
 // Two values as BF16 hi + lo (lo = bf16(v - hi)), packed (a in the low half): one paired
 // conversion per plane.
@@ -515,67 +512,24 @@ __device__ __forceinline__ void splitBf16x2(float a, float b, uint32_t &hi, uint
    lo = *(const uint32_t *) &l;
 }
 
-// Stage one tile's signal planes: sample i of the tile (64 per 128-byte block
-// k = i / 64) goes to block k, 16-byte chunk c = (i % 64) / 8 stored at
-// k*128 + ((c ^ (k & 7)) * 16), as hi and lo BF16.  Sample i is input index
-// q0 + i of x, zero outside [0, inLen).  All loads of a thread are issued
-// before any conversion so they overlap.
-__device__ __forceinline__ void bfStage(const float *x, long long q0, long long inLen, int nb, unsigned char *Ahi,
-                                        unsigned char *Alo, int tid)
-{
-   float f[kBfChunksPerThread][8];
-   // chunk starts are 8 floats apart, so all share one misalignment (in floats)
-   const int mis = (int) ((((uintptr_t) (x + q0)) >> 2) & 3);
-#pragma unroll
-   for (int u = 0; u < kBfChunksPerThread; u++) {
-      const int cidx = tid + u * kBfThreads;
-      if (cidx < nb * 8) {
-         const long long q = q0 + (long long) (cidx >> 3) * 64 + (cidx & 7) * 8;
-         if (mis == 0 && q >= 0 && q + 8 <= inLen) {
-            *(float4 *) &f[u][0] = *(const float4 *) (x + q);
-            *(float4 *) &f[u][4] = *(const float4 *) (x + q + 4);
-         }
-         else if (mis != 0 && q - mis >= 0 && q - mis + 12 <= inLen) {
-            // three aligned vectors around the chunk, then pick its 8 samples
-            const float4 a = *(const float4 *) (x + q - mis);
-            const float4 b = *(const float4 *) (x + q - mis + 4);
-            const float4 cc = *(const float4 *) (x + q - mis + 8);
-            const float w[12] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, cc.x, cc.y, cc.z, cc.w};
-#pragma unroll
-            for (int e = 0; e < 8; e++) f[u][e] = mis == 1 ? w[1 + e] : (mis == 2 ? w[2 + e] : w[3 + e]);
-         }
-         else {
-#pragma unroll
-            for (int e = 0; e < 8; e++) f[u][e] = (q + e >= 0 && q + e < inLen) ? x[q + e] : 0.0f;
-         }
-      }
-   }
-#pragma unroll
-   for (int u = 0; u < kBfChunksPerThread; u++) {
-      const int cidx = tid + u * kBfThreads;
-      if (cidx < nb * 8) {
-         const int k = cidx >> 3, c = cidx & 7;
-         uint4 hv, lv;
-         splitBf16x2(f[u][0], f[u][1], hv.x, lv.x);
-         splitBf16x2(f[u][2], f[u][3], hv.y, lv.y);
-         splitBf16x2(f[u][4], f[u][5], hv.z, lv.z);
-         splitBf16x2(f[u][6], f[u][7], hv.w, lv.w);
-         const int off = k * 128 + ((c ^ (k & 7)) << 4);
-         *(uint4 *) (Ahi + off) = hv;
-         *(uint4 *) (Alo + off) = lv;
-      }
-   }
-}
-
 // A run of consecutive output tiles [t0, t1) of one channel:
 //     y[j] = sum_{c<T} x[inShift + j + c] * g(c),  x zero outside [0, inLen),
 //     g(c) = h[T-1-c] (reverse = 1: DSPLIB_fir correlation order) or h[c] (reverse = 0).
+// A tile's window starts `lead` samples before its first output's, on a 16-byte boundary, and
+// the taps have as many zeros in front: every raw copy and every read of it is then aligned
+// (the same for all tiles of a channel: a tile is 8192 samples).
 struct BfRun {
    const float *x;
    const float *h;
    float *y;
    long long inShift, inLen;
    int outLen, T, reverse, t0, t1;
+   int lead, K; // K: taps contracted, leading zeros and phases included
+   __device__ void align()
+   {
+      lead = (int) ((((long long) ((uintptr_t) x >> 2)) + inShift) & 3);
+      K = bfK(T + lead);
+   }
 };
 
 // Pipeline of the split-BF16x3 FIR.  One persistent CTA per SM; the warps of a role
@@ -601,22 +555,22 @@ constexpr int kBfDrainWarps = 8;
 constexpr int kBfMmaWarp = kBfSplitWarps + kBfDrainWarps;
 constexpr int kBfFetchWarp = kBfMmaWarp + 1;
 constexpr int kBfCta = 32 * (kBfFetchWarp + 1);
-constexpr uint32_t kBfSplitBar = 1;   // the split threads' named barrier
 constexpr uint32_t kBfTmemCols = 256; // two accumulators of 128 columns
-constexpr int kBfMaxBlocks = bfBlocks(kBfMaxTaps);
+constexpr int kBfMaxBlocks = bfBlocks(kBfMaxTaps + 3);
 constexpr int kBfQuads = (kBfMaxBlocks * 16 + kBfSplitThreads - 1) / kBfSplitThreads; // 4-sample groups per split thread
 
 // Shared memory: barriers and the TMEM slot (1024 bytes), two sets of hi/lo planes, an
-// output tile, two raw tiles (with up to 3 samples before and 8 behind), two taps bands (runs alternate, so the next run's band is built while this one's is read).
-constexpr size_t kBfRawFloats = (size_t) kBfMaxBlocks * 64 + 32;
+// output tile, two raw tiles, two taps bands (runs alternate, so the next run's band is built while this one's is read).
+constexpr size_t kBfRawFloats = (size_t) kBfMaxBlocks * 64;
 constexpr size_t kBfPlane = (size_t) ((kBfMaxBlocks * 128 + 1023) & ~1023);
-__host__ __device__ constexpr size_t bfBandBytes(int T) { return (size_t) (bfK(T) / 8 + 8) * 256; }
+__host__ __device__ constexpr size_t bfBandBytes(int T) { return (size_t) (bfK(T + 3) / 8 + 8) * 256; }
 __host__ __device__ constexpr size_t bfSmemBytes(int Tmax) { return 2048 + 4 * kBfPlane + kBfTile * 4 + 8 * kBfRawFloats + 2 * bfBandBytes(Tmax); }
 static_assert(bfSmemBytes(kBfMaxTaps) <= 227 * 1024, "two plane sets and two of the longest bands fit");
 
 struct BfSmem {
    uint64_t *mmaDone, *planesFull, *accFree; // one per plane set / accumulator
    uint64_t *rawFull, *rawFree;              // one per raw slot
+   uint64_t *edges;                          // the split warps have written a raw tile's edges
    uint32_t *tslot;
    unsigned char *sets, *bands;
    float *stage; // one output tile, 1024 floats per drain warp
@@ -637,7 +591,8 @@ __device__ __forceinline__ BfSmem bfSmemLayout(unsigned char *smraw, int Tmax)
    L.accFree = L.planesFull + 2;
    L.rawFull = L.accFree + 2;
    L.rawFree = L.rawFull + 2;
-   L.tslot = (uint32_t *) (L.rawFree + 2);
+   L.edges = L.rawFree + 2;
+   L.tslot = (uint32_t *) (L.edges + 1);
    L.sets = sm + 1024;
    L.stage = (float *) (L.sets + 4 * kBfPlane);
    L.raw = L.stage + kBfTile;
@@ -651,117 +606,98 @@ __device__ __forceinline__ BfSmem bfSmemLayout(unsigned char *smraw, int Tmax)
 __device__ __forceinline__ int bfTileBlocks(const BfRun &r, int t)
 {
    const int outs = (int) min((long long) kBfTile, (long long) r.outLen - (long long) t * kBfTile);
-   return (outs + kBfPhases - 1) / kBfPhases + (bfK(r.T) + 63) / 64;
+   return (outs + kBfPhases - 1) / kBfPhases + (r.K + 63) / 64;
 }
 
-// Samples between the 16-byte boundary at or below a tile's first input and that input:
-// the same for every tile of a channel (a tile is 8192 samples).
-__device__ __forceinline__ int bfMis(const BfRun &r)
-{
-   return (int) ((((long long) ((uintptr_t) r.x >> 2)) + r.inShift) & 3);
-}
-
-// The raw window of tile t: `len` samples from input index w0 on, w0 on a 16-byte boundary.
-// The bulk copy takes its part inside the input, [lo, hi), both ends on 16-byte boundaries;
-// the split threads write the rest (up to 3 samples beside each end, and the zeros outside
-// the input).
+// A raw window: `len` samples from input index w0 on, w0 on a 16-byte boundary of the row x of
+// inLen samples.  The bulk copy takes its part inside the input, [lo, hi), both ends on
+// 16-byte boundaries; the split threads write the rest (up to 3 samples at each end, and the
+// zeros outside the input).
 struct BfWindow {
-   long long w0, lo, hi;
+   const float *x;
+   long long inLen, w0, lo, hi;
    int len;
+   __device__ uint32_t bytes() const { return (uint32_t) (hi - lo) * 4u; }
 };
-__device__ __forceinline__ BfWindow bfWindow(const BfRun &r, int t, int mis, int blocks)
+__device__ __forceinline__ BfWindow bfWindow(const float *x, long long inLen, long long w0, int len)
 {
-   BfWindow w;
-   w.w0 = r.inShift + (long long) t * kBfTile - mis;
-   w.len = blocks * kBfPhases + (mis ? 4 : 0);
-   w.lo = w.w0 >= 0 ? w.w0 : w.w0 + ((-w.w0 + 3) & ~3LL);
-   w.hi = w.w0 + ((min(w.w0 + w.len, r.inLen) - w.w0) & ~3LL);
+   BfWindow w{x, inLen, w0, w0, w0, len};
+   if (w0 < 0) w.lo = w0 + ((-w0 + 3) & ~3LL);
+   w.hi = w0 + ((min(w0 + len, inLen) - w0) & ~3LL);
    if (w.hi < w.lo) w.hi = w.lo;
    return w;
 }
-
-__device__ __forceinline__ void bfFixEdges(const BfRun &r, const BfWindow &w, float *raw, int tid)
+__device__ __forceinline__ void bfFixEdges(const BfWindow &w, float *raw, int tid)
 {
    for (int i = tid; i < (int) (w.lo - w.w0); i += kBfSplitThreads) {
       const long long q = w.w0 + i;
-      raw[i] = (q >= 0 && q < r.inLen) ? r.x[q] : 0.0f;
+      raw[i] = (q >= 0 && q < w.inLen) ? w.x[q] : 0.0f;
    }
    for (int i = (int) (w.hi - w.w0) + tid; i < w.len; i += kBfSplitThreads) {
       const long long q = w.w0 + i;
-      raw[i] = (q >= 0 && q < r.inLen) ? r.x[q] : 0.0f;
+      raw[i] = (q >= 0 && q < w.inLen) ? w.x[q] : 0.0f;
    }
+}
+// All split warps have written the edges: a bounded wait like the others (a warp that gave up
+// elsewhere would leave a named barrier waiting for good).
+__device__ __forceinline__ bool bfEdgesWritten(uint64_t *bar, uint32_t &phase, int lane)
+{
+   __syncwarp();
+   if (lane == 0) tc::mbarArrive(bar);
+   return tc::mbarWait(bar, phase++ & 1);
+}
+// The window of tile t of a run.
+__device__ __forceinline__ BfWindow bfTileWindow(const BfRun &r, int t, int blocks)
+{
+   return bfWindow(r.x, r.inLen, r.inShift - r.lead + (long long) t * kBfTile, blocks * kBfPhases);
 }
 
 // Split a raw tile into the planes: sample i (64 per 128-byte block k = i / 64) goes to
 // block k, 16-byte chunk c = (i % 64) / 8 stored at k * 128 + ((c ^ (k & 7)) * 16), as hi and lo
-// BF16.  Sample i is raw[MIS + i].  A thread takes 4 samples (consecutive lanes, consecutive
-// addresses) and writes half a chunk of each plane; its groups are 16 blocks apart, so they
-// share c and k & 7.  A full tile has at least 8 groups a thread (FULL: no test on those).
-template <int MIS, bool FULL>
-__device__ __forceinline__ void bfSplitMis(const float *raw, int nQuad, unsigned char *hi, unsigned char *lo, int tid)
+// BF16.  A thread takes 4 samples (consecutive lanes, consecutive addresses) and writes half a
+// chunk of each plane; its groups are 16 blocks apart, so they share c and k & 7.  The first
+// FULL of its up to GROUPS groups need no test.
+template <int FULL, int GROUPS>
+__device__ __forceinline__ void bfSplit(const float *raw, int nQuad, unsigned char *hi, unsigned char *lo, int tid)
 {
-   static_assert(8 * kBfSplitThreads <= kRows * 16 && kBfQuads == 9, "groups of a full tile");
    const int k = tid >> 4, off = k * 128 + ((((tid >> 1) & 7) ^ (k & 7)) << 4) + (tid & 1) * 8;
    const float4 *src = (const float4 *) raw + tid;
    hi += off;
    lo += off;
 #pragma unroll
-   for (int u0 = 0; u0 < kBfQuads; u0 += 3) {
-      float f[3][8];
+   for (int u0 = 0; u0 < GROUPS; u0 += 4) {
+      float4 f[4];
 #pragma unroll
-      for (int u = 0; u < 3; u++)
-         if ((FULL && u0 + u < 8) || tid + (u0 + u) * kBfSplitThreads < nQuad) {
-            *(float4 *) &f[u][0] = src[(u0 + u) * kBfSplitThreads];
-            if (MIS) *(float4 *) &f[u][4] = src[(u0 + u) * kBfSplitThreads + 1];
-         }
+      for (int u = 0; u < 4; u++)
+         if (u0 + u < GROUPS && (u0 + u < FULL || tid + (u0 + u) * kBfSplitThreads < nQuad))
+            f[u] = src[(u0 + u) * kBfSplitThreads];
 #pragma unroll
-      for (int u = 0; u < 3; u++)
-         if ((FULL && u0 + u < 8) || tid + (u0 + u) * kBfSplitThreads < nQuad) {
+      for (int u = 0; u < 4; u++)
+         if (u0 + u < GROUPS && (u0 + u < FULL || tid + (u0 + u) * kBfSplitThreads < nQuad)) {
             uint2 hv, lv;
-            splitBf16x2(f[u][MIS + 0], f[u][MIS + 1], hv.x, lv.x);
-            splitBf16x2(f[u][MIS + 2], f[u][MIS + 3], hv.y, lv.y);
+            splitBf16x2(f[u].x, f[u].y, hv.x, lv.x);
+            splitBf16x2(f[u].z, f[u].w, hv.y, lv.y);
             *(uint2 *) (hi + (u0 + u) * (kBfSplitThreads * 8)) = hv;
             *(uint2 *) (lo + (u0 + u) * (kBfSplitThreads * 8)) = lv;
          }
    }
 }
 
-__device__ __forceinline__ void bfSplit(const float *raw, int mis, int nQuad, unsigned char *hi, unsigned char *lo,
-                                        int tid)
-{
-   if (nQuad >= kRows * 16) {
-      switch (mis) { // uniform over the run
-      case 0: bfSplitMis<0, true>(raw, nQuad, hi, lo, tid); break;
-      case 1: bfSplitMis<1, true>(raw, nQuad, hi, lo, tid); break;
-      case 2: bfSplitMis<2, true>(raw, nQuad, hi, lo, tid); break;
-      default: bfSplitMis<3, true>(raw, nQuad, hi, lo, tid); break;
-      }
-   }
-   else {
-      switch (mis) {
-      case 0: bfSplitMis<0, false>(raw, nQuad, hi, lo, tid); break;
-      case 1: bfSplitMis<1, false>(raw, nQuad, hi, lo, tid); break;
-      case 2: bfSplitMis<2, false>(raw, nQuad, hi, lo, tid); break;
-      default: bfSplitMis<3, false>(raw, nQuad, hi, lo, tid); break;
-      }
-   }
-}
-
 // Taps band of a run.  Column n = 16 u + 8 v + i of the accumulator (u < 8, v = 0: hi taps,
 // 1: lo taps, i < 8) is phase b = 63 - (8 u + i); its operand row holds g[m - b], so the
-// 16-byte chunk q (taps m = 8 q .. 8 q + 7) of that row is G[8 (q + u) + i ..], G[k] = g[k - 63]:
+// 16-byte chunk q (taps m = 8 q .. 8 q + 7) of that row is G[8 (q + u) + i ..], G[k] = g[k - 63 - lead]:
 // it depends on q + u only.  With the phases in this order the K-major descriptor of the
 // band therefore reads one copy of each chunk, at (q + u) * 256 + v * 128 + i * 16 (256 bytes
 // between K chunks, 128 between groups of 8 columns), K / 8 + 8 rows of 256 bytes in all
 // instead of 256 bytes a tap.
 __device__ __forceinline__ void bfBand(const BfRun &r, unsigned char *band, int tid)
 {
-   const int T = r.T, n = bfK(T) + 64;
+   const int T = r.T, n = r.K + 64;
    for (int c = tid; c < n; c += kBfSplitThreads) { // c = 8 (q + u) + i
       uint32_t hv[4], lv[4];
 #pragma unroll
       for (int e = 0; e < 4; e++) {
-         const int k0 = c + 2 * e - 63, k1 = k0 + 1;
+         const int k0 = c + 2 * e - 63 - r.lead, k1 = k0 + 1;
          const float g0 = (k0 >= 0 && k0 < T) ? r.h[r.reverse ? T - 1 - k0 : k0] : 0.0f;
          const float g1 = (k1 >= 0 && k1 < T) ? r.h[r.reverse ? T - 1 - k1 : k1] : 0.0f;
          splitBf16x2(g0, g1, hv[e], lv[e]);
@@ -866,6 +802,7 @@ __device__ __forceinline__ void bfPipeline(const BfSmem &L, int nRuns, int *err,
          tc::mbarInit(L.rawFull + k, 1);
          tc::mbarInit(L.rawFree + k, kBfSplitWarps);
       }
+      tc::mbarInit(L.edges, kBfSplitWarps);
       tc::fenceMbarInit();
    }
    tc::fenceBeforeSync();
@@ -876,9 +813,9 @@ __device__ __forceinline__ void bfPipeline(const BfSmem &L, int nRuns, int *err,
    if (warp < kBfSplitWarps) {
       bool ok = true;
       int runs = 0, before = 0; // runs so far, tiles of the previous one
+      uint32_t edge = 0;
       for (int i = blockIdx.x; ok && i < nRuns; i += gridDim.x, runs++) {
          const BfRun r = get(i);
-         const int mis = bfMis(r);
          // The band's buffer was last read by the run before the previous one: its MMAs are
          // known to be complete (tile n - 3 or earlier) if the previous run had two tiles or
          // more, else once tile n - 2's are.
@@ -889,16 +826,17 @@ __device__ __forceinline__ void bfPipeline(const BfSmem &L, int nRuns, int *err,
             ok = n < 2 || tc::mbarWait(L.mmaDone + b, ((n >> 1) - 1) & 1);
             if (t == r.t0 && before < 2 && n >= 2) bfBand(r, L.band(runs), tid);
             ok = ok && tc::mbarWait(L.rawFull + b, (n >> 1) & 1);
-            const long long w0 = r.inShift - mis + (long long) t * kBfTile;
-            if (w0 < 0 || w0 + blocks * kBfPhases + 4 > r.inLen) { // the same for every split thread
-               if (ok) bfFixEdges(r, bfWindow(r, t, mis, blocks), L.slot(b), tid);
-               tc::namedSync(kBfSplitBar, kBfSplitThreads);
+            const long long w0 = r.inShift - r.lead + (long long) t * kBfTile;
+            if (w0 < 0 || w0 + blocks * kBfPhases > r.inLen) { // the same for every split thread
+               if (ok) bfFixEdges(bfTileWindow(r, t, blocks), L.slot(b), tid);
+               ok = ok && bfEdgesWritten(L.edges, edge, lane);
             }
             if (!ok) {
                raiseError(err);
                break;
             }
-            bfSplit(L.slot(b), mis, blocks * 16, L.hi(b), L.lo(b), tid);
+            if (blocks >= kRows) bfSplit<kRows * 16 / kBfSplitThreads, kBfQuads>(L.slot(b), blocks * 16, L.hi(b), L.lo(b), tid);
+            else bfSplit<0, kBfQuads>(L.slot(b), blocks * 16, L.hi(b), L.lo(b), tid);
             tc::fenceProxyAsync();
             __syncwarp();
             if (lane == 0) {
@@ -930,7 +868,7 @@ __device__ __forceinline__ void bfPipeline(const BfSmem &L, int nRuns, int *err,
       int runs = 0;
       for (int i = blockIdx.x; ok && i < nRuns; i += gridDim.x, runs++) {
          const BfRun r = get(i);
-         const int K = bfK(r.T);
+         const int K = r.K;
          const uint32_t bt = tc::smemAddr(L.band(runs));
          for (int t = r.t0; t < r.t1; t++, n++) {
             const int b = (int) (n & 1);
@@ -952,7 +890,6 @@ __device__ __forceinline__ void bfPipeline(const BfSmem &L, int nRuns, int *err,
       uint32_t issued = 0;
       for (int i = blockIdx.x; ok && i < nRuns; i += gridDim.x) {
          const BfRun r = get(i);
-         const int mis = bfMis(r);
          for (int t = r.t0; t < r.t1; t++, n++) {
             const int b = (int) (n & 1);
             if (n >= 2 && !tc::mbarWait(L.rawFree + b, ((n >> 1) - 1) & 1)) {
@@ -960,11 +897,10 @@ __device__ __forceinline__ void bfPipeline(const BfSmem &L, int nRuns, int *err,
                ok = false;
                break;
             }
-            const BfWindow w = bfWindow(r, t, mis, bfTileBlocks(r, t));
-            const uint32_t bytes = (uint32_t) (w.hi - w.lo) * 4u;
-            if (bytes) {
-               tc::mbarExpectTx(L.rawFull + b, bytes);
-               tc::bulkLoad(L.slot(b) + (w.lo - w.w0), r.x + w.lo, bytes, L.rawFull + b);
+            const BfWindow w = bfTileWindow(r, t, bfTileBlocks(r, t));
+            if (w.bytes()) {
+               tc::mbarExpectTx(L.rawFull + b, w.bytes());
+               tc::bulkLoad(L.slot(b) + (w.lo - w.w0), r.x + w.lo, w.bytes(), L.rawFull + b);
             }
             else tc::mbarArrive(L.rawFull + b);
             issued = n + 1;
@@ -999,6 +935,7 @@ __global__ void __launch_bounds__(kBfCta, 1) fir_bf16x3_tc_kernel(FirLaunch a, i
       r.reverse = 1;
       r.t0 = part * tilesPerRun;
       r.t1 = min(nt, r.t0 + tilesPerRun);
+      r.align();
       return r;
    });
 }
@@ -1015,9 +952,9 @@ __global__ void __launch_bounds__(kBfCta, 1)
       const int4 it = runs[i];
       const RaggedChan c = chans[it.x];
       BfRun r;
-      r.x = in + c.xOff;
+      r.x = in + (dx ? c.gOff : c.xOff);  // input gradient: the gradient plane of the scratch
       r.h = taps + c.hOff;
-      r.y = out + (dx ? c.xOff : c.pOff); // forward: plane 0 of the work buffer
+      r.y = out + (dx ? c.xOff : c.pOff); // forward: the FIR output plane of the work buffer
       r.T = c.T;
       r.inShift = dx ? -(long long) (c.T - 1) : 0;
       r.inLen = dx ? c.L - c.T + 1 : c.L;
@@ -1025,15 +962,12 @@ __global__ void __launch_bounds__(kBfCta, 1)
       r.reverse = dx ? 0 : 1;
       r.t0 = it.y;
       r.t1 = it.y + it.z;
+      r.align();
       return r;
    });
 }
 
 // ------------------------------------------------------------------ taps gradient (split-BF16x3)
-
-constexpr int kBfWorkers = kBfThreads;         // worker threads (16 warps)
-constexpr int kBfBlock = kBfWorkers + 32;      // + the MMA warp
-constexpr uint32_t kBfBar = 1;                 // the workers' named barrier
 
 // Taps gradient of the filter bank, dh_lag[c] = sum_j gu[j] x[j + c] (c < T), on the
 // tensor cores.  With j = 64 r + s (row r, phase s) and t' = c + s:
@@ -1043,20 +977,34 @@ constexpr uint32_t kBfBar = 1;                 // the workers' named barrier
 // (M = 128 positions t', 64 per 128-byte block, block r + t'/64 of the x plane, so the
 // second 64-wide atom of a tile starts one block (128 bytes) after the first), B = G
 // (N = 64 phases, block r of the gradient plane).  One accumulator tile per 128
-// positions (ceil((T + 63) / 128) <= 5 tiles of 64 TMEM columns) collects the three
-// split products x_hi g_hi + x_lo g_hi + x_hi g_lo over every row of a run of up to
-// four 8192-sample tiles; the diagonal sums are taken once per run, in a fixed order.
-// The next tile's planes are staged while the tensor core works on the current one.
-constexpr int kDhTile = kBfTile;                  // samples (128 rows) per staged tile
-constexpr int kDhMaxMt = (kBfMaxTaps + 63 + 127) / 128;
-constexpr int kDhXBlocks = 127 + 2 * kDhMaxMt;    // x blocks a tile's A operands reach
+// positions (Mt = ceil((T + 63) / 128) <= 5 tiles of 64 TMEM columns) collects the three
+// split products x_hi g_hi + x_lo g_hi + x_hi g_lo over every row of a run; the diagonal
+// sums are taken once per run, in a fixed order.
+//
+// The roles are those of the forward kernel: fetch (raw x and gradient tiles of 64 rows, a
+// ring of two), split (8 warps), MMA, and 8 warps that take the diagonal sums of run j
+// while the tensor core works on run j + 1 (accumulators of alternate runs 256 columns
+// apart; a run of five tiles takes 320 columns and waits for its neighbours).  Bound by the
+// shared-memory data path, as the forward kernel: per 64 rows 36 MMAs of 6 KB and 48 clocks
+// each (256 taps), and raw tiles, planes and their reads, about 900 clocks.  On the
+// 2048-channel bank 319 us against 404 us for one CTA a run that staged a tile of both signals
+// in lock step (100 clocks an MMA, set-up and diagonal sums of every run exposed).
+constexpr int kDhRows = 64;                       // rows (of 64 samples) per staged tile
+constexpr int kDhTile = kDhRows * kBfPhases;
+constexpr int kDhMaxMt = (kBfMaxTaps + 6 + 63 + 127) / 128;
+constexpr int kDhXBlocks = kDhRows - 1 + 2 * kDhMaxMt; // x blocks a tile's A operands reach
 constexpr size_t kDhXPlane = ((kDhXBlocks * 128 + 1023) / 1024) * 1024;
-constexpr size_t kDhGPlane = kRows * 128;
-constexpr size_t kDhBuf = 2 * kDhXPlane + 2 * kDhGPlane; // x hi, x lo, g hi, g lo
-constexpr size_t kDhSmem = 1024 + 2 * kDhBuf + 64;
+constexpr size_t kDhGPlane = kDhRows * 128;
+constexpr size_t kDhSet = 2 * kDhXPlane + 2 * kDhGPlane; // x hi, x lo, g hi, g lo
+constexpr int kDhRawX = kDhXBlocks * 64, kDhRawG = kDhTile; // floats
+constexpr int kDhXQuads = (kDhXBlocks * 16 + kBfSplitThreads - 1) / kBfSplitThreads;
+constexpr int kDhGQuads = kDhRows * 16 / kBfSplitThreads;
 constexpr int kDhPitch = 65;                      // floats per staged accumulator row
-static_assert((size_t) kRows * kDhPitch * 4 <= kDhBuf, "accumulator staging fits one buffer");
-static_assert(kDhMaxMt * 64 <= 512, "accumulator tiles fit the TMEM columns");
+constexpr size_t kDhSmem = 2048 + 2 * kDhSet + 8 * (size_t) (kDhRawX + kDhRawG) + 4 * (size_t) kRows * kDhPitch;
+constexpr int kDhDrainThreads = 32 * kBfDrainWarps;
+constexpr uint32_t kDhDrainBar = 2;
+static_assert(kDhSmem <= 227 * 1024, "plane sets, raw ring and accumulator staging fit");
+static_assert(kDhMaxMt * 64 <= 512 && 4 * 64 <= 256, "accumulator tiles fit the TMEM columns");
 
 // MN-major operand with 128-byte swizzle: 64-element atoms (128-byte rows, 8 rows per
 // 1024-byte swizzle atom along K), lbo = byte distance between atoms along M/N,
@@ -1072,140 +1020,242 @@ __device__ __forceinline__ uint64_t descSw128Mn(uint32_t saddr, uint32_t lbo, ui
    return d;
 }
 
-// Warp roles as in the split-BF16x3 FIR: warps 0-15 stage tiles into the two buffers
-// (planesFull[b] when buffer b holds tile k) and form the diagonal sums at the end; warp 16
-// issues the MMAs (mmaDone[b] when tile k's MMAs, reading buffer b, completed).
-__global__ void __launch_bounds__(kBfBlock, 1)
-    fir_dh_bf16x3_kernel(const RaggedChan *chans, const int4 *runs, const float *x, const float *gu, float *part,
-                         int *err)
+struct DhRun {
+   const float *x, *g;
+   int L, Lu, T, Mt, t0, t1, slot; // tiles [t0, t1) of kDhTile samples; slot: its partial sums
+   int leadX, leadG;               // samples before a tile that its windows start at, on 16-byte boundaries
+};
+
+// 16-row steps of tile t that hold gradient samples (the rows beyond are not contracted), and
+// its windows.
+__device__ __forceinline__ int dhSteps(const DhRun &r, int t)
+{
+   return min(kDhRows / 16, (r.Lu + r.leadG - t * kDhTile + 1023) / 1024);
+}
+__device__ __forceinline__ BfWindow dhWindowX(const DhRun &r, int t, int steps)
+{
+   return bfWindow(r.x, r.L, (long long) t * kDhTile - r.leadX, (16 * steps - 1 + 2 * r.Mt) * kBfPhases);
+}
+__device__ __forceinline__ BfWindow dhWindowG(const DhRun &r, int t, int steps)
+{
+   return bfWindow(r.g, r.Lu, (long long) t * kDhTile - r.leadG, 16 * steps * kBfPhases);
+}
+
+__global__ void __launch_bounds__(kBfCta, 1)
+    fir_dh_bf16x3_kernel(const RaggedChan *chans, const int4 *runs, int nRuns, const float *x, const float *gu,
+                         float *part, int *err)
 {
    extern __shared__ __align__(16) unsigned char smraw[];
    unsigned char *sm = (unsigned char *) (((uintptr_t) smraw + 1023) & ~(uintptr_t) 1023);
-   uint64_t *mbar = (uint64_t *) (sm + 2 * kDhBuf); // mmaDone, one per buffer
-   uint64_t *full = mbar + 2;                        // planesFull, one per buffer
-   uint32_t *tslot = (uint32_t *) (full + 2);
+   uint64_t *mmaDone = (uint64_t *) sm, *planesFull = mmaDone + 2; // per plane set
+   uint64_t *rawFull = mmaDone + 4, *rawFree = mmaDone + 6;        // per raw slot
+   uint64_t *accFull = mmaDone + 8, *accFree = mmaDone + 10;       // per parity of the run
+   uint64_t *edges = mmaDone + 12;
+   uint32_t *tslot = (uint32_t *) (mmaDone + 13);
+   unsigned char *sets = sm + 1024;
+   float *raw = (float *) (sets + 2 * kDhSet);
+   float *Ds = raw + 2 * (kDhRawX + kDhRawG);
+   auto set = [&](int b) { return sets + (size_t) b * kDhSet; };
+   auto slotX = [&](int b) { return raw + b * (kDhRawX + kDhRawG); };
+   auto slotG = [&](int b) { return raw + b * (kDhRawX + kDhRawG) + kDhRawX; };
    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-   const int4 run = runs[blockIdx.x]; // {channel, first tile, tiles, partial slot}
-   const RaggedChan c = chans[run.x];
-   const int T = c.T;
-   const int Mt = (T + 63 + 127) / 128;
-   const int nbX = 127 + 2 * Mt;
-   const float *xc = x + c.xOff, *gc = gu + c.xOff;
-   auto buf = [&](int b) { return sm + (size_t) b * kDhBuf; };
-   auto stage = [&](int t, int b) {
-      unsigned char *B = buf(b);
-      const long long q0 = (long long) t * kDhTile;
-      bfStage(xc, q0, c.L, nbX, B, B + kDhXPlane, tid);
-      bfStage(gc, q0, c.Lu, kRows, B + 2 * kDhXPlane, B + 2 * kDhXPlane + kDhGPlane, tid);
+   auto get = [&](int i) {
+      const int4 it = runs[i]; // {channel, first tile, tiles, partial slot}, tiles of 8192 samples
+      const RaggedChan c = chans[it.x];
+      DhRun r;
+      r.x = x + c.xOff;
+      r.g = gu + c.gOff;
+      r.L = c.L;
+      r.Lu = c.Lu;
+      r.T = c.T;
+      // windows on 16-byte boundaries, the input's at least as far ahead as the gradient's:
+      // position t' = c + s + leadX - leadG
+      r.leadG = (int) (((uintptr_t) r.g >> 2) & 3);
+      r.leadX = (int) (((uintptr_t) r.x >> 2) & 3);
+      if (r.leadX < r.leadG) r.leadX += 4;
+      r.Mt = (c.T + r.leadX - r.leadG + 63 + 127) / 128;
+      r.t0 = it.y * (kBfTile / kDhTile);
+      r.t1 = min((it.y + it.z) * (kBfTile / kDhTile), (c.Lu + r.leadG + kDhTile - 1) / kDhTile);
+      // the channel's last run takes a tile more where the lead pushes the last samples into it
+      if (it.y + it.z == (c.Lu + kBfTile - 1) / kBfTile) r.t1 = (c.Lu + r.leadG + kDhTile - 1) / kDhTile;
+      r.slot = it.w;
+      return r;
    };
    if (warp == 0) tc::tmemAlloc(tslot, 512);
    if (tid == 0) {
       for (int k = 0; k < 2; k++) {
-         tc::mbarInit(mbar + k, 1);
-         tc::mbarInit(full + k, 1);
+         tc::mbarInit(mmaDone + k, 1);
+         tc::mbarInit(planesFull + k, kBfSplitWarps);
+         tc::mbarInit(rawFull + k, 1);
+         tc::mbarInit(rawFree + k, kBfSplitWarps);
+         tc::mbarInit(accFull + k, 1);
+         tc::mbarInit(accFree + k, kBfDrainWarps);
       }
+      tc::mbarInit(edges, kBfSplitWarps);
       tc::fenceMbarInit();
    }
    tc::fenceBeforeSync();
    __syncthreads();
    tc::fenceAfterSync();
    const uint32_t tmem = *tslot;
-   bool fail = false;
-   if (tid < kBfWorkers) {
-      uint32_t par = 0; // mmaDone phase, one bit per buffer
-      for (int k = 0; k < run.z; k++) {
-         const int b = k & 1;
-         if (k >= 2) { // buffer b is free once tile k - 2's MMAs completed
-            const bool done = tid == 0 ? tc::mbarWait(mbar + b, (par >> b) & 1) : true;
-            par ^= 1u << b;
-            if (!done && tid == 0) raiseError(err);
-            if (tc::namedSyncOr(kBfBar, kBfWorkers, !done)) {
-               fail = true;
+   uint32_t n = 0; // tile n of this CTA uses plane set and raw slot n % 2, phase (n / 2) % 2
+   uint32_t j = 0; // run j likewise the accumulators
+   bool ok = true;
+   if (warp < kBfSplitWarps) {
+      uint32_t edge = 0;
+      for (int i = blockIdx.x; ok && i < nRuns; i += gridDim.x) {
+         const DhRun r = get(i);
+         for (int t = r.t0; t < r.t1; t++, n++) {
+            const int b = (int) (n & 1), steps = dhSteps(r, t);
+            ok = (n < 2 || tc::mbarWait(mmaDone + b, ((n >> 1) - 1) & 1)) && tc::mbarWait(rawFull + b, (n >> 1) & 1);
+            const long long e = (long long) t * kDhTile;
+            const int xb = 16 * steps - 1 + 2 * r.Mt, gb = 16 * steps;
+            // the same for every split thread
+            if ((t == 0 && r.leadX + r.leadG > 0) || e - r.leadX + xb * kBfPhases > r.L ||
+                e - r.leadG + gb * kBfPhases > r.Lu) {
+               if (ok) {
+                  bfFixEdges(dhWindowX(r, t, steps), slotX(b), tid);
+                  bfFixEdges(dhWindowG(r, t, steps), slotG(b), tid);
+                  ok = bfEdgesWritten(edges, edge, lane);
+               }
+            }
+            if (!ok) {
+               raiseError(err);
                break;
             }
-         }
-         stage(run.y + k, b);
-         tc::fenceProxyAsync();
-         tc::namedSync(kBfBar, kBfWorkers);
-         if (tid == 0) tc::mbarArrive(full + b);
-      }
-      // the last two tiles (bounded: after a failure, waits for tiles never issued give up)
-      for (int k = run.z >= 2 ? run.z - 2 : 0; !fail && k < run.z; k++) {
-         const int b = k & 1;
-         const bool done = tid == 0 ? tc::mbarWait(mbar + b, (par >> b) & 1) : true;
-         par ^= 1u << b;
-         if (!done && tid == 0) {
-            raiseError(err);
-            fail = true;
-         }
-      }
-   }
-   else if (tid == kBfWorkers) {
-      const uint32_t id = tc::idesc(1, 1, 1, kRows, 64) | (1u << 15) | (1u << 16); // both operands MN-major
-      uint32_t pf = 0;                                                               // planesFull phase per buffer
-      int commits = 0;
-      for (int k = 0; k < run.z; k++) {
-         const int b = k & 1;
-         if (!tc::mbarWait(full + b, (pf >> b) & 1)) {
-            raiseError(err);
-            fail = true;
-            break;
-         }
-         pf ^= 1u << b;
-         tc::fenceAfterSync();
-         unsigned char *B = buf(b);
-         const uint32_t xh = tc::smemAddr(B), xl = tc::smemAddr(B + kDhXPlane);
-         const uint32_t gh = tc::smemAddr(B + 2 * kDhXPlane), gl = tc::smemAddr(B + 2 * kDhXPlane + kDhGPlane);
-         for (int ks = 0; ks < kRows / 16; ks++) {
-            const uint64_t dGh = descSw128Mn(gh + ks * 2048, 128, 1024);
-            const uint64_t dGl = descSw128Mn(gl + ks * 2048, 128, 1024);
-            for (int m = 0; m < Mt; m++) {
-               const uint32_t off = (uint32_t) (ks * 16 + 2 * m) * 128;
-               const uint64_t dXh = descSw128Mn(xh + off, 128, 1024);
-               const uint64_t dXl = descSw128Mn(xl + off, 128, 1024);
-               const uint32_t d = tmem + 64 * m;
-               tc::mmaF16(d, dXh, dGh, id, k > 0 || ks > 0);
-               tc::mmaF16(d, dXl, dGh, id, true);
-               tc::mmaF16(d, dXh, dGl, id, true);
+            unsigned char *B = set(b);
+            bfSplit<0, kDhXQuads>(slotX(b), xb * 16, B, B + kDhXPlane, tid);
+            bfSplit<0, kDhGQuads>(slotG(b), gb * 16, B + 2 * kDhXPlane, B + 2 * kDhXPlane + kDhGPlane, tid);
+            tc::fenceProxyAsync();
+            __syncwarp();
+            if (lane == 0) {
+               tc::mbarArrive(planesFull + b);
+               tc::mbarArrive(rawFree + b);
             }
          }
-         tc::commit(mbar + b);
-         commits++;
       }
-      // after a failure: let the MMAs already committed finish before TMEM is released
-      // (tile n commits phase n / 2 of barrier n % 2)
-      if (fail)
-         for (int n = commits >= 2 ? commits - 2 : 0; n < commits; n++) (void) tc::mbarWait(mbar + (n & 1), (n >> 1) & 1);
    }
-   if (__syncthreads_or(fail)) {
-      tc::fenceAfterSync();
-      if (warp == 0) tc::tmemFree(tmem, 512);
-      return;
-   }
-   tc::fenceAfterSync();
-   // diagonal sums: lag c (thread c) adds D[c + s][s] over s, accumulator tile by tile
-   float acc = 0.0f;
-   float *Ds = (float *) buf(0);
-   for (int m = 0; m < Mt; m++) {
-      if (warp < 16) {
-         const int quad = warp & 3, cg = warp >> 2; // TMEM lanes 32 quad.., columns 16 cg..
-         uint32_t r[16];
-         tc::tmemLoad16(tmem + ((uint32_t) (quad * 32) << 16) + 64 * m + 16 * cg, r);
-         tc::tmemWaitLoad();
-         float *row = Ds + (quad * 32 + lane) * kDhPitch + 16 * cg;
+   else if (warp < kBfMmaWarp) {
+      const int dt = tid - kBfSplitThreads, quad = warp & 3, half = (warp - kBfSplitWarps) >> 2;
+      for (int i = blockIdx.x; ok && i < nRuns; i += gridDim.x, j++) {
+         const DhRun r = get(i);
+         const uint32_t base = tmem + (r.Mt > 4 ? 0 : (j & 1) * 256) + ((uint32_t) (quad * 32) << 16) + half * 32;
+         ok = tc::mbarWait(accFull + (j & 1), (j >> 1) & 1);
+         if (tc::namedSyncOr(kDhDrainBar, kDhDrainThreads, !ok)) {
+            raiseError(err);
+            ok = false;
+            break;
+         }
+         tc::fenceAfterSync();
+         // lag c adds D[c + shift + s][s] over s, accumulator tile by tile; a thread takes two lags
+         float acc[2] = {0.0f, 0.0f};
+         const int shift = r.leadX - r.leadG;
+         for (int m = 0; m < r.Mt; m++) {
+            uint32_t d[32];
+            tc::tmemLoad32(base + 64 * m, d);
+            tc::tmemWaitLoad();
+            if (m + 1 == r.Mt) {
+               tc::fenceBeforeSync();
+               __syncwarp();
+               if (lane == 0) tc::mbarArrive(accFree + (j & 1));
+            }
+            float *row = Ds + (quad * 32 + lane) * kDhPitch + half * 32;
 #pragma unroll
-         for (int i = 0; i < 16; i++) row[i] = __uint_as_float(r[i]);
+            for (int k = 0; k < 32; k++) row[k] = __uint_as_float(d[k]);
+            tc::namedSync(kDhDrainBar, kDhDrainThreads);
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+               const int c = dt + u * kDhDrainThreads, first = c + shift - 128 * m; // row of s = 0 in this tile
+               if (c < r.T && first > -64 && first < 128) {
+                  const float *diag = Ds + first * kDhPitch; // row first + sp, column sp
+                  for (int s0 = 0; s0 < 64; s0 += 16) { // 16 loads in flight
+                     float v[16];
+#pragma unroll
+                     for (int k = 0; k < 16; k++) {
+                        const int row = first + s0 + k;
+                        v[k] = (row >= 0 && row < 128) ? diag[(s0 + k) * (kDhPitch + 1)] : 0.0f;
+                     }
+#pragma unroll
+                     for (int k = 0; k < 16; k++) acc[u] += v[k];
+                  }
+               }
+            }
+            tc::namedSync(kDhDrainBar, kDhDrainThreads);
+         }
+#pragma unroll
+         for (int u = 0; u < 2; u++) {
+            const int c = dt + u * kDhDrainThreads;
+            if (c < r.T) part[(long long) r.slot * kBfMaxTaps + c] = acc[u];
+         }
       }
-      __syncthreads();
-      if (tid < T) {
-         const int lo = max(0, 128 * m - tid), hi = min(63, 128 * m + 127 - tid);
-         for (int sp = lo; sp <= hi; sp++) acc += Ds[(tid + sp - 128 * m) * kDhPitch + sp];
-      }
-      __syncthreads();
    }
-   if (tid < T) part[(long long) run.w * kBfMaxTaps + tid] = acc;
+   else if (warp == kBfMmaWarp && tc::electOne()) {
+      const uint32_t id = tc::idesc(1, 1, 1, kRows, 64) | (1u << 15) | (1u << 16); // both operands MN-major
+      bool wide = false; // the run before took five tiles
+      for (int i = blockIdx.x; ok && i < nRuns; i += gridDim.x, j++) {
+         const DhRun r = get(i);
+         const uint32_t base = tmem + (r.Mt > 4 ? 0 : (j & 1) * 256);
+         // the run before the previous one has been read, and the previous one too where its columns overlap
+         if ((j >= 2 && !tc::mbarWait(accFree + (j & 1), ((j >> 1) - 1) & 1)) ||
+             (j >= 1 && (wide || r.Mt > 4) && !tc::mbarWait(accFree + ((j - 1) & 1), ((j - 1) >> 1) & 1))) {
+            raiseError(err);
+            ok = false;
+            break;
+         }
+         wide = r.Mt > 4;
+         const int Mt = r.Mt;
+         for (int t = r.t0; t < r.t1; t++, n++) {
+            const int b = (int) (n & 1), steps = dhSteps(r, t);
+            if (!tc::mbarWait(planesFull + b, (n >> 1) & 1)) {
+               raiseError(err);
+               ok = false;
+               break;
+            }
+            tc::fenceAfterSync();
+            unsigned char *B = set(b);
+            // descriptor addresses count 16 bytes: a block is 8, the lo planes follow the hi ones
+            uint64_t dX = descSw128Mn(tc::smemAddr(B), 128, 1024);
+            uint64_t dG = descSw128Mn(tc::smemAddr(B + 2 * kDhXPlane), 128, 1024);
+            for (int ks = 0; ks < steps; ks++, dX += 128, dG += 128) {
+#pragma unroll
+               for (int m = 0; m < kDhMaxMt; m++)
+                  if (m < Mt) {
+                     tc::mmaF16(base + 64 * m, dX + 16 * m, dG, id, t > r.t0 || ks > 0);
+                     tc::mmaF16(base + 64 * m, dX + (16 * m + kDhXPlane / 16), dG, id, true);
+                     tc::mmaF16(base + 64 * m, dX + 16 * m, dG + kDhGPlane / 16, id, true);
+                  }
+            }
+            tc::commit(mmaDone + b);
+         }
+         if (ok) tc::commit(accFull + (j & 1));
+      }
+      // wait (bounded) for the last two tiles' MMAs before TMEM is released
+      for (uint32_t k = n >= 2 ? n - 2 : 0; k < n; k++) (void) tc::mbarWait(mmaDone + (k & 1), (k >> 1) & 1);
+   }
+   else if (warp == kBfFetchWarp && tc::electOne()) {
+      for (int i = blockIdx.x; ok && i < nRuns; i += gridDim.x) {
+         const DhRun r = get(i);
+         for (int t = r.t0; t < r.t1; t++, n++) {
+            const int b = (int) (n & 1), steps = dhSteps(r, t);
+            if (n >= 2 && !tc::mbarWait(rawFree + b, ((n >> 1) - 1) & 1)) {
+               raiseError(err);
+               ok = false;
+               break;
+            }
+            const BfWindow wx = dhWindowX(r, t, steps), wg = dhWindowG(r, t, steps);
+            const uint32_t bytes = wx.bytes() + wg.bytes();
+            if (bytes) tc::mbarExpectTx(rawFull + b, bytes);
+            else tc::mbarArrive(rawFull + b);
+            if (wx.bytes()) tc::bulkLoad(slotX(b) + (wx.lo - wx.w0), r.x + wx.lo, wx.bytes(), rawFull + b);
+            if (wg.bytes()) tc::bulkLoad(slotG(b) + (wg.lo - wg.w0), r.g + wg.lo, wg.bytes(), rawFull + b);
+         }
+      }
+      // copies still in flight land (bounded) before shared memory is given up
+      for (uint32_t k = n >= 2 ? n - 2 : 0; k < n; k++) (void) tc::mbarWait(rawFull + (k & 1), (k >> 1) & 1);
+   }
    tc::fenceBeforeSync();
    __syncthreads();
+   tc::fenceAfterSync();
    if (warp == 0) tc::tmemFree(tmem, 512);
 }
 } // namespace
@@ -1332,7 +1382,8 @@ cudaError_t launchFirDhBf16x3Ragged(const RaggedChan *chans, const int4 *runs, i
    cudaError_t e =
        cudaFuncSetAttribute(fir_dh_bf16x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kDhSmem);
    if (e != cudaSuccess) return e;
-   fir_dh_bf16x3_kernel<<<nRuns, kBfBlock, kDhSmem, s>>>(chans, runs, x, gu, part, err);
+   const int sms = deviceSms() > 0 ? deviceSms() : 148;
+   fir_dh_bf16x3_kernel<<<nRuns < sms ? nRuns : sms, kBfCta, kDhSmem, s>>>(chans, runs, nRuns, x, gu, part, err);
    countLaunch();
    return cudaGetLastError();
 }

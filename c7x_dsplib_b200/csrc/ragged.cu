@@ -291,7 +291,7 @@ static DSPLIB_STATUS raggedPlanBuild(DSPLIB_gpu_raggedPlan *plan, int32_t numCha
       }
       const int Lu = L - T + 1;
       const int nu = (Lu + kBankSpan - 1) / kBankSpan;
-      ch[c] = RaggedChan{xo, ho, co, po, L, T, S, Lu, ck, ph, gr};
+      ch[c] = RaggedChan{xo, ho, co, po, L, T, S, Lu, xo, ck, ph, gr};
       gr += 2LL * S * ((nu + 31) / 32);
       po += (Lu + 15) & ~15;
       ck += (long long) nu * S;
@@ -314,6 +314,18 @@ static DSPLIB_STATUS raggedPlanBuild(DSPLIB_gpu_raggedPlan *plan, int32_t numCha
       addRuns(firDx, c, L);
    }
    start[numChannels] = (int) dhRuns.size();
+   // Gradient plane of the scratch: channels on 16-byte boundaries (the tensor-core kernels
+   // copy whole 16-byte groups) where that fits in the packed length, as it does unless most
+   // channels have fewer than four taps; else packed as the input is.
+   long long go = 0;
+   for (const RaggedChan &q : ch) go += (q.Lu + 3) & ~3;
+   if (go <= xo) {
+      go = 0;
+      for (RaggedChan &q : ch) {
+         q.gOff = go;
+         go += (q.Lu + 3) & ~3;
+      }
+   }
    // longest runs first, so the short ones fill in behind them
    auto longer = [](const int4 &a, const int4 &b) { return a.z > b.z; };
    std::stable_sort(firFwd.begin(), firFwd.end(), longer);

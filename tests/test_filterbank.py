@@ -181,6 +181,24 @@ def test_bank_long_taps():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("T", [2, 65, 66, 193, 444, 512])
+def test_bank_gradient_tile_edges(T):
+    """Channels whose outputs end around a 64-sample row, a 1024-sample step, a 4096-sample
+    gradient tile, an 8192-output FIR tile and a 16-tile run of the taps gradient; taps around
+    the 128-position accumulator tiles, next to channels of few taps (accumulators of
+    neighbouring runs); with two taps the gradient plane keeps the input's packing."""
+    outs = [1, 63, 65, 1023, 1025, 4095, 4097, 8191, 8193, 12289, 16 * 8192 + 3]
+    taps = [T if k % 3 else min(T, 3) for k in range(len(outs))]
+    rng = np.random.default_rng(T)
+    lengths = [n + t - 1 for n, t in zip(outs, taps)]
+    stages = [k % 3 for k in range(len(outs))]
+    x = rng.standard_normal(sum(lengths))
+    h = np.concatenate([rng.standard_normal(t) / np.sqrt(t) for t in taps])
+    c = np.concatenate([stable_sections(rng, S).reshape(-1) for S in stages])
+    _check_bank(lengths, taps, stages, x, h, c, seed=T)
+
+
+@pytest.mark.gpu
 def test_bank_many_channels():
     _check_bank(*_bank_case(4, 300, Lrange=(256, 4000), Tmax=64, Smax=6))
 
