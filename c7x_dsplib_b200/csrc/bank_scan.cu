@@ -1,30 +1,38 @@
 // Cascade of direct-form-II biquads of the batched filter bank, forward and
-// adjoint, split along time into 512-sample units that warps filter
+// adjoint, split along time into 1024-sample units that warps filter
 // independently, with no wait between CTAs and no CTA barrier.
 //
-// A unit is one warp; each lane owns a chunk of 16 consecutive samples.  Per
-// stage the chunk is filtered from a zero state (the only serial pass), the
-// chunk end states are combined by a warp scan of the affine maps
+// A unit is one warp; each lane owns 32 consecutive samples as two chunks of 16, A and B, held
+// as packed pairs (A_i, B_i): every FP32 operation on samples is a packed one (fma.rn.f32x2,
+// each half rounded as fmaf).  The FMA pipe's rate is the same, but a packed instruction takes
+// half the issue slots, which bound these passes (73 - 81 % of them used with the pipe at 55 %),
+// and one warp scan serves 1024 samples instead of 512.  Per
+// stage the chunks are run from a zero state for their end states, a lane's two
+// end states combine, the lanes' end states are combined by a warp scan of the affine maps
 // s -> M s + e (M = A^16 and its powers, A the stage's 2x2 companion matrix,
 // formed in FP64 and rounded once; the unit's entry state joins the first
-// chunk's end state before the scan), and the true output follows without a
-// serial chain: w[i] = w_zs[i] + alpha_i w1 + beta_i w2 with (alpha_i, beta_i)
-// the first row of A^(i+1) and (w1, w2) the chunk's initial state, then
-// y[i] = b0 w[i] + b1 w[i-1] + b2 w[i-2].
+// lane's end state before the scan), and the chunks run again from their true initial states:
+// w[i] = u[i] - a1 w[i-1] - a2 w[i-2], y[i] = b0 w[i] + b1 w[i-1] + b2 w[i-2].  (Correcting the
+// first run's sequence by the free response instead, w[i] += alpha_i w1 + beta_i w2, has no
+// second serial chain but keeps the sequence in 32 registers a lane and reads 16 more
+// table vectors a stage: slower, with 250 registers in the adjoint.)
 //
 // Units are chained through the whole cascade at once.  With the state of
 // all S stages at a unit's start as one 2S-vector z, the state at its end is
 // Phi z + e, where e is the end state when every stage starts the unit from
-// zero and Phi = A_c^512, A_c the cascade's 2S x 2S one-step transition (block
+// zero and Phi = A_c^1024, A_c the cascade's 2S x 2S one-step transition (block
 // lower-triangular: stage p's output drives stage p + 1).  So:
-//   pass 1 (bank_unit_kernel<AGG>): every unit, all stages from a zero state:
-//           e, 2 floats per stage;
+//   pass 1 (bank_agg_kernel): e of every unit but the channel's last, as dot products of
+//           the unit's input with the impulse responses k_s from the cascade's input to each
+//           stage's internal sequence (bank_impulse_kernel, once per channel):
+//           e_s = (sum_t k_s[1023 - t] u[t], sum_t k_s[1022 - t] u[t]), two multiply-adds a
+//           sample and stage instead of the seven of a filtering pass;
 //   pass 2 (bank_chain_fast_kernel up to 16 stages, bank_chain_kernel beyond):
 //           per channel, z_0 = 0, z_{j+1} = Phi z_j + e_j, j over the
 //           channel's units (in two levels through Phi^32 over groups of 32
 //           units in FP32, or one unit after another in FP64); z_j is stored
 //           (2 floats per unit and stage): the checkpoints;
-//   pass 3 (bank_unit_kernel<OUT>): every unit again from its checkpoint: y.
+//   pass 3 (bank_unit_kernel): every unit from its checkpoint: y.
 // The adjoint is the same cascade run backwards in time with the stages in
 // reverse order (v[t] = g[t] - a1 v[t+1] - a2 v[t+2], lambda[t] = b0 v[t] +
 // b1 v[t+1] + b2 v[t+2]: g the stage's output gradient, lambda its input
@@ -46,21 +54,22 @@ namespace {
 using scan::M2;
 using scan::M2f;
 
-constexpr int kL = 16;          // samples per chunk (lane)
-constexpr int kUnit = 32 * kL;  // samples per unit (warp): 512
+constexpr int kL = 16;          // samples per chunk
+constexpr int kLane = 2 * kL;   // samples per lane: chunks A and B
+constexpr int kUnit = 32 * kLane; // samples per unit (warp): 1024
 constexpr int kWarps = 4;       // units per CTA
 constexpr int kThreads = 32 * kWarps;
-constexpr int kOutPad = kL + 1; // padded shared row per chunk (conflict-free staging)
-constexpr int kUnitLog2 = 9;    // Phi = A_c^(2^9)
+constexpr int kRow = kLane + 2; // staging row of a lane's samples, pairs (A_i, B_i) adjacent (conflict-free)
+constexpr int kStage = 32 * kRow;
+constexpr int kUnitLog2 = 10;   // Phi = A_c^(2^10)
 constexpr int kChainFastStages = 16; // cascades the FP32 register chain takes
 
 static_assert(kUnit == kBankSpan, "unit size");
 
 // Stage table (floats): [0, 5) b0 b1 b2 a1 a2; [8 + 4k, 12 + 4k) P[k] = M^(2^k), M = A^16,
-// k = 0..8, row-major; [44 + 2i, 46 + 2i) alpha_i, beta_i = row 0 of A^(i+1), i = 0..15.
+// k = 0..8, row-major.
 constexpr int kTabP = 8;
-constexpr int kTabAB = 44;
-static_assert(kTabAB + 2 * kL <= kBankTabFloats, "stage table layout");
+static_assert(kTabP + 4 * 9 <= kBankTabFloats && kBankTabFloats % 4 == 0, "stage table layout");
 
 __device__ __forceinline__ M2f tabP(const float *tb, int k)
 {
@@ -86,15 +95,6 @@ __global__ void __launch_bounds__(128) bank_tables_kernel(const float *coefs, in
    for (int k = 0; k < 5; k++) tb[k] = cf[k];
    for (int k = 5; k < kTabP; k++) tb[k] = 0.0f;
    const double a1 = cf[3], a2 = cf[4];
-   // row 0 of A^(i+1): row0(A^(i+2)) = row0(A^(i+1)) A, A = [[-a1, -a2], [1, 0]]
-   double r0 = -a1, r1 = -a2;
-   for (int i = 0; i < kL; i++) {
-      tb[kTabAB + 2 * i] = (float) r0;
-      tb[kTabAB + 2 * i + 1] = (float) r1;
-      const double n0 = fma(r0, -a1, r1), n1 = r0 * -a2;
-      r0 = n0;
-      r1 = n1;
-   }
    M2 M = {-a1, -a2, 1.0, 0.0};
    for (int r = 1; r < kL; r <<= 1) M = scan::mmul(M, M);
    for (int k = 0; k <= 8; k++) {
@@ -102,7 +102,6 @@ __global__ void __launch_bounds__(128) bank_tables_kernel(const float *coefs, in
       *(float4 *) (tb + kTabP + 4 * k) = make_float4(f.a, f.b, f.c, f.d);
       M = scan::mmul(M, M);
    }
-   for (int k = kTabAB + 2 * kL; k < kBankTabFloats; k++) tb[k] = 0.0f;
 }
 
 // ------------------------------------------------------------------ cascade transitions
@@ -114,7 +113,7 @@ __host__ __device__ inline int blk(int p, int q) { return p * (p + 1) / 2 + q; }
 // Processing position p -> stage: forward p, adjoint S - 1 - p.
 __device__ __forceinline__ int stageAt(int p, int S, bool adj) { return adj ? S - 1 - p : p; }
 
-// Phi = A_c^512 for one channel and direction, one CTA: A_c in shared memory, nine
+// Phi = A_c^1024 for one channel and direction, one CTA: A_c in shared memory, ten
 // squarings C(p,q) = sum_{m=q..p} B(p,m) B(m,q) between two shared buffers; then
 // Phi^32.  Per channel: Phi forward, Phi adjoint, Phi^32 forward, Phi^32 adjoint.
 __global__ void __launch_bounds__(128) bank_transition_kernel(const RaggedChan *chans, const float *coefs,
@@ -380,155 +379,216 @@ __global__ void __launch_bounds__(kChainWarps * 32) bank_chain_fast_kernel(const
 
 // ------------------------------------------------------------------ unit passes
 
-// Load the 16 samples of a chunk from a 16-float-aligned plane row, zero at t >= n.
-__device__ __forceinline__ void loadChunk(float (&v)[kL], const float *row, int t0, int n)
+// Two FP32 values in a register pair, and the packed operations on them.
+struct P2 {
+   unsigned long long v;
+};
+__device__ __forceinline__ P2 pk(float a, float b)
 {
-   const int np = (n + 15) & ~15; // the row is allocated to a multiple of 16 floats
-   if (t0 < np) {
+   P2 r;
+   asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+   return r;
+}
+__device__ __forceinline__ float2 up(P2 a)
+{
+   float2 r;
+   asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+   return r;
+}
+__device__ __forceinline__ P2 dup(float a) { return pk(a, a); }
+__device__ __forceinline__ P2 fma2(P2 a, P2 b, P2 c)
+{
+   P2 r;
+   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+   return r;
+}
+__device__ __forceinline__ P2 mul2(P2 a, P2 b)
+{
+   P2 r;
+   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+   return r;
+}
+
+// A warp's staging area: row l holds lane l's 32 samples, sample i at column
+// 2 (i % 16) + i / 16, so that a lane's pair i is one 8-byte access and 32 consecutive
+// samples are 32 distinct banks.
+__device__ __forceinline__ int stageCol(int i) { return 2 * (i & 15) + (i >> 4); }
+
+__device__ __forceinline__ void stageRead(P2 (&v)[kL], const float *stage, int lane)
+{
+   __syncwarp();
 #pragma unroll
-      for (int q = 0; q < kL / 4; q++) {
-         const float4 f = *(const float4 *) (row + t0 + 4 * q);
-         v[4 * q + 0] = t0 + 4 * q + 0 < n ? f.x : 0.0f;
-         v[4 * q + 1] = t0 + 4 * q + 1 < n ? f.y : 0.0f;
-         v[4 * q + 2] = t0 + 4 * q + 2 < n ? f.z : 0.0f;
-         v[4 * q + 3] = t0 + 4 * q + 3 < n ? f.w : 0.0f;
-      }
+   for (int i = 0; i < kL; i++) v[i].v = *(const unsigned long long *) (stage + lane * kRow + 2 * i);
+   __syncwarp();
+}
+
+// The unit's samples of a row, zero at t >= n.  fetchUnit issues the coalesced loads (sample
+// t0 + lane + 32 j in r[j]); stageUnit turns them into the lane's pairs, so that a kernel can
+// put other work between the two.
+__device__ __forceinline__ void fetchUnit(float (&r)[kLane], const float *row, int t0, int n, int lane)
+{
+   const float *p = row + t0 + lane;
+   if (t0 + kUnit <= n) {
+#pragma unroll
+      for (int j = 0; j < kLane; j++) r[j] = p[32 * j];
    }
    else {
 #pragma unroll
-      for (int i = 0; i < kL; i++) v[i] = 0.0f;
+      for (int j = 0; j < kLane; j++) r[j] = t0 + lane + 32 * j < n ? p[32 * j] : 0.0f;
    }
 }
-
-// The chunk of an unaligned packed row (x, y, gradients), through the warp's staging
-// area so that every access of the warp covers 32 consecutive samples.  fetchPacked
-// issues the unit's coalesced loads (sample t0 + lane + 32 j in r[j]); stagePacked turns
-// them into the lane's chunk, so that a kernel can put other work between the two.
-__device__ __forceinline__ void fetchPacked(float (&r)[kL], const float *row, int t0, int n, int lane)
+__device__ __forceinline__ void stageUnit(P2 (&v)[kL], const float (&r)[kLane], float *stage, int lane)
 {
+   const int col = stageCol(lane);
 #pragma unroll
-   for (int j = 0; j < kL; j++) {
-      const int k = lane + 32 * j;
-      r[j] = t0 + k < n ? row[t0 + k] : 0.0f;
+   for (int j = 0; j < kLane; j++) stage[j * kRow + col] = r[j];
+   stageRead(v, stage, lane);
+}
+// The same of a 16-byte-aligned row allocated to a multiple of 16 floats (the FIR output
+// plane): 16-byte loads, samples 4 (lane + 32 j) .. + 3 in r[j].
+__device__ __forceinline__ void fetchPlane(float4 (&r)[kL / 2], const float *row, int t0, int n, int lane)
+{
+   const int np = (n + 15) & ~15;
+#pragma unroll
+   for (int j = 0; j < kL / 2; j++) {
+      const int t = t0 + 4 * (lane + 32 * j);
+      r[j] = t < np ? *(const float4 *) (row + t) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (t0 + kUnit > n) {
+         if (t + 0 >= n) r[j].x = 0.0f;
+         if (t + 1 >= n) r[j].y = 0.0f;
+         if (t + 2 >= n) r[j].z = 0.0f;
+         if (t + 3 >= n) r[j].w = 0.0f;
+      }
    }
 }
-__device__ __forceinline__ void stagePacked(float (&v)[kL], const float (&r)[kL], float *stage, int lane)
+__device__ __forceinline__ void stagePlane(P2 (&v)[kL], const float4 (&r)[kL / 2], float *stage, int lane)
+{
+   const int i = 4 * (lane & 7); // sample within its lane's row lane / 8 + 4 j
+   float *d = stage + (lane >> 3) * kRow + stageCol(i);
+#pragma unroll
+   for (int j = 0; j < kL / 2; j++) {
+      d[4 * j * kRow + 0] = r[j].x;
+      d[4 * j * kRow + 2] = r[j].y;
+      d[4 * j * kRow + 4] = r[j].z;
+      d[4 * j * kRow + 6] = r[j].w;
+   }
+   stageRead(v, stage, lane);
+}
+
+__device__ __forceinline__ void storeUnit(const P2 (&v)[kL], float *row, int t0, int n, float *stage, int lane)
 {
 #pragma unroll
-   for (int j = 0; j < kL; j++) {
-      const int k = lane + 32 * j;
-      stage[(k >> 4) * kOutPad + (k & 15)] = r[j];
+   for (int i = 0; i < kL; i++) *(unsigned long long *) (stage + lane * kRow + 2 * i) = v[i].v;
+   __syncwarp();
+   const float *s = stage + stageCol(lane);
+   float *p = row + t0 + lane;
+   if (t0 + kUnit <= n) {
+#pragma unroll
+      for (int j = 0; j < kLane; j++) p[32 * j] = s[j * kRow];
+   }
+   else {
+#pragma unroll
+      for (int j = 0; j < kLane; j++)
+         if (t0 + lane + 32 * j < n) p[32 * j] = s[j * kRow];
    }
    __syncwarp();
-#pragma unroll
-   for (int i = 0; i < kL; i++) v[i] = stage[lane * kOutPad + i];
-   __syncwarp();
 }
 
-__device__ __forceinline__ void storePacked(const float (&v)[kL], float *row, int t0, int n, float *stage, int lane)
+// Coefficients of a stage as packed operands.
+struct StageCoef {
+   P2 b0, b1, b2, na1, na2;
+};
+__device__ __forceinline__ StageCoef stageCoef(const float *tb)
 {
-#pragma unroll
-   for (int i = 0; i < kL; i++) stage[lane * kOutPad + i] = v[i];
-   __syncwarp();
-   for (int k = lane; k < kUnit && t0 + k < n; k += 32) row[t0 + k] = stage[(k >> 4) * kOutPad + (k & 15)];
-   __syncwarp();
+   const float4 q = *(const float4 *) tb;
+   return {dup(q.x), dup(q.y), dup(q.z), dup(-q.w), dup(-tb[4])};
 }
 
-// DF2 over the chunk from a zero state (w[i]), returning the end state (w[15], w[14]).
-__device__ __forceinline__ float2 zeroStatePass(const float (&v)[kL], float (&w)[kL], float a1, float a2)
+// End states of both chunks from a zero state: (w[15], w[14]).
+__device__ __forceinline__ void zeroStateEnd(const P2 (&v)[kL], const StageCoef &c, P2 &w15, P2 &w14)
 {
-   float p1 = 0.0f, p2 = 0.0f;
+   P2 p1 = dup(0.0f), p2 = p1;
 #pragma unroll
    for (int i = 0; i < kL; i++) {
-      w[i] = fmaf(-a1, p1, fmaf(-a2, p2, v[i]));
+      const P2 w = fma2(c.na1, p1, fma2(c.na2, p2, v[i]));
       p2 = p1;
-      p1 = w[i];
+      p1 = w;
    }
-   return make_float2(w[kL - 1], w[kL - 2]);
+   w15 = p1;
+   w14 = p2;
 }
 
-// The same in reverse time: v[i] = g[i] - a1 v[i+1] - a2 v[i+2]; end state (v[0], v[1]).
-__device__ __forceinline__ float2 zeroStatePassRev(const float (&g)[kL], float (&v)[kL], float a1, float a2)
+// The same in reverse time, v[i] = g[i] - a1 v[i+1] - a2 v[i+2]: (v[0], v[1]).
+__device__ __forceinline__ void zeroStateEndRev(const P2 (&g)[kL], const StageCoef &c, P2 &v0, P2 &v1)
 {
-   float p1 = 0.0f, p2 = 0.0f;
+   P2 p1 = dup(0.0f), p2 = p1;
 #pragma unroll
    for (int i = kL - 1; i >= 0; i--) {
-      v[i] = fmaf(-a1, p1, fmaf(-a2, p2, g[i]));
+      const P2 v = fma2(c.na1, p1, fma2(c.na2, p2, g[i]));
       p2 = p1;
-      p1 = v[i];
+      p1 = v;
    }
-   return make_float2(v[0], v[1]);
+   v0 = p1;
+   v1 = p2;
 }
 
-// Initial state of this lane's chunk, forward time: M^lane entry + the scan of the lanes
-// before.  The first chunk's end state takes the unit's entry (M entry + its zero-state end)
-// before the scan, which then carries it to every lane with the chunks' own contributions.
-// Returns the inclusive scan in *incl (the unit's aggregate in the last lane when ZERO_ENTRY).
-template <bool ZERO_ENTRY = false>
-__device__ __forceinline__ float2 chunkStateUp(float2 end, float2 entry, const float *tb, int lane, float2 *incl)
+// Initial states (w1, w2) of this lane's chunks, packed, from the zero-state end states.  Forward
+// time: the lane's end state is M e_A + e_B; the first lane's takes the unit's entry before
+// the scan over the lanes (maps of 32 samples: powers of M^2 = P[1]), which then carries it on.
+__device__ __forceinline__ void chunkStateUp(P2 e1, P2 e2, float2 entry, const float *tb, int lane, P2 &w1, P2 &w2)
 {
-   float2 val = end;
-   if (!ZERO_ENTRY && lane == 0) val = scan::affine(tabP(tb, 0), entry, val);
+   const float2 x = up(e1), y = up(e2);
+   const float2 eA = make_float2(x.x, y.x), eB = make_float2(x.y, y.y);
+   const M2f M = tabP(tb, 0);
+   float2 val = scan::affine(M, eA, eB);
+   if (lane == 0) val = scan::affine(tabP(tb, 1), entry, val);
 #pragma unroll
    for (int k = 0; k < 5; k++) {
       const float2 o = scan::shflUp(val, 1 << k, 32);
-      if (lane >= (1 << k)) val = scan::affine(tabP(tb, k), o, val);
+      if (lane >= (1 << k)) val = scan::affine(tabP(tb, k + 1), o, val);
    }
-   float2 ex = scan::shflUp(val, 1, 32);
-   if (lane == 0) ex = ZERO_ENTRY ? make_float2(0.0f, 0.0f) : entry;
-   *incl = val;
-   return ex;
+   float2 a = scan::shflUp(val, 1, 32);
+   if (lane == 0) a = entry;
+   const float2 b = scan::affine(M, a, eA);
+   w1 = pk(a.x, b.x);
+   w2 = pk(a.y, b.y);
 }
 
-// Reverse time: M^(31 - lane) entry + the scan of the lanes after (lane 31 holds the chunk
-// processed first).
-template <bool ZERO_ENTRY = false>
-__device__ __forceinline__ float2 chunkStateDown(float2 end, float2 entry, const float *tb, int lane, float2 *incl)
+// Reverse time: chunk B comes before A, lane 31 first.
+__device__ __forceinline__ void chunkStateDown(P2 e1, P2 e2, float2 entry, const float *tb, int lane, P2 &v1, P2 &v2)
 {
-   float2 val = end;
-   if (!ZERO_ENTRY && lane == 31) val = scan::affine(tabP(tb, 0), entry, val);
+   const float2 x = up(e1), y = up(e2);
+   const float2 eA = make_float2(x.x, y.x), eB = make_float2(x.y, y.y);
+   const M2f M = tabP(tb, 0);
+   float2 val = scan::affine(M, eB, eA);
+   if (lane == 31) val = scan::affine(tabP(tb, 1), entry, val);
 #pragma unroll
    for (int k = 0; k < 5; k++) {
       const float2 o = shflDown(val, 1 << k);
-      if (lane + (1 << k) < 32) val = scan::affine(tabP(tb, k), o, val);
+      if (lane + (1 << k) < 32) val = scan::affine(tabP(tb, k + 1), o, val);
    }
-   float2 ex = shflDown(val, 1);
-   if (lane == 31) ex = ZERO_ENTRY ? make_float2(0.0f, 0.0f) : entry;
-   *incl = val;
-   return ex;
+   float2 b = shflDown(val, 1);
+   if (lane == 31) b = entry;
+   const float2 a = scan::affine(M, b, eB);
+   v1 = pk(a.x, b.x);
+   v2 = pk(a.y, b.y);
 }
 
-// True internal sequence (in place of the zero-state one) and stage output, from the
-// chunk's initial state (w1, w2) = (w[-1], w[-2]).
-__device__ __forceinline__ void correctAndOutput(float (&w)[kL], float (&out)[kL], const float *tb, float w1, float w2)
+// One stage of the forward cascade over a unit, in place; keep(i, w) takes its internal sequence.
+template <typename Keep>
+__device__ __forceinline__ void forwardStage(P2 (&v)[kL], float2 entry, const float *tb, int lane, Keep keep)
 {
-   const float b0 = tb[0], b1 = tb[1], b2 = tb[2];
-   float q1 = w1, q2 = w2;
+   const StageCoef c = stageCoef(tb);
+   P2 q1, q2;
+   zeroStateEnd(v, c, q1, q2);
+   chunkStateUp(q1, q2, entry, tb, lane, q1, q2);
 #pragma unroll
    for (int i = 0; i < kL; i++) {
-      const float2 ab = *(const float2 *) (tb + kTabAB + 2 * i);
-      const float wt = fmaf(ab.x, w1, fmaf(ab.y, w2, w[i]));
-      out[i] = fmaf(b0, wt, fmaf(b1, q1, b2 * q2));
-      w[i] = wt;
+      const P2 w = fma2(c.na1, q1, fma2(c.na2, q2, v[i]));
+      v[i] = fma2(c.b0, w, fma2(c.b1, q1, mul2(c.b2, q2)));
+      keep(i, w);
       q2 = q1;
-      q1 = wt;
-   }
-}
-
-// Reverse time, from (v[16], v[17]): lambda[i] = b0 v[i] + b1 v[i+1] + b2 v[i+2].
-__device__ __forceinline__ void correctAndOutputRev(float (&v)[kL], float (&lam)[kL], const float *tb, float v16,
-                                                    float v17)
-{
-   const float b0 = tb[0], b1 = tb[1], b2 = tb[2];
-   float n1 = v16, n2 = v17;
-#pragma unroll
-   for (int i = kL - 1; i >= 0; i--) {
-      const float2 ab = *(const float2 *) (tb + kTabAB + 2 * (kL - 1 - i));
-      const float vt = fmaf(ab.x, v16, fmaf(ab.y, v17, v[i]));
-      lam[i] = fmaf(b0, vt, fmaf(b1, n1, b2 * n2));
-      v[i] = vt;
-      n2 = n1;
-      n1 = vt;
+      q1 = w;
    }
 }
 
@@ -555,11 +615,12 @@ struct UnitArgs {
    int nUnits;
    int Smax;
    const float *tables;
+   const float *impulse; // impulse responses of the aggregates
    const float *in;   // forward: FIR output plane; adjoint aggregates: output gradient (packed)
-   float *out;        // OUT: y (packed, tail zeros)
-   float2 *agg;       // AGG: unit aggregates, 2 floats per stage (processing order)
+   float *out;        // y (packed, tail zeros)
+   float2 *agg;       // unit aggregates, 2 floats per stage (processing order)
    const float2 *ckpt;
-   // OUT_MSE: loss gradient gy = scale (y - target) on the valid samples, the unit's
+   // with the loss: gradient gy = scale (y - target) on the valid samples, the unit's
    // sum of (y - target)^2 in lossPart[unit], and the adjoint's unit aggregates in aggA
    const float *target;
    float *gy;
@@ -569,7 +630,7 @@ struct UnitArgs {
 };
 
 // Copy the channel's stage tables into the warp's slice of shared memory, four loads
-// per lane in flight before their stores (up to 6 stages in one round).
+// per lane in flight before their stores.
 __device__ __forceinline__ void loadTables(float *dst, const float *tables, const RaggedChan &c, int lane)
 {
    const float4 *src = (const float4 *) (tables + (c.cOff / 5) * kBankTabFloats);
@@ -586,31 +647,140 @@ __device__ __forceinline__ void loadTables(float *dst, const float *tables, cons
    __syncwarp();
 }
 
-// Forward passes: AGG = from a zero state, write the unit aggregate of every stage;
-// OUT = from the checkpoints, write y.  ADJ_AGG: adjoint aggregates over the output
-// gradient (reverse time, stages in reverse order).
-enum UnitMode { UNIT_AGG = 0, UNIT_OUT = 1, UNIT_ADJ_AGG = 2, UNIT_OUT_MSE = 3 };
-
-// The adjoint's zero-entry pass over a unit (reverse time, stages in reverse order):
-// g holds the output gradient on entry, the unit aggregate of every stage goes to agg.
-__device__ __forceinline__ void adjointAggregates(float (&g)[kL], const float *sTab, int S, float2 *agg, int lane)
+// ---- unit aggregates by impulse responses
+//
+// Tables of a channel of two units or more, per direction and processing position p, 1024
+// floats in the order the dot products read them: 16-byte group 32 j + l holds lane l's pairs
+// 2 j and 2 j + 1 of the sequence r, r[t] = k_p[1023 - t] forward, k_p[t] adjoint.
+__device__ __forceinline__ const float *impulseOf(const float *impulse, const RaggedChan &c, bool adj, int p)
 {
-   for (int p = 0; p < S; p++) {
-      const float *tb = sTab + (S - 1 - p) * kBankTabFloats;
-      float w[kL];
-      float2 incl;
-      const float2 st =
-          chunkStateDown<true>(zeroStatePassRev(g, w, tb[3], tb[4]), make_float2(0.0f, 0.0f), tb, lane, &incl);
-      correctAndOutputRev(w, g, tb, st.x, st.y);
-      if (lane == 0) agg[p] = incl;
+   return impulse + c.impOff + (long long) ((adj ? c.S : 0) + p) * kUnit;
+}
+
+// One warp per channel and direction: the cascade's response to a unit impulse at the unit's
+// start, every stage's internal sequence written out.
+__global__ void __launch_bounds__(64) bank_impulse_kernel(const RaggedChan *chans, const int *list, int Smax,
+                                                          const float *tables, float *impulse)
+{
+   extern __shared__ float4 dynI[];
+   const int lane = threadIdx.x & 31, adj = threadIdx.x >> 5;
+   const RaggedChan c = chans[list[blockIdx.x]];
+   float *sTab = (float *) dynI + (size_t) adj * Smax * kBankTabFloats;
+   loadTables(sTab, tables, c, lane);
+   P2 v[kL], w[kL];
+#pragma unroll
+   for (int i = 0; i < kL; i++) v[i] = dup(0.0f);
+   if (lane == 0) v[0] = pk(1.0f, 0.0f);
+   for (int p = 0; p < c.S; p++) {
+      forwardStage(v, make_float2(0.0f, 0.0f), sTab + stageAt(p, c.S, adj) * kBankTabFloats, lane,
+                   [&](int i, P2 q) { w[i] = q; });
+      float4 *dst = (float4 *) (impulse + c.impOff + (long long) ((adj ? c.S : 0) + p) * kUnit);
+#pragma unroll
+      for (int j = 0; j < kL / 2; j++) {
+         if (adj) {
+            const float2 a = up(w[2 * j]), b = up(w[2 * j + 1]);
+            dst[32 * j + lane] = make_float4(a.x, a.y, b.x, b.y);
+         }
+         else { // reversed: lane 31 - l, chunks exchanged
+            const float2 a = up(w[kL - 1 - 2 * j]), b = up(w[kL - 2 - 2 * j]);
+            dst[32 * j + 31 - lane] = make_float4(a.y, a.x, b.y, b.x);
+         }
+      }
    }
 }
 
-template <int MODE>
+// Aggregates of one or two (N) units of a channel whose samples the warp holds: two dot
+// products a stage and unit.  Bound by the tables' reads through L1, 36 cycles a stage, which
+// two units share.
+template <bool ADJ, int N>
+__device__ __forceinline__ void unitAggregates(const P2 (&v)[N][kL], const float *impulse, const RaggedChan &c,
+                                               float2 *agg0, float2 *agg1, int lane)
+{
+   for (int p = 0; p < c.S; p++) {
+      const ulonglong2 *src = (const ulonglong2 *) impulseOf(impulse, c, ADJ, p) + lane;
+      P2 k[kL];
+#pragma unroll
+      for (int j = 0; j < kL / 2; j++) {
+         const ulonglong2 q = src[32 * j];
+         k[2 * j] = P2{q.x};
+         k[2 * j + 1] = P2{q.y};
+      }
+      // second component: r[t - 1] (adjoint) or r[t + 1]; the pair that reaches into the next lane's
+      P2 edge;
+      if (ADJ) {
+         const float2 e = up(k[kL - 1]);
+         const float before = __shfl_up_sync(0xffffffffu, e.y, 1);
+         edge = pk(lane == 0 ? 0.0f : before, e.x);
+      }
+      else {
+         const float2 e = up(k[0]);
+         const float after = __shfl_down_sync(0xffffffffu, e.x, 1);
+         edge = pk(e.y, lane == 31 ? 0.0f : after);
+      }
+#pragma unroll
+      for (int n = 0; n < N; n++) {
+         P2 x = mul2(k[0], v[n][0]), y = mul2(edge, v[n][ADJ ? 0 : kL - 1]);
+#pragma unroll
+         for (int i = 1; i < kL; i++) {
+            x = fma2(k[i], v[n][i], x);
+            y = ADJ ? fma2(k[i - 1], v[n][i], y) : fma2(k[i], v[n][i - 1], y);
+         }
+         const float2 xs = up(x), ys = up(y);
+         const float sx = xs.x + xs.y, sy = ys.x + ys.y;
+         // both sums over the warp: the upper half keeps the second component
+         const bool hi = lane & 16;
+         float r = (hi ? sy : sx) + __shfl_xor_sync(0xffffffffu, hi ? sx : sy, 16);
+#pragma unroll
+         for (int o = 8; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+         if ((lane & 15) == 0) ((float *) ((n ? agg1 : agg0) + p))[lane >> 4] = r;
+      }
+   }
+}
+
+// Pass 1.  ADJ = false: every unit of the FIR output plane but its channel's last (whose end
+// no unit starts from); ADJ = true: every unit of the packed output gradient but the first.
+// A warp takes two consecutive units of the list, mostly of one channel.
+template <bool ADJ> __global__ void __launch_bounds__(kThreads) bank_agg_kernel(UnitArgs a)
+{
+   __shared__ __align__(16) float sStage[kWarps][kStage];
+   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+   const int ui = 2 * (blockIdx.x * kWarps + warp);
+   if (ui >= a.nUnits) return;
+   const int2 U0 = a.units[ui], U1 = ui + 1 < a.nUnits ? a.units[ui + 1] : make_int2(-1, 0);
+   const RaggedChan c0 = a.chans[U0.x], c1 = a.chans[U1.x < 0 ? U0.x : U1.x];
+   const bool need0 = ADJ ? U0.y > 0 : (U0.y + 1) * kUnit < c0.Lu;
+   const bool need1 = U1.x >= 0 && (ADJ ? U1.y > 0 : (U1.y + 1) * kUnit < c1.Lu);
+   if (!need0 && !need1) return;
+   P2 v[2][kL];
+   if (ADJ) {
+      float r[kLane];
+      fetchUnit(r, a.in + c0.xOff, U0.y * kUnit, need0 ? c0.Lu : 0, lane);
+      stageUnit(v[0], r, sStage[warp], lane);
+      fetchUnit(r, a.in + c1.xOff, U1.y * kUnit, need1 ? c1.Lu : 0, lane);
+      stageUnit(v[1], r, sStage[warp], lane);
+   }
+   else {
+      float4 r0[kL / 2], r1[kL / 2];
+      fetchPlane(r0, a.in + c0.pOff, U0.y * kUnit, need0 ? c0.Lu : 0, lane);
+      fetchPlane(r1, a.in + c1.pOff, U1.y * kUnit, need1 ? c1.Lu : 0, lane);
+      stagePlane(v[0], r0, sStage[warp], lane);
+      stagePlane(v[1], r1, sStage[warp], lane);
+   }
+   float2 *agg0 = a.agg + c0.ckOff + (long long) U0.y * c0.S, *agg1 = a.agg + c1.ckOff + (long long) U1.y * c1.S;
+   if (need0 && need1 && U0.x == U1.x) unitAggregates<ADJ, 2>(v, a.impulse, c0, agg0, agg1, lane);
+   else {
+      if (need0) unitAggregates<ADJ, 1>(*(const P2 (*)[1][kL]) &v[0], a.impulse, c0, agg0, agg0, lane);
+      if (need1) unitAggregates<ADJ, 1>(*(const P2 (*)[1][kL]) &v[1], a.impulse, c1, agg1, agg1, lane);
+   }
+}
+
+// Pass 3: y from the checkpoints; with MSE also the loss gradient, the unit's sum of squares
+// and the adjoint's aggregates.
+template <bool MSE>
 __global__ void __launch_bounds__(kThreads) bank_unit_kernel(UnitArgs a)
 {
    extern __shared__ float4 dynU[];
-   __shared__ float sStage[kWarps][32 * kOutPad];
+   __shared__ __align__(16) float sStage[kWarps][kStage];
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
    const int ui = blockIdx.x * kWarps + warp;
    if (ui >= a.nUnits) return;
@@ -619,55 +789,48 @@ __global__ void __launch_bounds__(kThreads) bank_unit_kernel(UnitArgs a)
    const RaggedChan c = a.chans[U.x];
    const int S = c.S, Lu = c.Lu, t0 = U.y * kUnit;
    const long long base = c.ckOff + (long long) U.y * S;
-   constexpr bool OUT = MODE == UNIT_OUT || MODE == UNIT_OUT_MSE;
    // the unit's entry states and input are requested before the tables' copy waits on its own loads
-   UnitStates ent = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
-   if (OUT) ent = loadStates(a.ckpt + base, S, lane);
-   float v[kL], tg[kL];
-   if (MODE == UNIT_ADJ_AGG) {
-      fetchPacked(tg, a.in + c.xOff, t0, Lu, lane);
+   const UnitStates ent = loadStates(a.ckpt + base, S, lane);
+   P2 v[kL];
+   {
+      float4 r[kL / 2];
+      fetchPlane(r, a.in + c.pOff, t0, Lu, lane);
       loadTables(sTab, a.tables, c, lane);
-      stagePacked(v, tg, sStage[warp], lane);
-      adjointAggregates(v, sTab, S, a.agg + base, lane);
-      return;
+      stagePlane(v, r, sStage[warp], lane);
    }
-   loadChunk(v, a.in + c.pOff, t0 + lane * kL, Lu);
-   loadTables(sTab, a.tables, c, lane);
-   for (int p = 0; p < S; p++) {
-      const float *tb = sTab + p * kBankTabFloats;
-      float w[kL];
-      const float2 entry = OUT ? entryAt(ent, p) : make_float2(0.0f, 0.0f);
-      float2 incl;
-      const float2 st = OUT ? chunkStateUp(zeroStatePass(v, w, tb[3], tb[4]), entry, tb, lane, &incl)
-                            : chunkStateUp<true>(zeroStatePass(v, w, tb[3], tb[4]), entry, tb, lane, &incl);
-      correctAndOutput(w, v, tb, st.x, st.y);
-      if (MODE == UNIT_AGG && lane == 31) a.agg[base + p] = incl;
-   }
-   if (OUT) {
-      storePacked(v, a.out + c.xOff, t0, Lu, sStage[warp], lane);
-      if (t0 + kUnit >= Lu)
-         for (int t = Lu + lane; t < c.L; t += 32) a.out[c.xOff + t] = 0.0f;
-   }
-   if (MODE == UNIT_OUT_MSE) {
-      // the target is read here, not with the unit's other loads: held across the stages
-      // it costs 16 registers a thread and the occupancy they buy (measured 1 % slower)
-      fetchPacked(tg, a.target + c.xOff, t0, Lu, lane);
-      stagePacked(tg, tg, sStage[warp], lane);
+   for (int p = 0; p < S; p++) forwardStage(v, entryAt(ent, p), sTab + p * kBankTabFloats, lane, [](int, P2) {});
+   storeUnit(v, a.out + c.xOff, t0, Lu, sStage[warp], lane);
+   if (t0 + kUnit >= Lu)
+      for (int t = Lu + lane; t < c.L; t += 32) a.out[c.xOff + t] = 0.0f;
+   if (MSE) {
+      // the target is read here, not with the unit's other loads: held across the stages it
+      // costs 32 registers a thread and the occupancy they buy, and copied to a second staging
+      // area meanwhile (cp.async) the step took 1820 us instead of 1804
+      P2 tg[kL];
+      {
+         float r[kLane];
+         fetchUnit(r, a.target + c.xOff, t0, Lu, lane);
+         stageUnit(tg, r, sStage[warp], lane);
+      }
       double sq = 0.0;
 #pragma unroll
       for (int i = 0; i < kL; i++) {
-         const bool valid = t0 + lane * kL + i < Lu;
-         const float d = v[i] - tg[i];
-         v[i] = valid ? a.scale * d : 0.0f;
-         if (valid) sq += (double) d * d;
+         const float2 y = up(v[i]), t = up(tg[i]);
+         const int ta = t0 + lane * kLane + i;
+         const float da = y.x - t.x, db = y.y - t.y;
+         const bool va = ta < Lu, vb = ta + kL < Lu;
+         v[i] = pk(va ? a.scale * da : 0.0f, vb ? a.scale * db : 0.0f);
+         if (va) sq += (double) da * da;
+         if (vb) sq += (double) db * db;
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
       if (lane == 0) a.lossPart[ui] = sq;
-      storePacked(v, a.gy + c.xOff, t0, Lu, sStage[warp], lane);
+      storeUnit(v, a.gy + c.xOff, t0, Lu, sStage[warp], lane);
       if (t0 + kUnit >= Lu)
          for (int t = Lu + lane; t < c.L; t += 32) a.gy[c.xOff + t] = 0.0f;
-      adjointAggregates(v, sTab, S, a.aggA + base, lane);
+      if (U.y > 0)
+         unitAggregates<true, 1>(*(const P2 (*)[1][kL]) &v, a.impulse, c, a.aggA + base, a.aggA + base, lane);
    }
 }
 
@@ -686,9 +849,15 @@ struct AdjArgs {
    int first;            // this launch's first unit (a bucket of one stage count)
 };
 
-// Stage sequences of one unit in shared memory: per stage (the last excepted, which
-// stays in registers) 16 rows of 32 lanes, so that the lanes of the warp touch
-// distinct banks.  One warp per CTA: the sequences are the bulk of the CTA's
+// Stages whose sequences a unit keeps in shared memory at once; deeper cascades are taken in
+// groups of stages, last group first, the forward run again up to each: a unit of eight
+// stages runs twelve forward stages instead of eight but takes 17 KB instead of 34, and the
+// SM holds twelve warps instead of six (2048-channel bank step 1856 -> 1804 us; groups of
+// three 1803, five 1817, six 1844).
+constexpr int kAdjStages = 4;
+
+// Stage sequences of one unit in shared memory: per stage of a group 16 rows of 32 pairs, so that
+// the lanes of the warp touch distinct banks.  One warp per CTA: the sequences are the bulk of the CTA's
 // shared memory, and single-warp CTAs pack the SM most tightly.
 __global__ void __launch_bounds__(32) bank_adjoint_kernel(AdjArgs a)
 {
@@ -697,89 +866,105 @@ __global__ void __launch_bounds__(32) bank_adjoint_kernel(AdjArgs a)
    float *sTab = (float *) dynA;
    const int2 U = a.units[a.first + blockIdx.x];
    const RaggedChan c = a.chans[U.x];
-   float *W = sTab + (size_t) c.S * kBankTabFloats; // the launch sized shared memory for c.S stages
-   // The staging rows of the packed gradient loads and stores share the stage sequences'
-   // space: the output gradient is read before the sequences are written, the input
-   // gradient stored after the last of them was read (at least 32 x 17 floats: adjointShared).
-   float *sStage = W;
+   unsigned long long *W = (unsigned long long *) (sTab + (size_t) c.S * kBankTabFloats); // sized for c.S stages
+   // The staging rows of the loads and stores share the stage sequences' space: the inputs are
+   // read before the sequences are written, the input gradient stored after the last of them
+   // was read (at least 32 x 34 floats: adjointShared).
+   float *sStage = (float *) W;
    const int S = c.S, Lu = c.Lu, t0 = U.y * kUnit;
    const long long base = c.ckOff + (long long) U.y * S;
    const UnitStates entF = loadStates(a.ckptF + base, S, lane), entA = loadStates(a.ckptA + base, S, lane);
-   float v[kL], w[kL], g[kL];
-   loadChunk(v, a.u + c.pOff, t0 + lane * kL, Lu);
-   fetchPacked(w, a.gy + c.xOff, t0, Lu, lane);
-   loadTables(sTab, a.tables, c, lane);
-   stagePacked(g, w, sStage, lane);
-   // 1. the forward of this unit from its checkpoints; every stage's sequence kept
-   for (int s = 0; s < S; s++) {
-      const float *tb = sTab + s * kBankTabFloats;
-      float2 incl;
-      const float2 st = chunkStateUp(zeroStatePass(v, w, tb[3], tb[4]), entryAt(entF, s), tb, lane, &incl);
-      correctAndOutput(w, v, tb, st.x, st.y);
-      if (s + 1 < S) {
-         float *Ws = W + s * kL * 32 + lane;
-#pragma unroll
-         for (int i = 0; i < kL; i++) Ws[i * 32] = w[i];
-      }
+   P2 v[kL], g[kL];
+   {
+      float4 r[kL / 2];
+      float q[kLane];
+      fetchPlane(r, a.u + c.pOff, t0, Lu, lane);
+      fetchUnit(q, a.gy + c.xOff, t0, Lu, lane);
+      loadTables(sTab, a.tables, c, lane);
+      stageUnit(g, q, sStage, lane);
+      stagePlane(v, r, sStage, lane);
    }
-   // 2. the stages' adjoints, last stage first, in reverse time
-   for (int p = 0; p < S; p++) {
-      const int s = S - 1 - p;
-      const float *tb = sTab + s * kBankTabFloats;
-      float vz[kL], lam[kL];
-      float2 incl;
-      const float2 st = chunkStateDown(zeroStatePassRev(g, vz, tb[3], tb[4]), entryAt(entA, p), tb, lane, &incl);
-      correctAndOutputRev(vz, lam, tb, st.x, st.y);
-      // forward sequence of this stage: wr[i + 2] = w[i]; w[-1], w[-2] are the previous
-      // lane's last two samples (lane 0: the unit's checkpoint state)
-      float wr[kL + 2];
-      if (p > 0) {
-         const float *Ws = W + s * kL * 32 + lane;
-#pragma unroll
-         for (int i = 0; i < kL; i++) wr[i + 2] = Ws[i * 32];
+   for (int s1 = S; s1 > 0;) {
+      const int s0 = max(0, s1 - kAdjStages);
+      if (s1 < S) { // a further group: the unit's input again
+         float4 r[kL / 2];
+         __syncwarp();
+         fetchPlane(r, a.u + c.pOff, t0, Lu, lane);
+         stagePlane(v, r, sStage, lane);
       }
-      else {
-#pragma unroll
-         for (int i = 0; i < kL; i++) wr[i + 2] = w[i];
-      }
-      wr[1] = __shfl_up_sync(0xffffffffu, wr[kL + 1], 1);
-      wr[0] = __shfl_up_sync(0xffffffffu, wr[kL], 1);
-      {
-         const float2 e = entryAt(entF, s);
-         if (lane == 0) {
-            wr[1] = e.x;
-            wr[0] = e.y;
+      // 1. the forward of this unit from its checkpoints; the group's sequences kept
+      for (int s = 0; s < s1; s++) {
+         const float *tb = sTab + s * kBankTabFloats;
+         if (s >= s0) {
+            unsigned long long *Ws = W + (s - s0) * kL * 32 + lane;
+            forwardStage(v, entryAt(entF, s), tb, lane, [&](int i, P2 q) { Ws[i * 32] = q.v; });
          }
+         else forwardStage(v, entryAt(entF, s), tb, lane, [](int, P2) {});
       }
-      float pr[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+      // 2. the stages' adjoints, last stage first, in reverse time
+      for (int s = s1 - 1; s >= s0; s--) {
+         const float *tb = sTab + s * kBankTabFloats;
+         const StageCoef cf = stageCoef(tb);
+         const unsigned long long *Ws = W + (s - s0) * kL * 32 + lane;
+         P2 n1, n2;
+         zeroStateEndRev(g, cf, n1, n2);
+         chunkStateDown(n1, n2, entryAt(entA, S - 1 - s), tb, lane, n1, n2);
+         // forward sequence of this stage: before chunk A the previous lane's chunk B (lane 0:
+         // the unit's checkpoint state), before chunk B chunk A
+         P2 w0 = P2{Ws[(kL - 1) * 32]}, w1 = P2{Ws[(kL - 2) * 32]}, m1, m2; // w[i], w[i-1]; w[-1], w[-2]
+         {
+            const float2 l1 = up(w0), l2 = up(w1), e = entryAt(entF, s);
+            const float p1 = __shfl_up_sync(0xffffffffu, l1.y, 1), p2 = __shfl_up_sync(0xffffffffu, l2.y, 1);
+            m1 = pk(lane == 0 ? e.x : p1, l1.x);
+            m2 = pk(lane == 0 ? e.y : p2, l2.x);
+         }
+         P2 pp[5];
 #pragma unroll
-      for (int i = 0; i < kL; i++) {
-         pr[0] = fmaf(g[i], wr[i + 2], pr[0]);
-         pr[1] = fmaf(g[i], wr[i + 1], pr[1]);
-         pr[2] = fmaf(g[i], wr[i], pr[2]);
-         pr[3] = fmaf(-lam[i], wr[i + 1], pr[3]);
-         pr[4] = fmaf(-lam[i], wr[i], pr[4]);
-         g[i] = lam[i];
+         for (int k = 0; k < 5; k++) pp[k] = dup(0.0f);
+#pragma unroll
+         for (int i = kL - 1; i >= 0; i--) {
+            const P2 w2 = i >= 2 ? P2{Ws[(i - 2) * 32]} : (i == 1 ? m1 : m2);
+            const P2 vt = fma2(cf.na1, n1, fma2(cf.na2, n2, g[i]));
+            const P2 lam = fma2(cf.b0, vt, fma2(cf.b1, n1, mul2(cf.b2, n2)));
+            pp[0] = fma2(g[i], w0, pp[0]);
+            pp[1] = fma2(g[i], w1, pp[1]);
+            pp[2] = fma2(g[i], w2, pp[2]);
+            pp[3] = fma2(lam, w1, pp[3]);
+            pp[4] = fma2(lam, w2, pp[4]);
+            g[i] = lam;
+            n2 = n1;
+            n1 = vt;
+            w0 = w1;
+            w1 = w2;
+         }
+         float pr[5];
+#pragma unroll
+         for (int k = 0; k < 5; k++) {
+            const float2 h = up(pp[k]);
+            pr[k] = k < 3 ? h.x + h.y : -(h.x + h.y);
+         }
+         // the five sums over the warp by halving: at each step a lane keeps half of its
+         // values and adds the partner's copy of them; lane 4 k ends with sum k (9 shuffles)
+         const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+         float q[4], q2[2];
+#pragma unroll
+         for (int j = 0; j < 4; j++) {
+            const float lo = pr[j], hi = j == 0 ? pr[4] : 0.0f;
+            q[j] = (b4 ? hi : lo) + __shfl_xor_sync(0xffffffffu, b4 ? lo : hi, 16);
+         }
+#pragma unroll
+         for (int j = 0; j < 2; j++)
+            q2[j] = (b3 ? q[j + 2] : q[j]) + __shfl_xor_sync(0xffffffffu, b3 ? q[j] : q[j + 2], 8);
+         float r = (b2 ? q2[1] : q2[0]) + __shfl_xor_sync(0xffffffffu, b2 ? q2[0] : q2[1], 4);
+         r += __shfl_xor_sync(0xffffffffu, r, 2);
+         r += __shfl_xor_sync(0xffffffffu, r, 1);
+         const int k = lane >> 2;
+         if ((lane & 3) == 0 && k < 5) a.part[(base + s) * 5 + k] = r;
       }
-      // the five sums over the warp by halving: at each step a lane keeps half of its
-      // values and adds the partner's copy of them; lane 4 k ends with sum k (9 shuffles)
-      const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
-      float q[4], q2[2];
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-         const float lo = pr[j], hi = j == 0 ? pr[4] : 0.0f;
-         q[j] = (b4 ? hi : lo) + __shfl_xor_sync(0xffffffffu, b4 ? lo : hi, 16);
-      }
-#pragma unroll
-      for (int j = 0; j < 2; j++) q2[j] = (b3 ? q[j + 2] : q[j]) + __shfl_xor_sync(0xffffffffu, b3 ? q[j] : q[j + 2], 8);
-      float r = (b2 ? q2[1] : q2[0]) + __shfl_xor_sync(0xffffffffu, b2 ? q2[0] : q2[1], 4);
-      r += __shfl_xor_sync(0xffffffffu, r, 2);
-      r += __shfl_xor_sync(0xffffffffu, r, 1);
-      const int k = lane >> 2;
-      if ((lane & 3) == 0 && k < 5) a.part[(base + s) * 5 + k] = r;
+      s1 = s0;
    }
    __syncwarp(); // every lane's last read of the stage sequences precedes the staging writes
-   storePacked(g, a.g + c.gOff, t0, Lu, sStage, lane);
+   storeUnit(g, a.g + c.gOff, t0, Lu, sStage, lane);
 }
 
 // Coefficient gradients of one channel (one CTA, coefficients spread over its warps): per
@@ -814,34 +999,52 @@ __global__ void __launch_bounds__(32 * kCoefWarps) bank_coef_kernel(const Ragged
 
 long long bankTransitionDoubles(int S) { return 8LL * S * (S + 1); } // Phi and Phi^32, both directions
 
-cudaError_t launchBankTables(const RaggedChan *chans, int C, const float *coefs, int totalStages, int Smax,
-                             float *tables, double *phi, cudaStream_t s)
+cudaError_t launchBankTables(const BankLaunch &b, const float *coefs, int totalStages, float *tables, double *phi,
+                             float *impulse, cudaStream_t s)
 {
    if (totalStages <= 0) return cudaSuccess;
    bank_tables_kernel<<<(totalStages + 127) / 128, 128, 0, s>>>(coefs, totalStages, tables);
-   const size_t dyn = (size_t) 8 * Smax * (Smax + 1) / 2 * sizeof(double);
+   const size_t dyn = (size_t) 8 * b.Smax * (b.Smax + 1) / 2 * sizeof(double);
    cudaError_t e = cudaFuncSetAttribute(bank_transition_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dyn);
    if (e != cudaSuccess) return e;
    // one warp per (channel, direction) while the block count is small (up to 36 blocks of
    // 2 x 2 for 8 stages): the squarings' barriers then cost a warp, not four
-   bank_transition_kernel<<<dim3(C, 2), Smax <= 8 ? 32 : 128, dyn, s>>>(chans, coefs, phi);
+   bank_transition_kernel<<<dim3(b.C, 2), b.Smax <= 8 ? 32 : 128, dyn, s>>>(b.chans, coefs, phi);
    countLaunch(2);
+   if (b.nImpulse > 0) {
+      const size_t dynI = (size_t) 2 * b.Smax * kBankTabFloats * sizeof(float);
+      if ((e = cudaFuncSetAttribute(bank_impulse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dynI)) !=
+          cudaSuccess)
+         return e;
+      bank_impulse_kernel<<<b.nImpulse, 64, dynI, s>>>(b.chans, b.impulseList, b.Smax, tables, impulse);
+      countLaunch();
+   }
    return cudaGetLastError();
 }
 
 static size_t unitShared(int Smax) { return (size_t) kWarps * Smax * kBankTabFloats * sizeof(float); }
 static size_t adjointShared(int Smax)
 {
-   const size_t seq = (size_t) (Smax > 0 ? Smax - 1 : 0) * kL * 32, stage = (size_t) 32 * kOutPad;
+   const int kept = Smax < kAdjStages ? Smax : kAdjStages;
+   const size_t seq = (size_t) kept * kL * 32 * 2, stage = kStage;
    return ((size_t) Smax * kBankTabFloats + (seq > stage ? seq : stage)) * sizeof(float);
 }
 
-template <int MODE> static cudaError_t launchUnits(const UnitArgs &a, cudaStream_t s)
+template <bool MSE> static cudaError_t launchUnits(const UnitArgs &a, cudaStream_t s)
 {
    const size_t dyn = unitShared(a.Smax);
-   cudaError_t e = cudaFuncSetAttribute(bank_unit_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dyn);
+   cudaError_t e = cudaFuncSetAttribute(bank_unit_kernel<MSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dyn);
    if (e != cudaSuccess) return e;
-   bank_unit_kernel<MODE><<<(a.nUnits + kWarps - 1) / kWarps, kThreads, dyn, s>>>(a);
+   bank_unit_kernel<MSE><<<(a.nUnits + kWarps - 1) / kWarps, kThreads, dyn, s>>>(a);
+   countLaunch();
+   return cudaGetLastError();
+}
+
+// Aggregates of every unit that another starts from; none where every channel is one unit.
+template <bool ADJ> static cudaError_t launchAggregates(const BankLaunch &b, const UnitArgs &a, cudaStream_t s)
+{
+   if (b.nImpulse <= 0) return cudaSuccess;
+   bank_agg_kernel<ADJ><<<(a.nUnits + 2 * kWarps - 1) / (2 * kWarps), kThreads, 0, s>>>(a);
    countLaunch();
    return cudaGetLastError();
 }
@@ -849,8 +1052,8 @@ template <int MODE> static cudaError_t launchUnits(const UnitArgs &a, cudaStream
 cudaError_t launchBankForward(const BankLaunch &b, cudaStream_t s)
 {
    if (b.nUnits <= 0) return cudaSuccess;
-   UnitArgs a{b.chans, b.units, b.nUnits, b.Smax, b.tables, b.u, nullptr, b.aggF, nullptr};
-   cudaError_t e = launchUnits<UNIT_AGG>(a, s);
+   UnitArgs a{b.chans, b.units, b.nUnits, b.Smax, b.tables, b.impulse, b.u, nullptr, b.aggF, nullptr};
+   cudaError_t e = launchAggregates<false>(b, a, s);
    if (e != cudaSuccess) return e;
    const size_t dynC = (size_t) (4 * b.Smax * (b.Smax + 1) / 2 + 2 * b.Smax) * sizeof(double);
    if ((e = cudaFuncSetAttribute(bank_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dynC)) !=
@@ -870,9 +1073,9 @@ cudaError_t launchBankForward(const BankLaunch &b, cudaStream_t s)
       a.lossPart = b.lossPart;
       a.aggA = b.aggA;
       a.scale = b.scale;
-      return launchUnits<UNIT_OUT_MSE>(a, s);
+      return launchUnits<true>(a, s);
    }
-   return launchUnits<UNIT_OUT>(a, s);
+   return launchUnits<false>(a, s);
 }
 
 cudaError_t launchBankBackward(const BankLaunch &b, cudaStream_t s)
@@ -880,8 +1083,8 @@ cudaError_t launchBankBackward(const BankLaunch &b, cudaStream_t s)
    if (b.nUnits <= 0) return cudaSuccess;
    cudaError_t e = cudaSuccess;
    if (!b.aggReady) {
-      UnitArgs a{b.chans, b.units, b.nUnits, b.Smax, b.tables, b.gy, nullptr, b.aggA, nullptr};
-      if ((e = launchUnits<UNIT_ADJ_AGG>(a, s)) != cudaSuccess) return e;
+      UnitArgs a{b.chans, b.units, b.nUnits, b.Smax, b.tables, b.impulse, b.gy, nullptr, b.aggA, nullptr};
+      if ((e = launchAggregates<true>(b, a, s)) != cudaSuccess) return e;
    }
    const size_t dynC = (size_t) (4 * b.Smax * (b.Smax + 1) / 2 + 2 * b.Smax) * sizeof(double);
    if ((e = cudaFuncSetAttribute(bank_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dynC)) !=

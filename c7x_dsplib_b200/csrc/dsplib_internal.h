@@ -301,9 +301,10 @@ struct RaggedChan {
    long long xOff, hOff, cOff, pOff;
    int L, T, S, Lu;
    long long gOff;   // its slice of the gradient plane of the scratch (gradient at the FIR output)
-   long long ckOff;  // first unit state (float2) of the channel: one per 512-sample unit and stage
+   long long ckOff;  // first unit state (float2) of the channel: one per 1024-sample unit and stage
    long long phiOff; // first double of the channel's unit transitions
    long long grpOff; // first float of the channel's chain group states (2S per 32 units)
+   long long impOff; // first float of its impulse responses (channels of two units or more)
 };
 // Split-BF16x3 tensor-core FIR over a list of runs {channel, first tile, tiles, 0}
 // of kFirBfTile outputs: forward (valid correlation of the channel's x with its
@@ -324,9 +325,10 @@ cudaError_t launchFirBf16x3Ragged(const RaggedChan *chans, const int4 *runs, int
 // Cascade of the filter bank split along time (bank_scan.cu): units of kBankSpan
 // samples (one warp each), chained per channel through the 2S-dimensional cascade
 // state; per stage a table of kBankTabFloats floats (coefficients, transition
-// powers, free-response rows), per channel the unit transitions of both directions.
-constexpr int kBankSpan = 512;
-constexpr int kBankTabFloats = 80;
+// powers), per channel the unit transitions and, where it has two units
+// or more, the impulse responses of both directions.
+constexpr int kBankSpan = 1024;
+constexpr int kBankTabFloats = 44;
 
 struct BankLaunch {
    const RaggedChan *chans;
@@ -336,6 +338,9 @@ struct BankLaunch {
    int Smax;
    const float *tables;
    const double *phi;
+   const float *impulse;
+   const int *impulseList; // the channels of two units or more
+   int nImpulse;
    const float *u;    // FIR output plane
    float *y;          // forward output
    const float *gy;   // adjoint: output gradient
@@ -365,8 +370,8 @@ struct BankLaunch {
 };
 // Doubles of both unit transitions of a channel of S stages.
 long long bankTransitionDoubles(int S);
-cudaError_t launchBankTables(const RaggedChan *chans, int C, const float *coefs, int totalStages, int Smax,
-                             float *tables, double *phi, cudaStream_t s);
+cudaError_t launchBankTables(const BankLaunch &b, const float *coefs, int totalStages, float *tables, double *phi,
+                             float *impulse, cudaStream_t s);
 cudaError_t launchBankForward(const BankLaunch &b, cudaStream_t s);
 cudaError_t launchBankBackward(const BankLaunch &b, cudaStream_t s);
 

@@ -13,7 +13,7 @@
 //                          8192-output tiles, one run per CTA.
 //   bank_tables_kernel, bank_transition_kernel, bank_unit_kernel, bank_chain_kernel,
 //   bank_adjoint_kernel, bank_coef_kernel (bank_scan.cu)
-//                          the cascade split along time into 512-sample units
+//                          the cascade split along time into 1024-sample units
 //                          (one warp each) chained per channel through the
 //                          cascade's 2S-dimensional state: unit aggregates, the
 //                          chain (one state per unit and stage: the checkpoints),
@@ -65,10 +65,12 @@ struct RaggedPlan {
    int nDhRuns = 0;
    int2 *dUnits = nullptr;      // cascade units (channel, unit index)
    int *dChainOrder = nullptr;  // channels by unit count, most first: the chains' CTA order
+   int *dImpulse = nullptr;     // channels of two units or more (with stages): impulse responses
+   int nImpulse = 0;
    int *err = nullptr;          // error word of the tensor-core kernels (mapped page-locked)
    int device = 0;
    // work buffer layout (float offsets)
-   long long wCk = 0, wAgg = 0, wTab = 0, wPhi = 0, wGrp = 0, wTotal = 0;
+   long long wCk = 0, wAgg = 0, wTab = 0, wPhi = 0, wGrp = 0, wImp = 0, wTotal = 0;
    // scratch layout (float offsets)
    long long sAgg = 0, sCk = 0, sGrp = 0, sPart = 0, sLoss = 0, sDh = 0, sTotal = 0;
    // host-buffer steps: the channel table, and contiguous channel segments (each with a
@@ -213,6 +215,7 @@ static void freePlan(RaggedPlan *p)
    cudaFree(p->dDhRuns);
    cudaFree(p->dUnits);
    cudaFree(p->dChainOrder);
+   cudaFree(p->dImpulse);
    freeErrorWord(p->err);
    for (RaggedPlan::Segment &g : p->segs) freePlan(g.plan);
    for (int i = 0; i < p->nAux; i++) {
@@ -282,7 +285,8 @@ static DSPLIB_STATUS raggedPlanBuild(DSPLIB_gpu_raggedPlan *plan, int32_t numCha
       const int tiles = (outLen + kFirBfTile - 1) / kFirBfTile;
       for (int t = 0; t < tiles; t += runTiles) runs.push_back(make_int4(c, t, std::min(runTiles, tiles - t), 0));
    };
-   long long xo = 0, ho = 0, co = 0, po = 0, ck = 0, ph = 0, gr = 0;
+   long long xo = 0, ho = 0, co = 0, po = 0, ck = 0, ph = 0, gr = 0, im = 0;
+   std::vector<int> impulse;
    for (int c = 0; c < numChannels; c++) {
       const int L = length[c], T = taps[c], S = stages[c];
       if (T < 1 || T > kFirBfMaxTaps || L < T || S < 0 || S > kRaggedMaxStages) {
@@ -291,7 +295,11 @@ static DSPLIB_STATUS raggedPlanBuild(DSPLIB_gpu_raggedPlan *plan, int32_t numCha
       }
       const int Lu = L - T + 1;
       const int nu = (Lu + kBankSpan - 1) / kBankSpan;
-      ch[c] = RaggedChan{xo, ho, co, po, L, T, S, Lu, xo, ck, ph, gr};
+      ch[c] = RaggedChan{xo, ho, co, po, L, T, S, Lu, xo, ck, ph, gr, im};
+      if (nu > 1 && S > 0) {
+         impulse.push_back(c);
+         im += 2LL * S * kBankSpan;
+      }
       gr += 2LL * S * ((nu + 31) / 32);
       po += (Lu + 15) & ~15;
       ck += (long long) nu * S;
@@ -381,13 +389,16 @@ static DSPLIB_STATUS raggedPlanBuild(DSPLIB_gpu_raggedPlan *plan, int32_t numCha
       }
       (void) cudaGetLastError(); // without auxiliary streams the buckets run in sequence
    }
-   // work buffer: u | forward checkpoints | forward aggregates | stage tables | unit transitions
+   // work buffer: u | forward checkpoints | forward aggregates | stage tables | unit transitions |
+   // chain group states | impulse responses
    p->wCk = align4(p->planeStride);
    p->wAgg = p->wCk + align4(2 * p->nCk);
    p->wTab = p->wAgg + align4(2 * p->nCk);
    p->wPhi = p->wTab + (long long) kBankTabFloats * p->totalStages;
    p->wGrp = p->wPhi + align4(2 * p->nPhi);
-   p->wTotal = p->wGrp + align4(p->nGrp);
+   p->wImp = p->wGrp + align4(p->nGrp);
+   p->wTotal = p->wImp + im;
+   p->nImpulse = (int) impulse.size();
    // scratch: g | adjoint aggregates | adjoint checkpoints | coefficient partials | taps partials
    p->sAgg = align4(p->totalLen);
    p->sCk = p->sAgg + align4(2 * p->nCk);
@@ -399,7 +410,8 @@ static DSPLIB_STATUS raggedPlanBuild(DSPLIB_gpu_raggedPlan *plan, int32_t numCha
    const bool ok = upload(&p->dChan, ch) == cudaSuccess && upload(&p->dFwdItems, fwd) == cudaSuccess &&
                    upload(&p->dFirFwdRuns, firFwd) == cudaSuccess && upload(&p->dFirDxRuns, firDx) == cudaSuccess &&
                    upload(&p->dDhStart, start) == cudaSuccess && upload(&p->dDhRuns, dhRuns) == cudaSuccess &&
-                   upload(&p->dUnits, units) == cudaSuccess && upload(&p->dChainOrder, chainOrder) == cudaSuccess;
+                   upload(&p->dUnits, units) == cudaSuccess && upload(&p->dChainOrder, chainOrder) == cudaSuccess &&
+                   upload(&p->dImpulse, impulse) == cudaSuccess;
    if (!ok) {
       freePlan(p);
       return DSPLIB_ERR_FAILURE;
@@ -546,6 +558,9 @@ static BankLaunch bankLaunch(const RaggedPlan *p, const float *work)
    b.Smax = p->Smax;
    b.tables = work + p->wTab;
    b.phi = (const double *) (work + p->wPhi);
+   b.impulse = work + p->wImp;
+   b.impulseList = p->dImpulse;
+   b.nImpulse = p->nImpulse;
    b.u = work;
    b.aggF = (float2 *) (work + p->wAgg);
    b.ckptF = (float2 *) (work + p->wCk);
@@ -573,8 +588,7 @@ DSPLIB_STATUS DSPLIB_gpu_firBiquadBatched_fwd(DSPLIB_gpu_raggedPlan plan, const 
    b.y = y;
    if (launchFirBf16x3Ragged(p->dChan, p->dFirFwdRuns, p->nFirFwdRuns, x, taps, u, false, p->Tmax, p->err, s) != cudaSuccess)
       return DSPLIB_ERR_FAILURE;
-   if (launchBankTables(p->dChan, p->C, coefs, p->totalStages, p->Smax, work + p->wTab, (double *) (work + p->wPhi),
-                        s) != cudaSuccess ||
+   if (launchBankTables(b, coefs, p->totalStages, work + p->wTab, (double *) (work + p->wPhi), work + p->wImp, s) != cudaSuccess ||
        launchBankForward(b, s) != cudaSuccess)
       return DSPLIB_ERR_FAILURE;
    return DSPLIB_SUCCESS;
@@ -635,8 +649,7 @@ static DSPLIB_STATUS stepMseCore(RaggedPlan *p, const float *x, const float *tap
    // forward, loss gradient and the adjoint's first pass in one sweep over the units
    if (launchFirBf16x3Ragged(p->dChan, p->dFirFwdRuns, p->nFirFwdRuns, x, taps, work, false, p->Tmax, p->err, s) !=
            cudaSuccess ||
-       launchBankTables(p->dChan, p->C, coefs, p->totalStages, p->Smax, work + p->wTab, (double *) (work + p->wPhi),
-                        s) != cudaSuccess ||
+       launchBankTables(b, coefs, p->totalStages, work + p->wTab, (double *) (work + p->wPhi), work + p->wImp, s) != cudaSuccess ||
        launchBankForward(b, s) != cudaSuccess)
       return DSPLIB_ERR_FAILURE;
    mse_reduce_kernel<<<1, 1024, 0, s>>>(b.lossPart, p->nUnits, invCount, loss, lossSum);

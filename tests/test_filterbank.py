@@ -199,6 +199,27 @@ def test_bank_gradient_tile_edges(T):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("S", [1, 4, 5, 9, 16, 17, 33, 64])
+def test_bank_cascade_unit_edges(S):
+    """Channels that end around a 16-sample chunk, a lane's 32 samples, a 1024-sample unit and a
+    group of 32 units; stage counts around the adjoint's groups of four, the two chain
+    kernels and a warp's entry states, next to channels without stages.  All-pass sections
+    (poles of radius up to 0.6) keep every stage's signal at unit level; a stage's FP32
+    rounding is a few 2^-24 / (1 - r) of it, 64 stages stay below the bar of 1e-4."""
+    outs = [1, 16, 17, 32, 33, 1023, 1024, 1025, 2047, 2049, 32 * 1024, 32 * 1024 + 1, 5000]
+    rng = np.random.default_rng(500 + S)
+    taps = [1 + k % 4 for k in range(len(outs))]
+    stages = [S if k != 3 else 0 for k in range(len(outs))]
+    lengths = [n + t - 1 for n, t in zip(outs, taps)]
+    x = rng.standard_normal(sum(lengths))
+    h = np.concatenate([rng.standard_normal(t) / np.sqrt(t) + (np.arange(t) == 0) for t in taps])
+    r, th = rng.uniform(0.2, 0.6, sum(stages)), rng.uniform(0.3, 2.8, sum(stages))
+    a1, a2 = -2 * r * np.cos(th), r * r
+    c = np.stack([a2, a1, np.ones_like(a1), a1, a2], 1).reshape(-1)
+    _check_bank(lengths, taps, stages, x, h, c, seed=S)
+
+
+@pytest.mark.gpu
 def test_bank_many_channels():
     _check_bank(*_bank_case(4, 300, Lrange=(256, 4000), Tmax=64, Smax=6))
 
