@@ -53,6 +53,12 @@ namespace {
 
 using scan::M2;
 using scan::M2f;
+using scan::P2;
+using scan::dup;
+using scan::fma2;
+using scan::mul2;
+using scan::pk;
+using scan::up;
 
 constexpr int kL = 16;          // samples per chunk
 constexpr int kLane = 2 * kL;   // samples per lane: chunks A and B
@@ -378,36 +384,6 @@ __global__ void __launch_bounds__(kChainWarps * 32) bank_chain_fast_kernel(const
 }
 
 // ------------------------------------------------------------------ unit passes
-
-// Two FP32 values in a register pair, and the packed operations on them.
-struct P2 {
-   unsigned long long v;
-};
-__device__ __forceinline__ P2 pk(float a, float b)
-{
-   P2 r;
-   asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
-   return r;
-}
-__device__ __forceinline__ float2 up(P2 a)
-{
-   float2 r;
-   asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
-   return r;
-}
-__device__ __forceinline__ P2 dup(float a) { return pk(a, a); }
-__device__ __forceinline__ P2 fma2(P2 a, P2 b, P2 c)
-{
-   P2 r;
-   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-   return r;
-}
-__device__ __forceinline__ P2 mul2(P2 a, P2 b)
-{
-   P2 r;
-   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-   return r;
-}
 
 // A warp's staging area: row l holds lane l's 32 samples, sample i at column
 // 2 (i % 16) + i / 16, so that a lane's pair i is one 8-byte access and 32 consecutive

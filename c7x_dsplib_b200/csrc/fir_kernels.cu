@@ -8,17 +8,23 @@
 //                      floats are summed in tap order with separately rounded
 //                      multiply and add.  MODE_Q keeps the exact accumulator
 //                      and applies round-half-up / shift / saturate.
-//   fir_f32_simt_kernel the plain FP32 CUDA-core kernel: 8 consecutive outputs
-//                      per thread held in registers, taps unrolled by 8, fused
-//                      multiply-add.
+//   fir_f32_simt_kernel the plain FP32 CUDA-core kernel: 8 consecutive outputs and
+//                      the 8 half a tile further per thread as packed pairs in
+//                      registers, taps unrolled by 8, packed fused multiply-add.
+//   fir_f32_few_kernel  the same arithmetic for few outputs of many taps: the taps
+//                      split over groups of threads and the CTAs of a cluster.
 //
 // Layout (channel-major, DSPLIB_fir_cn.cpp:57-58): x[l*inPitch + t],
 // y[l*outPitch + j]; stored taps h[T-1-c] multiply x[j+c].
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
 #include "dsplib_internal.h"
+#include "scan_common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace dsplib {
 
@@ -153,58 +159,199 @@ __global__ void __launch_bounds__(kDirThreads) fir_floatq_kernel(FirLaunch a)
    }
 }
 
-constexpr int kSimtTile = 2048; // outputs per CTA, 8 per thread
+using scan::P2;
+using scan::dup;
+using scan::fma2;
+using scan::pk;
+using scan::up;
+
+// Plain FP32 FIR.  A thread keeps 8 pairs (y[j], y[j + H]) of outputs, H half the tile, so that
+// every multiply-add is a packed one (each half rounded as fmaf) on pairs (x[k], x[k + H]) kept
+// interleaved in shared memory and taps stored twice.  The taps are added in ascending order.
+// Bound by the FMA pipe: per 8 taps 64 packed multiply-adds (128 cycles of the pipe) against
+// 8 vector loads (20 shared-memory cycles); with scalar multiply-adds the issue slots and the
+// shared-memory reads (two-way conflicts) held the pipe at 40 %.  256 channels x 32768 samples x
+// 255 taps: 145 -> 91 us (47 of the 67 TFLOP/s that packed multiply-adds alone reach).
+constexpr int kSimtTile = 2048; // outputs per CTA, 16 per thread
 constexpr int kSimtTaps = 256;  // taps per shared-memory block
-constexpr int kSimtThreads = 256;
+constexpr int kSimtThreads = kSimtTile / 16;
+
+// Pair k of a window: 8 pairs (64 bytes) and 16 bytes of padding, so that the vector loads of
+// eight threads, 8 pairs apart, touch distinct banks.
+__device__ __forceinline__ int pairAt(int k) { return k + (k >> 3) * 2; }
+constexpr int pairsPadded(int n) { return n / 8 * 10; } // n a multiple of 8
+
+// acc[r] += sum_{c < n} w[8 t + r + c] g[c] for the thread at w = window + pairAt(8 t); n a multiple
+// of 8 (taps beyond the filter are zero), the window 8 pairs longer.
+__device__ __forceinline__ void simtTaps(P2 (&acc)[8], const P2 *w, const P2 *g, int n)
+{
+   P2 v[16];
+   auto load8 = [](P2 *d, const P2 *src) {
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+         const ulonglong2 u = *(const ulonglong2 *) (src + 2 * q);
+         d[2 * q].v = u.x;
+         d[2 * q + 1].v = u.y;
+      }
+   };
+   load8(v, w);
+#pragma unroll 2
+   for (int c = 0; c < n; c += 8) {
+      w += 10;
+      P2 h[8];
+      load8(v + 8, w);
+      load8(h, g + c);
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+#pragma unroll
+         for (int r = 0; r < 8; r++) acc[r] = fma2(v[r + i], h[i], acc[r]);
+#pragma unroll
+      for (int r = 0; r < 8; r++) v[r] = v[r + 8];
+   }
+}
 
 __global__ void __launch_bounds__(kSimtThreads) fir_f32_simt_kernel(FirLaunch a)
 {
-   __shared__ __align__(16) float xs[kSimtTile + kSimtTaps + 8];
-   __shared__ __align__(16) float gs[kSimtTaps];
+   __shared__ __align__(16) P2 xs[pairsPadded(kSimtTile / 2 + kSimtTaps + 8)];
+   __shared__ __align__(16) P2 gs[kSimtTaps];
+   const int tid = threadIdx.x;
    const int j0 = blockIdx.x * kSimtTile;
+   const int outs = min(kSimtTile, a.outSize - j0);
+   const int H = ((outs + 1) / 2 + 7) & ~7; // a short tile is halved too
    const long long inExtent = (long long) a.outSize + a.T - 1;
    for (int l = blockIdx.y; l < a.batch; l += gridDim.y) {
       const float *x = (const float *) a.x + (long long) l * a.inPitch;
       const float *h = (const float *) a.h + (long long) l * a.filtPitch;
-      float *y = (float *) a.y + (long long) l * a.outPitch;
-      float acc[8];
+      float *y = (float *) a.y + (long long) l * a.outPitch + j0;
+      P2 acc[8];
 #pragma unroll
-      for (int r = 0; r < 8; r++) acc[r] = 0.0f;
+      for (int r = 0; r < 8; r++) acc[r] = dup(0.0f);
       for (int cb = 0; cb < a.T; cb += kSimtTaps) {
          const int tb = min(kSimtTaps, a.T - cb);
          const int tbr = (tb + 7) & ~7;
-         for (int k = threadIdx.x; k < kSimtTile + tbr + 8; k += kSimtThreads) {
-            long long idx = (long long) j0 + cb + k;
-            xs[k] = idx < inExtent ? x[idx] : 0.0f;
+         const long long q0 = (long long) j0 + cb;
+         for (int k = tid; k < H + tbr + 8; k += kSimtThreads) {
+            const long long q = q0 + k;
+            xs[pairAt(k)] = pk(q < inExtent ? x[q] : 0.0f, q + H < inExtent ? x[q + H] : 0.0f);
          }
-         for (int k = threadIdx.x; k < tbr; k += kSimtThreads) gs[k] = k < tb ? h[a.T - 1 - (cb + k)] : 0.0f;
+         for (int k = tid; k < tbr; k += kSimtThreads) gs[k] = dup(k < tb ? h[a.T - 1 - (cb + k)] : 0.0f);
          __syncthreads();
-         const float *xw = xs + 8 * threadIdx.x;
-         for (int c = 0; c < tbr; c += 8) {
-            float w[16], g[8];
-            *(float4 *) &w[0] = *(const float4 *) &xw[c];
-            *(float4 *) &w[4] = *(const float4 *) &xw[c + 4];
-            *(float4 *) &w[8] = *(const float4 *) &xw[c + 8];
-            *(float4 *) &w[12] = *(const float4 *) &xw[c + 12];
-            *(float4 *) &g[0] = *(const float4 *) &gs[c];
-            *(float4 *) &g[4] = *(const float4 *) &gs[c + 4];
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-#pragma unroll
-               for (int r = 0; r < 8; r++) acc[r] = fmaf(w[r + i], g[i], acc[r]);
-            }
-         }
+         if (8 * tid < H) simtTaps(acc, xs + 10 * tid, gs, tbr);
          __syncthreads();
       }
-      // Stage the 8 consecutive outputs per thread through shared memory so
-      // the global stores are coalesced.
+      // the outputs through shared memory, so that the global stores are coalesced (rows of 8
+      // padded to 9: distinct banks)
+      float *os = (float *) xs;
+      if (8 * tid < H) {
 #pragma unroll
-      for (int r = 0; r < 8; r++) xs[8 * threadIdx.x + r] = acc[r];
+         for (int r = 0; r < 8; r++) {
+            const float2 v = up(acc[r]);
+            os[9 * tid + r] = v.x;
+            os[9 * (tid + H / 8) + r] = v.y;
+         }
+      }
       __syncthreads();
-      for (int k = threadIdx.x; k < kSimtTile; k += kSimtThreads)
-         if (j0 + k < a.outSize) y[j0 + k] = xs[k];
+      for (int k = tid; k < outs; k += kSimtThreads) y[k] = os[k + (k >> 3)];
       __syncthreads();
    }
+}
+
+// Few outputs of many taps (the taps gradient of an FIR layer is such a filter): one cluster of
+// kFewCluster CTAs per channel, each a range of the taps, and in it groups of GT threads that
+// hold all outputs (8 pairs a thread, up to 16 GT outputs) and take 64 taps in turn; the
+// groups' sums and then the CTAs' are added in order through (distributed) shared memory, so
+// results repeat bit for bit.  With the kernel above one CTA a channel ran all taps, 16 of 256
+// threads on 128 outputs: 434 -> 16 us for 64 channels, 128 outputs, 16257 taps.
+constexpr int kFewThreads = 128, kFewTaps = 64, kFewCluster = 8;
+
+template <int GT> __global__ void __launch_bounds__(kFewThreads) fir_f32_few_kernel(FirLaunch a)
+{
+   constexpr int H = 8 * GT, Q = kFewThreads / GT, TB = Q * kFewTaps; // half tile, groups, taps per block
+   constexpr int kWindow = pairsPadded(H + TB + 8), kSums = Q * 9 * GT; // pairs; the groups' sums reuse the window
+   __shared__ __align__(16) P2 xs[kWindow > kSums ? kWindow : kSums];
+   __shared__ __align__(16) P2 gs[TB];
+   __shared__ float part[2 * H];
+   float *red = (float *) xs; // [Q][9 * 2 GT]
+   const int tid = threadIdx.x, grp = tid / GT, t = tid % GT;
+   cg::cluster_group cl = cg::this_cluster();
+   const int rank = (int) cl.block_rank(), K = (int) cl.num_blocks();
+   const int l = blockIdx.y;
+   const float *x = (const float *) a.x + (long long) l * a.inPitch;
+   const float *h = (const float *) a.h + (long long) l * a.filtPitch;
+   float *y = (float *) a.y + (long long) l * a.outPitch;
+   const long long inExtent = (long long) a.outSize + a.T - 1;
+   // this CTA's taps: whole blocks
+   const int blocks = (a.T + TB - 1) / TB, per = (blocks + K - 1) / K;
+   const int c1 = (int) min((long long) a.T, (long long) (rank + 1) * per * TB);
+   P2 acc[8];
+#pragma unroll
+   for (int r = 0; r < 8; r++) acc[r] = dup(0.0f);
+   for (long long cb = (long long) rank * per * TB; cb < c1; cb += TB) {
+      const int tb = (int) min((long long) TB, c1 - cb);
+      for (int k = tid; k < H + TB + 8; k += kFewThreads) {
+         const long long q = cb + k;
+         xs[pairAt(k)] = pk(q < inExtent ? x[q] : 0.0f, q + H < inExtent ? x[q + H] : 0.0f);
+      }
+      for (int k = tid; k < TB; k += kFewThreads) gs[k] = dup(k < tb ? h[a.T - 1 - (cb + k)] : 0.0f);
+      __syncthreads();
+      const int left = tb - grp * kFewTaps; // in steps of 8 taps, as the other kernel: no sample further off meets a zero tap
+      if (left > 0)
+         simtTaps(acc, xs + pairsPadded(grp * kFewTaps) + 10 * t, gs + grp * kFewTaps, min(kFewTaps, (left + 7) & ~7));
+      __syncthreads();
+   }
+#pragma unroll
+   for (int r = 0; r < 8; r++) {
+      const float2 v = up(acc[r]);
+      red[grp * (18 * GT) + 9 * t + r] = v.x;
+      red[grp * (18 * GT) + 9 * (t + GT) + r] = v.y;
+   }
+   __syncthreads();
+   for (int o = tid; o < 2 * H; o += kFewThreads) {
+      float v = 0.0f;
+      for (int q = 0; q < Q; q++) v += red[q * (18 * GT) + o + (o >> 3)];
+      part[o] = v;
+   }
+   cl.sync();
+   for (int o = rank * kFewThreads + tid; o < a.outSize; o += K * kFewThreads) {
+      float v = 0.0f;
+      for (int d = 0; d < K; d++) v += cl.map_shared_rank(part, d)[o];
+      y[o] = v;
+   }
+   cl.sync(); // no CTA leaves while others read its sums
+}
+
+template <int GT> cudaError_t launchFew(const FirLaunch &a, cudaStream_t s)
+{
+   for (int l0 = 0; l0 < a.batch; l0 += 65535) {
+      FirLaunch b = a;
+      b.x = (const float *) a.x + (long long) l0 * a.inPitch;
+      b.h = (const float *) a.h + (long long) l0 * a.filtPitch;
+      b.y = (float *) a.y + (long long) l0 * a.outPitch;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(kFewCluster, a.batch - l0 < 65535 ? a.batch - l0 : 65535);
+      cfg.blockDim = dim3(kFewThreads);
+      cfg.stream = s;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = kFewCluster;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      const cudaError_t e = cudaLaunchKernelEx(&cfg, fir_f32_few_kernel<GT>, b);
+      if (e != cudaSuccess) return e;
+      countLaunch();
+   }
+   return cudaGetLastError();
+}
+
+// Up to 512 outputs of at least 1024 taps: the taps are split.  Both kernels do the same
+// multiply-adds, so the line lies where one CTA a channel (or a tile) leaves the GPU idle: a
+// batch below two CTAs an SM.
+bool firFewOutputs(const FirLaunch &a)
+{
+   const int sms = deviceSms() > 0 ? deviceSms() : 148;
+   return a.outSize <= 512 && a.T >= 1024 && a.batch < 16 * sms;
 }
 
 template <typename T, int MODE> cudaError_t launchDirect(const FirLaunch &a, cudaStream_t s)
@@ -240,6 +387,11 @@ cudaError_t launchFir(const FirLaunch &a, FirKernelKind kind, cudaStream_t s)
       }
    case FIR_F32_SIMT: {
       if (a.dtype != DSPLIB_FLOAT32) return cudaErrorInvalidValue;
+      if (firFewOutputs(a)) {
+         if (a.outSize <= 128) return launchFew<8>(a, s);
+         if (a.outSize <= 256) return launchFew<16>(a, s);
+         return launchFew<32>(a, s);
+      }
       dim3 grid((a.outSize + kSimtTile - 1) / kSimtTile, a.batch < 65535 ? a.batch : 65535);
       fir_f32_simt_kernel<<<grid, kSimtThreads, 0, s>>>(a);
       countLaunch();

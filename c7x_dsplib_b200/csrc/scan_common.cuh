@@ -1,4 +1,4 @@
-// 2x2 affine-map helpers shared by the chunked parallel-in-time biquad scans.
+// 2x2 affine-map helpers shared by the chunked parallel-in-time biquad scans, and packed FP32.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -62,6 +62,36 @@ __device__ __forceinline__ float2 shflIdx(float2 v, int src)
    v.x = __shfl_sync(0xffffffffu, v.x, src);
    v.y = __shfl_sync(0xffffffffu, v.y, src);
    return v;
+}
+
+// Two FP32 values in a register pair, and the packed operations on them.
+struct P2 {
+   unsigned long long v;
+};
+__device__ __forceinline__ P2 pk(float a, float b)
+{
+   P2 r;
+   asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+   return r;
+}
+__device__ __forceinline__ float2 up(P2 a)
+{
+   float2 r;
+   asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+   return r;
+}
+__device__ __forceinline__ P2 dup(float a) { return pk(a, a); }
+__device__ __forceinline__ P2 fma2(P2 a, P2 b, P2 c)
+{
+   P2 r;
+   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+   return r;
+}
+__device__ __forceinline__ P2 mul2(P2 a, P2 b)
+{
+   P2 r;
+   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+   return r;
 }
 
 } // namespace scan

@@ -174,6 +174,31 @@ def test_simt_float_accuracy(nch):
         assert np.max(np.abs(y - oracle.fir(x, h, T, nch=nch))) <= TOL_REF
 
 
+@pytest.mark.parametrize("out,T", [(1, 1), (7, 8), (9, 7), (17, 257), (2047, 9), (2048, 255), (2049, 256), (4097, 700),
+                                   (1, 1024), (127, 1025), (128, 16257), (129, 8191), (256, 4096), (257, 1023),
+                                   (257, 1024), (512, 2049), (513, 1500)])
+def test_simt_float_edges(out, T):
+    """Outputs around 8 a thread, half tiles and whole ones, taps around a step of 8 and a block;
+    few outputs of many taps (split over groups and CTAs) on both sides of that rule's lines.
+    Rows off the 16-byte boundary, nothing written between them.  Outputs have unit variance:
+    the bar is 2e-6 of max(1, the channel's peak), as above."""
+    rng = np.random.default_rng(out * 7 + T)
+    B, N = 3, out + T - 1
+    x = np.zeros((B, N + 1), np.float32)
+    x[:, :N] = rng.standard_normal((B, N))
+    hh = (rng.standard_normal((B, T)) / np.sqrt(T)).astype(np.float32)
+    args, pin, pfilt, pout = D.fir_setup(D.FLOAT32, B, N, T, nch=1, in_pitch=N + 1, out_pitch=out + 3)
+    pout.dim_x = out
+    h = D.FirHandle()
+    assert h.init(args, pin, pfilt, pout) == D.SUCCESS
+    xd, hd, od = dev(x), dev(hh), dev(np.full((B, out + 3), 7.5, np.float32))
+    assert h.exec(xd, hd, od) == D.SUCCESS, h.last_error()
+    got = host(od)
+    y64 = oracle.fir_f64(np.ascontiguousarray(x[:, :N]), hh, T, nch=1)
+    assert (np.abs(got[:, :out] - y64).max(axis=1) <= 2e-6 * np.maximum(1, np.abs(y64).max(axis=1))).all()
+    assert (got[:, out:] == 7.5).all()
+
+
 def lowpass(rng, rows, T):
     """Hamming-windowed sinc low-pass, cutoff U[0.05, 0.45], unit DC gain (stored tap order)."""
     n = np.arange(T) - (T - 1) / 2.0
