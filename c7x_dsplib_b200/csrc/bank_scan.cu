@@ -1097,6 +1097,12 @@ cudaError_t launchBankBackward(const BankLaunch &b, cudaStream_t s)
       if ((e = cudaEventRecord(b.join[i], b.aux[i])) != cudaSuccess) return e;
       if ((e = cudaStreamWaitEvent(s, b.join[i], 0)) != cudaSuccess) return e;
    }
+   return cudaGetLastError();
+}
+
+cudaError_t launchBankCoefGradients(const BankLaunch &b, cudaStream_t s)
+{
+   if (b.nUnits <= 0) return cudaSuccess;
    bank_coef_kernel<<<b.C, 32 * kCoefWarps, 0, s>>>(b.chans, b.part, b.gcoefs);
    countLaunch();
    return cudaGetLastError();

@@ -374,6 +374,8 @@ cudaError_t launchBankTables(const BankLaunch &b, const float *coefs, int totalS
                              float *impulse, cudaStream_t s);
 cudaError_t launchBankForward(const BankLaunch &b, cudaStream_t s);
 cudaError_t launchBankBackward(const BankLaunch &b, cudaStream_t s);
+// The coefficient gradients from the partial sums that the backward pass leaves.
+cudaError_t launchBankCoefGradients(const BankLaunch &b, cudaStream_t s);
 
 struct BiquadLaunch {
    const float *x;

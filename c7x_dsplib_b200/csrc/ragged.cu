@@ -86,13 +86,15 @@ struct RaggedPlan {
    std::vector<Segment> segs;
    // units ordered by their channel's stage count, deepest first, in buckets of one count
    std::vector<int> bucketS, bucketStart; // bucketStart has one entry more (the end)
-   // auxiliary streams and events of the adjoint's bucket launches (created with the plan)
+   // auxiliary streams and events (created with the plan): the adjoint's bucket launches
+   // spread over them, and small kernels that only a later one needs run on the first beside
+   // the main stream's (sideFork / sideDone)
    static constexpr int kAux = 3;
    cudaStream_t aux[kAux] = {};
-   cudaEvent_t fork = nullptr, join[kAux] = {};
+   cudaEvent_t fork = nullptr, join[kAux] = {}, sideFork = nullptr, sideDone = nullptr;
    int nAux = 0;
-   // the fork / join events are per plan: calls on one plan from several host threads
-   // queue their adjoints one at a time
+   // the events are per plan: calls on one plan from several host threads are queued one at
+   // a time
    std::mutex forkMu;
    long long segWork = 0, segScratch = 0; // largest work / scratch of one segment
    // device buffers of the host-buffer step (allocated by its first call, kept with the
@@ -222,7 +224,8 @@ static void freePlan(RaggedPlan *p)
       cudaStreamDestroy(p->aux[i]);
       cudaEventDestroy(p->join[i]);
    }
-   if (p->fork) cudaEventDestroy(p->fork);
+   for (cudaEvent_t e : {p->fork, p->sideFork, p->sideDone})
+      if (e) cudaEventDestroy(e);
    cudaFree(p->hBlk);
    cudaFree(p->hWork);
    cudaFree(p->hScratch);
@@ -377,9 +380,12 @@ static DSPLIB_STATUS raggedPlanBuild(DSPLIB_gpu_raggedPlan *plan, int32_t numCha
    p->hStages.assign(stages, stages + numChannels);
    cudaGetDevice(&p->device);
    p->err = allocErrorWord();
-   if (p->bucketS.size() > 1) {
-      bool ok = cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming) == cudaSuccess;
-      for (int i = 0; ok && i < RaggedPlan::kAux; i++) {
+   {
+      bool ok = true;
+      for (cudaEvent_t *e : {&p->fork, &p->sideFork, &p->sideDone})
+         ok = ok && cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess;
+      const int streams = p->bucketS.size() > 1 ? RaggedPlan::kAux : 1;
+      for (int i = 0; ok && i < streams; i++) {
          ok = cudaStreamCreateWithFlags(&p->aux[i], cudaStreamNonBlocking) == cudaSuccess;
          if (ok && cudaEventCreateWithFlags(&p->join[i], cudaEventDisableTiming) != cudaSuccess) {
             cudaStreamDestroy(p->aux[i]);
@@ -387,7 +393,7 @@ static DSPLIB_STATUS raggedPlanBuild(DSPLIB_gpu_raggedPlan *plan, int32_t numCha
          }
          if (ok) p->nAux = i + 1;
       }
-      (void) cudaGetLastError(); // without auxiliary streams the buckets run in sequence
+      (void) cudaGetLastError(); // without auxiliary streams everything runs in sequence
    }
    // work buffer: u | forward checkpoints | forward aggregates | stage tables | unit transitions |
    // chain group states | impulse responses
@@ -575,6 +581,62 @@ static BankLaunch bankLaunch(const RaggedPlan *p, const float *work)
    return b;
 }
 
+// Work beside the main stream s: sideBegin returns the plan's first auxiliary stream, ordered
+// behind what s holds so far (s itself without auxiliary streams), sideEnd marks its end and
+// sideJoin orders s behind that.  Capturable; the caller holds forkMu.
+static cudaError_t sideBegin(const RaggedPlan *p, cudaStream_t s, cudaStream_t *side)
+{
+   *side = s;
+   if (p->nAux == 0) return cudaSuccess;
+   cudaError_t e = cudaEventRecord(p->sideFork, s);
+   if (e == cudaSuccess) e = cudaStreamWaitEvent(p->aux[0], p->sideFork, 0);
+   if (e == cudaSuccess) *side = p->aux[0];
+   return e;
+}
+static cudaError_t sideJoin(const RaggedPlan *p, cudaStream_t s)
+{
+   if (p->nAux == 0) return cudaSuccess;
+   const cudaError_t e = cudaEventRecord(p->sideDone, p->aux[0]);
+   return e != cudaSuccess ? e : cudaStreamWaitEvent(s, p->sideDone, 0);
+}
+
+// FIR forward, and beside it the stage tables, unit transitions and impulse responses, which
+// depend on the coefficients alone (77 us on the 2048-channel bank, 45 us on 256 channels).
+static cudaError_t launchFirAndTables(const RaggedPlan *p, const BankLaunch &b, const float *x, const float *taps,
+                                      const float *coefs, float *work, cudaStream_t s)
+{
+   cudaStream_t side = s;
+   cudaError_t e = sideBegin(p, s, &side);
+   if (e == cudaSuccess)
+      e = launchFirBf16x3Ragged(p->dChan, p->dFirFwdRuns, p->nFirFwdRuns, x, taps, work, false, p->Tmax, p->err, s);
+   if (e == cudaSuccess)
+      e = launchBankTables(b, coefs, p->totalStages, work + p->wTab, (double *) (work + p->wPhi), work + p->wImp, side);
+   const cudaError_t j = sideJoin(p, s);
+   return e != cudaSuccess ? e : j;
+}
+
+// The adjoint behind the output gradient's aggregates: cascade, then the FIR's input and taps
+// gradients, with the coefficient gradients' sums beside them.
+static cudaError_t launchAdjoint(const RaggedPlan *p, BankLaunch &b, const float *x, const float *taps, float *gx,
+                                 float *gtaps, float *scratch, cudaStream_t s)
+{
+   cudaError_t e = launchBankBackward(b, s);
+   cudaStream_t side = s;
+   if (e == cudaSuccess) e = sideBegin(p, s, &side);
+   if (e == cudaSuccess) e = launchBankCoefGradients(b, side);
+   float *part = scratch + p->sDh;
+   if (e == cudaSuccess)
+      e = launchFirBf16x3Ragged(p->dChan, p->dFirDxRuns, p->nFirDxRuns, b.g, taps, gx, true, p->Tmax, p->err, s);
+   if (e == cudaSuccess) e = launchFirDhBf16x3Ragged(p->dChan, p->dDhRuns, p->nDhRuns, x, b.g, part, p->err, s);
+   if (e == cudaSuccess) {
+      fir_dh_reduce_kernel<<<p->C, 256, 0, s>>>(p->dChan, p->dDhStart, part, gtaps);
+      countLaunch();
+      e = cudaGetLastError();
+   }
+   const cudaError_t j = sideJoin(p, s);
+   return e != cudaSuccess ? e : j;
+}
+
 DSPLIB_STATUS DSPLIB_gpu_firBiquadBatched_fwd(DSPLIB_gpu_raggedPlan plan, const float *x, const float *taps,
                                               const float *coefs, float *y, float *work, void *stream)
 {
@@ -583,13 +645,10 @@ DSPLIB_STATUS DSPLIB_gpu_firBiquadBatched_fwd(DSPLIB_gpu_raggedPlan plan, const 
    PlanDevice dev(p);
    if (!dev.ok()) return DSPLIB_ERR_FAILURE;
    cudaStream_t s = (cudaStream_t) stream;
-   float *u = work;
    BankLaunch b = bankLaunch(p, work);
    b.y = y;
-   if (launchFirBf16x3Ragged(p->dChan, p->dFirFwdRuns, p->nFirFwdRuns, x, taps, u, false, p->Tmax, p->err, s) != cudaSuccess)
-      return DSPLIB_ERR_FAILURE;
-   if (launchBankTables(b, coefs, p->totalStages, work + p->wTab, (double *) (work + p->wPhi), work + p->wImp, s) != cudaSuccess ||
-       launchBankForward(b, s) != cudaSuccess)
+   std::lock_guard<std::mutex> lock(p->forkMu);
+   if (launchFirAndTables(p, b, x, taps, coefs, work, s) != cudaSuccess || launchBankForward(b, s) != cudaSuccess)
       return DSPLIB_ERR_FAILURE;
    return DSPLIB_SUCCESS;
 }
@@ -604,27 +663,16 @@ DSPLIB_STATUS DSPLIB_gpu_firBiquadBatched_bwd(DSPLIB_gpu_raggedPlan plan, const 
    PlanDevice dev(p);
    if (!dev.ok()) return DSPLIB_ERR_FAILURE;
    cudaStream_t s = (cudaStream_t) stream;
-   float *g = scratch;              // gradient w.r.t. the FIR output
-   float *part = scratch + p->sDh; // per-tile taps-gradient partials
    BankLaunch b = bankLaunch(p, work);
    b.gy = gy;
-   b.g = g;
+   b.g = scratch; // gradient w.r.t. the FIR output
    b.aggA = (float2 *) (scratch + p->sAgg);
    b.ckptA = (float2 *) (scratch + p->sCk);
    b.groupA = scratch + p->sGrp;
    b.part = scratch + p->sPart;
    b.gcoefs = gcoefs;
-   {
-      std::lock_guard<std::mutex> lock(p->forkMu);
-      if (launchBankBackward(b, s) != cudaSuccess) return DSPLIB_ERR_FAILURE;
-   }
-   if (launchFirBf16x3Ragged(p->dChan, p->dFirDxRuns, p->nFirDxRuns, g, taps, gx, true, p->Tmax, p->err, s) != cudaSuccess)
-      return DSPLIB_ERR_FAILURE;
-   if (launchFirDhBf16x3Ragged(p->dChan, p->dDhRuns, p->nDhRuns, x, g, part, p->err, s) != cudaSuccess)
-      return DSPLIB_ERR_FAILURE;
-   fir_dh_reduce_kernel<<<p->C, 256, 0, s>>>(p->dChan, p->dDhStart, part, gtaps);
-   countLaunch(1);
-   return cudaGetLastError() == cudaSuccess ? DSPLIB_SUCCESS : DSPLIB_ERR_FAILURE;
+   std::lock_guard<std::mutex> lock(p->forkMu);
+   return launchAdjoint(p, b, x, taps, gx, gtaps, scratch, s) == cudaSuccess ? DSPLIB_SUCCESS : DSPLIB_ERR_FAILURE;
 }
 
 } // extern "C"
@@ -638,7 +686,6 @@ static DSPLIB_STATUS stepMseCore(RaggedPlan *p, const float *x, const float *tap
                                  float *gtaps, float *gcoefs, float *work, float *scratch, float scale,
                                  double invCount, cudaStream_t s)
 {
-   float *g = scratch;
    BankLaunch b = bankLaunch(p, work);
    b.y = y;
    b.target = target;
@@ -646,35 +693,24 @@ static DSPLIB_STATUS stepMseCore(RaggedPlan *p, const float *x, const float *tap
    b.lossPart = (double *) (scratch + p->sLoss);
    b.scale = scale;
    b.aggA = (float2 *) (scratch + p->sAgg);
+   std::lock_guard<std::mutex> lock(p->forkMu);
    // forward, loss gradient and the adjoint's first pass in one sweep over the units
-   if (launchFirBf16x3Ragged(p->dChan, p->dFirFwdRuns, p->nFirFwdRuns, x, taps, work, false, p->Tmax, p->err, s) !=
-           cudaSuccess ||
-       launchBankTables(b, coefs, p->totalStages, work + p->wTab, (double *) (work + p->wPhi), work + p->wImp, s) != cudaSuccess ||
-       launchBankForward(b, s) != cudaSuccess)
+   if (launchFirAndTables(p, b, x, taps, coefs, work, s) != cudaSuccess || launchBankForward(b, s) != cudaSuccess)
       return DSPLIB_ERR_FAILURE;
-   mse_reduce_kernel<<<1, 1024, 0, s>>>(b.lossPart, p->nUnits, invCount, loss, lossSum);
+   // the loss beside the adjoint (joined at its end)
+   cudaStream_t side = s;
+   if (sideBegin(p, s, &side) != cudaSuccess) return DSPLIB_ERR_FAILURE;
+   mse_reduce_kernel<<<1, 1024, 0, side>>>(b.lossPart, p->nUnits, invCount, loss, lossSum);
    countLaunch();
-   // adjoint
    b.target = nullptr;
    b.gy = gy;
-   b.g = g;
+   b.g = scratch;
    b.ckptA = (float2 *) (scratch + p->sCk);
    b.groupA = scratch + p->sGrp;
    b.part = scratch + p->sPart;
    b.gcoefs = gcoefs;
    b.aggReady = true;
-   cudaError_t be;
-   {
-      std::lock_guard<std::mutex> lock(p->forkMu);
-      be = launchBankBackward(b, s);
-   }
-   if (be != cudaSuccess ||
-       launchFirBf16x3Ragged(p->dChan, p->dFirDxRuns, p->nFirDxRuns, g, taps, gx, true, p->Tmax, p->err, s) != cudaSuccess ||
-       launchFirDhBf16x3Ragged(p->dChan, p->dDhRuns, p->nDhRuns, x, g, scratch + p->sDh, p->err, s) != cudaSuccess)
-      return DSPLIB_ERR_FAILURE;
-   fir_dh_reduce_kernel<<<p->C, 256, 0, s>>>(p->dChan, p->dDhStart, scratch + p->sDh, gtaps);
-   countLaunch();
-   return cudaGetLastError() == cudaSuccess ? DSPLIB_SUCCESS : DSPLIB_ERR_FAILURE;
+   return launchAdjoint(p, b, x, taps, gx, gtaps, scratch, s) == cudaSuccess ? DSPLIB_SUCCESS : DSPLIB_ERR_FAILURE;
 }
 
 // Input bytes (x and target) per segment of a host-buffer step.
