@@ -10,7 +10,8 @@
 //
 // biquad_scan_kernel  chunked parallel-in-time scan.  Lane = channel (32
 //                     channels per CTA, so every time row is one coalesced
-//                     128-byte access), warp = chunk of L consecutive samples,
+//                     128-byte access; or half rows of 16), warp = chunk of L consecutive
+//                     samples (its two halves run at once as packed FP32 pairs),
 //                     CTA = W chunks, cluster of K CTAs = one window of K*W*L
 //                     samples.  For each stage:
 //                       1. every chunk runs the stage recursion from a zero
@@ -40,6 +41,7 @@
 #include <cstdio>
 
 #include "dsplib_internal.h"
+#include "scan_common.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -272,10 +274,130 @@ __device__ __forceinline__ void runChunkAny(float (&v)[L], int len, const Coef &
    else runChunk<FORM, L, WRITE, false>(v, len, c, st, tail);
 }
 
-constexpr int kScanL = 32;      // samples per chunk
+using scan::P2;
+using scan::add2;
+using scan::dup;
+using scan::fma2;
+using scan::mul2;
+using scan::pk;
+using scan::up;
+
+// A stage's recursion over a lane's 2 H samples held as packed pairs (sample i, sample H + i):
+// both halves run at once from their own states s1, s2 (packed), every operation a packed one in
+// the order of runChunk.  k: the stage's coefficients as scanCoef keeps them.  WRITE = false
+// gives the end states only.  FULL = false: the state (and for DF1 the last two inputs and
+// outputs) after sample len - 1 is taken on the way; the samples beyond are zeros.
+template <int FORM, bool WRITE, bool FULL, int H>
+__device__ __forceinline__ void runPairs(P2 (&v)[H], int len, const float (&k)[5], P2 &s1, P2 &s2, float2 *fin, float4 *tail)
+{
+   constexpr bool DF1 = FORM == DSPLIB_BIQUAD_DF1;
+   const P2 k0 = dup(k[0]), k1 = dup(k[1]), k2 = dup(k[2]), n3 = dup(-k[3]), n4 = dup(-k[4]), a11 = dup(k[3]);
+   P2 u1 = dup(0.0f), u2 = u1, y1 = u1, y2 = u1;
+#pragma unroll
+   for (int i = 0; i < H; i++) {
+      const P2 x = v[i];
+      if (FORM == DSPLIB_BIQUAD_DF2) {
+         const P2 w = fma2(n3, s1, fma2(n4, s2, x));
+         if (WRITE) v[i] = fma2(k0, w, fma2(k1, s1, mul2(k2, s2)));
+         s2 = s1;
+         s1 = w;
+      }
+      else if (FORM == DSPLIB_BIQUAD_TIF) { // k: c0, c1, a12, a11
+         const P2 o = add2(x, s1);
+         const P2 d0 = fma2(a11, s1, fma2(x, k0, s2));
+         s2 = fma2(k1, x, mul2(k2, s1));
+         s1 = d0;
+         if (WRITE) v[i] = o;
+      }
+      else { // k: b0, b1 - a1 b0, b2 - a2 b0, a1, a2
+         if (WRITE) {
+            const P2 y = fma2(x, k0, s1);
+            v[i] = y;
+            if (DF1) {
+               u2 = u1;
+               u1 = x;
+               y2 = y1;
+               y1 = y;
+            }
+         }
+         const P2 n = fma2(n3, s1, fma2(x, k1, s2));
+         s2 = fma2(n4, s1, mul2(x, k2));
+         s1 = n;
+      }
+      if (WRITE && !FULL) {
+         const float2 a = up(s1), b = up(s2);
+         if (i + 1 == len) *fin = make_float2(a.x, b.x);
+         if (i + H + 1 == len) *fin = make_float2(a.y, b.y);
+         if (DF1) {
+            const float2 p = up(u1), q = up(u2), r = up(y1), t = up(y2);
+            if (i + 1 == len) *tail = make_float4(p.x, q.x, r.x, t.x);
+            if (i + H + 1 == len) *tail = make_float4(p.y, q.y, r.y, t.y);
+         }
+      }
+   }
+   if (WRITE && FULL) {
+      const float2 a = up(s1), b = up(s2);
+      *fin = make_float2(a.y, b.y);
+      if (DF1) *tail = make_float4(up(u1).y, up(u2).y, up(y1).y, up(y2).y);
+   }
+}
+
+// The same recursion over the lane's samples one after another (scalar operations, the same
+// values as runPairs over halves of this length would see): from the state st, which becomes the
+// end state; FULL = false as above, with fin and tail.
+template <int FORM, bool WRITE, bool FULL, int H>
+__device__ __forceinline__ void runSerial(P2 (&v)[H], int len, const float (&k)[5], float2 &st, float2 *fin, float4 *tail)
+{
+   constexpr bool DF1 = FORM == DSPLIB_BIQUAD_DF1;
+   float s1 = st.x, s2 = st.y, u1 = 0.0f, u2 = 0.0f, y1 = 0.0f, y2 = 0.0f;
+#pragma unroll
+   for (int i = 0; i < 2 * H; i++) {
+      const float2 p = up(v[i % H]);
+      const float x = i < H ? p.x : p.y;
+      float o = 0.0f;
+      if (FORM == DSPLIB_BIQUAD_DF2) {
+         const float w = fmaf(-k[3], s1, fmaf(-k[4], s2, x));
+         o = fmaf(k[0], w, fmaf(k[1], s1, k[2] * s2));
+         s2 = s1;
+         s1 = w;
+      }
+      else if (FORM == DSPLIB_BIQUAD_TIF) {
+         o = x + s1;
+         const float d0 = fmaf(k[3], s1, fmaf(x, k[0], s2));
+         s2 = fmaf(k[1], x, k[2] * s1);
+         s1 = d0;
+      }
+      else {
+         o = fmaf(x, k[0], s1);
+         u2 = u1;
+         u1 = x;
+         y2 = y1;
+         y1 = o;
+         const float n = fmaf(-k[3], s1, fmaf(x, k[1], s2));
+         s2 = fmaf(-k[4], s1, x * k[2]);
+         s1 = n;
+      }
+      if (WRITE) v[i % H] = i < H ? pk(o, p.y) : pk(p.x, o);
+      if (WRITE && !FULL && i + 1 == len) {
+         *fin = make_float2(s1, s2);
+         if (DF1) *tail = make_float4(u1, u2, y1, y2);
+      }
+   }
+   st = make_float2(s1, s2);
+   if (WRITE && FULL) {
+      *fin = st;
+      if (DF1) *tail = make_float4(u1, u2, y1, y2);
+   }
+}
+
+// Samples per chunk: short chunks (32, run serially) where latency counts, long ones (64, run as
+// two packed halves of 32) where many channels do (launchScanForm).  States pass between spans
+// of 32 samples either way: halves of 16 in the short chunks ran no faster, and doubled the
+// error where the output nearly cancels.
+constexpr int kShortChunk = 32, kLongChunk = 64;
 constexpr int kPad = 33;        // row pitch (double2) of the chunk x channel tables
 constexpr int kMaxCluster = 16; // CTAs per cluster
-constexpr int kPowTableBytes = 64 * 1024;
+constexpr int kPowTableBytes = 80 * 1024;
 
 __host__ __device__ constexpr int ilog2c(int x) { return x <= 1 ? 0 : 1 + ilog2c(x / 2); }
 
@@ -292,11 +414,11 @@ __device__ __forceinline__ float2 affinef(const M2f &m, float2 v, float2 e)
    return make_float2(fmaf(m.a, v.x, fmaf(m.b, v.y, e.x)), fmaf(m.c, v.x, fmaf(m.d, v.y, e.y)));
 }
 
-// Matrix powers kept per stage and channel: M^(2^k), M = A^L, for
-// k = 0 .. log2(W) (the last one is the CTA span A^(W*L)).
+// Matrix powers kept per stage and channel: A^(L/2) (between a chunk's halves), then M^(2^k),
+// M = A^L, for k = 0 .. log2(W) (the last one is the CTA span A^(W*L)).
 template <int W> struct ScanShape {
    static constexpr int LOGW = ilog2c(W);
-   static constexpr int NP = LOGW + 1;
+   static constexpr int NP = LOGW + 2;
 };
 
 struct ScanSmem {
@@ -304,12 +426,12 @@ struct ScanSmem {
    bool powTable;
 };
 
-template <int W> __host__ __device__ inline ScanSmem scanLayout(int S)
+template <int W, int SUB = 1> __host__ __device__ inline ScanSmem scanLayout(int S)
 {
    ScanSmem o;
    size_t off = 0;
    o.E = off;
-   off += (size_t) W * kPad * sizeof(float2);
+   off += (size_t) 2 * W * SUB * kPad * sizeof(float2); // two phases
    o.Mine = off;
    off += (size_t) 32 * sizeof(float2);
    o.Win = off;
@@ -328,11 +450,11 @@ template <int W> __host__ __device__ inline ScanSmem scanLayout(int S)
 // Shared memory of a scan launch: the tables, plus the next-window buffer when the
 // input is device memory and spans more than one window, plus (clusters) the
 // exchange buffer: two phases of every CTA's 32 chunk-span aggregates.
-template <int W> inline size_t scanSmemBytes(const BiquadLaunch &a, int K)
+template <int W, int L, int SUB> inline size_t scanSmemBytes(const BiquadLaunch &a, int K)
 {
-   const ScanSmem lay = scanLayout<W>(a.S);
-   const bool next = a.prefetch && (long long) a.N > (long long) K * W * kScanL;
-   return lay.total + (next ? (size_t) kScanL * W * 32 * sizeof(float) : 0) +
+   const ScanSmem lay = scanLayout<W, SUB>(a.S);
+   const bool next = a.prefetch && (long long) a.N > (long long) K * W * SUB * L;
+   return lay.total + (next ? (size_t) L * W * 32 * sizeof(float) : 0) +
           (K > 1 ? (size_t) 2 * K * 32 * sizeof(float2) : 0);
 }
 
@@ -342,12 +464,12 @@ __device__ __forceinline__ void cpAsync4(float *dst, const float *src)
    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
 }
 
-// Writes M^(2^k), k = 0 .. NP-1, of M = A^L to out[] (formed in FP64, rounded once).
-template <int FORM, int W> __device__ __forceinline__ void stagePowersF(const Coef &c, M2f *out)
+// Writes A^(L/2) and M^(2^k), M = A^L, to out[] (formed in FP64, rounded once).
+template <int FORM, int W, int L> __device__ __forceinline__ void stagePowersF(const Coef &c, M2f *out)
 {
    M2 P = transition<FORM>(c);
 #pragma unroll
-   for (int r = 1; r < kScanL; r <<= 1) P = mmul(P, P);
+   for (int r = 1; r < L / 2; r <<= 1) P = mmul(P, P);
    out[0] = {(float) P.a, (float) P.b, (float) P.c, (float) P.d};
 #pragma unroll
    for (int k = 1; k < ScanShape<W>::NP; k++) {
@@ -356,22 +478,28 @@ template <int FORM, int W> __device__ __forceinline__ void stagePowersF(const Co
    }
 }
 
-// Horner's rule acc <- M acc + e_i over i = 0 .. n-1 (n <= MAXN), e_i = src[i * stride].
-// The loads are issued eight at a time ahead of the dependent multiply-adds, so the chain
-// costs about one FMA latency pair per step rather than a shared-memory round trip.
+// Horner's rule acc <- M acc + e_i over i = 0 .. n-1 (n <= MAXN, the same for the warp), e_i =
+// src[i * stride].  The loads are issued four at a time ahead of the dependent multiply-adds, so
+// the chain costs about one FMA latency pair per step rather than a shared-memory round trip.
 template <int MAXN>
 __device__ __forceinline__ float2 hornerF(const M2f &M, float2 acc, const float2 *src, int stride, int n)
 {
 #pragma unroll
-   for (int g = 0; g < MAXN; g += 8) {
-      if (g >= n) break;
-      float2 e[8];
+   for (int g = 0; g < MAXN; g += 4) {
+      if (g + 4 > n) break;
+      float2 e[4];
 #pragma unroll
-      for (int i = 0; i < 8; i++) e[i] = (g + i < n) ? src[(g + i) * stride] : make_float2(0.f, 0.f);
+      for (int i = 0; i < 4; i++) e[i] = src[(g + i) * stride];
 #pragma unroll
-      for (int i = 0; i < 8; i++)
-         if (g + i < n) acc = affinef(M, acc, e[i]);
+      for (int i = 0; i < 4; i++) acc = affinef(M, acc, e[i]);
    }
+   src += (n & ~3) * stride;
+   if (n & 2) {
+      const float2 e0 = src[0], e1 = src[stride];
+      acc = affinef(M, affinef(M, acc, e0), e1);
+      src += 2 * stride;
+   }
+   if (n & 1) acc = affinef(M, acc, src[0]);
    return acc;
 }
 
@@ -385,33 +513,41 @@ __device__ __forceinline__ float2 powApplyF(const M2f *P, int n, int nb, float2 
    return v;
 }
 
-template <int FORM, int W, bool CLUSTER>
+// SUB = 1: lane = channel.  SUB = 2 (no cluster): 16 channels, the warp's two half rows take
+// consecutive chunks.
+template <int FORM, int W, int L, int SUB, bool CLUSTER>
 __global__ void __launch_bounds__(W * 32, 16 / W) biquad_scan_kernel(BiquadLaunch a)
 {
-   constexpr int L = kScanL;
+   static_assert(SUB == 1 || !CLUSTER, "half rows take one CTA a window");
+   constexpr int CH = 32 / SUB;
+   constexpr bool PAIRS = L == kLongChunk;
    constexpr int nv = FORM == DSPLIB_BIQUAD_DF1 ? 4 : 2;
    constexpr int LOGW = ScanShape<W>::LOGW;
    constexpr int NP = ScanShape<W>::NP;
    extern __shared__ __align__(16) unsigned char smem[];
-   const ScanSmem lay = scanLayout<W>(a.S);
-   float2 *sE = (float2 *) (smem + lay.E);
+   const ScanSmem lay = scanLayout<W, SUB>(a.S);
+   float2 *sE2 = (float2 *) (smem + lay.E);
    float2 *sMine = (float2 *) (smem + lay.Mine);
    float2 *sWin = (float2 *) (smem + lay.Win);
    M2f *sPow = (M2f *) (smem + lay.Pow);
    float *sCf = (float *) (smem + lay.Cf);
    float *sNext = (float *) (smem + lay.Next);
 
-   const int lane = threadIdx.x & 31;
+   const int lane = threadIdx.x & (CH - 1); // channel within the CTA's
+   const int sub = SUB > 1 ? (threadIdx.x & 31) / CH : 0;
    const int w = threadIdx.x >> 5;
-   const int ch = blockIdx.y * 32 + lane;
-   const bool active = ch < a.C;
+   const int cw = w * SUB + sub; // chunk within the CTA's
+   // lanes beyond the last channel run along on that channel's data and store nothing, so that
+   // lengths are the same over the warp
+   const bool active = blockIdx.y * CH + lane < a.C;
+   const int ch = active ? blockIdx.y * CH + lane : a.C - 1;
    int K = 1, rank = 0;
    if (CLUSTER) {
       cg::cluster_group cl = cg::this_cluster();
       K = (int) cl.num_blocks();
       rank = (int) cl.block_rank();
    }
-   const long long windowLen = (long long) K * W * L;
+   const long long windowLen = (long long) K * W * SUB * L;
    // Device-memory input over several windows: the next window's samples are copied into
    // shared memory (each thread its own slots) while this one is filtered.
    const bool usePrefetch = a.prefetch && a.N > windowLen;
@@ -419,31 +555,35 @@ __global__ void __launch_bounds__(W * 32, 16 / W) biquad_scan_kernel(BiquadLaunc
    float2 *sAggIn = (float2 *) (smem + lay.Next + (usePrefetch ? (size_t) L * W * 32 * sizeof(float) : 0));
 
    // First window's input, issued before the table set-up so the loads overlap it.
-   long long t0 = ((long long) rank * W + w) * L;
-   int len = (active && t0 < a.N) ? (int) ((a.N - t0) < L ? (a.N - t0) : L) : 0;
-   float v[L];
-   {
+   long long t0 = ((long long) rank * W * SUB + cw) * L;
+   int len = t0 < a.N ? (int) ((a.N - t0) < L ? (a.N - t0) : L) : 0;
+   const int inPitch = (int) a.inPitch, outPitch = (int) a.outPitch;
+   P2 v[L / 2]; // pairs (sample i, sample L / 2 + i)
+   auto loadWindow = [&]() {
       const float *xp = a.x + t0 * a.inPitch + ch;
       if (len == L) {
 #pragma unroll
-         for (int i = 0; i < L; i++) v[i] = xp[i * a.inPitch];
+         for (int i = 0; i < L / 2; i++) v[i] = pk(xp[(long long) i * inPitch], xp[(long long) (i + L / 2) * inPitch]);
       }
       else {
 #pragma unroll
-         for (int i = 0; i < L; i++) v[i] = i < len ? xp[i * a.inPitch] : 0.0f;
+         for (int i = 0; i < L / 2; i++)
+            v[i] = pk(i < len ? xp[(long long) i * inPitch] : 0.0f, i + L / 2 < len ? xp[(long long) (i + L / 2) * inPitch] : 0.0f);
       }
-   }
+   };
+   loadWindow();
 
    // Coefficients, matrix powers and the initial state (scan coordinates) per stage and channel.
    for (int s = w; s < a.S; s += W) {
-      Coef c;
-      if (active) c = loadCoef(a, s, ch);
-      else
-         for (int k = 0; k < 5; k++) c.k[k] = 0.0f;
+      const Coef c = loadCoef(a, s, ch);
       for (int k = 0; k < 5; k++) sCf[(s * 32 + lane) * 5 + k] = c.k[k];
-      if (lay.powTable) stagePowersF<FORM, W>(c, sPow + (s * 32 + lane) * NP);
-      float2 st0 = make_float2(0.0, 0.0);
-      if (active) {
+      if (FORM == DSPLIB_BIQUAD_DF1 || FORM == DSPLIB_BIQUAD_TDF2) { // as runPairs reads them
+         sCf[(s * 32 + lane) * 5 + 1] = (float) ((double) c.k[1] - (double) c.k[3] * c.k[0]);
+         sCf[(s * 32 + lane) * 5 + 2] = (float) ((double) c.k[2] - (double) c.k[4] * c.k[0]);
+      }
+      if (lay.powTable) stagePowersF<FORM, W, L>(c, sPow + (s * 32 + lane) * NP);
+      float2 st0;
+      {
          const float *sp = a.state + (long long) (s * nv) * a.varPitch + ch;
          if (FORM == DSPLIB_BIQUAD_DF1) { // DF1 (xd1, xd2, yd1, yd2) -> transposed-form state
             const double xd1 = sp[0], xd2 = sp[a.varPitch], yd1 = sp[2 * a.varPitch], yd2 = sp[3 * a.varPitch];
@@ -462,32 +602,35 @@ __global__ void __launch_bounds__(W * 32, 16 / W) biquad_scan_kernel(BiquadLaunc
    int phase = 0;
    for (long long win0 = 0; win0 < a.N; win0 += windowLen) {
       if (win0 > 0) {
-         t0 = win0 + ((long long) rank * W + w) * L;
-         len = (active && t0 < a.N) ? (int) ((a.N - t0) < L ? (a.N - t0) : L) : 0;
+         t0 = win0 + ((long long) rank * W * SUB + cw) * L;
+         len = t0 < a.N ? (int) ((a.N - t0) < L ? (a.N - t0) : L) : 0;
          if (usePrefetch) {
             asm volatile("cp.async.wait_all;" ::: "memory");
-#pragma unroll
-            for (int i = 0; i < L; i++) v[i] = i < len ? sNext[i * (W * 32) + threadIdx.x] : 0.0f;
-         }
-         else {
-            const float *xp = a.x + t0 * a.inPitch + ch;
             if (len == L) {
 #pragma unroll
-               for (int i = 0; i < L; i++) v[i] = xp[i * a.inPitch];
+               for (int i = 0; i < L / 2; i++)
+                  v[i] = pk(sNext[i * (W * 32) + threadIdx.x], sNext[(i + L / 2) * (W * 32) + threadIdx.x]);
             }
-            else {
+            else
 #pragma unroll
-               for (int i = 0; i < L; i++) v[i] = i < len ? xp[i * a.inPitch] : 0.0f;
-            }
+            for (int i = 0; i < L / 2; i++)
+               v[i] = pk(i < len ? sNext[i * (W * 32) + threadIdx.x] : 0.0f,
+                         i + L / 2 < len ? sNext[(i + L / 2) * (W * 32) + threadIdx.x] : 0.0f);
          }
+         else loadWindow();
       }
       if (usePrefetch && win0 + windowLen < a.N) {
-         const long long tn = win0 + windowLen + ((long long) rank * W + w) * L;
-         const int ln = (active && tn < a.N) ? (int) ((a.N - tn) < L ? (a.N - tn) : L) : 0;
+         const long long tn = win0 + windowLen + ((long long) rank * W * SUB + cw) * L;
+         const int ln = tn < a.N ? (int) ((a.N - tn) < L ? (a.N - tn) : L) : 0;
          const float *xp = a.x + tn * a.inPitch + ch;
+         if (ln == L) {
+#pragma unroll
+            for (int i = 0; i < L; i++) cpAsync4(&sNext[i * (W * 32) + threadIdx.x], xp + (long long) i * inPitch);
+         }
+         else
 #pragma unroll
          for (int i = 0; i < L; i++)
-            if (i < ln) cpAsync4(&sNext[i * (W * 32) + threadIdx.x], xp + i * a.inPitch);
+            if (i < ln) cpAsync4(&sNext[i * (W * 32) + threadIdx.x], xp + (long long) i * inPitch);
          asm volatile("cp.async.commit_group;" ::: "memory");
       }
       for (int s = 0; s < a.S; s++) {
@@ -495,22 +638,42 @@ __global__ void __launch_bounds__(W * 32, 16 / W) biquad_scan_kernel(BiquadLaunc
 #pragma unroll
          for (int k = 0; k < 5; k++) c.k[k] = sCf[(s * 32 + lane) * 5 + k];
          // Matrix powers of this stage for channel `lane`: the table, or (deep cascades) this
-         // stage's powers formed by warp 0 into the buffer of this iteration's parity.  A buffer
-         // is rewritten two iterations later, once every warp has passed the barrier between.
-         const M2f *P;
+         // stage's powers formed by warp 0 into the buffer of this iteration's parity, A^(L/2)
+         // by every warp (it is used before the barrier).  A buffer is rewritten two iterations
+         // later, once every warp has passed the barrier between.
+         const M2f *Ph; // A^(L/2)
+         M2f half;
          if (lay.powTable) {
-            P = sPow + (s * 32 + lane) * NP;
+            Ph = sPow + (s * 32 + lane) * NP;
+            if (PAIRS) half = Ph[0];
          }
          else {
-            P = sPow + ((phase & 1) * 32 + lane) * NP;
-            if (w == 0) stagePowersF<FORM, W>(c, (M2f *) P);
+            Ph = sPow + ((phase & 1) * 32 + lane) * NP;
+            if (w == 0) stagePowersF<FORM, W, L>(c, (M2f *) Ph);
+            if (PAIRS) {
+               M2 q = transition<FORM>(c);
+#pragma unroll
+               for (int r = 1; r < L / 2; r <<= 1) q = mmul(q, q);
+               half = {(float) q.a, (float) q.b, (float) q.c, (float) q.d};
+            }
          }
-         // 1. zero-state end state of this chunk.  The window's entry state for this stage
-         //    is read before the barrier: it is replaced after it.
-         float2 e = make_float2(0.f, 0.f);
-         runChunkAny<FORM, L, false>(v, len, c, e, nullptr);
+         const M2f *P = Ph + 1;
+         // 1. zero-state end states of this chunk's halves, and of the chunk.  The window's entry
+         //    state for this stage is read before the barrier: it is replaced after it.
+         float2 eA, e = make_float2(0.0f, 0.0f);
+         if (!PAIRS) runSerial<FORM, false, true>(v, L, c.k, e, nullptr, nullptr);
+         else {
+            P2 z1 = dup(0.0f), z2 = z1;
+            runPairs<FORM, false, true>(v, L, c.k, z1, z2, nullptr, nullptr);
+            const float2 p = up(z1), q = up(z2);
+            eA = make_float2(p.x, q.x);
+            e = affinef(half, eA, make_float2(p.y, q.y));
+         }
          const float2 win = sWin[s * 32 + lane];
-         sE[w * kPad + lane] = e;
+         // alternate buffers: a warp may be a stage ahead of one that still reads the last stage's
+         // end states, never two (the barrier of the stage between)
+         float2 *sE = sE2 + (phase & 1) * (W * SUB * kPad);
+         sE[cw * kPad + lane] = e;
          __syncthreads();
 
          // 2. chunk-boundary states, lane = channel, by Horner's rule over the chunks before
@@ -558,21 +721,41 @@ __global__ void __launch_bounds__(W * 32, 16 / W) biquad_scan_kernel(BiquadLaunc
             st = make_float2(tv.x + pre.x, tv.y + pre.y);
          }
          else {
-            const float2 acc = hornerF<W>(M, win, sE + lane, kPad, w);
+            float2 acc = hornerF<W * SUB>(M, win, sE + lane, kPad, w * SUB);
+            if (SUB > 1 && sub > 0) acc = affinef(M, acc, sE[(w * SUB) * kPad + lane]);
             st = acc;
-            if (w == W - 1) sWin[s * 32 + lane] = affinef(M, acc, e); // state at the window's end
+            if (cw == W * SUB - 1) sWin[s * 32 + lane] = affinef(M, acc, e); // state at the window's end
          }
 
-         // 4. rerun from the true state, producing the stage output in place
+         // 4. rerun from the true states, producing the stage output in place
          float4 tail = make_float4(0.f, 0.f, 0.f, 0.f);
-         runChunkAny<FORM, L, true>(v, len, c, st, &tail);
+         if (!PAIRS) {
+            float2 z = st;
+            if (len == L) runSerial<FORM, true, true>(v, L, c.k, z, &st, &tail);
+            else runSerial<FORM, true, false>(v, len, c.k, z, &st, &tail);
+         }
+         else {
+            const float2 sb = affinef(half, st, eA);
+            P2 z1 = pk(st.x, sb.x), z2 = pk(st.y, sb.y);
+            if (len == L) runPairs<FORM, true, true>(v, L, c.k, z1, z2, &st, &tail);
+            else {
+               float2 prev = make_float2(0.0f, 0.0f);
+               if (FORM == DSPLIB_BIQUAD_DF1 && len == L / 2 + 1) prev.x = up(v[L / 2 - 1]).x;
+               runPairs<FORM, true, false>(v, len, c.k, z1, z2, &st, &tail);
+               // one sample into the second half: the one before is the first half's last
+               if (FORM == DSPLIB_BIQUAD_DF1 && len == L / 2 + 1) {
+                  tail.y = prev.x;
+                  tail.w = up(v[L / 2 - 1]).x;
+               }
+            }
+         }
          if (FORM == DSPLIB_BIQUAD_TIF && c.k[4] != 1.0f) {
-            const float g = c.k[4];
+            const P2 g = dup(c.k[4]);
 #pragma unroll
-            for (int i = 0; i < L; i++) v[i] *= g;
+            for (int i = 0; i < L / 2; i++) v[i] = mul2(v[i], g);
          }
          float *sp = a.state + (long long) (s * nv) * a.varPitch + ch;
-         if (len > 0 && t0 + len == a.N) { // chunk holding the last sample: final state
+         if (active && len > 0 && t0 + len == a.N) { // chunk holding the last sample: final state
             if (FORM == DSPLIB_BIQUAD_DF1) {
                // With a single sample the stage's old xd1 / yd1 shift into xd2 / yd2: read
                // them before they are overwritten (no other thread writes this stage's state).
@@ -593,22 +776,33 @@ __global__ void __launch_bounds__(W * 32, 16 / W) biquad_scan_kernel(BiquadLaunc
                sp[a.varPitch] = st.y;
             }
          }
-         if (FORM == DSPLIB_BIQUAD_DF1 && len == L && t0 + L == a.N - 1) { // next chunk holds one sample
+         if (FORM == DSPLIB_BIQUAD_DF1 && active && len == L && t0 + L == a.N - 1) { // next chunk holds one sample
             sp[a.varPitch] = tail.x;
             sp[3 * a.varPitch] = tail.z;
          }
          phase++;
       }
+      // One stage: nothing else orders the last warp's write of the window's end state before the
+      // next window's read of it.
+      if (a.S == 1 && K == 1 && win0 + windowLen < a.N) __syncthreads();
       {
          float *yp = a.y + t0 * a.outPitch + ch;
-         if (len == L) {
+         if (!active) {}
+         else if (len == L) {
 #pragma unroll
-            for (int i = 0; i < L; i++) yp[i * a.outPitch] = v[i];
+            for (int i = 0; i < L / 2; i++) {
+               const float2 o = up(v[i]);
+               yp[(long long) i * outPitch] = o.x;
+               yp[(long long) (i + L / 2) * outPitch] = o.y;
+            }
          }
          else {
 #pragma unroll
-            for (int i = 0; i < L; i++)
-               if (i < len) yp[i * a.outPitch] = v[i];
+            for (int i = 0; i < L / 2; i++) {
+               const float2 o = up(v[i]);
+               if (i < len) yp[(long long) i * outPitch] = o.x;
+               if (i + L / 2 < len) yp[(long long) (i + L / 2) * outPitch] = o.y;
+            }
          }
       }
    }
@@ -635,6 +829,9 @@ constexpr int kChWindow = kChThreads * kChL;
 constexpr int kChPowers = 10; // M^(2^k), k = 0..9: M^512 spans a window
 constexpr int kChanKernelMaxChannels = 16;
 constexpr int kChanTuneMaxChannels = 128; // the autotuner may pick the per-channel kernel up to here
+constexpr int kTuneHalfRows = 32;         // ... for 8 warps of two half rows of 16 channels, short chunks
+constexpr int kTuneHalfRowsLong = 33;     // ... the same, long chunks
+constexpr int kTuneLongChunk = 64;        // ... and for 8 warps of 64-sample chunks (in place of the warps)
 constexpr int kTuneChanKernel = 1;        // the autotuner's choice value for the per-channel kernel
 
 size_t chanSmemBytes(int S) { return (size_t) S * (kChPowers * sizeof(M2) + sizeof(double2) + 5 * sizeof(float)); }
@@ -784,16 +981,15 @@ template <int FORM> __global__ void __launch_bounds__(kChThreads, 1) biquad_chan
 }
 
 // Largest power-of-two cluster <= want that can be resident (<= 8 portable, 16 opt-in).
-template <int FORM, int W> int pickCluster(int want, size_t smemBytes)
+template <int FORM, int W, int L> int pickCluster(int want, size_t smemBytes)
 {
    static int cached[17] = {0};
-   if (want > W) want = W;
    if (want > kMaxCluster) want = kMaxCluster;
    int K = 1;
    while (K * 2 <= want) K *= 2;
    if (K <= 1) return 1;
    if (cached[K]) return cached[K];
-   auto fn = biquad_scan_kernel<FORM, W, true>;
+   auto fn = biquad_scan_kernel<FORM, W, L, 1, true>;
    int chosen = 1;
    for (int k = K; k >= 2; k >>= 1) {
       if (k > 8 && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
@@ -822,29 +1018,30 @@ template <int FORM, int W> int pickCluster(int want, size_t smemBytes)
    return chosen;
 }
 
-template <int FORM, int W> cudaError_t launchScanShape(const BiquadLaunch &a, int want, cudaStream_t s)
+template <int FORM, int W, int L, int SUB = 1> cudaError_t launchScanShape(const BiquadLaunch &a, int want, cudaStream_t s)
 {
-   const ScanSmem lay = scanLayout<W>(a.S);
-   const int groups = (a.C + 31) / 32;
+   const ScanSmem lay = scanLayout<W, SUB>(a.S);
+   const int groups = (a.C + 32 / SUB - 1) / (32 / SUB);
    dim3 block(W * 32);
    cudaError_t e;
-   auto fn1 = biquad_scan_kernel<FORM, W, false>;
-   auto fnK = biquad_scan_kernel<FORM, W, true>;
+   auto fn1 = biquad_scan_kernel<FORM, W, L, SUB, false>;
+   auto fnK = biquad_scan_kernel<FORM, W, L, 1, true>;
    // the largest footprint this launch can take (tables + next-window buffer)
-   const size_t maxBytes = lay.total + (a.prefetch ? (size_t) kScanL * W * 32 * sizeof(float) : 0) +
+   const size_t maxBytes = lay.total + (a.prefetch ? (size_t) L * W * 32 * sizeof(float) : 0) +
                            (size_t) 2 * kMaxCluster * 32 * sizeof(float2);
    static bool attrSet = false;
    static size_t attrBytes = 0;
    if (!attrSet || attrBytes < maxBytes) {
       if ((e = cudaFuncSetAttribute(fn1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) maxBytes)) != cudaSuccess)
          return e;
-      if ((e = cudaFuncSetAttribute(fnK, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) maxBytes)) != cudaSuccess)
+      if (SUB == 1 &&
+          (e = cudaFuncSetAttribute(fnK, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) maxBytes)) != cudaSuccess)
          return e;
       attrSet = true;
       attrBytes = maxBytes;
    }
-   const int K = want > 1 ? pickCluster<FORM, W>(want, maxBytes) : 1;
-   const size_t bytes = scanSmemBytes<W>(a, K);
+   const int K = SUB == 1 && want > 1 ? pickCluster<FORM, W, L>(want, maxBytes) : 1;
+   const size_t bytes = scanSmemBytes<W, L, SUB>(a, K);
    dim3 grid(K, groups);
    if (K == 1) {
       fn1<<<grid, block, bytes, s>>>(a);
@@ -882,30 +1079,49 @@ template <int FORM> cudaError_t launchChanForm(const BiquadLaunch &a, cudaStream
    return cudaGetLastError();
 }
 
-// Shape choice, from timings of 1 .. 4096 channels x 8192 samples x 4 stages on B200:
+// Shape choice, from timings of 20 .. 4096 channels x 300 .. 20011 samples, 2 .. 7 stages, on
+// B200 (us, DF2 with 4 stages unless said otherwise):
 //  * up to 16 channels, lane = channel leaves most lanes idle: one CTA per channel
 //    scanning along time;
-//  * otherwise 32 channels per CTA (W = 16 warps: one CTA per SM at 128 registers),
-//    and time split over a cluster of K CTAs: the largest power of two <= 16 that keeps
-//    groups x K <= 128 CTAs resident in one wave; clusters of 16 are only taken while at
-//    most 7 of them are needed (no more are co-resident).  Fewer windows per CTA beat
-//    more CTAs once a second wave would be needed.
-// The autotuner's choice, where it has one for this problem class, replaces the rule:
-// 8 or 16 warps per CTA (windows of 256 or 512 samples) and up to 16 CTAs per cluster.
+//  * below 2048 samples, half rows of 16 channels: twice the CTAs, without the cluster barriers
+//    that would pay only from four windows on (512 channels x 300: 8.4 against 10.5; x 1024: 10.5
+//    against 12.5 in clusters of two; 203 x 1500: 18.6 against 24.9);
+//  * DF2 and TIF: 64-sample chunks in clusters, the largest power of two that its windows fill:
+//    16 for up to 7 groups of 32 channels (no more are co-resident), 8 or fewer with at most
+//    384 CTAs, two an SM (32 x 8192: 12.5 against 14.6 in 32-sample chunks; 1024 x 8192: 36
+//    against 70; TIF, 7 stages, 203 x 20011: 64 against 70); above 96 groups half rows, whose
+//    CTAs' loads, stores and barriers pass under each other's arithmetic (4096 x 8192: 99
+//    against 113 in clusters of two, 119 in one CTA of 16 warps a group);
+//  * DF1 and TDF2, whose packed long chunks spill registers: 32-sample chunks in clusters of at
+//    most 112 CTAs of 16 warps, one an SM (TDF2, 5 stages, 32 x 8192: 17.3 against 18.6), long
+//    chunks where these give a group more CTAs (DF1, 2 stages, 1024 x 8192: 30 against 45 in half
+//    rows), half rows above 32 groups (DF1, 4096 x 8192: 80 against 93).
+// The autotuner's choice, where it has one for this problem class, replaces the rule.
 template <int FORM> cudaError_t launchScanForm(const BiquadLaunch &a, cudaStream_t s)
 {
    if (a.C <= kChanKernelMaxChannels || a.tuneChoice == kTuneChanKernel) return launchChanForm<FORM>(a, s);
    if (a.tuneChoice > 0) {
       const int W = a.tuneChoice / 100, K = a.tuneChoice % 100;
-      if (W == 8 && K >= 1) return launchScanShape<FORM, 8>(a, K, s);
-      if (W == 16 && K >= 1) return launchScanShape<FORM, 16>(a, K, s);
+      if (W == 8 && K >= 1) return launchScanShape<FORM, 8, kShortChunk>(a, K, s);
+      if (W == 16 && K >= 1) return launchScanShape<FORM, 16, kShortChunk>(a, K, s);
+      if (W == kTuneHalfRows) return launchScanShape<FORM, 8, kShortChunk, 2>(a, 1, s);
+      if (W == kTuneHalfRowsLong) return launchScanShape<FORM, 8, kLongChunk, 2>(a, 1, s);
+      if (W == kTuneLongChunk && K >= 1) return launchScanShape<FORM, 8, kLongChunk>(a, K, s);
    }
    const int groups = (a.C + 31) / 32;
-   const long long chunks = (a.N + kScanL - 1) / kScanL;
-   int K = 1;
-   while (K < 16 && (long long) K * 2 * 16 <= chunks && groups * K * 2 <= 128 && !(K * 2 == 16 && groups > 7))
-      K *= 2;
-   return launchScanShape<FORM, 16>(a, K, s);
+   constexpr bool packed = FORM == DSPLIB_BIQUAD_DF2 || FORM == DSPLIB_BIQUAD_TIF;
+   const int windows = a.N / 512;
+   if (windows < 4) return launchScanShape<FORM, 8, kShortChunk, 2>(a, 1, s);
+   int K = 1, KL = 1;
+   while (K < 16 && K * 2 <= windows && groups * K * 2 <= 112) K *= 2;
+   while (KL < 8 && KL * 2 <= windows && groups * KL * 2 <= (packed ? 384 : 256)) KL *= 2;
+   if (packed) {
+      if (groups > 96) return launchScanShape<FORM, 8, kLongChunk, 2>(a, 1, s);
+      return launchScanShape<FORM, 8, kLongChunk>(a, K > KL ? K : KL, s);
+   }
+   if (groups > 32) return launchScanShape<FORM, 8, kShortChunk, 2>(a, 1, s);
+   if (KL > K) return launchScanShape<FORM, 8, kLongChunk>(a, KL, s);
+   return launchScanShape<FORM, 16, kShortChunk>(a, K, s);
 }
 
 template <int FORM> cudaError_t launchSeqForm(const BiquadLaunch &a, cudaStream_t s)
@@ -949,10 +1165,14 @@ std::vector<int> biquadTuneCandidates(const BiquadLaunch &a)
    if (biquadTuneKey(a).empty()) return c;
    // a few dozen channels: one CTA per channel along time (more SMs than one cluster) is a candidate
    if (a.C <= kChanTuneMaxChannels) c.push_back(kTuneChanKernel);
-   const long long chunks = (a.N + kScanL - 1) / kScanL;
+   const long long chunks = (a.N + kShortChunk - 1) / kShortChunk;
    for (int W : {8, 16})
       for (int K = 1; K <= (W < kMaxCluster ? W : kMaxCluster); K *= 2)
          if (K == 1 || (long long) K * W <= chunks) c.push_back(100 * W + K);
+   c.push_back(100 * kTuneHalfRows + 1);
+   c.push_back(100 * kTuneHalfRowsLong + 1);
+   for (int K = 1; K <= kMaxCluster; K *= 2) // long chunks: windows of 512 samples, as 16 warps of short ones
+      if (K == 1 || (long long) K * 16 <= chunks) c.push_back(100 * kTuneLongChunk + K);
    return c;
 }
 

@@ -94,5 +94,11 @@ __device__ __forceinline__ P2 mul2(P2 a, P2 b)
    return r;
 }
 
+__device__ __forceinline__ P2 add2(P2 a, P2 b)
+{
+   P2 r;
+   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+   return r;
+}
 } // namespace scan
 } // namespace dsplib

@@ -86,6 +86,37 @@ def test_biquad_scan_every_candidate(table, form):
             check_accuracy(st, st32, s64, f"final state, form {form} choice {c}")
 
 
+@pytest.mark.parametrize("form", [D.DF1, D.DF2, D.TDF2, D.TIF])
+@pytest.mark.parametrize("choice", [801, 1601, 1602, 3201, 3301, 6401, 6402])
+def test_biquad_scan_shape_edges(table, form, choice):
+    """Every shape of the scan at lengths around half a chunk, a chunk, a window and a cluster's
+    windows, channel counts around half a row and a row, from a random state (TIF, whose state
+    is in its own coordinates, from zero): outputs and final states."""
+    from test_biquad_gpu import check_accuracy, nv, oracle_run, stable_sections
+
+    rng = np.random.default_rng(60 + form)
+    S = 3
+    for C, N in ((17, 1), (33, 2), (47, 16), (37, 17), (48, 18), (31, 32), (37, 33), (20, 34), (40, 63), (37, 65),
+                 (33, 97), (37, 255), (37, 257), (49, 511), (37, 513), (65, 1024), (37, 1041), (19, 1057), (37, 2081)):
+        nch = N % 2
+        x = rng.standard_normal((N, C)).astype(np.float32)
+        nat = stable_sections(rng, C if nch else 1, S)
+        st0 = (0.1 * rng.standard_normal((S * nv(form), C)) * (form != D.TIF)).astype(np.float32)
+        y32, st32, y64, s64 = oracle_run(form, x, nat, st0.copy(), nch)
+        opt, _ = D.opt_coefficients(nat, form, nch, C)
+        hd = D.BiquadHandle()
+        st = st0.copy()
+        D.cascade_biquad(x, opt, st, form=form, nch=nch, handle=hd)
+        key, _ = hd.tune_key()
+        assert table.DSPLIB_gpu_autotuneStore(key.encode(), choice) == 0
+        st = torch.from_numpy(st0.copy()).cuda()
+        xd = torch.from_numpy(x).cuda()
+        y = D.cascade_biquad(xd, torch.from_numpy(opt).cuda(), st, form=form, nch=nch, handle=hd).cpu().numpy()
+        check_accuracy(y, y32, y64, f"form {form} choice {choice} C {C} N {N}")
+        if form != D.TIF:
+            check_accuracy(st.cpu().numpy(), st32, s64, f"state, form {form} choice {choice} C {C} N {N}")
+
+
 def test_bank_run_length_every_candidate(table):
     from c7x_dsplib_b200.filterbank import RaggedFilterBank
 
