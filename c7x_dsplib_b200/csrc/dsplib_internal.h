@@ -235,7 +235,7 @@ struct FirLaunch {
    long long filtPitch; // elements between tap rows, 0 = shared
    int shift;
    int *err = nullptr; // tensor-core kernels: error word for an expired bounded wait
-   int tuneTpc = 0;    // tensor-core kernels: output tiles per CTA (0: the built-in rule)
+   int tuneTpc = 0;    // tensor-core kernels: output tiles per run (0: the built-in rule)
    int tunePerSm = 0;  // int8/int16 tensor-core kernel: resident CTAs per SM (0: the built-in rule)
 };
 

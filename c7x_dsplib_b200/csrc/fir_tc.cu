@@ -8,9 +8,10 @@
 // The Hankel matrix A is never expanded: the shared-memory descriptors make
 // consecutive rows overlap inside the raw signal segment.
 //
-// int8/int16 (kind::i8, P = 16, N = 16, tile 2048): an 8-bit core-matrix row
-//   is 16 bytes = 16 samples, so the no-swizzle K-major descriptor with
-//   LBO = 16 B and SBO = 128 B reads row a at byte 16a of the segment.
+// int8/int16 (kind::i8, P = N = 16 or 32, tile 2048 or 4096): an 8-bit core-matrix row
+//   is 16 bytes = 16 samples, so with P = 16 the no-swizzle K-major descriptor with
+//   LBO = 16 B and SBO = 128 B reads row a at byte 16a of the segment; with P = 32 the
+//   segment's even and odd 16-byte chunks lie in two parts, LBO apart.
 //   int8: one s8 x s8 product.  int16: x = 256*xh + xl, g = 256*gh + gl (xh, gh
 //   signed bytes, xl, gl unsigned); y = 65536*hh + 256*(hl + lh) + ll, each an
 //   exact int32 kind::i8 accumulation recombined exactly in 64 bits; modulo
@@ -31,9 +32,9 @@
 //   fourth rides in the same MMA (N = 128 instead of 64 for the lo plane) at no
 //   measurable cost here (the tile loop is not MMA-bound) and brings it to 8.7e-6.
 //
-// All kernels are persistent: one wave of CTAs strides over runs of consecutive tiles of one
-// channel.  The integer kernel keeps a band of shared taps for all of a CTA's runs
-// and fetches each run's first segment during the previous run's last tile.
+// All kernels are persistent: one wave of CTAs strides over runs of consecutive tiles.  The
+// integer kernel keeps a band of shared taps for all of a CTA's tiles and fetches each tile's
+// segment during the one before.
 // All waits on the tensor core are bounded; on expiry the kernel sets the error word it
 // was given (the calling handle's or plan's), frees its TMEM and exits.
 #include <algorithm>
@@ -61,24 +62,35 @@ constexpr int kRows = 128;
 
 // ------------------------------------------------------------------ integer
 
-constexpr int kPhases = 16;
-constexpr int kTile = kRows * kPhases;
 constexpr int kThreads = 128;
 constexpr int kMaxTapsTc = 2048;
+constexpr int kIntTuneTile = 2048; // outputs a tile counts as in the autotuner's keys
 
-__host__ __device__ inline int bandK(int T) { return ((T + 15 + 31) / 32) * 32; }
-
-template <typename T> struct IntLimits;
-template <> struct IntLimits<int8_t> { static constexpr long long lo = -128, hi = 127; };
-template <> struct IntLimits<int16_t> { static constexpr long long lo = -32768, hi = 32767; };
-
-// int8: |acc| <= 2048 * 2^14 fits 32 bits, so the output stage stays in 32-bit arithmetic.
-template <int QMODE> __device__ __forceinline__ int8_t outStage8(int acc, int shift)
-{
-   if (!QMODE) return (int8_t) acc; // modulo 2^8
-   if (shift > 0) acc = (acc + (1 << (shift - 1))) >> shift;
-   return (int8_t) max(-128, min(127, acc));
-}
+// Sizes of a form with P outputs a row (16 or 32), for T taps and the longest lead.
+template <typename T, int P> struct IntShape {
+   static constexpr int tile = kRows * P;
+   static constexpr int planes = sizeof(T);              // byte planes of a sample
+   static constexpr int per = 16 / (int) sizeof(T);      // samples a 16-byte vector
+   static constexpr int align = P * sizeof(T) >= 32 ? 32 / (int) sizeof(T) : 16; // outputs a row starts at a multiple of
+   static constexpr int cols(bool q) { return planes == 1 ? P : (q ? 3 : 2) * P; } // accumulator columns
+   static constexpr uint32_t tmemCols(bool q) { return cols(q) <= 32 ? 32 : cols(q) <= 64 ? 64 : 128; }
+   static constexpr int perSm(bool q) { return planes == 1 ? 8 : tmemCols(q) == 128 ? 4 : 6; } // CTAs an SM
+   static constexpr int pre = (tile + kMaxTapsTc + 64) * (int) sizeof(T) / 16 / kThreads + 1; // vectors a thread
+   __host__ __device__ static int K(int taps) { return ((P - 1 + taps + per - 1 + 31) / 32) * 32; }
+   __host__ __device__ static int seg(int taps) { return tile - P + K(taps); }
+   // Chunk c (16 samples) of the segment is chunk c / (P / 16) of part c % (P / 16): with P = 16
+   // bytes a row the rows of a core matrix follow one another; a longer row is read as P / 16
+   // such parts.  The padding spreads the parts over the banks.
+   __host__ __device__ static int part(int taps)
+   {
+      const int n = P / 16, chunks = (seg(taps) / 16 + n - 1) / n;
+      return n == 1 ? chunks * 16 : ((chunks * 16 + 63) / 128) * 128 + 64;
+   }
+   __host__ __device__ static int plane(int taps) { return P / 16 * part(taps); }
+   __host__ __device__ static int taps(int t) { return (K(t) + P + 4 + 15) / 16 * 16; }    // bytes of gb, one plane
+   __host__ __device__ static int band(int t) { return (K(t) - 16 + P) * 16; }             // bytes, one plane
+   __host__ __device__ static size_t smem(int t) { return 16 + (size_t) planes * (taps(t) + band(t) + 2 * plane(t)); }
+};
 
 // Four int8 Q-mode outputs (round half up, shift, saturate) packed into one word, byte k =
 // output k: two saturating pack conversions instead of a clamp per output and byte moves.
@@ -110,185 +122,160 @@ __device__ __forceinline__ uint32_t outStage16x2(long long v0, long long v1, int
    return d;
 }
 
-template <typename T, int QMODE>
-__device__ __forceinline__ T outStage(long long acc, int shift)
+__device__ __forceinline__ void cpAsync16(void *dst, const void *src)
 {
-   if (!QMODE) return (T) acc; // modulo 2^bits
-   if (shift > 0) acc = (acc + (1LL << (shift - 1))) >> shift;
-   if (acc < IntLimits<T>::lo) acc = IntLimits<T>::lo;
-   if (acc > IntLimits<T>::hi) acc = IntLimits<T>::hi;
-   return (T) acc;
+   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc::smemAddr(dst)), "l"(src) : "memory");
 }
 
-// One 16-byte vector (16 / sizeof(T) samples) of the segment starting at xs, the
-// samples at or beyond `avail` read as zero: whole vectors load as one access, the one
-// vector that straddles the row end element by element.
-template <typename T> __device__ __forceinline__ int4 loadSegVec(const T *xs, long long k, long long avail)
+__device__ __forceinline__ void cpAsyncWaitAll() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Store 32 bytes to a 32-byte aligned address as one access.
+__device__ __forceinline__ void store32(void *p, const uint32_t *w)
 {
-   constexpr int per = 16 / sizeof(T);
-   const long long s0 = k * per;
-   if (s0 + per <= avail) return ((const int4 *) xs)[k];
-   __align__(16) T tmp[per];
-#pragma unroll
-   for (int e = 0; e < per; e++) tmp[e] = (s0 + e < avail) ? xs[s0 + e] : (T) 0;
-   return *(const int4 *) tmp;
+   asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+                "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                : "memory");
 }
 
-// Write one 16-byte vector of samples into the byte plane(s): int8 -> A0; int16 ->
-// A0 = high (signed) bytes, A1 = low (unsigned) bytes.
-template <typename T>
-__device__ __forceinline__ void putSegVec(const int4 &v, int k, unsigned char *A0, unsigned char *A1)
+// Integer FIR.  Integer sums do not depend on how they are grouped, so a channel's tile grid is
+// laid to suit its rows: a row of P outputs starts on a 16- or 32-byte boundary of y (`shift`
+// outputs before the channel's first one, never stored), and the input window of a tile starts
+// `lead` samples before its first output's, on a 16-byte boundary, with as many zero taps in
+// front.  Every load and store is then a whole aligned vector but those at a channel's ends, and
+// a row goes from its TMEM lane to memory through one thread's registers.
+//
+// Runs are equal shares of all tiles of all channels in turn, one for each resident CTA, so
+// no SM waits for another's last channel (runs of whole or half channels: 3.4 waves of 888
+// CTAs on 1000 channels).  A tile is a chain of fetch, barrier, MMAs, drain of some 4000 clk,
+// hidden by the 4 to 8 CTAs of an SM; the MMAs take a third of the shared memory's rate and
+// instructions 60 % of the issue slots (4096 x 16384 int8, 128 taps).  An earlier form with
+// tiles of 2048 from each channel's first sample on read rows off the 16-byte boundary sample by
+// sample, and assembled the output vectors through shared memory with funnel shifts: 4096
+// channels x 16384 int8 samples x 128 taps 63.5 us, now 41.8 (20.5 at the copy rate); 1000
+// channels x 10007 int16 samples x 201 taps 85.4, now 25.8; 4096 x 16384 int16 111, now 91,
+// in Q mode 171, now 118.
+template <typename T> struct IntRow {
+   const T *x;
+   T *y;
+   int l, shift, lead;
+};
+
+// Tiles of a channel, with the largest shift any channel needs.
+template <typename T, int P> __host__ __device__ inline int intTiles(const FirLaunch &a)
 {
-   if (sizeof(T) == 1) {
-      ((int4 *) A0)[k] = v;
-   }
-   else {
-      const int16_t *e = (const int16_t *) &v;
-      __align__(8) unsigned char hb[8], lb[8];
-#pragma unroll
-      for (int i = 0; i < 8; i++) {
-         hb[i] = (unsigned char) (e[i] >> 8);
-         lb[i] = (unsigned char) (e[i] & 0xFF);
-      }
-      ((uint2 *) A0)[k] = *(uint2 *) hb;
-      ((uint2 *) A1)[k] = *(uint2 *) lb;
-   }
+   constexpr int al = IntShape<T, P>::align;
+   const bool aligned = ((uintptr_t) a.y & (al * sizeof(T) - 1)) == 0 && a.outPitch % al == 0;
+   return (int) (((long long) a.outSize + (aligned ? 0 : al - 1) + kRows * P - 1) / (kRows * P));
 }
 
-// Stage seg samples of xs (row positions j0 .. j0 + seg - 1, zero from inExtent on) into
-// the byte plane(s).  16-byte vectors when xs is aligned, samples otherwise.
-template <typename T>
-__device__ __forceinline__ void intStage(const T *xs, long long j0, long long inExtent, int seg, unsigned char *A0,
-                                         unsigned char *A1, int tid)
+template <typename T, int QMODE, int P>
+__global__ void __launch_bounds__(kThreads, IntShape<T, P>::perSm(QMODE)) fir_int_tc_kernel(FirLaunch a, uint32_t tilesPerRun)
 {
+   using Sh = IntShape<T, P>;
    constexpr bool SPLIT = sizeof(T) == 2;
-   constexpr int per = 16 / sizeof(T); // samples per 16-byte vector
-   const long long avail = inExtent - j0;
-   if ((((uintptr_t) xs) & 15) == 0) {
-      for (int k = tid; k < seg / per; k += kThreads) putSegVec<T>(loadSegVec<T>(xs, k, avail), k, A0, A1);
-   }
-   else {
-      for (int k = tid; k < seg; k += kThreads) {
-         const int v = (k < avail) ? (int) xs[k] : 0;
-         if (SPLIT) {
-            A0[k] = (unsigned char) (v >> 8);
-            A1[k] = (unsigned char) (v & 0xFF);
-         }
-         else {
-            A0[k] = (unsigned char) v;
-         }
-      }
-   }
-}
-
-// Write n consecutive outputs dst[0..n) of one tile from shared memory, where
-// the tile's 16-byte chunk ci (bytes 16ci .. 16ci+15 of the output run) sits at
-// byte offset cpos(ci) of stage.  The accumulator drain leaves one output row
-// per lane, so storing straight from registers would make every lane of a warp
-// hit a different row (one memory transaction per lane and instruction); from
-// shared memory a warp writes contiguous 16-byte vectors instead.  The vectors
-// are aligned to the destination: when dst is not 16-byte aligned (row pitches
-// such as N - T + 1 elements), each vector is assembled from two stage chunks
-// with a funnel shift, and a head and tail of scalar stores cover the ends.
-template <typename T, typename ChunkPos>
-__device__ __forceinline__ void storeTile(T *dst, int n, const unsigned char *stage, ChunkPos cpos, int tid,
-                                          int nthreads)
-{
-   auto elem = [&](int k) {
-      const int byte = k * (int) sizeof(T);
-      return *(const T *) (stage + cpos(byte >> 4) + (byte & 15));
-   };
-   const int hb = (16 - (int) ((uintptr_t) dst & 15)) & 15; // bytes before the first 16-byte boundary
-   const int head = min(n, hb / (int) sizeof(T));
-   const int nvec = (n - head) * (int) sizeof(T) / 16;
-   if (tid < head) dst[tid] = elem(tid);
-   const int q = hb >> 2, r = (hb & 3) * 8;
-   unsigned char *dv = (unsigned char *) dst + hb;
-   for (int v = tid; v < nvec; v += nthreads) {
-      const uint4 a = *(const uint4 *) (stage + cpos(v));
-      uint4 o = a;
-      if (hb) {
-         const uint4 b = *(const uint4 *) (stage + cpos(v + 1));
-         uint32_t w0, w1, w2, w3, w4;
-         switch (q) { // uniform across the CTA
-         case 0: w0 = a.x, w1 = a.y, w2 = a.z, w3 = a.w, w4 = b.x; break;
-         case 1: w0 = a.y, w1 = a.z, w2 = a.w, w3 = b.x, w4 = b.y; break;
-         case 2: w0 = a.z, w1 = a.w, w2 = b.x, w3 = b.y, w4 = b.z; break;
-         default: w0 = a.w, w1 = b.x, w2 = b.y, w3 = b.z, w4 = b.w; break;
-         }
-         o.x = __funnelshift_r(w0, w1, r);
-         o.y = __funnelshift_r(w1, w2, r);
-         o.z = __funnelshift_r(w2, w3, r);
-         o.w = __funnelshift_r(w3, w4, r);
-      }
-      *(uint4 *) (dv + 16 * v) = o;
-   }
-   for (int k = head + nvec * (16 / (int) sizeof(T)) + tid; k < n; k += nthreads) dst[k] = elem(k);
-}
-
-template <typename T, int QMODE>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 6 : 8) fir_int_tc_kernel(FirLaunch a, int tilesPerCta)
-{
-   constexpr bool SPLIT = sizeof(T) == 2;
-   constexpr uint32_t kCols = SPLIT ? 64 : 32; // TMEM columns (accumulators of 16 columns each)
+   constexpr int per = Sh::per, kTile = Sh::tile, kParts = P / 16;
    const int T_ = a.T;
-   const int Kt = bandK(T_);
-   const int seg = kTile + Kt;            // samples one tile reads (multiple of 32)
-   const int nplane = SPLIT ? 2 : 1;
+   const int Kt = Sh::K(T_), seg = Sh::seg(T_), part = Sh::part(T_), planeBytes = Sh::plane(T_);
    extern __shared__ __align__(128) unsigned char sm[];
    uint64_t *mbar = (uint64_t *) sm;
    uint32_t *tslot = (uint32_t *) (sm + 8);
-   // Reversed taps g[c] = h[T-1-c] as bytes (int16: high and low byte planes) at
-   // byte 16 + c of gb0 / gb1, zero elsewhere: one 32-bit word per thread to build.
-   const int gbWords = (Kt + 20) / 4;
+   // Reversed taps g[c] = h[T-1-c] as bytes (int16: high and low byte planes) at byte
+   // P - 1 + lead + c of gb0 / gb1, zero elsewhere: one 32-bit word per thread to build.
    uint32_t *gb0 = (uint32_t *) (sm + 16);
-   uint32_t *gb1 = gb0 + gbWords;
-   unsigned char *B0 = sm + 16 + ((gbWords * 4 * nplane + 15) & ~15);
-   unsigned char *B1 = B0 + (size_t) Kt * 16;
-   unsigned char *Abase = B0 + (size_t) Kt * 16 * nplane;
-   // A[buf][plane]: seg bytes each
-   auto A = [&](int buf, int plane) { return Abase + (size_t) (buf * nplane + plane) * seg; };
-   T *ostage = (T *) (Abase + (size_t) 2 * nplane * seg); // one tile of outputs, row-major
+   uint32_t *gb1 = (uint32_t *) (sm + 16 + Sh::taps(T_));
+   unsigned char *B0 = sm + 16 + Sh::planes * Sh::taps(T_);
+   unsigned char *B1 = B0 + Sh::band(T_);
+   unsigned char *Abase = B0 + (size_t) Sh::planes * Sh::band(T_);
+   auto A = [&](int buf, int plane) { return Abase + (buf * Sh::planes + plane) * planeBytes; };
 
    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-   if (warp == 0) tc::tmemAlloc(tslot, kCols);
+   if (warp == 0) tc::tmemAlloc(tslot, Sh::tmemCols(QMODE));
    if (tid == 0) tc::mbarInit(mbar, 1);
    tc::fenceBeforeSync();
    __syncthreads();
    tc::fenceAfterSync();
    const uint32_t tmem = *tslot;
 
-   const int nt = (a.outSize + kTile - 1) / kTile;
-   const long long inExtent = (long long) a.outSize + T_ - 1;
-   // Work item = tiles [part * tilesPerCta, ...) of one channel; CTAs stride over the items
-   // (persistent: the taps band of shared taps is built once per CTA, and each item's first
-   // segment is fetched during the previous item's last tile).
-   const int nParts = (nt + tilesPerCta - 1) / tilesPerCta;
-   const long long nItems = (long long) a.batch * nParts;
+   const int inExtent = a.outSize + T_ - 1;
+   // Runs of tilesPerRun consecutive tiles (of all channels in turn); CTAs stride over the runs.
+   // The band is built anew when the channel's taps or its lead are others than the last tile's.
+   const uint32_t nt = (uint32_t) intTiles<T, P>(a);
+   const uint32_t nTiles = (uint32_t) a.batch * nt; // with the grid below 2^32: memory bounds it
+   auto rowOf = [&](int l) {
+      IntRow<T> r;
+      r.l = l;
+      r.x = (const T *) a.x + (long long) l * a.inPitch;
+      r.y = (T *) a.y + (long long) l * a.outPitch;
+      r.shift = (int) ((uintptr_t) r.y / sizeof(T)) & (Sh::align - 1);
+      r.lead = (int) (((uintptr_t) r.x / sizeof(T)) - r.shift) & (per - 1);
+      return r;
+   };
+   // The segment of tile t as 16-byte vectors, samples outside the row zero: int8 straight into
+   // shared memory, int16 into registers (its byte planes are parted when the tile's turn comes).
+   constexpr int kPre = SPLIT ? Sh::pre : 1;
+   const int nvec = (seg + per - 1) / per;
+   int4 pre[kPre];
+   auto slot8 = [&](int buf, int k) { return (int4 *) (A(buf, 0) + (k % kParts) * part + (k / kParts) * 16); };
+   auto fetch = [&](const IntRow<T> &r, uint32_t t, int buf) {
+      const long long s0 = (long long) t * kTile - r.shift - r.lead;
+      const T *p = r.x + s0;
+      auto edge = [&](int k) {
+         const long long q = s0 + (long long) k * per;
+         if (q <= -per || q >= inExtent) return make_int4(0, 0, 0, 0);
+         __align__(16) T tmp[per];
+#pragma unroll
+         for (int e = 0; e < per; e++) tmp[e] = (q + e >= 0 && q + e < inExtent) ? p[k * per + e] : (T) 0;
+         return *(const int4 *) tmp;
+      };
+      // vectors [v0, v1) lie inside the row
+      const int v0 = s0 < 0 ? (int) ((-s0 + per - 1) / per) : 0;
+      const int v1 = (int) min((long long) nvec, (inExtent - s0) / per);
+      if (SPLIT) {
+#pragma unroll
+         for (int i = 0; i < kPre; i++) {
+            const int k = tid + i * kThreads;
+            if (k >= v0 && k < v1) pre[i] = ((const int4 *) p)[k];
+            else if (k < nvec) pre[i] = edge(k);
+         }
+      }
+      else {
+         for (int k = tid; k < nvec; k += kThreads) {
+            if (k >= v0 && k < v1) cpAsync16(slot8(buf, k), (const int4 *) p + k);
+            else *slot8(buf, k) = edge(k);
+         }
+      }
+   };
    uint32_t iter = 0;
-   bool failed = false;
-   int bandOf = -1; // channel whose taps the band holds
+   int bandOf = -1, bandLead = -1; // channel and lead of the taps the band holds
    int buf = 0;
-   long long item = blockIdx.x;
-   if (item < nItems) {
-      const int l = (int) (item / nParts), t0 = (int) (item % nParts) * tilesPerCta;
-      intStage<T>((const T *) a.x + (long long) l * a.inPitch + (long long) t0 * kTile, (long long) t0 * kTile,
-                  inExtent, seg, A(0, 0), A(0, 1), tid);
-   }
-   for (; item < nItems && !failed; item += gridDim.x) {
-      const int l = (int) (item / nParts);
-      const int t0 = (int) (item % nParts) * tilesPerCta;
-      const int t1 = min(nt, t0 + tilesPerCta);
-      const T *x = (const T *) a.x + (long long) l * a.inPitch;
-      T *y = (T *) a.y + (long long) l * a.outPitch;
-      if (bandOf < 0 || (a.filtPitch != 0 && bandOf != l)) {
-         const T *h = (const T *) a.h + (long long) l * a.filtPitch;
-         __syncthreads(); // the previous band's last MMAs are complete (waited) before it changes
-         for (int wd = tid; wd < gbWords; wd += kThreads) {
+   bool bad = false; // this thread's wait gave up
+   const uint32_t nRuns = (nTiles + tilesPerRun - 1) / tilesPerRun;
+   uint32_t run = blockIdx.x, tile = run * tilesPerRun;
+   bool more = run < nRuns;
+   IntRow<T> r = rowOf(more ? (int) (tile / nt) : 0);
+   uint32_t t = tile % nt, end = min(nTiles, tile + tilesPerRun);
+   if (more) fetch(r, t, 0);
+   while (more) {
+      if (SPLIT) {
+#pragma unroll
+         for (int i = 0; i < kPre; i++) {
+            const int k = tid + i * kThreads, c = k >> 1; // vector k = half of chunk c
+            const int o = (c % kParts) * part + (c / kParts) * 16 + (k & 1) * 8;
+            const int4 &v = pre[i];
+            if (k < nvec) {
+               *(uint2 *) (A(buf, 0) + o) = make_uint2(__byte_perm(v.x, v.y, 0x7531), __byte_perm(v.z, v.w, 0x7531));
+               *(uint2 *) (A(buf, 1) + o) = make_uint2(__byte_perm(v.x, v.y, 0x6420), __byte_perm(v.z, v.w, 0x6420));
+            }
+         }
+      }
+      if (bandOf < 0 || (a.filtPitch != 0 && bandOf != r.l) || bandLead != r.lead) {
+         const T *h = (const T *) a.h + (long long) r.l * a.filtPitch;
+         // the previous band's last MMAs are complete (waited); its words were read before that
+         for (int wd = tid; wd < Sh::taps(T_) / 4; wd += kThreads) {
             uint32_t w0 = 0, w1 = 0;
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-               const int c = 4 * wd + j - 16;
+               const int c = 4 * wd + j - (P - 1) - r.lead;
                const int g = (c >= 0 && c < T_) ? (int) h[T_ - 1 - c] : 0;
                if (SPLIT) {
                   w0 |= (uint32_t) ((g >> 8) & 0xFF) << (8 * j);
@@ -302,14 +289,14 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 6 : 8) fir_int_tc_k
             if (SPLIT) gb1[wd] = w1;
          }
          __syncthreads();
-         // Taps band, K-major no-swizzle: 16-byte chunk ch = 16q + 8i + r (byte 16 ch) holds
-         // B[m = 16q + e][b = 8i + r] = g[16q + e - 8i - r], e < 16: bytes gb[16 + 16q - 8i - r + e],
-         // gathered from five words with funnel shifts.
-         for (int ch = tid; ch < Kt; ch += kThreads) {
-            const int base = 16 + 16 * (ch >> 4) - 8 * ((ch >> 3) & 1) - (ch & 7);
-            const int w = base >> 2, sh = (base & 3) * 8;
+         // Taps band, K-major no-swizzle, phases in reverse (column n = phase P-1-n): element
+         // (m, n) = g[m + n - (P-1) - lead] = byte m + n of gb, so the 16-byte chunk of m = 16q,
+         // column n depends on 16q + n alone and is held once, at 16 (16q + n); gathered from
+         // five words with funnel shifts.
+         for (int ch = tid; ch < Kt - 16 + P; ch += kThreads) {
+            const int w = ch >> 2, sh = (ch & 3) * 8;
 #pragma unroll
-            for (int pl = 0; pl < (SPLIT ? 2 : 1); pl++) {
+            for (int pl = 0; pl < Sh::planes; pl++) {
                const uint32_t *gb = pl ? gb1 : gb0;
                const uint32_t v0 = gb[w], v1 = gb[w + 1], v2 = gb[w + 2], v3 = gb[w + 3], v4 = gb[w + 4];
                uint4 o;
@@ -320,176 +307,169 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 6 : 8) fir_int_tc_k
                *(uint4 *) ((pl ? B1 : B0) + 16 * ch) = o;
             }
          }
-         bandOf = l;
+         bandOf = r.l;
+         bandLead = r.lead;
       }
-      for (int t = t0; t < t1; t++) {
-         const long long j0 = (long long) t * kTile;
-         tc::fenceProxyAsync();
-         __syncthreads(); // segment[buf] and band written; previous accumulators drained
-         if (tid == 0) {
-            tc::fenceAfterSync();
-            const uint32_t a0 = tc::smemAddr(A(buf, 0)), a1 = tc::smemAddr(A(buf, 1));
-            const uint32_t b0 = tc::smemAddr(B0), b1 = tc::smemAddr(B1);
-            for (int kk = 0; kk < Kt / 32; kk++) {
-               const uint64_t dA0 = tc::descNoSwizzle(a0 + 32 * kk, 16, 128);
-               const uint64_t dB0 = tc::descNoSwizzle(b0 + 512 * kk, 256, 128);
-               if (!SPLIT) {
-                  tc::mmaI8(tmem, dA0, dB0, tc::idesc(2, 1, 1, kRows, kPhases), kk > 0);
-               }
-               else {
-                  const uint64_t dA1 = tc::descNoSwizzle(a1 + 32 * kk, 16, 128);
-                  const uint64_t dB1 = tc::descNoSwizzle(b1 + 512 * kk, 256, 128);
-                  if (QMODE) tc::mmaI8(tmem, dA0, dB0, tc::idesc(2, 1, 1, kRows, kPhases), kk > 0); // hi*hi
-                  tc::mmaI8(tmem + 16, dA0, dB1, tc::idesc(2, 1, 0, kRows, kPhases), kk > 0);       // hi*lo
-                  tc::mmaI8(tmem + 16, dA1, dB0, tc::idesc(2, 0, 1, kRows, kPhases), true);         // lo*hi
-                  tc::mmaI8(tmem + 32, dA1, dB1, tc::idesc(2, 0, 0, kRows, kPhases), kk > 0);       // lo*lo
-               }
-            }
-            tc::commit(mbar);
-         }
-         // Fetch the next segment (this item's next tile, or the next item's first) into
-         // registers now; it is written to shared memory after this tile's drain, so the
-         // load latency hides behind the MMAs and the drain.
-         constexpr int kPre = SPLIT ? 5 : 3; // 16-byte vectors per thread: (2048 + 2080) * sizeof(T) / 16 / 128
-         int4 pre[kPre];
-         const T *xn = nullptr;
-         long long jn = 0;
-         if (t + 1 < t1) {
-            xn = x;
-            jn = j0 + kTile;
-         }
-         else if (item + gridDim.x < nItems) {
-            const long long ni = item + gridDim.x;
-            xn = (const T *) a.x + (long long) (ni / nParts) * a.inPitch;
-            jn = (long long) (ni % nParts) * tilesPerCta * kTile;
-         }
-         const bool preVec = xn != nullptr && ((((uintptr_t) (xn + jn)) & 15) == 0);
-         const int nvec = seg * (int) sizeof(T) / 16;
-         if (preVec) {
-#pragma unroll
-            for (int i = 0; i < kPre; i++) {
-               const int k = tid + i * kThreads;
-               if (k < nvec) pre[i] = loadSegVec<T>(xn + jn, k, inExtent - jn);
-            }
-         }
-         const bool done = tc::mbarWait(mbar, iter & 1);
-         if (!done && tid == 0) raiseError(a.err);
-         failed = __syncthreads_or(!done) != 0;
-         iter++;
+      if (!SPLIT) cpAsyncWaitAll();
+      tc::fenceProxyAsync();
+      tc::fenceBeforeSync();
+      // segment[buf] and band written, previous accumulators drained by every warp; a wait that gave
+      // up ends all together
+      if (__syncthreads_or(bad)) break;
+      if (warp == 0 && tc::electOne()) {
          tc::fenceAfterSync();
-         if (!failed) {
-            // Drain: warp w owns TMEM lanes 32w..32w+31 = rows a; 16 consecutive outputs per row.
-            const uint32_t lanes = (uint32_t) (warp * 32) << 16;
-            uint32_t acc[3][16];
-            tc::tmemLoad16(tmem + lanes, acc[0]);
-            if (SPLIT) {
-               tc::tmemLoad16(tmem + lanes + 16, acc[1]);
-               tc::tmemLoad16(tmem + lanes + 32, acc[2]);
+         constexpr uint32_t al = kParts == 1 ? 16 : 0;
+         const uint32_t lbo = al ? al : (uint32_t) part;
+         const uint64_t dA0 = tc::descNoSwizzle(tc::smemAddr(A(buf, 0)), lbo, 128);
+         const uint64_t dA1 = tc::descNoSwizzle(tc::smemAddr(A(buf, 1)), lbo, 128);
+         uint64_t dB0 = tc::descNoSwizzle(tc::smemAddr(B0), 256, 128), dB1 = tc::descNoSwizzle(tc::smemAddr(B1), 256, 128);
+         // 32 taps a step: two chunks of the segment, 512 bytes of the band (descriptor addresses count 16)
+         for (int kk = 0; kk < Kt / 32; kk++, dB0 += 32, dB1 += 32) {
+            const uint32_t off = (2 * kk % kParts) * (part / 16) + 2 * kk / kParts;
+            if (!SPLIT) tc::mmaI8(tmem, dA0 + off, dB0, tc::idesc(2, 1, 1, kRows, P), kk > 0);
+            else {
+               tc::mmaI8(tmem, dA0 + off, dB1, tc::idesc(2, 1, 0, kRows, P), kk > 0);     // hi*lo
+               tc::mmaI8(tmem, dA1 + off, dB0, tc::idesc(2, 0, 1, kRows, P), true);       // lo*hi
+               tc::mmaI8(tmem + P, dA1 + off, dB1, tc::idesc(2, 0, 0, kRows, P), kk > 0); // lo*lo
+               if (QMODE) tc::mmaI8(tmem + 2 * P, dA0 + off, dB0, tc::idesc(2, 1, 1, kRows, P), kk > 0); // hi*hi
             }
-            tc::tmemWaitLoad();
-            const int row = warp * 32 + lane;
-            __align__(16) T out[16];
-            if (SPLIT && QMODE) {
-               uint32_t w[8];
+         }
+         tc::commit(mbar);
+      }
+      __syncwarp();
+      // fetch the next tile's segment now; int16 samples are written to shared memory after this
+      // tile's drain
+      const IntRow<T> cur = r;
+      const uint32_t tNow = t;
+      if (++tile == end) {
+         run += gridDim.x;
+         more = run < nRuns;
+         if (more) {
+            tile = run * tilesPerRun;
+            end = min(nTiles, tile + tilesPerRun);
+            r = rowOf((int) (tile / nt));
+            t = tile % nt;
+         }
+      }
+      else if (++t == nt) {
+         r = rowOf(r.l + 1);
+         t = 0;
+      }
+      if (more) fetch(r, t, buf ^ 1);
+      if (!tc::mbarWait(mbar, iter & 1)) {
+         bad = true;
+         raiseError(a.err);
+      }
+      iter++;
+      buf ^= 1;
+      tc::fenceAfterSync();
+      if (!bad) {
+         // Drain: warp w owns TMEM lanes 32w..32w+31 = rows; P consecutive outputs a row, columns reversed.
+         const uint32_t lanes = tmem + ((uint32_t) (warp * 32) << 16);
+         const long long j0 = (long long) tNow * kTile - cur.shift + (warp * 32 + lane) * P;
+         constexpr int kPiece = Sh::align; // outputs a store
+         constexpr int kGroups = kPiece / 16;
+         constexpr int kWords = kPiece * (int) sizeof(T) / 4;
 #pragma unroll
-               for (int b = 0; b < 16; b += 2) {
-                  const long long v0 = ((long long) (int) acc[0][b] << 16) + ((long long) (int) acc[1][b] << 8) +
-                                       (long long) (int) acc[2][b];
-                  const long long v1 = ((long long) (int) acc[0][b + 1] << 16) +
-                                       ((long long) (int) acc[1][b + 1] << 8) + (long long) (int) acc[2][b + 1];
-                  w[b / 2] = outStage16x2(v0, v1, a.shift);
+         for (int h = 0; h < P / kPiece; h++) {
+            __align__(16) uint32_t w[kWords];
+#pragma unroll
+            for (int g = 0; g < kGroups; g++) {
+               const int col = P - 16 - kPiece * h - 16 * g;
+               uint32_t acc[3][16];
+               tc::tmemLoad16(lanes + col, acc[0]);
+               if (SPLIT) tc::tmemLoad16(lanes + P + col, acc[1]);
+               if (SPLIT && QMODE) tc::tmemLoad16(lanes + 2 * P + col, acc[2]);
+               tc::tmemWaitLoad();
+#pragma unroll
+               for (int b = 0; b < 16; b += 4) { // outputs b..b+3 = columns 15-b..12-b
+                  const int c = 15 - b;
+                  uint32_t *d = w + (16 * g + b) * (int) sizeof(T) / 4;
+                  if (SPLIT && QMODE) {
+#pragma unroll
+                     for (int e = 0; e < 4; e += 2) {
+                        auto sum = [&](int k) {
+                           return ((long long) (int) acc[2][k] << 16) + ((long long) (int) acc[0][k] << 8) +
+                                  (long long) (int) acc[1][k];
+                        };
+                        d[e / 2] = outStage16x2(sum(c - e), sum(c - e - 1), a.shift);
+                     }
+                  }
+                  else if (SPLIT) { // modulo 2^16 the hi*hi term vanishes
+#pragma unroll
+                     for (int e = 0; e < 4; e += 2)
+                        d[e / 2] = __byte_perm((acc[0][c - e] << 8) + acc[1][c - e],
+                                               (acc[0][c - e - 1] << 8) + acc[1][c - e - 1], 0x5410);
+                  }
+                  else if (QMODE)
+                     d[0] = outStage8x4((int) acc[0][c], (int) acc[0][c - 1], (int) acc[0][c - 2], (int) acc[0][c - 3],
+                                        a.shift);
+                  else // modulo 2^8
+                     d[0] = __byte_perm(__byte_perm(acc[0][c], acc[0][c - 1], 0x0040),
+                                        __byte_perm(acc[0][c - 2], acc[0][c - 3], 0x0040), 0x5410);
                }
-               *(uint4 *) &out[0] = make_uint4(w[0], w[1], w[2], w[3]);
-               *(uint4 *) &out[8] = make_uint4(w[4], w[5], w[6], w[7]);
             }
-            if (!SPLIT && QMODE) {
-               uint4 w;
-               w.x = outStage8x4((int) acc[0][0], (int) acc[0][1], (int) acc[0][2], (int) acc[0][3], a.shift);
-               w.y = outStage8x4((int) acc[0][4], (int) acc[0][5], (int) acc[0][6], (int) acc[0][7], a.shift);
-               w.z = outStage8x4((int) acc[0][8], (int) acc[0][9], (int) acc[0][10], (int) acc[0][11], a.shift);
-               w.w = outStage8x4((int) acc[0][12], (int) acc[0][13], (int) acc[0][14], (int) acc[0][15], a.shift);
-               *(uint4 *) &out[0] = w;
+            const long long j = j0 + kPiece * h;
+            if (j >= 0 && j + kPiece <= a.outSize) {
+               if (kWords == 8) store32(cur.y + j, w);
+               else *(uint4 *) (cur.y + j) = *(const uint4 *) w;
             }
+            else if (j > -kPiece && j < a.outSize) {
+               const int b0 = j < 0 ? (int) -j : 0, b1 = (int) min((long long) kPiece, a.outSize - j);
 #pragma unroll
-            for (int b = 0; b < 16; b++) {
-               long long v;
-               if (!SPLIT) {
-                  if (!QMODE) out[b] = (T) outStage8<QMODE>((int) acc[0][b], a.shift);
-                  continue;
-               }
-               if (QMODE) continue; // packed above
-               v = (long long) (int) (((uint32_t) acc[1][b] << 8) + (uint32_t) acc[2][b]);
-               out[b] = outStage<T, QMODE>(v, a.shift);
-            }
-            int4 *os = (int4 *) (ostage + row * kPhases);
-            os[0] = *(int4 *) &out[0];
-            if (SPLIT) os[1] = *(int4 *) &out[8];
-         }
-         tc::fenceBeforeSync();
-         if (failed) break;
-         __syncthreads(); // the output tile is complete in shared memory
-         storeTile<T>(y + j0, (int) min((long long) kTile, (long long) a.outSize - j0),
-                      (const unsigned char *) ostage, [](int ci) { return ci * 16; }, tid, kThreads);
-         if (preVec) {
-            unsigned char *N0 = A(buf ^ 1, 0), *N1 = A(buf ^ 1, 1);
-#pragma unroll
-            for (int i = 0; i < kPre; i++) {
-               const int k = tid + i * kThreads;
-               if (k < nvec) putSegVec<T>(pre[i], k, N0, N1);
+               for (int b = 0; b < kPiece; b++)
+                  if (b >= b0 && b < b1)
+                     cur.y[j + b] = SPLIT ? (T) (w[b / (SPLIT ? 2 : 4)] >> (16 * (b & 1))) : (T) (w[b / 4] >> (8 * (b & 3)));
             }
          }
-         else if (xn != nullptr) {
-            intStage<T>(xn + jn, jn, inExtent, seg, A(buf ^ 1, 0), A(buf ^ 1, 1), tid); // unaligned row
-         }
-         buf ^= 1;
       }
    }
+   if (!SPLIT) cpAsyncWaitAll();
+   tc::fenceBeforeSync();
    __syncthreads();
-   if (warp == 0) tc::tmemFree(tmem, kCols);
+   if (warp == 0) tc::tmemFree(tmem, Sh::tmemCols(QMODE));
 }
 
-// Tiles per CTA (the built-in rule, when the autotuner has no entry): a whole channel
-// when there are enough channels to fill the GPU several times over, else split so that
-// at least ~2 waves of CTAs exist.
-inline int tilesPerCtaFor(int nt, int batch, int ctasPerSm)
-{
-   const long long sms = deviceSms() > 0 ? deviceSms() : 148;
-   int tpc = nt;
-   while (tpc > 1 && (long long) ((nt + tpc - 1) / tpc) * batch < sms * ctasPerSm * 2) tpc = (tpc + 1) / 2;
-   return tpc;
-}
-
+// CTAs per SM of the longest wave the autotuner may ask for.
 template <typename T> constexpr int intLaunchBound() { return sizeof(T) == 2 ? 6 : 8; }
 
-template <typename T, int QMODE> cudaError_t launchIntTc(const FirLaunch &a, cudaStream_t s)
+template <typename T, int QMODE, int P> static cudaError_t launchIntTcP(const FirLaunch &a, cudaStream_t s)
 {
-   constexpr bool SPLIT = sizeof(T) == 2;
-   const int Kt = bandK(a.T);
-   const int nplane = SPLIT ? 2 : 1;
-   const size_t gbBytes = (size_t) ((Kt + 20) / 4) * 4 * nplane;
-   const size_t smem = 16 + ((gbBytes + 15) & ~(size_t) 15) + (size_t) Kt * 16 * nplane +
-                       2 * (size_t) nplane * (kTile + Kt) + (size_t) kTile * sizeof(T);
-   auto fn = fir_int_tc_kernel<T, QMODE>;
+   using Sh = IntShape<T, P>;
+   const size_t smem = Sh::smem(a.T);
+   auto fn = fir_int_tc_kernel<T, QMODE, P>;
    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
    if (e != cudaSuccess) return e;
-   const int nt = (a.outSize + kTile - 1) / kTile;
-   const int tpc = a.tuneTpc > 0 ? (a.tuneTpc < nt ? a.tuneTpc : nt) : tilesPerCtaFor(nt, a.batch, 8);
-   const long long items = (long long) a.batch * ((nt + tpc - 1) / tpc);
-   // persistent: one wave of resident CTAs striding over the work items (CTAs per SM: the
-   // autotuner's choice or the launch bound, fewer when shared memory runs out first)
+   const uint32_t nt = (uint32_t) intTiles<T, P>(a);
+   // persistent: one wave of resident CTAs striding over the runs (CTAs per SM: the autotuner's
+   // choice or the launch bound, fewer when shared memory runs out first)
    const int bySmem = (int) ((228u * 1024u) / (smem + 1024u));
-   const int want = a.tunePerSm > 0 ? a.tunePerSm : intLaunchBound<T>();
-   const int perSm = want < bySmem ? want : bySmem;
-   const int sms = deviceSms() > 0 ? deviceSms() : 148;
-   const long long wave = (long long) (perSm > 0 ? perSm : 1) * sms;
-   const int grid = (int) (items < wave ? items : wave);
+   int perSm = a.tunePerSm > 0 ? a.tunePerSm : Sh::perSm(QMODE);
+   perSm = std::max(1, std::min({perSm, bySmem, Sh::perSm(QMODE)}));
+   const long long wave = (long long) perSm * (deviceSms() > 0 ? deviceSms() : 148);
+   const long long total = (long long) a.batch * nt;
+   const long long tpr = a.tuneTpc > 0 ? std::min<long long>(a.tuneTpc, nt) : (total + wave - 1) / wave;
+   const long long runs = (total + tpr - 1) / tpr;
    FirLaunch k = a;
    // int8: |acc| <= 2048 * 2^14 = 2^25, so every shift from 27 up rounds to zero, as 31
    // (the largest the 32-bit output stage can take) does.
-   if (!SPLIT && k.shift > 31) k.shift = 31;
-   fn<<<grid, kThreads, smem, s>>>(k, tpc);
+   if (sizeof(T) == 1 && k.shift > 31) k.shift = 31;
+   fn<<<(unsigned) std::min(runs, wave), kThreads, smem, s>>>(k, (uint32_t) tpr);
    countLaunch();
    return cudaGetLastError();
+}
+
+// Rows of 32 outputs read each byte of the segment half as often in the MMAs (40 clk of shared
+// memory a step of 32 taps for 4096 outputs instead of 36 for 2048); rows of 16 do where half the
+// larger tile would be empty (a channel within 2048 outputs) and where every tile has an SM of
+// its own, for the shorter way through it.  In us, 32 against 16: int8 4096 channels x 16384
+// samples x 128 taps 39.3 / 55.5, int16 1000 x 10007 x 201 25.8 / 27.4; int16 4096 x 1100 x 33
+// 22.8 / 18.7, int8 4096 x 2048 x 16 18.6 / 16.5, int8 16 x 4096 x 64 6.05 / 5.0.
+template <typename T, int QMODE> static cudaError_t launchIntTc(const FirLaunch &a, cudaStream_t s)
+{
+   const int nt = intTiles<T, 16>(a);
+   if (nt == 1 || (long long) nt * a.batch <= (deviceSms() > 0 ? deviceSms() : 148)) return launchIntTcP<T, QMODE, 16>(a, s);
+   return launchIntTcP<T, QMODE, 32>(a, s);
 }
 
 // ------------------------------------------------------------------ split-BF16x3
@@ -1329,7 +1309,7 @@ std::string firTuneKey(const FirLaunch &a, FirKernelKind kind)
       return buf;
    }
    if ((kind == FIR_INT_WRAP_TC || kind == FIR_INT_Q_TC) && firIntTcSupported(a)) {
-      const int nt = (a.outSize + kTile - 1) / kTile;
+      const int nt = (a.outSize + kIntTuneTile - 1) / kIntTuneTile;
       snprintf(buf, sizeof(buf), "fir_int|dtype=%d|q=%d|T=%d|tiles=2^%d|batch=2^%d|sms=%d", a.dtype,
                kind == FIR_INT_Q_TC ? 1 : 0, a.T, tuneClass(nt), tuneClass(a.batch), deviceSms());
       return buf;
@@ -1337,7 +1317,8 @@ std::string firTuneKey(const FirLaunch &a, FirKernelKind kind)
    return std::string();
 }
 
-// bf16x3: the choice is the tiles per CTA; int: tiles per CTA * 16 + CTAs per SM.
+// bf16x3: the choice is the tiles per CTA; int: tiles per run (0: the built-in even split) * 16 +
+// CTAs per SM.
 std::vector<int> firTuneCandidates(const FirLaunch &a, FirKernelKind kind)
 {
    std::vector<int> c;
@@ -1355,9 +1336,9 @@ std::vector<int> firTuneCandidates(const FirLaunch &a, FirKernelKind kind)
       c = tileCounts(nt, bfTilesPerRun(nt, a.batch));
    }
    else {
-      const int nt = (a.outSize + kTile - 1) / kTile;
+      const int nt = (a.outSize + kIntTuneTile - 1) / kIntTuneTile;
       const int bound = a.dtype == DSPLIB_INT16 ? intLaunchBound<int16_t>() : intLaunchBound<int8_t>();
-      for (int t : tileCounts(nt, tilesPerCtaFor(nt, a.batch, 8)))
+      for (int t : tileCounts(nt, 0))
          for (int per = 4; per <= bound; per += 2) c.push_back(t * 16 + per);
    }
    std::sort(c.begin(), c.end());

@@ -77,7 +77,8 @@ int64_t DSPLIB_gpu_kernelLaunchCount(void);
  * measured choice per problem class and GPU instead, where a kernel has shapes to
  * choose from:
  *   fir_bf16x3  output tiles per CTA of the split-BF16x3 FIR;
- *   fir_int     output tiles per CTA and resident CTAs per SM of the int8/int16 FIR;
+ *   fir_int     output tiles per run (0: an even share for each CTA) and resident CTAs per SM
+ *               of the int8/int16 FIR;
  *   bq_scan     warps per CTA (the 32-sample chunks of one window: its length), half rows or
  *               64-sample chunks, and CTAs per cluster of the cascade-biquad scan;
  *   bank_runs   output tiles per run of the batched filter bank's FIR work lists.

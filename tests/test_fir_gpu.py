@@ -158,6 +158,33 @@ def test_int_tensor_core_unaligned_rows():
     assert np.array_equal(host(od)[:, : N - T + 1], want)
 
 
+@pytest.mark.parametrize("qmode", [False, True])
+@pytest.mark.parametrize("dt", [np.int8, np.int16])
+def test_int_tensor_core_grid_edges(dt, qmode):
+    """Rows off the vector boundary in x and y, by other amounts from channel to channel, outputs
+    around the edges of rows and tiles of both tile sizes, more tiles than CTAs; what lies
+    between the output rows stays as it was."""
+    rng = np.random.default_rng(24)
+    for (B, outs, T, offx, offy, padx, pady, nch) in [
+            (160, 4096, 33, 0, 0, 0, 0, 0), (150, 4097, 64, 1, 5, 3, 1, 1), (149, 4095, 1, 7, 0, 0, 17, 0),
+            (75, 2049, 200, 0, 31, 5, 16, 1), (37, 8193, 97, 3, 3, 13, 2, 0), (1300, 2100, 16, 2, 1, 0, 3, 1),
+            (9, 2048, 31, 5, 9, 1, 0, 1), (200, 17, 20, 1, 2, 3, 4, 0), (2, 200001, 256, 9, 11, 2, 1, 1)]:
+        N, pin, pout = outs + T - 1, outs + T - 1 + padx, outs + pady
+        buf = rand(dt, (B * pin + offx,), rng)
+        x = np.ascontiguousarray(buf[offx:].reshape(B, pin)[:, :N])
+        hh = rand(dt, (B if nch else 1, T), rng)
+        args, ain, afilt, aout = D.fir_setup(_NP_CODE[dt], B, N, T, nch=nch, shift=6, in_pitch=pin, out_pitch=pout)
+        h = D.FirHandle()
+        assert h.init(args, ain, afilt, aout) == D.SUCCESS
+        h.set_qmode(qmode)
+        od = dev(np.full(B * pout + offy + 40, 77, dt))
+        assert h.exec(dev(buf)[offx:], dev(hh), od[offy:]) == D.SUCCESS, h.last_error()
+        want = np.full(B * pout + offy + 40, 77, dt)
+        y = oracle.fir_q(x, hh, T, 6, nch=nch) if qmode else oracle.fir(x, hh, T, nch=nch)
+        want[offy:offy + B * pout].reshape(B, pout)[:, :outs] = y
+        assert np.array_equal(host(od), want), (B, outs, T, offx, offy, padx, pady)
+
+
 def _relerr(y, y64):
     return np.max(np.abs(y.astype(np.float64) - y64), axis=1) / np.maximum(np.max(np.abs(y64), axis=1), 1e-30)
 
