@@ -285,6 +285,8 @@ struct AddNChLaunch {
 cudaError_t launchAddNCh(const AddNChLaunch &a, cudaStream_t s);
 bool firIntTcSupported(const FirLaunch &a);
 bool firBf16x3Supported(const FirLaunch &a);
+cudaError_t launchStreamWindow(char *win, long long pitch, const void *in, long long inPitch, int channels, int hist,
+                               int block, int elt, cudaStream_t s);
 cudaError_t launchFirIntTc(const FirLaunch &a, bool qmode, cudaStream_t s);
 // Autotuner entries of the tensor-core FIR kernels (kind FIR_F32_BF16X3, FIR_INT_WRAP_TC,
 // FIR_INT_Q_TC): the key of a launch's problem class ("" for kernels without shapes to

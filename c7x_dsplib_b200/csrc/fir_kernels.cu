@@ -415,4 +415,57 @@ cudaError_t launchFir(const FirLaunch &a, FirKernelKind kind, cudaStream_t s)
    return cudaErrorInvalidValue;
 }
 
+// ------------------------------------------------------------------ streaming window
+
+// Advance the windows of a streaming filter, [hist | block] elements a channel: the last `hist`
+// elements move to the front and the new block takes the place behind them.  Element i of the
+// history is read, and the element that replaces it written, by one thread, and no other
+// touches its two places (block >= hist), so nothing has to wait.  V elements a copy where the
+// rows of `in` allow (a window's block starts on a 16-byte boundary).  Bound by its launch.
+template <typename E, int V>
+__global__ void __launch_bounds__(256) stream_window_kernel(char *win, long long pitch, const char *in,
+                                                            long long inPitch, int channels, int hist, int block)
+{
+   const int body = block - hist, nv = body / V, items = hist + nv + (body - nv * V);
+   for (int c = blockIdx.y; c < channels; c += gridDim.y) {
+      E *w = (E *) (win + c * pitch);
+      const E *x = (const E *) (in + c * inPitch);
+      for (long long k = (long long) blockIdx.x * blockDim.x + threadIdx.x; k < items; k += (long long) gridDim.x * blockDim.x) {
+         if (k < hist) {
+            w[k] = w[block + k];
+            w[block + k] = x[body + k];
+         }
+         else if (k - hist < nv) {
+            const long long q = (k - hist) * V;
+            if (V > 1) *(int4 *) (w + hist + q) = *(const int4 *) (x + q);
+            else w[hist + q] = x[q];
+         }
+         else {
+            const long long q = k - hist - nv + (long long) nv * V;
+            w[hist + q] = x[q];
+         }
+      }
+   }
+}
+
+cudaError_t launchStreamWindow(char *win, long long pitch, const void *in, long long inPitch, int channels, int hist,
+                               int block, int elt, cudaStream_t s)
+{
+   const int V = 16 / elt;
+   const bool wide = ((((uintptr_t) win + (size_t) hist * elt) | (uintptr_t) pitch | (uintptr_t) in | (uintptr_t) inPitch) & 15) == 0;
+   const long long items = wide ? hist + (long long) (block - hist) / V + V - 1 : block;
+   const dim3 grid((unsigned) std::min<long long>((items + 255) / 256, 1024), (unsigned) std::min(channels, 65535));
+   auto go = [&](auto e) {
+      using E = decltype(e);
+      if (wide) stream_window_kernel<E, 16 / (int) sizeof(E)><<<grid, 256, 0, s>>>(win, pitch, (const char *) in, inPitch, channels, hist, block);
+      else stream_window_kernel<E, 1><<<grid, 256, 0, s>>>(win, pitch, (const char *) in, inPitch, channels, hist, block);
+   };
+   if (elt == 1) go((uint8_t) 0);
+   else if (elt == 2) go((uint16_t) 0);
+   else if (elt == 4) go((uint32_t) 0);
+   else return cudaErrorInvalidValue;
+   countLaunch();
+   return cudaGetLastError();
+}
+
 } // namespace dsplib

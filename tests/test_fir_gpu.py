@@ -461,6 +461,34 @@ def test_fir_stream_matches_one_call(dt, style, precision, qmode, C, T, N, block
     assert np.array_equal(again, got[:, :N])
 
 
+@pytest.mark.parametrize("dt", [np.int8, np.int16, np.int32, np.float32])
+@pytest.mark.parametrize("C,T,N", [(1, 1, 5), (5, 2, 1), (3, 38, 37), (3, 37, 37), (4, 64, 4096), (2, 301, 300),
+                                   (3, 301, 299), (7, 5, 1021)])
+def test_fir_stream_block_places(dt, C, T, N):
+    """Blocks on and off the 16-byte boundary and in host memory in turn, block lengths around the
+    history's; a refused call (Q mode with a shift beyond 62) leaves the history as it was."""
+    rng = np.random.default_rng(C * T + N)
+    x = rand(dt, (C, 6 * N), rng)
+    h = rand(dt, (C, T), rng)
+    code = {**_NP_CODE, np.float32: D.FLOAT32}[dt]
+    st = D.FirStream(code, C, N, T, nch=1, shift=63)
+    want = oracle.fir(np.concatenate([np.zeros((C, T - 1), dt), x], axis=1), h, T, nch=1)
+    for b in range(6):
+        xb = np.ascontiguousarray(x[:, b * N:(b + 1) * N])
+        if b in (2, 4) and dt != np.float32:
+            D.lib().DSPLIB_gpu_firSetQMode(st.h, 1)
+            with pytest.raises(D.DsplibError):
+                st.exec(dev(xb) if b == 4 else xb, dev(h), dev(xb))
+            D.lib().DSPLIB_gpu_firSetQMode(st.h, 0)
+        if b % 3 == 2:
+            got = st.exec(xb, h, np.zeros((C, N), dt))
+        else:
+            buf = dev(np.concatenate([np.zeros(b % 3, dt), xb.ravel()]))
+            got = host(st.exec(buf[b % 3:], dev(h), torch.zeros((C, N), dtype=buf.dtype, device="cuda")))
+        w = want[:, b * N:(b + 1) * N]
+        assert np.array_equal(got, w) if dt != np.float32 else np.max(np.abs(got - w)) <= TOL_REF, b
+
+
 def test_handles_on_concurrent_host_threads():
     """Handles are independent: host threads filtering pageable host buffers at the same
     time (per-thread staging buffers and copy pipelines) give the oracle's results."""
