@@ -157,6 +157,8 @@ SIGNATURES = {
     "DSPLIB_gpu_firStreamExec": (ctypes.c_int, [_VP, _VP, _VP, _VP]),
     "DSPLIB_gpu_firStreamReset": (ctypes.c_int, [_VP]),
     "DSPLIB_gpu_firStreamDestroy": (ctypes.c_int, [_VP]),
+    "DSPLIB_gpu_firAdjointScratch": (ctypes.c_int64, [ctypes.c_int32] * 6),
+    "DSPLIB_gpu_firAdjoint": (ctypes.c_int, [ctypes.c_int32] * 4 + [_VP] * 7),
     "DSPLIB_gpu_raggedPlanCreate": (ctypes.c_int, [_P(_VP), ctypes.c_int32, _P(ctypes.c_int32),
                                                    _P(ctypes.c_int32), _P(ctypes.c_int32)]),
     "DSPLIB_gpu_raggedPlanSize": (ctypes.c_int64, [_VP, ctypes.c_int32]),

@@ -285,6 +285,9 @@ struct AddNChLaunch {
 cudaError_t launchAddNCh(const AddNChLaunch &a, cudaStream_t s);
 bool firIntTcSupported(const FirLaunch &a);
 bool firBf16x3Supported(const FirLaunch &a);
+size_t firAdjointScratch(int batch, int rows, int N, int T, bool wantX, bool wantH); // floats
+cudaError_t launchFirAdjoint(const float *gy, const float *x, const float *h, float *gx, float *gh, float *scratch,
+                             int batch, int rows, int N, int T, cudaStream_t s);
 cudaError_t launchStreamWindow(char *win, long long pitch, const void *in, long long inPitch, int channels, int hist,
                                int block, int elt, cudaStream_t s);
 cudaError_t launchFirIntTc(const FirLaunch &a, bool qmode, cudaStream_t s);

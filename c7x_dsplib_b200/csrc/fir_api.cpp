@@ -427,4 +427,24 @@ void DSPLIB_fir_perfEst(DSPLIB_kernelHandle handle,
    if (estCycles) *estCycles = (uint64_t) (t * 1e9) + 4000; // + launch and sync
 }
 
+int64_t DSPLIB_gpu_firAdjointScratch(int32_t batch, int32_t tapRows, int32_t dataSize, int32_t filterSize,
+                                     int32_t wantX, int32_t wantH)
+{
+   if (batch < 1 || (tapRows != 1 && tapRows != batch) || filterSize < 1 || dataSize < filterSize) return -1;
+   return (int64_t) firAdjointScratch(batch, tapRows, dataSize, filterSize, wantX != 0, wantH != 0);
+}
+
+DSPLIB_STATUS DSPLIB_gpu_firAdjoint(int32_t batch, int32_t tapRows, int32_t dataSize, int32_t filterSize, const float *gy,
+                                    const float *x, const float *h, float *gx, float *gh, float *scratch, void *stream)
+{
+   const int64_t n = DSPLIB_gpu_firAdjointScratch(batch, tapRows, dataSize, filterSize, gx != nullptr, gh != nullptr);
+   if (n < 0) return DSPLIB_ERR_INVALID_DIMENSION;
+   if (!gy || !x || !h || (n > 0 && !scratch)) return DSPLIB_ERR_NULL_POINTER;
+   if (launchFirAdjoint(gy, x, h, gx, gh, scratch, batch, tapRows, dataSize, filterSize, (cudaStream_t) stream) != cudaSuccess) {
+      (void) cudaGetLastError();
+      return DSPLIB_ERR_FAILURE;
+   }
+   return DSPLIB_SUCCESS;
+}
+
 } // extern "C"

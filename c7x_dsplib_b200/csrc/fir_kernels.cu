@@ -468,4 +468,92 @@ cudaError_t launchStreamWindow(char *win, long long pitch, const void *in, long 
    return cudaGetLastError();
 }
 
+// ------------------------------------------------------------------ adjoint
+
+// The operands of the two filters of the adjoint, from rows gy [batch, M] and h [rows, T]
+// (M = N - T + 1): gy with T - 1 zeros on both sides, the taps reversed, gy reversed.
+__global__ void __launch_bounds__(256) fir_adjoint_operands_kernel(const float *gy, const float *h, float *wide, float *hrev,
+                                                                   float *grev, int batch, int rows, int M, int T)
+{
+   const long long W = M + 2LL * (T - 1);
+   const long long nw = wide ? batch * W : 0, nh = wide ? (long long) rows * T : 0, ng = grev ? (long long) batch * M : 0;
+   for (long long k = (long long) blockIdx.x * blockDim.x + threadIdx.x; k < nw + nh + ng; k += (long long) gridDim.x * blockDim.x) {
+      if (k < nw) {
+         const long long l = k / W, j = k - l * W - (T - 1);
+         wide[k] = j >= 0 && j < M ? gy[l * M + j] : 0.f;
+      }
+      else if (k < nw + nh) {
+         const long long q = k - nw, l = q / T;
+         hrev[q] = h[l * T + (T - 1 - (q - l * T))];
+      }
+      else {
+         const long long q = k - nw - nh, l = q / M;
+         grev[q] = gy[l * M + (M - 1 - (q - l * M))];
+      }
+   }
+}
+
+__global__ void __launch_bounds__(256) reverse_rows_kernel(const float *in, float *out, int rows, int n)
+{
+   for (long long k = (long long) blockIdx.x * blockDim.x + threadIdx.x; k < (long long) rows * n; k += (long long) gridDim.x * blockDim.x) {
+      const long long l = k / n;
+      out[k] = in[l * n + (n - 1 - (k - l * n))];
+   }
+}
+
+size_t firAdjointScratch(int batch, int rows, int N, int T, bool wantX, bool wantH)
+{
+   const size_t M = (size_t) (N - T + 1);
+   auto up = [](size_t n) { return (n + 31) & ~(size_t) 31; };
+   return (wantX ? up(batch * (M + 2 * (size_t) (T - 1))) + up((size_t) rows * T) : 0) +
+          (wantH ? up(batch * M) + up((size_t) batch * T) : 0);
+}
+
+// dx = FIR of the widened gy with the reversed taps, dh = the FIR of x with each channel's
+// reversed gy as its taps, reversed.  One launch makes the operands (five of the framework's
+// took 27 us of host time).
+cudaError_t launchFirAdjoint(const float *gy, const float *x, const float *h, float *gx, float *gh, float *scratch,
+                             int batch, int rows, int N, int T, cudaStream_t s)
+{
+   const int M = N - T + 1;
+   auto up = [](size_t n) { return (n + 31) & ~(size_t) 31; };
+   const size_t W = (size_t) M + 2 * (size_t) (T - 1);
+   float *wide = nullptr, *hrev = nullptr, *grev = nullptr, *lag = nullptr;
+   if (gx) {
+      wide = scratch;
+      hrev = wide + up(batch * W);
+      scratch = hrev + up((size_t) rows * T);
+   }
+   if (gh) {
+      grev = scratch;
+      lag = grev + up((size_t) batch * M);
+   }
+   auto blocks = [](size_t n) { return (unsigned) std::min<size_t>((n + 255) / 256, 148 * 16); };
+   const size_t items = (gx ? batch * W + (size_t) rows * T : 0) + (gh ? (size_t) batch * M : 0);
+   if (items == 0) return cudaSuccess;
+   fir_adjoint_operands_kernel<<<blocks(items), 256, 0, s>>>(gy, h, wide, hrev, grev, batch, rows, M, T);
+   countLaunch();
+   cudaError_t e = cudaGetLastError();
+   FirLaunch a{};
+   a.dtype = DSPLIB_FLOAT32;
+   a.batch = batch;
+   if (gx && e == cudaSuccess) {
+      a.x = wide, a.h = hrev, a.y = gx;
+      a.T = T, a.outSize = N;
+      a.inPitch = (long long) W, a.outPitch = N, a.filtPitch = rows > 1 ? T : 0;
+      e = launchFir(a, FIR_F32_SIMT, s);
+   }
+   if (gh && e == cudaSuccess) {
+      a.x = x, a.h = grev, a.y = lag;
+      a.T = M, a.outSize = T;
+      a.inPitch = N, a.outPitch = T, a.filtPitch = M;
+      e = launchFir(a, FIR_F32_SIMT, s);
+      if (e != cudaSuccess) return e;
+      reverse_rows_kernel<<<blocks((size_t) batch * T), 256, 0, s>>>(lag, gh, batch, T);
+      countLaunch();
+      e = cudaGetLastError();
+   }
+   return e;
+}
+
 } // namespace dsplib

@@ -161,6 +161,17 @@ DSPLIB_STATUS DSPLIB_gpu_firStreamExec(DSPLIB_gpu_firStream stream, const void *
 DSPLIB_STATUS DSPLIB_gpu_firStreamReset(DSPLIB_gpu_firStream stream);
 DSPLIB_STATUS DSPLIB_gpu_firStreamDestroy(DSPLIB_gpu_firStream stream);
 
+/** Adjoint of DSPLIB_fir (FLOAT32, FP32 CUDA-core kernels) over dense device rows, queued on the
+ *  given cudaStream_t: from gy [batch, dataSize - filterSize + 1], x [batch, dataSize] and stored
+ *  taps h [tapRows, filterSize] (1 row shared by all channels, or batch) the gradients
+ *  gx [batch, dataSize] and gh [batch, filterSize] (per channel also for shared taps: their sum
+ *  over the channels is the caller's).  Either may be NULL.  scratch:
+ *  DSPLIB_gpu_firAdjointScratch floats (-1: sizes refused). */
+int64_t DSPLIB_gpu_firAdjointScratch(int32_t batch, int32_t tapRows, int32_t dataSize, int32_t filterSize,
+                                     int32_t wantX, int32_t wantH);
+DSPLIB_STATUS DSPLIB_gpu_firAdjoint(int32_t batch, int32_t tapRows, int32_t dataSize, int32_t filterSize, const float *gy,
+                                    const float *x, const float *h, float *gx, float *gh, float *scratch, void *stream);
+
 /* ---------------------------------------------------------------------------
  * Batched filter bank over channels of uneven length, forward and adjoint.
  * Per channel c (length L_c, T_c taps, S_c second-order stages):

@@ -104,6 +104,52 @@ def test_fir_operator_gradients_match_fp64(nch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("nch", [False, True])
+@pytest.mark.parametrize("B,N,T", [(1, 1, 1), (3, 40, 1), (2, 33, 33), (5, 1500, 64), (2, 700, 600), (1, 9, 4)])
+def test_fir_operator_gradients_edges(B, N, T, nch):
+    """The one-call gradients of torch.ops.dsplib_gpu.fir: one or both wanted, rows with gaps,
+    several gradients at once, gradients that are differentiated again, and meta shapes."""
+    import c7x_dsplib_b200.torch_ops  # noqa: F401
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    g = torch.Generator().manual_seed(B * N + T)
+    M = N - T + 1
+    x, h = torch.randn(B, N, generator=g), torch.randn(B if nch else 1, T, generator=g)
+    w, v = torch.randn(B, M, generator=g), torch.randn(B, N, generator=g)
+
+    def fir64(xx, hh):
+        rows = hh if nch else hh.expand(B, T)
+        return torch.stack([torch.nn.functional.conv1d(xx[l].view(1, 1, -1), rows[l].flip(0).view(1, 1, -1)).view(-1)
+                            for l in range(B)])
+
+    def near(got, want):
+        # float32 sums of at most N products against float64: N * 2^-24 of the terms' size each
+        scale = N * 2.0 ** -22 * max(1.0, float(w.abs().max())) * max(float(x.abs().max()), float(h.abs().max()))
+        assert got.shape == want.shape
+        assert float((got.double().cpu() - want).abs().max()) <= scale * max(1.0, N ** 0.5)
+
+    x64, h64 = x.double().requires_grad_(), h.double().requires_grad_()
+    want = torch.autograd.grad(fir64(x64, h64), (x64, h64), w.double(), create_graph=True)
+    fir = torch.ops.dsplib_gpu.fir
+    gap = torch.empty(B, 2 * N, device="cuda")[:, ::2].copy_(x)
+    gapw = torch.empty(M, B, device="cuda").t().copy_(w.cuda())
+    for need_x, need_h in ((True, True), (True, False), (False, True)):
+        xd, hd = gap.detach().requires_grad_(need_x), h.cuda().requires_grad_(need_h)
+        wrt = [t for t in (xd, hd) if t.requires_grad]
+        got = torch.autograd.grad(fir(xd, hd, nch, 0, False, 0), wrt, gapw)
+        for a, b in zip(got, [q for q, n in zip(want, (need_x, need_h)) if n]):
+            near(a, b.detach())
+    xd, hd = x.cuda().requires_grad_(), h.cuda().requires_grad_()
+    gx, gh = torch.autograd.grad(fir(xd, hd, nch, 0, False, 0), (xd, hd), w.cuda(), create_graph=True)
+    near(gx.detach(), want[0].detach())
+    near(torch.autograd.grad((gx * v.cuda()).sum(), hd)[0], torch.autograd.grad((want[0] * v.double()).sum(), h64)[0])
+    with FakeTensorMode():
+        xf, hf = (torch.empty(t.shape, device="cuda", requires_grad=True) for t in (x, h))
+        gx, gh = torch.autograd.grad(fir(xf, hf, nch, 0, False, 0), (xf, hf), torch.empty(B, M, device="cuda"))
+        assert gx.shape == x.shape and gh.shape == h.shape
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("form", [0, 1, 2, 3])
 @pytest.mark.parametrize("nch", [False, True])
 def test_cascade_operator_gradients_match_fp64(form, nch):
