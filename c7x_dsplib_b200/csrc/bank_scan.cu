@@ -1032,12 +1032,12 @@ cudaError_t launchBankForward(const BankLaunch &b, cudaStream_t s)
    cudaError_t e = launchAggregates<false>(b, a, s);
    if (e != cudaSuccess) return e;
    const size_t dynC = (size_t) (4 * b.Smax * (b.Smax + 1) / 2 + 2 * b.Smax) * sizeof(double);
-   if ((e = cudaFuncSetAttribute(bank_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dynC)) !=
-       cudaSuccess)
-      return e;
    bank_chain_fast_kernel<<<b.C, kChainWarps * 32, 0, s>>>(b.chans, b.chainOrder, b.phi, b.aggF, b.ckptF, b.groupF, 0);
    countLaunch();
    if (b.Smax > kChainFastStages) {
+      if ((e = cudaFuncSetAttribute(bank_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dynC)) !=
+          cudaSuccess)
+         return e;
       bank_chain_kernel<<<b.C, 32, dynC, s>>>(b.chans, b.chainOrder, b.phi, b.aggF, b.ckptF, 0);
       countLaunch();
    }
@@ -1063,12 +1063,12 @@ cudaError_t launchBankBackward(const BankLaunch &b, cudaStream_t s)
       if ((e = launchAggregates<true>(b, a, s)) != cudaSuccess) return e;
    }
    const size_t dynC = (size_t) (4 * b.Smax * (b.Smax + 1) / 2 + 2 * b.Smax) * sizeof(double);
-   if ((e = cudaFuncSetAttribute(bank_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dynC)) !=
-       cudaSuccess)
-      return e;
    bank_chain_fast_kernel<<<b.C, kChainWarps * 32, 0, s>>>(b.chans, b.chainOrder, b.phi, b.aggA, b.ckptA, b.groupA, 1);
    countLaunch();
    if (b.Smax > kChainFastStages) {
+      if ((e = cudaFuncSetAttribute(bank_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dynC)) !=
+          cudaSuccess)
+         return e;
       bank_chain_kernel<<<b.C, 32, dynC, s>>>(b.chans, b.chainOrder, b.phi, b.aggA, b.ckptA, 1);
       countLaunch();
    }
