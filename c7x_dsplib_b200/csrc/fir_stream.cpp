@@ -11,11 +11,13 @@
 // Each channel has a device window [T - 1 history | N new]; between calls its last T - 1
 // samples are the history.  Per call, on the handle's stream, one kernel moves the history to
 // the window's head and the new block behind it, and DSPLIB_fir_exec runs over the windows;
-// if it refuses, the head is moved back.  Blocks in host memory (or on another device), and
-// blocks shorter than the history, whose old and new place overlap, are moved by copies.
+// if it refuses, the head is moved back.  Blocks in host memory (or on another device), blocks
+// shorter than the history, whose old and new place overlap, and blocks whose rows do not all
+// start on a multiple of the sample size are moved by copies.
 // (Three 2-D copies around the filter, with the history in a buffer of its own, took 18.4 us
 // a call on 16 channels x 4096 int16 samples x 64 taps; now 10.2.)
 #include <climits>
+#include <cstdint>
 #include <cstdlib>
 #include <cstring>
 
@@ -134,7 +136,8 @@ DSPLIB_STATUS DSPLIB_gpu_firStreamExec(DSPLIB_gpu_firStream stream, const void *
    const cudaStream_t cs = hc->stream;
    cudaError_t e = cudaSuccess;
    const bool own = onThisDevice(pIn);
-   if (own && s->N >= s->T - 1) {
+   const bool whole = (((uintptr_t) pIn | s->inPitch) & (size_t) (s->elt - 1)) == 0; // the kernel loads whole samples
+   if (own && whole && s->N >= s->T - 1) {
       if ((e = launchStreamWindow(s->win, (long long) s->pitch, pIn, (long long) s->inPitch, s->channels, s->T - 1,
                                   s->N, s->elt, cs)))
          return cudaFail(hc, e, "stream: fill window");

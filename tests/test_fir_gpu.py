@@ -489,6 +489,36 @@ def test_fir_stream_block_places(dt, C, T, N):
         assert np.array_equal(got, w) if dt != np.float32 else np.max(np.abs(got - w)) <= TOL_REF, b
 
 
+@pytest.mark.parametrize("dt", [np.int16, np.int32, np.float32])
+@pytest.mark.parametrize("T,N", [(1, 5), (38, 37), (64, 257), (65, 16), (9, 4096)])
+@pytest.mark.parametrize("offset,gap", [(1, 0), (0, 1), (3, 5), (2, 2)])
+def test_fir_stream_block_bytes(dt, T, N, offset, gap):
+    """Device blocks whose rows start on any byte: offset bytes into the buffer, the pitch gap bytes
+    longer than the row."""
+    import ctypes
+
+    C, blocks, elt = 3, 3, np.dtype(dt).itemsize
+    rng = np.random.default_rng(T * N + offset)
+    x = rand(dt, (C, blocks * N), rng)
+    h = rand(dt, (C, T), rng)
+    code = {**_NP_CODE, np.float32: D.FLOAT32}[dt]
+    args = D.FirInitArgs(funcStyle=D.NATC, dataSize=N, batchSize=C, filterSize=T, shift=0, enableNchCoefs=1, enableMMA=0,
+                         MMA_SIZE=D.MMA_SIZE[elt], enableQ=0, Q=0)
+    st = D.FirStream.__new__(D.FirStream)
+    st.s = ctypes.c_void_p()
+    descs = [D.bp(code, N, C, N * elt + gap), D.bp(code, T, C, T * elt), D.bp(code, N, C, N * elt)]
+    assert D.lib().DSPLIB_gpu_firStreamCreate(ctypes.byref(st.s), ctypes.byref(args),
+                                              *map(ctypes.byref, descs)) == D.SUCCESS
+    st.h = D.lib().DSPLIB_gpu_firStreamHandle(st.s)
+    want = oracle.fir(np.concatenate([np.zeros((C, T - 1), dt), x], axis=1), h, T, nch=1)
+    for b in range(blocks):
+        rows = np.zeros((C, N * elt + gap), np.uint8)
+        rows[:, :N * elt] = np.ascontiguousarray(x[:, b * N:(b + 1) * N]).view(np.uint8)
+        buf = dev(np.concatenate([np.zeros(offset, np.uint8), rows.ravel()]))
+        out = torch.zeros((C, N), dtype=torch.from_numpy(x).dtype, device="cuda")
+        assert np.array_equal(host(st.exec(buf[offset:], dev(h), out)), want[:, b * N:(b + 1) * N]), b
+
+
 def test_handles_on_concurrent_host_threads():
     """Handles are independent: host threads filtering pageable host buffers at the same
     time (per-thread staging buffers and copy pipelines) give the oracle's results."""
