@@ -147,6 +147,7 @@ void freeErrorWord(int *w);
 // operation (counted over the calls of injectCheck) reports cudaErrorUnknown.
 void injectArm(HandleCommon *h);
 void injectDisarm();
+void injectPass(HandleCommon *h); // what is left of the count goes to the exec that this call makes next
 cudaError_t injectCheck(cudaError_t e);
 DSPLIB_STATUS cudaFail(HandleCommon *h, cudaError_t e, const char *what);
 void countLaunch(int n = 1);

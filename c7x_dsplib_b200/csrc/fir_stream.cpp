@@ -11,7 +11,7 @@
 // Each channel has a device window [T - 1 history | N new]; between calls its last T - 1
 // samples are the history.  Per call, on the handle's stream, one kernel moves the history to
 // the window's head and the new block behind it, and DSPLIB_fir_exec runs over the windows;
-// if it refuses, the head is moved back.  Blocks in host memory (or on another device), blocks
+// if it refuses, or a copy does, the history is moved back.  Blocks in host memory (or on another device), blocks
 // shorter than the history, whose old and new place overlap, and blocks whose rows do not all
 // start on a multiple of the sample size are moved by copies.
 // (Three 2-D copies around the filter, with the history in a buffer of its own, took 18.4 us
@@ -39,13 +39,16 @@ struct FirStream {
    char *tail() const { return win + blockBytes(); }
 };
 
-// History between the window's tail and its head through the buffer: the two may overlap.
-static cudaError_t moveHistory(const FirStream *s, char *to, const char *from, cudaStream_t cs)
+// History between the window's tail and its head goes through the buffer: the two may overlap.
+static cudaError_t takeHistory(const FirStream *s, const char *from, cudaStream_t cs)
 {
    const size_t hb = s->histBytes();
-   if (!hb) return cudaSuccess;
-   cudaError_t e = cudaMemcpy2DAsync(s->hist, hb, from, s->pitch, hb, s->channels, cudaMemcpyDeviceToDevice, cs);
-   return e ? e : cudaMemcpy2DAsync(to, s->pitch, s->hist, hb, hb, s->channels, cudaMemcpyDeviceToDevice, cs);
+   return hb ? cudaMemcpy2DAsync(s->hist, hb, from, s->pitch, hb, s->channels, cudaMemcpyDeviceToDevice, cs) : cudaSuccess;
+}
+static cudaError_t putHistory(const FirStream *s, char *to, cudaStream_t cs)
+{
+   const size_t hb = s->histBytes();
+   return hb ? cudaMemcpy2DAsync(to, s->pitch, s->hist, hb, hb, s->channels, cudaMemcpyDeviceToDevice, cs) : cudaSuccess;
 }
 
 // Whether a kernel on the current device may read p.
@@ -143,14 +146,24 @@ DSPLIB_STATUS DSPLIB_gpu_firStreamExec(DSPLIB_gpu_firStream stream, const void *
          return cudaFail(hc, e, "stream: fill window");
    }
    else {
-      if ((e = moveHistory(s, s->win, s->tail(), cs))) return cudaFail(hc, e, "stream: restore history");
-      if ((e = cudaMemcpy2DAsync(s->win + s->histBytes(), s->pitch, pIn, s->inPitch, s->blockBytes(), s->channels,
-                                 cudaMemcpyDefault, cs)))
-         return cudaFail(hc, e, "stream: copy block");
+      const char *what = "stream: restore history";
+      injectArm(hc);
+      if ((e = injectCheck(takeHistory(s, s->tail(), cs))) != cudaSuccess) return cudaFail(hc, e, what);
+      e = injectCheck(putHistory(s, s->win, cs));
+      if (e == cudaSuccess) {
+         what = "stream: copy block";
+         e = injectCheck(cudaMemcpy2DAsync(s->win + s->histBytes(), s->pitch, pIn, s->inPitch, s->blockBytes(),
+                                           s->channels, cudaMemcpyDefault, cs));
+      }
+      if (e != cudaSuccess) {
+         (void) putHistory(s, s->tail(), cs); // the head or the block may have gone over it
+         return cudaFail(hc, e, what);
+      }
+      injectPass(hc);
    }
    const DSPLIB_STATUS st = DSPLIB_fir_exec(s->handle, s->win, pFilter, pOut);
-   if (st != DSPLIB_SUCCESS) {
-      (void) moveHistory(s, s->tail(), s->win, cs); // a refused call leaves the history as it was
+   if (st != DSPLIB_SUCCESS) { // a refused call leaves the history as it was
+      if (takeHistory(s, s->win, cs) == cudaSuccess) (void) putHistory(s, s->tail(), cs);
       return st;
    }
    // a host block is copied in asynchronously: complete before returning unless async level 2

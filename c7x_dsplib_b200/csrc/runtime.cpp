@@ -113,6 +113,12 @@ void injectArm(HandleCommon *h)
 
 void injectDisarm() { t_injectLeft = 0; }
 
+void injectPass(HandleCommon *h)
+{
+   h->injectAt = t_injectLeft;
+   t_injectLeft = 0;
+}
+
 cudaError_t injectCheck(cudaError_t e)
 {
    if (e != cudaSuccess || t_injectLeft <= 0) return e;

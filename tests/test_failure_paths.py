@@ -51,6 +51,31 @@ def test_fir_injected_failures_drain_and_recover(B, N):
     assert failed >= 3
 
 
+@pytest.mark.parametrize("on_device", [False, True])
+@pytest.mark.parametrize("T,N", [(64, 16), (64, 63), (20, 500)])
+def test_fir_stream_injected_failures_keep_the_history(T, N, on_device):
+    """A call of which any operation fails leaves the history as it was, also where the block is
+    shorter than the history."""
+    C, blocks = 3, 9
+    rng = np.random.default_rng(T + N)
+    x = rng.integers(-4096, 4096, size=(C, blocks * N)).astype(np.int16)
+    h = rng.integers(-4096, 4096, size=(1, T)).astype(np.int16)
+    want = oracle.fir(np.concatenate([np.zeros((C, T - 1), np.int16), x], axis=1), h, T, nch=0)
+    dev = lambda a: torch.from_numpy(a).cuda() if on_device else a
+    st = D.FirStream(D.INT16, C, N, T, nch=0)
+    failed = 0
+    for b in range(blocks):
+        xb, hd, out = (dev(np.ascontiguousarray(a)) for a in (x[:, b * N:(b + 1) * N], h, np.zeros((C, N), np.int16)))
+        assert D.lib().DSPLIB_gpu_injectFault(st.h, b + 1) == D.SUCCESS
+        try:
+            y = st.exec(xb, hd, out)
+        except D.DsplibError:
+            failed += 1
+            y = st.exec(xb, hd, out)
+        assert np.array_equal(y.cpu().numpy() if on_device else y, want[:, b * N:(b + 1) * N]), b
+    assert failed >= 3
+
+
 @pytest.mark.parametrize("N,pinned", [(65536, True), (1000, False)])
 def test_biquad_injected_failures_drain_and_recover(N, pinned):
     C, S = 32, 4
