@@ -539,8 +539,9 @@ __global__ void __launch_bounds__(W * 32, 16 / W) biquad_scan_kernel(BiquadLaunc
    const int cw = w * SUB + sub; // chunk within the CTA's
    // lanes beyond the last channel run along on that channel's data and store nothing, so that
    // lengths are the same over the warp
-   const bool active = blockIdx.y * CH + lane < a.C;
-   const int ch = active ? blockIdx.y * CH + lane : a.C - 1;
+   const int c0 = (int) (CLUSTER ? blockIdx.y : blockIdx.x) * CH; // without clusters the groups lie along x, which takes more than 65535
+   const bool active = c0 + lane < a.C;
+   const int ch = active ? c0 + lane : a.C - 1;
    int K = 1, rank = 0;
    if (CLUSTER) {
       cg::cluster_group cl = cg::this_cluster();
@@ -1042,13 +1043,12 @@ template <int FORM, int W, int L, int SUB = 1> cudaError_t launchScanShape(const
    }
    const int K = SUB == 1 && want > 1 ? pickCluster<FORM, W, L>(want, maxBytes) : 1;
    const size_t bytes = scanSmemBytes<W, L, SUB>(a, K);
-   dim3 grid(K, groups);
    if (K == 1) {
-      fn1<<<grid, block, bytes, s>>>(a);
+      fn1<<<groups, block, bytes, s>>>(a);
    }
    else {
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = grid;
+      cfg.gridDim = dim3(K, groups);
       cfg.blockDim = block;
       cfg.dynamicSmemBytes = bytes;
       cfg.stream = s;

@@ -207,6 +207,22 @@ def test_opt_single_sample_multi_stage(C):
         assert np.max(np.abs(host(sd) - s_ref)) <= 1e-5 * max(1.0, float(np.max(np.abs(s_ref)))), form
 
 
+@pytest.mark.parametrize("form", FORMS)
+def test_opt_more_than_a_million_channels(form):
+    """More groups of 16 channels than a grid's second dimension holds (65535)."""
+    N, C, S = 2, 16 * 65535 + 21, 1
+    rng = np.random.default_rng(form)
+    x = rng.standard_normal((N, C)).astype(np.float32)
+    nat = stable_sections(rng, 1, S)
+    st = np.zeros((S * nv(form), C), np.float32)
+    opt, _ = D.opt_coefficients(nat, form, 0, C)
+    sd = dev(st)
+    y = host(D.cascade_biquad(dev(x), dev(opt), sd, form=form, nch=0))
+    y32, st32, y64, _ = oracle_run(form, x, nat, st, 0)
+    assert np.max(np.abs(y - y64)) <= 1e-5 * np.max(np.abs(y64))
+    assert np.max(np.abs(host(sd) - st32)) <= 1e-5 * np.max(np.abs(st32))
+
+
 def test_opt_in_place():
     rng = np.random.default_rng(3)
     N, C, S = 10000, 32, 4
