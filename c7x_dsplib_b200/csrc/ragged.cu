@@ -575,7 +575,7 @@ static BankLaunch bankLaunch(const RaggedPlan *p, const float *work)
    b.bucketStart = p->bucketStart.data();
    b.nBuckets = (int) p->bucketS.size();
    b.aux = p->aux;
-   b.nAux = p->nAux;
+   b.nAux = p->bucketS.size() > 1 ? p->nAux : 0; // one bucket stays on the caller's stream
    b.fork = p->fork;
    b.join = p->join;
    return b;

@@ -366,6 +366,60 @@ def test_bank_poles_near_unit_circle(radius):
         xo, ho, co = xo + L, ho + T, co + 5 * S
 
 
+def _bank_tensors(lengths, taps, stages, seed):
+    """A bank and two sets of tensors for its calls: (bank, x, h, c, gy, sets), a set being
+    y, work, gx, gtaps, gcoefs, scratch."""
+    import torch
+
+    from c7x_dsplib_b200.filterbank import RaggedFilterBank
+
+    bank = RaggedFilterBank(lengths, taps, stages)
+    gen = torch.Generator("cuda").manual_seed(seed)
+    n, nh, nk, nw, ns = (bank.sizes[k] for k in range(5))
+    x, gy = (torch.randn(n, device="cuda", generator=gen) for _ in range(2))
+    h = torch.randn(nh, device="cuda", generator=gen) / 4
+    c = torch.tensor([0.5, 0.2, 0.1, -0.9, 0.4], device="cuda").repeat(nk // 5)
+    sets = [[torch.empty(k, device="cuda") for k in (n, nw, n, nh, nk, ns)] for _ in range(2)]
+    return bank, x, h, c, gy, sets
+
+
+def _beside_a_capture(lengths, taps, stages):
+    """Forward and adjoint of a plan, eager on another stream, while a capture that holds a forward of
+    the same plan goes on: both give what they give alone."""
+    import torch
+
+    bank, x, h, c, gy, (a, b) = _bank_tensors(lengths, taps, stages, len(lengths))
+
+    def call(t):
+        bank.forward_raw(x, h, c, t[0], t[1])
+        bank.backward_raw(x, h, c, t[1], gy, *t[2:])
+
+    call(a)
+    want = [t.clone() for t in (a[0], *a[2:5])]
+    side = torch.cuda.Stream()
+    for t in (*a, *b):
+        t.fill_(7.0)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        bank.forward_raw(x, h, c, a[0], a[1])
+        with torch.cuda.stream(side):
+            call(b)
+        bank.backward_raw(x, h, c, a[1], gy, *a[2:])
+    g.replay()
+    torch.cuda.synchronize()
+    for t in (a, b):
+        for u, v in zip((t[0], *t[2:5]), want):
+            assert torch.equal(u, v)
+    del g
+
+
+@pytest.mark.gpu
+def test_uniform_plan_eager_beside_a_capture():
+    """One stage count, few samples: the eager calls stay on their stream altogether."""
+    _beside_a_capture([3000] * 5, [17] * 5, [3] * 5)
+
+
 @pytest.mark.gpu
 def test_bank_deep_cascades_beyond_shared_memory():
     """24 and 22 stages beside shallow ones: the unit transitions of deep cascades
