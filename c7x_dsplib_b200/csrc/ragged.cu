@@ -575,30 +575,44 @@ static BankLaunch bankLaunch(const RaggedPlan *p, const float *work)
    b.bucketStart = p->bucketStart.data();
    b.nBuckets = (int) p->bucketS.size();
    b.aux = p->aux;
-   b.nAux = p->bucketS.size() > 1 ? p->nAux : 0; // one bucket stays on the caller's stream
    b.fork = p->fork;
    b.join = p->join;
    return b;
 }
 
+// Whether a call on s may use the plan's auxiliary streams: between the first use in a capture of s
+// and the capture's end they belong to that capture, and calls on other streams do without.
+// The caller holds forkMu.
+static bool auxFree(const RaggedPlan *p, cudaStream_t s)
+{
+   cudaStreamCaptureStatus mine = cudaStreamCaptureStatusNone, theirs = cudaStreamCaptureStatusNone;
+   unsigned long long id = 0, other = 0;
+   bool ok = cudaStreamGetCaptureInfo(s, &mine, &id) == cudaSuccess;
+   for (int i = 0; ok && i < p->nAux; i++)
+      ok = cudaStreamGetCaptureInfo(p->aux[i], &theirs, &other) == cudaSuccess &&
+           (theirs == cudaStreamCaptureStatusNone ||
+            (theirs == cudaStreamCaptureStatusActive && mine == cudaStreamCaptureStatusActive && other == id));
+   if (!ok) (void) cudaGetLastError();
+   return ok && p->nAux > 0;
+}
+
 // Work beside the main stream s: sideBegin returns the plan's first auxiliary stream, ordered
 // behind what s holds so far (s itself where the side stream is not used), sideJoin orders s
 // behind its end.  Capturable; the caller holds forkMu.
-// Outside a capture the small plans stay on one stream: there the host sets the pace, and a fork
+// Outside a capture the small plans' side work stays on the one stream: there the host sets the pace, and a fork
 // and a join are four calls to it (forward and backward of 8 channels of at most 4096 samples: 176 us
 // with, 166 without, 256 channels of at most 30 thousand 253 to 268 with, 226 to 261 without, at
 // most 262 thousand 398 with, 412 without; a captured step of 57 channels 105 with, 115 without).
+// (The adjoint's buckets of units are spread at any size: launchBankBackward.)
 constexpr long long kSideMinSamples = 2LL << 20;
 static bool sideUsed(const RaggedPlan *p, cudaStream_t s)
 {
-   if (p->nAux == 0) return false;
-   if (p->totalLen >= kSideMinSamples) return true;
-   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-   if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
-      (void) cudaGetLastError();
-      return false;
+   if (p->totalLen < kSideMinSamples) {
+      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+      if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) (void) cudaGetLastError();
+      if (cs != cudaStreamCaptureStatusActive) return false;
    }
-   return cs == cudaStreamCaptureStatusActive;
+   return auxFree(p, s);
 }
 static cudaError_t sideBegin(const RaggedPlan *p, cudaStream_t s, cudaStream_t *side)
 {
@@ -636,6 +650,7 @@ static cudaError_t launchFirAndTables(const RaggedPlan *p, const BankLaunch &b, 
 static cudaError_t launchAdjoint(const RaggedPlan *p, BankLaunch &b, const float *x, const float *taps, float *gx,
                                  float *gtaps, float *scratch, cudaStream_t s)
 {
+   b.nAux = p->bucketS.size() > 1 && auxFree(p, s) ? p->nAux : 0; // one bucket stays on the caller's stream
    cudaError_t e = launchBankBackward(b, s);
    cudaStream_t side = s;
    if (e == cudaSuccess) e = sideBegin(p, s, &side);

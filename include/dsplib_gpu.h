@@ -208,7 +208,8 @@ typedef enum {
 
 /** Build a plan (per-channel offsets and work lists, uploaded to the current
  *  device).  1 <= T_c <= 512, T_c <= L_c, 0 <= S_c <= 64, else
- *  DSPLIB_ERR_INVALID_DIMENSION.  The plan may be used from any stream of that device. */
+ *  DSPLIB_ERR_INVALID_DIMENSION.  The plan may be used from any stream of that device,
+ *  also while one of its calls is in a stream capture. */
 DSPLIB_STATUS DSPLIB_gpu_raggedPlanCreate(DSPLIB_gpu_raggedPlan *plan, int32_t numChannels, const int32_t *length,
                                           const int32_t *taps, const int32_t *stages);
 /** Buffer sizes in floats (DSPLIB_gpu_raggedSize); -1 for an unknown query. */

@@ -421,6 +421,48 @@ def test_uniform_plan_eager_beside_a_capture():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("lengths", [[3000, 700, 5000, 1100], [600_000] * 4], ids=["small", "large"])
+def test_plan_eager_beside_a_capture(lengths):
+    """Several stage counts, and more samples than calls outside a capture leave on one stream."""
+    _beside_a_capture(lengths, [17, 16, 3, 1], [3, 1, 2, 0])
+
+
+@pytest.mark.gpu
+def test_plan_in_two_captures_at_once():
+    import torch
+
+    bank, x, h, c, gy, sets = _bank_tensors([3000, 700, 5000], [17, 16, 3], [3, 1, 2], 4)
+
+    def call(t):
+        bank.forward_raw(x, h, c, t[0], t[1])
+        bank.backward_raw(x, h, c, t[1], gy, *t[2:])
+
+    call(sets[0])
+    want = [t.clone() for t in (sets[0][0], *sets[0][2:5])]
+    streams, graphs = [torch.cuda.Stream() for _ in sets], [torch.cuda.CUDAGraph() for _ in sets]
+    for t in (*sets[0], *sets[1]):
+        t.fill_(7.0)
+    torch.cuda.synchronize()
+    for s, g in zip(streams, graphs):
+        with torch.cuda.stream(s):
+            g.capture_begin(capture_error_mode="relaxed")
+    for _ in range(2):  # in turn
+        for s, t in zip(streams, sets):
+            with torch.cuda.stream(s):
+                call(t)
+    for s, g in zip(streams, graphs):
+        with torch.cuda.stream(s):
+            g.capture_end()
+    for g in graphs:
+        g.replay()
+    torch.cuda.synchronize()
+    for t in sets:
+        for u, v in zip((t[0], *t[2:5]), want):
+            assert torch.equal(u, v)
+    del graphs
+
+
+@pytest.mark.gpu
 def test_bank_deep_cascades_beyond_shared_memory():
     """24 and 22 stages beside shallow ones: the unit transitions of deep cascades
     (48 x 48 state) and the adjoint's per-stage sequences in shared memory."""
