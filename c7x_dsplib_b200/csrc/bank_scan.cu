@@ -568,6 +568,24 @@ __device__ __forceinline__ void forwardStage(P2 (&v)[kL], float2 entry, const fl
    }
 }
 
+// One stage of the reverse cascade over a unit that starts (at its end in time) from a zero state,
+// in place; lane 0 returns the state at the unit's beginning in time.
+__device__ __forceinline__ float2 reverseStageZero(P2 (&g)[kL], const float *tb, int lane)
+{
+   const StageCoef c = stageCoef(tb);
+   P2 n1, n2;
+   zeroStateEndRev(g, c, n1, n2);
+   chunkStateDown(n1, n2, make_float2(0.0f, 0.0f), tb, lane, n1, n2);
+#pragma unroll
+   for (int i = kL - 1; i >= 0; i--) {
+      const P2 v = fma2(c.na1, n1, fma2(c.na2, n2, g[i]));
+      g[i] = fma2(c.b0, v, fma2(c.b1, n1, mul2(c.b2, n2)));
+      n2 = n1;
+      n1 = v;
+   }
+   return make_float2(up(n1).x, up(n2).x);
+}
+
 // A unit's per-stage states, read once: lane l holds stage l in lo and stage l + 32 in hi
 // (up to 64 stages); entryAt broadcasts stage p.
 struct UnitStates {
@@ -591,7 +609,6 @@ struct UnitArgs {
    int nUnits;
    int Smax;
    const float *tables;
-   const float *impulse; // impulse responses of the aggregates
    const float *in;   // forward: FIR output plane; adjoint aggregates: output gradient (packed)
    float *out;        // y (packed, tail zeros)
    float2 *agg;       // unit aggregates, 2 floats per stage (processing order)
@@ -623,131 +640,55 @@ __device__ __forceinline__ void loadTables(float *dst, const float *tables, cons
    __syncwarp();
 }
 
-// ---- unit aggregates by impulse responses
-//
-// Tables of a channel of two units or more, per direction and processing position p, 1024
-// floats in the order the dot products read them: 16-byte group 32 j + l holds lane l's pairs
-// 2 j and 2 j + 1 of the sequence r, r[t] = k_p[1023 - t] forward, k_p[t] adjoint.
-__device__ __forceinline__ const float *impulseOf(const float *impulse, const RaggedChan &c, bool adj, int p)
+// Aggregates of a unit (held by the warp, overwritten): its stages' end states from a zero state.
+template <bool ADJ>
+__device__ __forceinline__ void unitAggregates(P2 (&v)[kL], const float *sTab, int S, float2 *agg, int lane)
 {
-   return impulse + c.impOff + (long long) ((adj ? c.S : 0) + p) * kUnit;
-}
-
-// One warp per channel and direction: the cascade's response to a unit impulse at the unit's
-// start, every stage's internal sequence written out.
-__global__ void __launch_bounds__(64) bank_impulse_kernel(const RaggedChan *chans, const int *list, int Smax,
-                                                          const float *tables, float *impulse)
-{
-   extern __shared__ float4 dynI[];
-   const int lane = threadIdx.x & 31, adj = threadIdx.x >> 5;
-   const RaggedChan c = chans[list[blockIdx.x]];
-   float *sTab = (float *) dynI + (size_t) adj * Smax * kBankTabFloats;
-   loadTables(sTab, tables, c, lane);
-   P2 v[kL], w[kL];
-#pragma unroll
-   for (int i = 0; i < kL; i++) v[i] = dup(0.0f);
-   if (lane == 0) v[0] = pk(1.0f, 0.0f);
-   for (int p = 0; p < c.S; p++) {
-      forwardStage(v, make_float2(0.0f, 0.0f), sTab + stageAt(p, c.S, adj) * kBankTabFloats, lane,
-                   [&](int i, P2 q) { w[i] = q; });
-      float4 *dst = (float4 *) (impulse + c.impOff + (long long) ((adj ? c.S : 0) + p) * kUnit);
-#pragma unroll
-      for (int j = 0; j < kL / 2; j++) {
-         if (adj) {
-            const float2 a = up(w[2 * j]), b = up(w[2 * j + 1]);
-            dst[32 * j + lane] = make_float4(a.x, a.y, b.x, b.y);
-         }
-         else { // reversed: lane 31 - l, chunks exchanged
-            const float2 a = up(w[kL - 1 - 2 * j]), b = up(w[kL - 2 - 2 * j]);
-            dst[32 * j + 31 - lane] = make_float4(a.y, a.x, b.y, b.x);
-         }
-      }
-   }
-}
-
-// Aggregates of one or two (N) units of a channel whose samples the warp holds: two dot
-// products a stage and unit.  Bound by the tables' reads through L1, 36 cycles a stage, which
-// two units share.
-template <bool ADJ, int N>
-__device__ __forceinline__ void unitAggregates(const P2 (&v)[N][kL], const float *impulse, const RaggedChan &c,
-                                               float2 *agg0, float2 *agg1, int lane)
-{
-   for (int p = 0; p < c.S; p++) {
-      const ulonglong2 *src = (const ulonglong2 *) impulseOf(impulse, c, ADJ, p) + lane;
-      P2 k[kL];
-#pragma unroll
-      for (int j = 0; j < kL / 2; j++) {
-         const ulonglong2 q = src[32 * j];
-         k[2 * j] = P2{q.x};
-         k[2 * j + 1] = P2{q.y};
-      }
-      // second component: r[t - 1] (adjoint) or r[t + 1]; the pair that reaches into the next lane's
-      P2 edge;
+   for (int p = 0; p < S; p++) {
+      const float *tb = sTab + stageAt(p, S, ADJ) * kBankTabFloats;
       if (ADJ) {
-         const float2 e = up(k[kL - 1]);
-         const float before = __shfl_up_sync(0xffffffffu, e.y, 1);
-         edge = pk(lane == 0 ? 0.0f : before, e.x);
+         const float2 e = reverseStageZero(v, tb, lane);
+         if (lane == 0) agg[p] = e;
       }
       else {
-         const float2 e = up(k[0]);
-         const float after = __shfl_down_sync(0xffffffffu, e.x, 1);
-         edge = pk(e.y, lane == 31 ? 0.0f : after);
-      }
-#pragma unroll
-      for (int n = 0; n < N; n++) {
-         P2 x = mul2(k[0], v[n][0]), y = mul2(edge, v[n][ADJ ? 0 : kL - 1]);
-#pragma unroll
-         for (int i = 1; i < kL; i++) {
-            x = fma2(k[i], v[n][i], x);
-            y = ADJ ? fma2(k[i - 1], v[n][i], y) : fma2(k[i], v[n][i - 1], y);
-         }
-         const float2 xs = up(x), ys = up(y);
-         const float sx = xs.x + xs.y, sy = ys.x + ys.y;
-         // both sums over the warp: the upper half keeps the second component
-         const bool hi = lane & 16;
-         float r = (hi ? sy : sx) + __shfl_xor_sync(0xffffffffu, hi ? sx : sy, 16);
-#pragma unroll
-         for (int o = 8; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-         if ((lane & 15) == 0) ((float *) ((n ? agg1 : agg0) + p))[lane >> 4] = r;
+         P2 w1, w2;
+         forwardStage(v, make_float2(0.0f, 0.0f), tb, lane, [&](int i, P2 w) {
+            if (i == kL - 1) w1 = w;
+            if (i == kL - 2) w2 = w;
+         });
+         if (lane == 31) agg[p] = make_float2(up(w1).y, up(w2).y);
       }
    }
 }
 
 // Pass 1.  ADJ = false: every unit of the FIR output plane but its channel's last (whose end
 // no unit starts from); ADJ = true: every unit of the packed output gradient but the first.
-// A warp takes two consecutive units of the list, mostly of one channel.
 template <bool ADJ> __global__ void __launch_bounds__(kThreads) bank_agg_kernel(UnitArgs a)
 {
+   extern __shared__ float4 dynG[];
    __shared__ __align__(16) float sStage[kWarps][kStage];
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-   const int ui = 2 * (blockIdx.x * kWarps + warp);
+   const int ui = blockIdx.x * kWarps + warp;
    if (ui >= a.nUnits) return;
-   const int2 U0 = a.units[ui], U1 = ui + 1 < a.nUnits ? a.units[ui + 1] : make_int2(-1, 0);
-   const RaggedChan c0 = a.chans[U0.x], c1 = a.chans[U1.x < 0 ? U0.x : U1.x];
-   const bool need0 = ADJ ? U0.y > 0 : (U0.y + 1) * kUnit < c0.Lu;
-   const bool need1 = U1.x >= 0 && (ADJ ? U1.y > 0 : (U1.y + 1) * kUnit < c1.Lu);
-   if (!need0 && !need1) return;
-   P2 v[2][kL];
+   float *sTab = (float *) dynG + (size_t) warp * a.Smax * kBankTabFloats;
+   const int2 U = a.units[ui];
+   const RaggedChan c = a.chans[U.x];
+   const int t0 = U.y * kUnit;
+   if (c.S == 0 || (ADJ ? U.y == 0 : t0 + kUnit >= c.Lu)) return;
+   P2 v[kL];
    if (ADJ) {
       float r[kLane];
-      fetchUnit(r, a.in + c0.xOff, U0.y * kUnit, need0 ? c0.Lu : 0, lane);
-      stageUnit(v[0], r, sStage[warp], lane);
-      fetchUnit(r, a.in + c1.xOff, U1.y * kUnit, need1 ? c1.Lu : 0, lane);
-      stageUnit(v[1], r, sStage[warp], lane);
+      fetchUnit(r, a.in + c.xOff, t0, c.Lu, lane);
+      loadTables(sTab, a.tables, c, lane);
+      stageUnit(v, r, sStage[warp], lane);
    }
    else {
-      float4 r0[kL / 2], r1[kL / 2];
-      fetchPlane(r0, a.in + c0.pOff, U0.y * kUnit, need0 ? c0.Lu : 0, lane);
-      fetchPlane(r1, a.in + c1.pOff, U1.y * kUnit, need1 ? c1.Lu : 0, lane);
-      stagePlane(v[0], r0, sStage[warp], lane);
-      stagePlane(v[1], r1, sStage[warp], lane);
+      float4 r[kL / 2];
+      fetchPlane(r, a.in + c.pOff, t0, c.Lu, lane);
+      loadTables(sTab, a.tables, c, lane);
+      stagePlane(v, r, sStage[warp], lane);
    }
-   float2 *agg0 = a.agg + c0.ckOff + (long long) U0.y * c0.S, *agg1 = a.agg + c1.ckOff + (long long) U1.y * c1.S;
-   if (need0 && need1 && U0.x == U1.x) unitAggregates<ADJ, 2>(v, a.impulse, c0, agg0, agg1, lane);
-   else {
-      if (need0) unitAggregates<ADJ, 1>(*(const P2 (*)[1][kL]) &v[0], a.impulse, c0, agg0, agg0, lane);
-      if (need1) unitAggregates<ADJ, 1>(*(const P2 (*)[1][kL]) &v[1], a.impulse, c1, agg1, agg1, lane);
-   }
+   unitAggregates<ADJ>(v, sTab, c.S, a.agg + c.ckOff + (long long) U.y * c.S, lane);
 }
 
 // Pass 3: y from the checkpoints; with MSE also the loss gradient, the unit's sum of squares
@@ -805,8 +746,7 @@ __global__ void __launch_bounds__(kThreads) bank_unit_kernel(UnitArgs a)
       storeUnit(v, a.gy + c.xOff, t0, Lu, sStage[warp], lane);
       if (t0 + kUnit >= Lu)
          for (int t = Lu + lane; t < c.L; t += 32) a.gy[c.xOff + t] = 0.0f;
-      if (U.y > 0)
-         unitAggregates<true, 1>(*(const P2 (*)[1][kL]) &v, a.impulse, c, a.aggA + base, a.aggA + base, lane);
+      if (U.y > 0) unitAggregates<true>(v, sTab, S, a.aggA + base, lane);
    }
 }
 
@@ -976,7 +916,7 @@ __global__ void __launch_bounds__(32 * kCoefWarps) bank_coef_kernel(const Ragged
 long long bankTransitionDoubles(int S) { return 8LL * S * (S + 1); } // Phi and Phi^32, both directions
 
 cudaError_t launchBankTables(const BankLaunch &b, const float *coefs, int totalStages, float *tables, double *phi,
-                             float *impulse, cudaStream_t s)
+                             cudaStream_t s)
 {
    if (totalStages <= 0) return cudaSuccess;
    bank_tables_kernel<<<(totalStages + 127) / 128, 128, 0, s>>>(coefs, totalStages, tables);
@@ -987,14 +927,6 @@ cudaError_t launchBankTables(const BankLaunch &b, const float *coefs, int totalS
    // 2 x 2 for 8 stages): the squarings' barriers then cost a warp, not four
    bank_transition_kernel<<<dim3(b.C, 2), b.Smax <= 8 ? 32 : 128, dyn, s>>>(b.chans, coefs, phi);
    countLaunch(2);
-   if (b.nImpulse > 0) {
-      const size_t dynI = (size_t) 2 * b.Smax * kBankTabFloats * sizeof(float);
-      if ((e = cudaFuncSetAttribute(bank_impulse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dynI)) !=
-          cudaSuccess)
-         return e;
-      bank_impulse_kernel<<<b.nImpulse, 64, dynI, s>>>(b.chans, b.impulseList, b.Smax, tables, impulse);
-      countLaunch();
-   }
    return cudaGetLastError();
 }
 
@@ -1019,8 +951,11 @@ template <bool MSE> static cudaError_t launchUnits(const UnitArgs &a, cudaStream
 // Aggregates of every unit that another starts from; none where every channel is one unit.
 template <bool ADJ> static cudaError_t launchAggregates(const BankLaunch &b, const UnitArgs &a, cudaStream_t s)
 {
-   if (b.nImpulse <= 0) return cudaSuccess;
-   bank_agg_kernel<ADJ><<<(a.nUnits + 2 * kWarps - 1) / (2 * kWarps), kThreads, 0, s>>>(a);
+   if (b.nUnits == b.C) return cudaSuccess;
+   const size_t dyn = unitShared(a.Smax);
+   cudaError_t e = cudaFuncSetAttribute(bank_agg_kernel<ADJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dyn);
+   if (e != cudaSuccess) return e;
+   bank_agg_kernel<ADJ><<<(a.nUnits + kWarps - 1) / kWarps, kThreads, dyn, s>>>(a);
    countLaunch();
    return cudaGetLastError();
 }
@@ -1028,7 +963,7 @@ template <bool ADJ> static cudaError_t launchAggregates(const BankLaunch &b, con
 cudaError_t launchBankForward(const BankLaunch &b, cudaStream_t s)
 {
    if (b.nUnits <= 0) return cudaSuccess;
-   UnitArgs a{b.chans, b.units, b.nUnits, b.Smax, b.tables, b.impulse, b.u, nullptr, b.aggF, nullptr};
+   UnitArgs a{b.chans, b.units, b.nUnits, b.Smax, b.tables, b.u, nullptr, b.aggF, nullptr};
    cudaError_t e = launchAggregates<false>(b, a, s);
    if (e != cudaSuccess) return e;
    const size_t dynC = (size_t) (4 * b.Smax * (b.Smax + 1) / 2 + 2 * b.Smax) * sizeof(double);
@@ -1059,7 +994,7 @@ cudaError_t launchBankBackward(const BankLaunch &b, cudaStream_t s)
    if (b.nUnits <= 0) return cudaSuccess;
    cudaError_t e = cudaSuccess;
    if (!b.aggReady) {
-      UnitArgs a{b.chans, b.units, b.nUnits, b.Smax, b.tables, b.impulse, b.gy, nullptr, b.aggA, nullptr};
+      UnitArgs a{b.chans, b.units, b.nUnits, b.Smax, b.tables, b.gy, nullptr, b.aggA, nullptr};
       if ((e = launchAggregates<true>(b, a, s)) != cudaSuccess) return e;
    }
    const size_t dynC = (size_t) (4 * b.Smax * (b.Smax + 1) / 2 + 2 * b.Smax) * sizeof(double);

@@ -310,7 +310,6 @@ struct RaggedChan {
    long long ckOff;  // first unit state (float2) of the channel: one per 1024-sample unit and stage
    long long phiOff; // first double of the channel's unit transitions
    long long grpOff; // first float of the channel's chain group states (2S per 32 units)
-   long long impOff; // first float of its impulse responses (channels of two units or more)
 };
 // Split-BF16x3 tensor-core FIR over a list of runs {channel, first tile, tiles, 0}
 // of kFirBfTile outputs: forward (valid correlation of the channel's x with its
@@ -331,8 +330,7 @@ cudaError_t launchFirBf16x3Ragged(const RaggedChan *chans, const int4 *runs, int
 // Cascade of the filter bank split along time (bank_scan.cu): units of kBankSpan
 // samples (one warp each), chained per channel through the 2S-dimensional cascade
 // state; per stage a table of kBankTabFloats floats (coefficients, transition
-// powers), per channel the unit transitions and, where it has two units
-// or more, the impulse responses of both directions.
+// powers), per channel the unit transitions of both directions.
 constexpr int kBankSpan = 1024;
 constexpr int kBankTabFloats = 44;
 
@@ -344,9 +342,6 @@ struct BankLaunch {
    int Smax;
    const float *tables;
    const double *phi;
-   const float *impulse;
-   const int *impulseList; // the channels of two units or more
-   int nImpulse;
    const float *u;    // FIR output plane
    float *y;          // forward output
    const float *gy;   // adjoint: output gradient
@@ -377,7 +372,7 @@ struct BankLaunch {
 // Doubles of both unit transitions of a channel of S stages.
 long long bankTransitionDoubles(int S);
 cudaError_t launchBankTables(const BankLaunch &b, const float *coefs, int totalStages, float *tables, double *phi,
-                             float *impulse, cudaStream_t s);
+                             cudaStream_t s);
 cudaError_t launchBankForward(const BankLaunch &b, cudaStream_t s);
 cudaError_t launchBankBackward(const BankLaunch &b, cudaStream_t s);
 // The coefficient gradients from the partial sums that the backward pass leaves.

@@ -27,7 +27,8 @@
 //   mse_partial_kernel / mse_reduce_kernel  loss and its gradient.
 //
 // Work buffer (forward -> adjoint, floats): FIR output plane (sum of round16(Lu)),
-// forward checkpoints, forward unit aggregates, stage tables, unit transitions.
+// forward checkpoints, forward unit aggregates, stage tables, unit transitions, chain group
+// states.
 // Scratch (adjoint): gradient w.r.t. u, adjoint aggregates and checkpoints,
 // coefficient-gradient partial sums per unit and stage, taps-gradient partials
 // (also the loss partials).
@@ -65,12 +66,10 @@ struct RaggedPlan {
    int nDhRuns = 0;
    int2 *dUnits = nullptr;      // cascade units (channel, unit index)
    int *dChainOrder = nullptr;  // channels by unit count, most first: the chains' CTA order
-   int *dImpulse = nullptr;     // channels of two units or more (with stages): impulse responses
-   int nImpulse = 0;
    int *err = nullptr;          // error word of the tensor-core kernels (mapped page-locked)
    int device = 0;
    // work buffer layout (float offsets)
-   long long wCk = 0, wAgg = 0, wTab = 0, wPhi = 0, wGrp = 0, wImp = 0, wTotal = 0;
+   long long wCk = 0, wAgg = 0, wTab = 0, wPhi = 0, wGrp = 0, wTotal = 0;
    // scratch layout (float offsets)
    long long sAgg = 0, sCk = 0, sGrp = 0, sPart = 0, sLoss = 0, sDh = 0, sTotal = 0;
    // host-buffer steps: the channel table, and contiguous channel segments (each with a
@@ -217,7 +216,6 @@ static void freePlan(RaggedPlan *p)
    cudaFree(p->dDhRuns);
    cudaFree(p->dUnits);
    cudaFree(p->dChainOrder);
-   cudaFree(p->dImpulse);
    freeErrorWord(p->err);
    for (RaggedPlan::Segment &g : p->segs) freePlan(g.plan);
    for (int i = 0; i < p->nAux; i++) {
@@ -288,8 +286,7 @@ static DSPLIB_STATUS raggedPlanBuild(DSPLIB_gpu_raggedPlan *plan, int32_t numCha
       const int tiles = (outLen + kFirBfTile - 1) / kFirBfTile;
       for (int t = 0; t < tiles; t += runTiles) runs.push_back(make_int4(c, t, std::min(runTiles, tiles - t), 0));
    };
-   long long xo = 0, ho = 0, co = 0, po = 0, ck = 0, ph = 0, gr = 0, im = 0;
-   std::vector<int> impulse;
+   long long xo = 0, ho = 0, co = 0, po = 0, ck = 0, ph = 0, gr = 0;
    for (int c = 0; c < numChannels; c++) {
       const int L = length[c], T = taps[c], S = stages[c];
       if (T < 1 || T > kFirBfMaxTaps || L < T || S < 0 || S > kRaggedMaxStages) {
@@ -298,11 +295,7 @@ static DSPLIB_STATUS raggedPlanBuild(DSPLIB_gpu_raggedPlan *plan, int32_t numCha
       }
       const int Lu = L - T + 1;
       const int nu = (Lu + kBankSpan - 1) / kBankSpan;
-      ch[c] = RaggedChan{xo, ho, co, po, L, T, S, Lu, xo, ck, ph, gr, im};
-      if (nu > 1 && S > 0) {
-         impulse.push_back(c);
-         im += 2LL * S * kBankSpan;
-      }
+      ch[c] = RaggedChan{xo, ho, co, po, L, T, S, Lu, xo, ck, ph, gr};
       gr += 2LL * S * ((nu + 31) / 32);
       po += (Lu + 15) & ~15;
       ck += (long long) nu * S;
@@ -396,15 +389,13 @@ static DSPLIB_STATUS raggedPlanBuild(DSPLIB_gpu_raggedPlan *plan, int32_t numCha
       (void) cudaGetLastError(); // without auxiliary streams everything runs in sequence
    }
    // work buffer: u | forward checkpoints | forward aggregates | stage tables | unit transitions |
-   // chain group states | impulse responses
+   // chain group states
    p->wCk = align4(p->planeStride);
    p->wAgg = p->wCk + align4(2 * p->nCk);
    p->wTab = p->wAgg + align4(2 * p->nCk);
    p->wPhi = p->wTab + (long long) kBankTabFloats * p->totalStages;
    p->wGrp = p->wPhi + align4(2 * p->nPhi);
-   p->wImp = p->wGrp + align4(p->nGrp);
-   p->wTotal = p->wImp + im;
-   p->nImpulse = (int) impulse.size();
+   p->wTotal = p->wGrp + align4(p->nGrp);
    // scratch: g | adjoint aggregates | adjoint checkpoints | coefficient partials | taps partials
    p->sAgg = align4(p->totalLen);
    p->sCk = p->sAgg + align4(2 * p->nCk);
@@ -416,8 +407,7 @@ static DSPLIB_STATUS raggedPlanBuild(DSPLIB_gpu_raggedPlan *plan, int32_t numCha
    const bool ok = upload(&p->dChan, ch) == cudaSuccess && upload(&p->dFwdItems, fwd) == cudaSuccess &&
                    upload(&p->dFirFwdRuns, firFwd) == cudaSuccess && upload(&p->dFirDxRuns, firDx) == cudaSuccess &&
                    upload(&p->dDhStart, start) == cudaSuccess && upload(&p->dDhRuns, dhRuns) == cudaSuccess &&
-                   upload(&p->dUnits, units) == cudaSuccess && upload(&p->dChainOrder, chainOrder) == cudaSuccess &&
-                   upload(&p->dImpulse, impulse) == cudaSuccess;
+                   upload(&p->dUnits, units) == cudaSuccess && upload(&p->dChainOrder, chainOrder) == cudaSuccess;
    if (!ok) {
       freePlan(p);
       return DSPLIB_ERR_FAILURE;
@@ -564,9 +554,6 @@ static BankLaunch bankLaunch(const RaggedPlan *p, const float *work)
    b.Smax = p->Smax;
    b.tables = work + p->wTab;
    b.phi = (const double *) (work + p->wPhi);
-   b.impulse = work + p->wImp;
-   b.impulseList = p->dImpulse;
-   b.nImpulse = p->nImpulse;
    b.u = work;
    b.aggF = (float2 *) (work + p->wAgg);
    b.ckptF = (float2 *) (work + p->wCk);
@@ -630,8 +617,8 @@ static cudaError_t sideJoin(const RaggedPlan *p, cudaStream_t s)
    return e != cudaSuccess ? e : cudaStreamWaitEvent(s, p->sideDone, 0);
 }
 
-// FIR forward, and beside it the stage tables, unit transitions and impulse responses, which
-// depend on the coefficients alone (77 us on the 2048-channel bank, 45 us on 256 channels).
+// FIR forward, and beside it the stage tables and unit transitions, which depend on the
+// coefficients alone.
 static cudaError_t launchFirAndTables(const RaggedPlan *p, const BankLaunch &b, const float *x, const float *taps,
                                       const float *coefs, float *work, cudaStream_t s)
 {
@@ -640,7 +627,7 @@ static cudaError_t launchFirAndTables(const RaggedPlan *p, const BankLaunch &b, 
    if (e == cudaSuccess)
       e = launchFirBf16x3Ragged(p->dChan, p->dFirFwdRuns, p->nFirFwdRuns, x, taps, work, false, p->Tmax, p->err, s);
    if (e == cudaSuccess)
-      e = launchBankTables(b, coefs, p->totalStages, work + p->wTab, (double *) (work + p->wPhi), work + p->wImp, side);
+      e = launchBankTables(b, coefs, p->totalStages, work + p->wTab, (double *) (work + p->wPhi), side);
    const cudaError_t j = sideJoin(p, s);
    return e != cudaSuccess ? e : j;
 }

@@ -197,12 +197,13 @@ typedef enum {
    DSPLIB_GPU_RAGGED_COEFS = 2,   /* floats in coefs / gcoefs (5 sum S_c) */
    DSPLIB_GPU_RAGGED_WORK = 3,    /* floats the forward leaves for the adjoint: the FIR output
                                      (sum_c round16(L_c - T_c + 1) floats), one 2-float state per
-                                     512 samples and stage (the cascade's checkpoints) and the
-                                     unit aggregates, per-stage tables and per-channel unit
-                                     transitions: about 4 bytes per sample plus 0.03 per sample
-                                     and stage; no stage output is kept */
+                                     1024 samples and stage (the cascade's checkpoints), as much
+                                     for the unit aggregates, and per channel 176 S + 64 S (S + 1)
+                                     bytes of stage tables and unit transitions: about 4 bytes
+                                     per sample plus 0.016 per sample and stage on long
+                                     channels; no stage output is kept */
    DSPLIB_GPU_RAGGED_SCRATCH = 4, /* floats of adjoint scratch (about 4 bytes per sample plus
-                                     0.07 per sample and stage) */
+                                     0.036 per sample and stage) */
    DSPLIB_GPU_RAGGED_OUTPUTS = 5, /* valid output samples (sum L_c - T_c + 1) */
 } DSPLIB_gpu_raggedSize;
 

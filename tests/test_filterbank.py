@@ -366,6 +366,22 @@ def test_bank_poles_near_unit_circle(radius):
         xo, ho, co = xo + L, ho + T, co + 5 * S
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("C,L,T,S", [(1, 5, 5, 1), (7, 1100, 64, 8), (5, 2049, 1, 64), (3, 5000, 17, 16), (2, 300000, 256, 4)])
+def test_plan_sizes(C, L, T, S):
+    """Work and scratch stay within the sizes that the header states."""
+    from c7x_dsplib_b200.filterbank import SCRATCH, WORK, RaggedFilterBank
+
+    sizes = RaggedFilterBank([L] * C, [T] * C, [S] * C).sizes
+    out = L - T + 1
+    units, groups = -(-out // 1024), -(-out // 32768)
+    work = 4 * -(-out // 16) * 16 + 16 * units * S + 176 * S + 64 * S * (S + 1) + 8 * S * groups
+    assert 4 * sizes[WORK] <= C * work + 6 * 16
+    runs = -(-out // 8192)
+    scratch = 4 * L + 36 * units * S + 8 * S * groups + 4 * 512 * runs
+    assert 4 * sizes[SCRATCH] <= C * (scratch + 8 * units) + 8 * 16
+
+
 def _bank_tensors(lengths, taps, stages, seed):
     """A bank and two sets of tensors for its calls: (bank, x, h, c, gy, sets), a set being
     y, work, gx, gtaps, gcoefs, scratch."""
