@@ -22,11 +22,14 @@
 // Phi z + e, where e is the end state when every stage starts the unit from
 // zero and Phi = A_c^1024, A_c the cascade's 2S x 2S one-step transition (block
 // lower-triangular: stage p's output drives stage p + 1).  So:
-//   pass 1 (bank_agg_kernel): e of every unit but the channel's last, as dot products of
-//           the unit's input with the impulse responses k_s from the cascade's input to each
-//           stage's internal sequence (bank_impulse_kernel, once per channel):
-//           e_s = (sum_t k_s[1023 - t] u[t], sum_t k_s[1022 - t] u[t]), two multiply-adds a
-//           sample and stage instead of the seven of a filtering pass;
+//   pass 1 (bank_agg_kernel): e of every unit but the channel's last, by filtering it from a
+//           zero state.  (As dot products with the impulse responses from the cascade's
+//           input to each stage's internal sequence, two multiply-adds a sample and stage
+//           instead of seven: 1603 us a step against 1604 on 2048 channels of up to 262144
+//           samples, the adjoint 4 % faster on a thousand channels of 20000 samples and 12 to 24
+//           stages, the forward up to 17 % slower on channels of 1100 to 6000 samples; and the
+//           responses take 8 KB of work buffer a channel and stage, 138 MB instead of 70 for
+//           work and scratch of 4096 channels of 1100 samples and 8 stages.)
 //   pass 2 (bank_chain_fast_kernel up to 16 stages, bank_chain_kernel beyond):
 //           per channel, z_0 = 0, z_{j+1} = Phi z_j + e_j, j over the
 //           channel's units (in two levels through Phi^32 over groups of 32
