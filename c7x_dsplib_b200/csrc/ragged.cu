@@ -586,11 +586,12 @@ static bool auxFree(const RaggedPlan *p, cudaStream_t s)
 // Work beside the main stream s: sideBegin returns the plan's first auxiliary stream, ordered
 // behind what s holds so far (s itself where the side stream is not used), sideJoin orders s
 // behind its end.  Capturable; the caller holds forkMu.
-// Outside a capture the small plans' side work stays on the one stream: there the host sets the pace, and a fork
-// and a join are four calls to it (forward and backward of 8 channels of at most 4096 samples: 176 us
-// with, 166 without, 256 channels of at most 30 thousand 253 to 268 with, 226 to 261 without, at
-// most 262 thousand 398 with, 412 without; a captured step of 57 channels 105 with, 115 without).
-// (The adjoint's buckets of units are spread at any size: launchBankBackward.)
+// The loss of a step is summed there beside the adjoint, the tables of small captured plans beside the FIR
+// (tablesBeside).  Step with the loss beside the adjoint and behind the forward: 2048 channels of at most
+// 262144 samples 1612 and 1624 us, 256 channels 370 and 373, captured 57 channels of at most 5169 86 and 88.
+// Outside a capture the small plans stay on the one stream: there the host sets the pace, and a fork
+// and a join are four calls to it (forward and backward of 8 channels of at most 4096 samples with two
+// forks 176 us, without 166).  (The adjoint's buckets of units are spread at any size: launchBankBackward.)
 constexpr long long kSideMinSamples = 2LL << 20;
 static bool sideUsed(const RaggedPlan *p, cudaStream_t s)
 {
@@ -617,31 +618,43 @@ static cudaError_t sideJoin(const RaggedPlan *p, cudaStream_t s)
    return e != cudaSuccess ? e : cudaStreamWaitEvent(s, p->sideDone, 0);
 }
 
-// FIR forward, and beside it the stage tables and unit transitions, which depend on the
-// coefficients alone.
+// FIR forward and the stage tables and unit transitions, which depend on the coefficients alone:
+// side by side where the FIR's CTAs (one an SM) leave SMs free for the transitions' two CTAs a
+// channel, one to an SM or, single warps, two; else in turn.  CTAs that find every SM held by the
+// FIR are all placed on the first SMs that it leaves, and share them: 512 channels of at
+// most 4096 samples, 8 stages, captured, forward 105 us side by side and 63 in turn, 50 channels
+// of 60000 and 32 stages 427 and 354, 256 of at most 262144 143 and 133, 2048 521 and 525; with
+// SMs free 20 channels of at most 20000 32 and 40, 70 of at most 5169 46 and 51.
+static bool tablesBeside(const RaggedPlan *p, cudaStream_t s)
+{
+   const int sms = deviceSms() > 0 ? deviceSms() : 148;
+   return p->nFirFwdRuns + (p->Smax <= 8 ? 1 : 2) * (long long) p->C <= sms && sideUsed(p, s);
+}
+
 static cudaError_t launchFirAndTables(const RaggedPlan *p, const BankLaunch &b, const float *x, const float *taps,
                                       const float *coefs, float *work, cudaStream_t s)
 {
    cudaStream_t side = s;
-   cudaError_t e = sideBegin(p, s, &side);
+   const bool beside = tablesBeside(p, s);
+   cudaError_t e = beside ? sideBegin(p, s, &side) : cudaSuccess;
    if (e == cudaSuccess)
       e = launchFirBf16x3Ragged(p->dChan, p->dFirFwdRuns, p->nFirFwdRuns, x, taps, work, false, p->Tmax, p->err, s);
    if (e == cudaSuccess)
       e = launchBankTables(b, coefs, p->totalStages, work + p->wTab, (double *) (work + p->wPhi), side);
-   const cudaError_t j = sideJoin(p, s);
+   const cudaError_t j = beside ? sideJoin(p, s) : cudaSuccess;
    return e != cudaSuccess ? e : j;
 }
 
-// The adjoint behind the output gradient's aggregates: cascade, then the FIR's input and taps
-// gradients, with the coefficient gradients' sums beside them.
+// The adjoint behind the output gradient's aggregates: cascade, the coefficient gradients' sums, then
+// the FIR's input and taps gradients.  The sums are not run beside the FIR's kernels: their CTAs
+// either come first by luck or find every SM held, as above (16 channels of 400 to 900 thousand
+// samples: 23 us, or 222; backward 342 us captured, 476 eager).
 static cudaError_t launchAdjoint(const RaggedPlan *p, BankLaunch &b, const float *x, const float *taps, float *gx,
                                  float *gtaps, float *scratch, cudaStream_t s)
 {
    b.nAux = p->bucketS.size() > 1 && auxFree(p, s) ? p->nAux : 0; // one bucket stays on the caller's stream
    cudaError_t e = launchBankBackward(b, s);
-   cudaStream_t side = s;
-   if (e == cudaSuccess) e = sideBegin(p, s, &side);
-   if (e == cudaSuccess) e = launchBankCoefGradients(b, side);
+   if (e == cudaSuccess) e = launchBankCoefGradients(b, s);
    float *part = scratch + p->sDh;
    if (e == cudaSuccess)
       e = launchFirBf16x3Ragged(p->dChan, p->dFirDxRuns, p->nFirDxRuns, b.g, taps, gx, true, p->Tmax, p->err, s);
@@ -651,8 +664,7 @@ static cudaError_t launchAdjoint(const RaggedPlan *p, BankLaunch &b, const float
       countLaunch();
       e = cudaGetLastError();
    }
-   const cudaError_t j = sideJoin(p, s);
-   return e != cudaSuccess ? e : j;
+   return e;
 }
 
 DSPLIB_STATUS DSPLIB_gpu_firBiquadBatched_fwd(DSPLIB_gpu_raggedPlan plan, const float *x, const float *taps,
@@ -728,7 +740,8 @@ static DSPLIB_STATUS stepMseCore(RaggedPlan *p, const float *x, const float *tap
    b.part = scratch + p->sPart;
    b.gcoefs = gcoefs;
    b.aggReady = true;
-   return launchAdjoint(p, b, x, taps, gx, gtaps, scratch, s) == cudaSuccess ? DSPLIB_SUCCESS : DSPLIB_ERR_FAILURE;
+   const cudaError_t e = launchAdjoint(p, b, x, taps, gx, gtaps, scratch, s), j = sideJoin(p, s);
+   return e == cudaSuccess && j == cudaSuccess ? DSPLIB_SUCCESS : DSPLIB_ERR_FAILURE;
 }
 
 // Input bytes (x and target) per segment of a host-buffer step.

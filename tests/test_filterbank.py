@@ -444,6 +444,26 @@ def test_plan_eager_beside_a_capture(lengths):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("C,S", [(8, 3), (74, 8), (75, 8), (49, 9), (50, 9)])
+def test_captured_step_beside_and_in_turn(C, S):
+    """Captured steps of plans whose tables are made beside the FIR and of plans just too large for that
+    (one run a channel on 148 SMs) equal the eager calls."""
+    import torch
+
+    bank, x, h, c, target, (a, b) = _bank_tensors([1500] * C, [20] * C, [S] * C, C)
+    y, work, gx, gh, gc, scratch = a
+    gy, loss = torch.empty_like(x), torch.empty(1, device="cuda")
+    bank.step_mse_raw(x, h, c, target, y, gy, loss, gx, gh, gc, work, scratch)
+    replay, out = bank.graph_step(x, h, c, target)
+    for t in out.values():
+        t.fill_(7.0)
+    replay()
+    torch.cuda.synchronize()
+    for k, t in (("y", y), ("gx", gx), ("gtaps", gh), ("gcoefs", gc), ("loss", loss)):
+        assert torch.equal(out[k], t), k
+
+
+@pytest.mark.gpu
 def test_plan_in_two_captures_at_once():
     import torch
 
