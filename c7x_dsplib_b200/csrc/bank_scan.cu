@@ -72,6 +72,7 @@ constexpr int kRow = kLane + 2; // staging row of a lane's samples, pairs (A_i, 
 constexpr int kStage = 32 * kRow;
 constexpr int kUnitLog2 = 10;   // Phi = A_c^(2^10)
 constexpr int kChainFastStages = 16; // cascades the FP32 register chain takes
+constexpr int kChainGroup = 32;      // units of one of its groups
 
 static_assert(kUnit == kBankSpan, "unit size");
 
@@ -123,8 +124,8 @@ __host__ __device__ inline int blk(int p, int q) { return p * (p + 1) / 2 + q; }
 __device__ __forceinline__ int stageAt(int p, int S, bool adj) { return adj ? S - 1 - p : p; }
 
 // Phi = A_c^1024 for one channel and direction, one CTA: A_c in shared memory, ten
-// squarings C(p,q) = sum_{m=q..p} B(p,m) B(m,q) between two shared buffers; then
-// Phi^32.  Per channel: Phi forward, Phi adjoint, Phi^32 forward, Phi^32 adjoint.
+// squarings C(p,q) = sum_{m=q..p} B(p,m) B(m,q) between two shared buffers; then, where it is
+// used, Phi^32.  Per channel: Phi forward, Phi adjoint, Phi^32 forward, Phi^32 adjoint.
 __global__ void __launch_bounds__(128) bank_transition_kernel(const RaggedChan *chans, const float *coefs,
                                                               double *phi)
 {
@@ -191,7 +192,9 @@ __global__ void __launch_bounds__(128) bank_transition_kernel(const RaggedChan *
    }
    double *dst = phi + c.phiOff + (adj ? 4LL * nb : 0);
    for (int i = threadIdx.x; i < 4 * nb; i += blockDim.x) dst[i] = B[i];
-   // five more squarings: Phi^32, the transition over a group of 32 units
+   // five more squarings: Phi^32, the transition over a group of 32 units, where there are two
+   // groups and the chain takes them (bank_chain_fast_kernel)
+   if (S > kChainFastStages || c.Lu <= kChainGroup * kUnit) return;
    for (int it = 0; it < 5; it++) {
       for (int b = threadIdx.x; b < nb; b += blockDim.x) {
          int p = 0;
@@ -274,7 +277,6 @@ __global__ void __launch_bounds__(32) bank_chain_kernel(const RaggedChan *chans,
 // transition in registers; z is broadcast by shuffles.  Group states sit in shared
 // memory for channels of up to 48 groups, in the caller's buffer beyond.
 constexpr int kChainWarps = 8;
-constexpr int kChainGroup = 32;
 constexpr int kChainSharedGroups = 48;
 
 // Row r of a transition (lane r's) at rows[r * kRowPad + k], zero beyond n2 and above the
@@ -349,7 +351,7 @@ __global__ void __launch_bounds__(kChainWarps * 32) bank_chain_fast_kernel(const
       return j0;
    };
    loadRows(sRow[0], phi + c.phiOff + (adj ? 4LL * nb : 0), n2, threadIdx.x, blockDim.x);
-   loadRows(sRow[1], phi + c.phiOff + 8LL * nb + (adj ? 4LL * nb : 0), n2, threadIdx.x, blockDim.x);
+   if (groups > 1) loadRows(sRow[1], phi + c.phiOff + 8LL * nb + (adj ? 4LL * nb : 0), n2, threadIdx.x, blockDim.x);
    __syncthreads();
    const float *row = sRow[0] + lane * kRowPad;
    // 1. group aggregates from a zero state (the last group's is not needed)
