@@ -768,14 +768,35 @@ struct AdjArgs {
    float *g;             // gradient w.r.t. the FIR output (the scratch's plane)
    float *part;          // 5 coefficient-gradient sums per unit and stage
    int first;            // this launch's first unit (a bucket of one stage count)
+   int group;            // stages kept at once (adjointGroup)
 };
 
 // Stages whose sequences a unit keeps in shared memory at once; deeper cascades are taken in
 // groups of stages, last group first, the forward run again up to each: a unit of eight
 // stages runs twelve forward stages instead of eight but takes 17 KB instead of 34, and the
 // SM holds twelve warps instead of six (2048-channel bank step 1856 -> 1804 us; groups of
-// three 1803, five 1817, six 1844).
+// three 1803, five 1817, six 1844).  Deeper ones (us of the backward by group): 1000 channels of
+// 20000, 16 stages 4: 786, 8: 812, 16: 1070; 24 stages 4: 1295, 8: 1243, 24: 2060.  Where all units of the
+// plan are resident at once anyway, they keep as many stages as leaves them so: nothing is gained from
+// more warps there (64 channels of 1100, 64 stages 4: 264, 11: 167, 48: 125).
 constexpr int kAdjStages = 4;
+constexpr int kAdjWarps = 16;                    // a warp takes 128 registers a thread
+constexpr size_t kSmemSm = 228 * 1024, kSmemCta = 227 * 1024; // shared memory of an SM, and of one CTA
+
+static size_t adjointShared(int S, int group)
+{
+   const size_t seq = (size_t) group * kL * 32 * 2, stage = kStage;
+   return ((size_t) S * kBankTabFloats + (seq > stage ? seq : stage)) * sizeof(float);
+}
+static int adjointGroup(int S, int nUnits)
+{
+   const int sms = deviceSms() > 0 ? deviceSms() : 148, each = (nUnits + sms - 1) / sms; // units an SM
+   int group = S < kAdjStages ? S : kAdjStages;
+   while (each <= kAdjWarps && group < S && adjointShared(S, group + 1) <= kSmemCta &&
+          each * (adjointShared(S, group + 1) + 1024) <= kSmemSm)
+      group++;
+   return group;
+}
 
 // Stage sequences of one unit in shared memory: per stage of a group 16 rows of 32 pairs, so that
 // the lanes of the warp touch distinct banks.  One warp per CTA: the sequences are the bulk of the CTA's
@@ -806,7 +827,7 @@ __global__ void __launch_bounds__(32) bank_adjoint_kernel(AdjArgs a)
       stagePlane(v, r, sStage, lane);
    }
    for (int s1 = S; s1 > 0;) {
-      const int s0 = max(0, s1 - kAdjStages);
+      const int s0 = max(0, s1 - a.group);
       if (s1 < S) { // a further group: the unit's input again
          float4 r[kL / 2];
          __syncwarp();
@@ -936,13 +957,6 @@ cudaError_t launchBankTables(const BankLaunch &b, const float *coefs, int totalS
 }
 
 static size_t unitShared(int Smax) { return (size_t) kWarps * Smax * kBankTabFloats * sizeof(float); }
-static size_t adjointShared(int Smax)
-{
-   const int kept = Smax < kAdjStages ? Smax : kAdjStages;
-   const size_t seq = (size_t) kept * kL * 32 * 2, stage = kStage;
-   return ((size_t) Smax * kBankTabFloats + (seq > stage ? seq : stage)) * sizeof(float);
-}
-
 template <bool MSE> static cudaError_t launchUnits(const UnitArgs &a, cudaStream_t s)
 {
    const size_t dyn = unitShared(a.Smax);
@@ -1012,10 +1026,11 @@ cudaError_t launchBankBackward(const BankLaunch &b, cudaStream_t s)
       bank_chain_kernel<<<b.C, 32, dynC, s>>>(b.chans, b.chainOrder, b.phi, b.aggA, b.ckptA, 1);
       countLaunch();
    }
-   if ((e = cudaFuncSetAttribute(bank_adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int) adjointShared(b.Smax))) != cudaSuccess)
+   // the same limit for every plan: calls on several threads do not lower each other's
+   if ((e = cudaFuncSetAttribute(bank_adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kSmemCta)) !=
+       cudaSuccess)
       return e;
-   AdjArgs d{b.chans, b.units, b.nUnits, b.Smax, b.tables, b.u, b.gy, b.ckptF, b.ckptA, b.g, b.part, 0};
+   AdjArgs d{b.chans, b.units, b.nUnits, b.Smax, b.tables, b.u, b.gy, b.ckptF, b.ckptA, b.g, b.part, 0, 0};
    // One launch per stage count, each with the shared memory its cascades need, spread over
    // the caller's stream and the auxiliary ones so that CTAs of different buckets share the
    // SMs (and no launch waits for another's tail).
@@ -1030,7 +1045,8 @@ cudaError_t launchBankBackward(const BankLaunch &b, cudaStream_t s)
       const int n = b.bucketStart[k + 1] - b.bucketStart[k];
       if (n <= 0) continue;
       const cudaStream_t st = (k % lanes) == 0 ? s : b.aux[(k % lanes) - 1];
-      bank_adjoint_kernel<<<n, 32, adjointShared(b.bucketS[k]), st>>>(d);
+      d.group = adjointGroup(b.bucketS[k], b.nUnits);
+      bank_adjoint_kernel<<<n, 32, adjointShared(b.bucketS[k], d.group), st>>>(d);
       countLaunch();
    }
    for (int i = 0; i < b.nAux; i++) {

@@ -444,6 +444,28 @@ def test_plan_eager_beside_a_capture(lengths):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("S", [5, 8, 17, 64])
+def test_adjoint_stage_groups(S):
+    """A channel's results do not depend on how many units the plan has, and so not on how many stages
+    a unit of the adjoint keeps at once (all of them down to four)."""
+    import torch
+
+    want = None
+    for more in (0, 300, 1000, 5000):  # units beside the channel's three
+        bank, x, h, c, gy, (a, b) = _bank_tensors([3000, 1] + [1024] * more, [17, 1] + [1] * more, [S, 0] + [1] * more, S)
+        rng = torch.Generator("cuda").manual_seed(S)
+        x[:3000], gy[:3000] = (torch.randn(3000, device="cuda", generator=rng) for _ in range(2))
+        h[:17] = torch.randn(17, device="cuda", generator=rng)
+        bank.forward_raw(x, h, c, a[0], a[1])
+        bank.backward_raw(x, h, c, a[1], gy, *a[2:])
+        torch.cuda.synchronize()
+        got = [t.clone() for t in (a[0][:3000], a[2][:3000], a[3][:17], a[4][:5 * S])]
+        want = want or got
+        for u, v in zip(got, want):
+            assert torch.isfinite(u).all() and torch.equal(u, v), more
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("C,S", [(8, 3), (74, 8), (75, 8), (49, 9), (50, 9)])
 def test_captured_step_beside_and_in_turn(C, S):
     """Captured steps of plans whose tables are made beside the FIR and of plans just too large for that
