@@ -783,6 +783,11 @@ constexpr int kAdjStages = 4;
 constexpr int kAdjWarps = 16;                    // a warp takes 128 registers a thread
 constexpr size_t kSmemSm = 228 * 1024, kSmemCta = 227 * 1024; // shared memory of an SM, and of one CTA
 
+// Dynamic shared memory by the deepest cascade of a plan.  The kernels' limits are set for the deepest
+// that any plan has, always the same: calls on several threads do not lower each other's.
+static size_t transitionShared(int S) { return (size_t) 8 * S * (S + 1) / 2 * sizeof(double); }
+static size_t chainShared(int S) { return (size_t) (4 * S * (S + 1) / 2 + 2 * S) * sizeof(double); }
+static size_t unitShared(int S) { return (size_t) kWarps * S * kBankTabFloats * sizeof(float); }
 static size_t adjointShared(int S, int group)
 {
    const size_t seq = (size_t) group * kL * 32 * 2, stage = kStage;
@@ -946,23 +951,22 @@ cudaError_t launchBankTables(const BankLaunch &b, const float *coefs, int totalS
 {
    if (totalStages <= 0) return cudaSuccess;
    bank_tables_kernel<<<(totalStages + 127) / 128, 128, 0, s>>>(coefs, totalStages, tables);
-   const size_t dyn = (size_t) 8 * b.Smax * (b.Smax + 1) / 2 * sizeof(double);
-   cudaError_t e = cudaFuncSetAttribute(bank_transition_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dyn);
+   cudaError_t e = cudaFuncSetAttribute(bank_transition_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int) transitionShared(kRaggedMaxStages));
    if (e != cudaSuccess) return e;
    // one warp per (channel, direction) while the block count is small (up to 36 blocks of
    // 2 x 2 for 8 stages): the squarings' barriers then cost a warp, not four
-   bank_transition_kernel<<<dim3(b.C, 2), b.Smax <= 8 ? 32 : 128, dyn, s>>>(b.chans, coefs, phi);
+   bank_transition_kernel<<<dim3(b.C, 2), b.Smax <= 8 ? 32 : 128, transitionShared(b.Smax), s>>>(b.chans, coefs, phi);
    countLaunch(2);
    return cudaGetLastError();
 }
 
-static size_t unitShared(int Smax) { return (size_t) kWarps * Smax * kBankTabFloats * sizeof(float); }
 template <bool MSE> static cudaError_t launchUnits(const UnitArgs &a, cudaStream_t s)
 {
-   const size_t dyn = unitShared(a.Smax);
-   cudaError_t e = cudaFuncSetAttribute(bank_unit_kernel<MSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dyn);
+   cudaError_t e = cudaFuncSetAttribute(bank_unit_kernel<MSE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int) unitShared(kRaggedMaxStages));
    if (e != cudaSuccess) return e;
-   bank_unit_kernel<MSE><<<(a.nUnits + kWarps - 1) / kWarps, kThreads, dyn, s>>>(a);
+   bank_unit_kernel<MSE><<<(a.nUnits + kWarps - 1) / kWarps, kThreads, unitShared(a.Smax), s>>>(a);
    countLaunch();
    return cudaGetLastError();
 }
@@ -971,10 +975,10 @@ template <bool MSE> static cudaError_t launchUnits(const UnitArgs &a, cudaStream
 template <bool ADJ> static cudaError_t launchAggregates(const BankLaunch &b, const UnitArgs &a, cudaStream_t s)
 {
    if (b.nUnits == b.C) return cudaSuccess;
-   const size_t dyn = unitShared(a.Smax);
-   cudaError_t e = cudaFuncSetAttribute(bank_agg_kernel<ADJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dyn);
+   cudaError_t e = cudaFuncSetAttribute(bank_agg_kernel<ADJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int) unitShared(kRaggedMaxStages));
    if (e != cudaSuccess) return e;
-   bank_agg_kernel<ADJ><<<(a.nUnits + kWarps - 1) / kWarps, kThreads, dyn, s>>>(a);
+   bank_agg_kernel<ADJ><<<(a.nUnits + kWarps - 1) / kWarps, kThreads, unitShared(a.Smax), s>>>(a);
    countLaunch();
    return cudaGetLastError();
 }
@@ -985,14 +989,13 @@ cudaError_t launchBankForward(const BankLaunch &b, cudaStream_t s)
    UnitArgs a{b.chans, b.units, b.nUnits, b.Smax, b.tables, b.u, nullptr, b.aggF, nullptr};
    cudaError_t e = launchAggregates<false>(b, a, s);
    if (e != cudaSuccess) return e;
-   const size_t dynC = (size_t) (4 * b.Smax * (b.Smax + 1) / 2 + 2 * b.Smax) * sizeof(double);
    bank_chain_fast_kernel<<<b.C, kChainWarps * 32, 0, s>>>(b.chans, b.chainOrder, b.phi, b.aggF, b.ckptF, b.groupF, 0);
    countLaunch();
    if (b.Smax > kChainFastStages) {
-      if ((e = cudaFuncSetAttribute(bank_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dynC)) !=
-          cudaSuccess)
+      if ((e = cudaFuncSetAttribute(bank_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int) chainShared(kRaggedMaxStages))) != cudaSuccess)
          return e;
-      bank_chain_kernel<<<b.C, 32, dynC, s>>>(b.chans, b.chainOrder, b.phi, b.aggF, b.ckptF, 0);
+      bank_chain_kernel<<<b.C, 32, chainShared(b.Smax), s>>>(b.chans, b.chainOrder, b.phi, b.aggF, b.ckptF, 0);
       countLaunch();
    }
    a.out = b.y;
@@ -1016,17 +1019,15 @@ cudaError_t launchBankBackward(const BankLaunch &b, cudaStream_t s)
       UnitArgs a{b.chans, b.units, b.nUnits, b.Smax, b.tables, b.gy, nullptr, b.aggA, nullptr};
       if ((e = launchAggregates<true>(b, a, s)) != cudaSuccess) return e;
    }
-   const size_t dynC = (size_t) (4 * b.Smax * (b.Smax + 1) / 2 + 2 * b.Smax) * sizeof(double);
    bank_chain_fast_kernel<<<b.C, kChainWarps * 32, 0, s>>>(b.chans, b.chainOrder, b.phi, b.aggA, b.ckptA, b.groupA, 1);
    countLaunch();
    if (b.Smax > kChainFastStages) {
-      if ((e = cudaFuncSetAttribute(bank_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) dynC)) !=
-          cudaSuccess)
+      if ((e = cudaFuncSetAttribute(bank_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int) chainShared(kRaggedMaxStages))) != cudaSuccess)
          return e;
-      bank_chain_kernel<<<b.C, 32, dynC, s>>>(b.chans, b.chainOrder, b.phi, b.aggA, b.ckptA, 1);
+      bank_chain_kernel<<<b.C, 32, chainShared(b.Smax), s>>>(b.chans, b.chainOrder, b.phi, b.aggA, b.ckptA, 1);
       countLaunch();
    }
-   // the same limit for every plan: calls on several threads do not lower each other's
    if ((e = cudaFuncSetAttribute(bank_adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kSmemCta)) !=
        cudaSuccess)
       return e;

@@ -398,6 +398,7 @@ constexpr int kShortChunk = 32, kLongChunk = 64;
 constexpr int kPad = 33;        // row pitch (double2) of the chunk x channel tables
 constexpr int kMaxCluster = 16; // CTAs per cluster
 constexpr int kPowTableBytes = 80 * 1024;
+constexpr int kMaxSmemCta = 227 * 1024; // dynamic shared memory a CTA can have
 
 __host__ __device__ constexpr int ilog2c(int x) { return x <= 1 ? 0 : 1 + ilog2c(x / 2); }
 
@@ -1030,16 +1031,14 @@ template <int FORM, int W, int L, int SUB = 1> cudaError_t launchScanShape(const
    // the largest footprint this launch can take (tables + next-window buffer)
    const size_t maxBytes = lay.total + (a.prefetch ? (size_t) L * W * 32 * sizeof(float) : 0) +
                            (size_t) 2 * kMaxCluster * 32 * sizeof(float2);
+   // the same limit for every call: calls on several threads do not lower each other's
    static bool attrSet = false;
-   static size_t attrBytes = 0;
-   if (!attrSet || attrBytes < maxBytes) {
-      if ((e = cudaFuncSetAttribute(fn1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) maxBytes)) != cudaSuccess)
-         return e;
+   if (!attrSet) {
+      if ((e = cudaFuncSetAttribute(fn1, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemCta)) != cudaSuccess) return e;
       if (SUB == 1 &&
-          (e = cudaFuncSetAttribute(fnK, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) maxBytes)) != cudaSuccess)
+          (e = cudaFuncSetAttribute(fnK, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemCta)) != cudaSuccess)
          return e;
       attrSet = true;
-      attrBytes = maxBytes;
    }
    const int K = SUB == 1 && want > 1 ? pickCluster<FORM, W, L>(want, maxBytes) : 1;
    const size_t bytes = scanSmemBytes<W, L, SUB>(a, K);

@@ -331,6 +331,7 @@ cudaError_t launchFirBf16x3Ragged(const RaggedChan *chans, const int4 *runs, int
 // samples (one warp each), chained per channel through the 2S-dimensional cascade
 // state; per stage a table of kBankTabFloats floats (coefficients, transition
 // powers), per channel the unit transitions of both directions.
+constexpr int kRaggedMaxStages = 64; // deepest cascade of a plan
 constexpr int kBankSpan = 1024;
 constexpr int kBankTabFloats = 44;
 

@@ -438,7 +438,8 @@ template <typename T, int QMODE, int P> static cudaError_t launchIntTcP(const Fi
    using Sh = IntShape<T, P>;
    const size_t smem = Sh::smem(a.T);
    auto fn = fir_int_tc_kernel<T, QMODE, P>;
-   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+   // the same limit for every call: calls on several threads do not lower each other's
+   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) Sh::smem(kMaxTapsTc));
    if (e != cudaSuccess) return e;
    const uint32_t nt = (uint32_t) intTiles<T, P>(a);
    // persistent: one wave of resident CTAs striding over the runs (CTAs per SM: the autotuner's
@@ -1270,7 +1271,7 @@ cudaError_t launchFirBf16x3(const FirLaunch &a, cudaStream_t s)
    if (!firBf16x3Supported(a)) return cudaErrorNotSupported;
    const size_t smem = bfSmemBytes(a.T);
    cudaError_t e =
-       cudaFuncSetAttribute(fir_bf16x3_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+       cudaFuncSetAttribute(fir_bf16x3_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bfSmemBytes(kBfMaxTaps));
    if (e != cudaSuccess) return e;
    const int nt = (a.outSize + kBfTile - 1) / kBfTile;
    const int tpr = a.tuneTpc > 0 ? (a.tuneTpc < nt ? a.tuneTpc : nt) : bfTilesPerRun(nt, a.batch);
@@ -1289,7 +1290,7 @@ cudaError_t launchFirBf16x3Ragged(const RaggedChan *chans, const int4 *runs, int
    if (nRuns <= 0) return cudaSuccess;
    const size_t smem = bfSmemBytes(Tmax);
    cudaError_t e =
-       cudaFuncSetAttribute(fir_bf16x3_ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+       cudaFuncSetAttribute(fir_bf16x3_ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bfSmemBytes(kBfMaxTaps));
    if (e != cudaSuccess) return e;
    int sms = 148, dev = 0;
    if (cudaGetDevice(&dev) == cudaSuccess) (void) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -106,7 +106,6 @@ namespace {
 
 
 constexpr int kRTile = 2048; // samples per item of the taps-gradient partials and the loss
-constexpr int kRaggedMaxStages = 64;
 
 // Taps gradient: the per-run partial sums of fir_dh_bf16x3_kernel (fir_tc.cu), one
 // 512-float slot per run, slots of a channel consecutive and in time order, summed in

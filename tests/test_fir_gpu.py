@@ -561,6 +561,39 @@ def test_handles_on_concurrent_host_threads():
             assert np.array_equal(y, want)
 
 
+def test_threads_with_short_and_long_filters():
+    """Host threads that filter with few and with many taps at the same time: the kernels' shared memory
+    differs, and neither thread's calls limit the other's."""
+    import threading
+
+    errors = []
+
+    def work(T, dt, precision):
+        try:
+            x = rand(dt, (3, 9000), np.random.default_rng(T))
+            h = rand(dt, (3, T), np.random.default_rng(T + 1))
+            xd, hd = dev(x), dev(h)
+            s = torch.cuda.Stream()
+            want = out = None
+            for _ in range(400):
+                out = torch.zeros((3, 9000 - T + 1), dtype=xd.dtype, device="cuda")
+                D.fir(xd, hd, T, nch=1, precision=precision, out=out, stream=s)
+                s.synchronize()
+                want = out if want is None else want
+                assert torch.equal(out, want)
+        except Exception as e:  # reported below
+            errors.append(repr(e))
+
+    jobs = [(T, dt, p) for T in (3, 500) for dt, p in ((np.int8, 0), (np.int16, 0), (np.float32, D.FIR_BF16X3))]
+    jobs += [(2048, np.int8, 0), (2048, np.int16, 0)]
+    threads = [threading.Thread(target=work, args=j) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+
+
 # ------------------------------------------------------------------ float Q mode
 
 
