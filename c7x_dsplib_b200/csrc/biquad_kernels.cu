@@ -399,6 +399,11 @@ constexpr int kPad = 33;        // row pitch (double2) of the chunk x channel ta
 constexpr int kMaxCluster = 16; // CTAs per cluster
 constexpr int kPowTableBytes = 80 * 1024;
 constexpr int kMaxSmemCta = 227 * 1024; // dynamic shared memory a CTA can have
+// Deepest cascade whose coefficient and carry tables fit the scan kernel's
+// shared memory beside the next-window buffer and the cluster exchange rows
+// (28 B per stage and channel: 160 stages take 226.5 KB of the 227 KB in CTAs of
+// 16 warps); deeper cascades use the sequential kernel.
+constexpr int kScanMaxStages = 160;
 
 __host__ __device__ constexpr int ilog2c(int x) { return x <= 1 ? 0 : 1 + ilog2c(x / 2); }
 
@@ -427,9 +432,9 @@ struct ScanSmem {
    bool powTable;
 };
 
-template <int W, int SUB = 1> __host__ __device__ inline ScanSmem scanLayout(int S)
+template <int W, int SUB = 1> __host__ __device__ constexpr ScanSmem scanLayout(int S)
 {
-   ScanSmem o;
+   ScanSmem o{};
    size_t off = 0;
    o.E = off;
    off += (size_t) 2 * W * SUB * kPad * sizeof(float2); // two phases
@@ -1028,9 +1033,10 @@ template <int FORM, int W, int L, int SUB = 1> cudaError_t launchScanShape(const
    cudaError_t e;
    auto fn1 = biquad_scan_kernel<FORM, W, L, SUB, false>;
    auto fnK = biquad_scan_kernel<FORM, W, L, 1, true>;
-   // the largest footprint this launch can take (tables + next-window buffer)
-   const size_t maxBytes = lay.total + (a.prefetch ? (size_t) L * W * 32 * sizeof(float) : 0) +
-                           (size_t) 2 * kMaxCluster * 32 * sizeof(float2);
+   // the largest footprint this launch can take (tables + next-window buffer + exchange rows)
+   constexpr size_t buffers = (size_t) L * W * 32 * sizeof(float) + (size_t) 2 * kMaxCluster * 32 * sizeof(float2);
+   static_assert(scanLayout<W, SUB>(kScanMaxStages).total + buffers <= kMaxSmemCta, "the deepest cascade fits");
+   const size_t maxBytes = lay.total + buffers - (a.prefetch ? 0 : (size_t) L * W * 32 * sizeof(float));
    // the same limit for every call: calls on several threads do not lower each other's
    static bool attrSet = false;
    if (!attrSet) {
@@ -1143,11 +1149,7 @@ cudaError_t launchBiquadSequential(const BiquadLaunch &a, cudaStream_t s)
    return cudaErrorInvalidValue;
 }
 
-// Deepest cascade whose coefficient and carry tables fit the scan kernel's
-// shared memory beside the next-window buffer and the cluster exchange rows
-// (28 B per stage and channel: 160 stages take 222 KB of the 227 KB); deeper
-// cascades use the sequential kernel.
-int biquadScanMaxStages() { return 160; }
+int biquadScanMaxStages() { return kScanMaxStages; }
 
 std::string biquadTuneKey(const BiquadLaunch &a)
 {
