@@ -345,13 +345,19 @@ template <int GT> cudaError_t launchFew(const FirLaunch &a, cudaStream_t s)
    return cudaGetLastError();
 }
 
-// Up to 512 outputs of at least 1024 taps: the taps are split.  Both kernels do the same
-// multiply-adds, so the line lies where one CTA a channel (or a tile) leaves the GPU idle: a
-// batch below two CTAs an SM.
+// Up to 512 outputs of at least 1024 taps: the taps are split where one CTA a channel leaves SMs idle,
+// or keeps most of its threads idle for long enough.  A split channel costs 8 CTAs (50 us a thousand
+// channels up to 2048 taps), an undivided one its taps in turn.  In us, undivided / split, 128 outputs: up
+// to two channels an SM, 150 of 1024 taps 19 / 13, 296 of 1024 19 / 21, of 1280 23 / 21; up to five, 700 of
+// 1024 31 / 39, of 1280 39 / 39, of 1536 45 / 39; more, 1184 of 1536 51 / 63, 8000 of 2304 479 / 478, of 2560
+// 529 / 485; with 512 outputs a block holds fewer taps: 1184 of 3072 102 / 120, of 4096 133 / 125.
 bool firFewOutputs(const FirLaunch &a)
 {
    const int sms = deviceSms() > 0 ? deviceSms() : 148;
-   return a.outSize <= 512 && a.T >= 1024 && a.batch < 16 * sms;
+   if (a.outSize > 512 || a.T < 1024) return false;
+   if (a.batch <= 2 * sms) return true;
+   if (a.batch <= 5 * sms) return a.T >= 1536;
+   return a.T >= (a.outSize <= 256 ? 2560 : 4096);
 }
 
 template <typename T, int MODE> cudaError_t launchDirect(const FirLaunch &a, cudaStream_t s)

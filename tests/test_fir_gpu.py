@@ -226,6 +226,19 @@ def test_simt_float_edges(out, T):
     assert (got[:, out:] == 7.5).all()
 
 
+@pytest.mark.parametrize("B,out,T", [(296, 3, 1024), (297, 3, 1024), (297, 130, 1535), (297, 130, 1536), (740, 9, 1536),
+                                     (741, 9, 1536), (741, 9, 2559), (741, 9, 2560), (741, 257, 4095), (741, 257, 4096)])
+def test_simt_float_few_outputs_by_batch(B, out, T):
+    """Few outputs of many taps by channel count, both sides of the lines (148 SMs).  T roundings of at most
+    2^-24 of a partial sum each, independent in sign: the bar is four of their deviations."""
+    rng = np.random.default_rng(B + T)
+    x = rng.standard_normal((B, out + T - 1)).astype(np.float32)
+    h = (rng.standard_normal((B, T)) / np.sqrt(T)).astype(np.float32)
+    y = host(D.fir(dev(x), dev(h), T, nch=1, precision=D.FIR_SIMT))
+    y64 = oracle.fir_f64(x, h, T, nch=1)
+    assert (np.abs(y - y64).max(axis=1) <= 4 * np.sqrt(T) * 2.0 ** -24 * np.maximum(1, np.abs(y64).max(axis=1))).all()
+
+
 def lowpass(rng, rows, T):
     """Hamming-windowed sinc low-pass, cutoff U[0.05, 0.45], unit DC gain (stored tap order)."""
     n = np.arange(T) - (T - 1) / 2.0
