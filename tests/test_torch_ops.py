@@ -150,6 +150,33 @@ def test_fir_operator_gradients_edges(B, N, T, nch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("nch", [False, True])
+@pytest.mark.parametrize("B,N,T", [(1, 1, 1), (3, 40, 1), (2, 33, 33), (5, 1500, 64), (2, 700, 600), (1, 9, 4), (3, 5000, 500)])
+def test_fir_operator_gradients_accuracy(B, N, T, nch):
+    """The one-call gradients row by row.  A gradient is a sum of n products (T for the input's, N - T + 1
+    for the taps', over all channels where they share them): n roundings of at most 2^-24 of a
+    partial sum each, independent in sign; the bar is four of their deviations."""
+    import c7x_dsplib_b200.torch_ops  # noqa: F401
+
+    g = torch.Generator().manual_seed(B + N + T)
+    M = N - T + 1
+    x, h = torch.randn(B, N, generator=g), torch.randn(B if nch else 1, T, generator=g)
+    w = torch.randn(B, M, generator=g)
+    xd, hd = x.cuda().requires_grad_(), h.cuda().requires_grad_()
+    gx, gh = torch.autograd.grad(torch.ops.dsplib_gpu.fir(xd, hd, nch, 0, False, 0), (xd, hd), w.cuda())
+    rows = h.double().expand(B, T)
+    pad = torch.nn.functional.pad(w.double(), (T - 1, T - 1))
+    wx = torch.stack([(pad[l].unfold(0, T, 1) * rows[l]).sum(1) for l in range(B)])
+    wh = torch.stack([(x[l].double().unfold(0, M, 1) * w[l].double()).sum(1).flip(0) for l in range(B)])
+    if not nch:
+        wh = wh.sum(0, keepdim=True)
+    for got, want, n in ((gx, wx, T), (gh, wh, M * (1 if nch else B))):
+        peak = want.abs().amax(dim=1).clamp(min=1)
+        err = (got.double().cpu() - want).abs().amax(dim=1)
+        assert got.shape == want.shape and bool((err <= 4 * n ** 0.5 * 2.0 ** -24 * peak).all()), (err / peak).tolist()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("form", [0, 1, 2, 3])
 @pytest.mark.parametrize("nch", [False, True])
 def test_cascade_operator_gradients_match_fp64(form, nch):
