@@ -546,6 +546,7 @@ constexpr size_t kBfRawFloats = (size_t) kBfMaxBlocks * 64;
 constexpr size_t kBfPlane = (size_t) ((kBfMaxBlocks * 128 + 1023) & ~1023);
 __host__ __device__ constexpr size_t bfBandBytes(int T) { return (size_t) (bfK(T + 3) / 8 + 8) * 256; }
 __host__ __device__ constexpr size_t bfSmemBytes(int Tmax) { return 2048 + 4 * kBfPlane + kBfTile * 4 + 8 * kBfRawFloats + 2 * bfBandBytes(Tmax); }
+static_assert(kBfSplitWarps == 8, "a tile's flags are one 64-bit word");
 static_assert(bfSmemBytes(kBfMaxTaps) <= 227 * 1024, "two plane sets and two of the longest bands fit");
 
 struct BfSmem {
@@ -553,6 +554,7 @@ struct BfSmem {
    uint64_t *rawFull, *rawFree;              // one per raw slot
    uint64_t *edges;                          // the split warps have written a raw tile's edges
    uint32_t *tslot;
+   unsigned char *notFinite; // per tile (eight in turn) and split warp: it met a sample that is not finite
    unsigned char *sets, *bands;
    float *stage; // one output tile, 1024 floats per drain warp
    float *raw;
@@ -574,6 +576,7 @@ __device__ __forceinline__ BfSmem bfSmemLayout(unsigned char *smraw, int Tmax)
    L.rawFree = L.rawFull + 2;
    L.edges = L.rawFree + 2;
    L.tslot = (uint32_t *) (L.edges + 1);
+   L.notFinite = sm + 512;
    L.sets = sm + 1024;
    L.stage = (float *) (L.sets + 4 * kBfPlane);
    L.raw = L.stage + kBfTile;
@@ -637,12 +640,14 @@ __device__ __forceinline__ BfWindow bfTileWindow(const BfRun &r, int t, int bloc
 // block k, 16-byte chunk c = (i % 64) / 8 stored at k * 128 + ((c ^ (k & 7)) * 16), as hi and lo
 // BF16.  A thread takes 4 samples (consecutive lanes, consecutive addresses) and writes half a
 // chunk of each plane; its groups are 16 blocks apart, so they share c and k & 7.  The first
-// FULL of its up to GROUPS groups need no test.
+// FULL of its up to GROUPS groups need no test.  Returns bits of its samples that BF16 holds no
+// finite value for.
 template <int FULL, int GROUPS>
-__device__ __forceinline__ void bfSplit(const float *raw, int nQuad, unsigned char *hi, unsigned char *lo, int tid)
+__device__ __forceinline__ uint32_t bfSplit(const float *raw, int nQuad, unsigned char *hi, unsigned char *lo, int tid)
 {
    const int k = tid >> 4, off = k * 128 + ((((tid >> 1) & 7) ^ (k & 7)) << 4) + (tid & 1) * 8;
    const float4 *src = (const float4 *) raw + tid;
+   uint32_t bad = 0;
    hi += off;
    lo += off;
 #pragma unroll
@@ -660,8 +665,11 @@ __device__ __forceinline__ void bfSplit(const float *raw, int nQuad, unsigned ch
             splitBf16x2(f[u].z, f[u].w, hv.y, lv.y);
             *(uint2 *) (hi + (u0 + u) * (kBfSplitThreads * 8)) = hv;
             *(uint2 *) (lo + (u0 + u) * (kBfSplitThreads * 8)) = lv;
+            // an exponent of all ones carries into the sign
+            bad |= (((hv.x & 0x7f807f80u) + 0x00800080u) | ((hv.y & 0x7f807f80u) + 0x00800080u)) & 0x80008000u;
          }
    }
+   return bad;
 }
 
 // Taps band of a run.  Column n = 16 u + 8 v + i of the accumulator (u < 8, v = 0: hi taps,
@@ -686,6 +694,45 @@ __device__ __forceinline__ void bfBand(const BfRun &r, unsigned char *band, int 
       unsigned char *d = band + (c >> 3) * 256 + (c & 7) * 16;
       *(uint4 *) d = make_uint4(hv[0], hv[1], hv[2], hv[3]);
       *(uint4 *) (d + 128) = make_uint4(lv[0], lv[1], lv[2], lv[3]);
+   }
+}
+
+// A sample that is not finite makes the 64 outputs of every row NaN whose window holds it: row a
+// contracts the samples [64 a, 64 a + bfK(T)), most of them with zeros of the band.  The lead
+// makes the contracted window begin up to 3 samples earlier and end up to 15 later.  Outputs that
+// only such a sample spoiled are computed anew, in FP32 as the plain kernel does: rows of 32
+// outputs y[64 i + lane], row i's window at input index q0 + 64 i, `first` outputs into the row's 64.
+__device__ __noinline__ void bfRestoreRows(const float *x, long long inLen, long long q0, const float *h, int T, int reverse,
+                                           int lead, float *y, long long left, int first)
+{
+   const int lane = threadIdx.x & 31, K0 = bfK(T), K = bfK(T + lead);
+   auto spoils = [](float v) { return (__float_as_uint(__bfloat162float(__float2bfloat16_rn(v))) & 0x7f800000u) == 0x7f800000u; };
+   auto bad = [&](long long q) { return q >= 0 && q < inLen && spoils(x[q]); };
+   // lane = row: spoiled from outside its window, and not by its first samples
+   bool mine = false;
+   if (lane * kBfPhases < left) {
+      const long long q = q0 + lane * kBfPhases;
+      for (int k = 1; k <= lead; k++) mine = mine || bad(q - k);
+      for (int k = K0; k < K - lead; k++) mine = mine || bad(q + k);
+      for (int k = 0; k < 2; k++) mine = mine && !bad(q + k);
+   }
+   uint32_t rows = __ballot_sync(0xffffffffu, mine);
+   if (!rows) return;
+   bool tap = false;
+   for (int c = lane; c < T; c += 32) tap = tap || spoils(h[c]);
+   if (__any_sync(0xffffffffu, tap)) return;
+   for (; rows; rows &= rows - 1) {
+      const int row = __ffs(rows) - 1;
+      const long long q = q0 + row * kBfPhases;
+      bool inside = false;
+      for (int k = lane; k < K0; k += 32) inside = inside || bad(q + k);
+      if (__any_sync(0xffffffffu, inside)) continue;
+      float sum = 0.0f;
+      for (int c = 0; c < T; c++) {
+         const long long i = q + first + lane + c;
+         if (i >= 0 && i < inLen) sum = fmaf(x[i], h[reverse ? T - 1 - c : c], sum);
+      }
+      if (row * kBfPhases + lane < left) y[row * kBfPhases + lane] = sum;
    }
 }
 
@@ -769,8 +816,9 @@ __device__ __forceinline__ void bfIssue(int K, uint32_t ahi, uint32_t alo, uint3
 
 // The kernel body: `get(i)` describes run i (i < nRuns); runs are taken in turn by the
 // CTAs of the grid.  Every wait is bounded: a role whose wait gives up raises the error word
-// and leaves, and the others follow as theirs give up.
-template <typename Get>
+// and leaves, and the others follow as theirs give up.  LEAD = false: every run's lead is zero (the test
+// for samples that are not finite takes 2 % of the time).
+template <bool LEAD, typename Get>
 __device__ __forceinline__ void bfPipeline(const BfSmem &L, int nRuns, int *err, Get get)
 {
    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -816,8 +864,13 @@ __device__ __forceinline__ void bfPipeline(const BfSmem &L, int nRuns, int *err,
                raiseError(err);
                break;
             }
-            if (blocks >= kRows) bfSplit<kRows * 16 / kBfSplitThreads, kBfQuads>(L.slot(b), blocks * 16, L.hi(b), L.lo(b), tid);
-            else bfSplit<0, kBfQuads>(L.slot(b), blocks * 16, L.hi(b), L.lo(b), tid);
+            const uint32_t bad =
+                blocks >= kRows ? bfSplit<kRows * 16 / kBfSplitThreads, kBfQuads>(L.slot(b), blocks * 16, L.hi(b), L.lo(b), tid)
+                                : bfSplit<0, kBfQuads>(L.slot(b), blocks * 16, L.hi(b), L.lo(b), tid);
+            if (LEAD) {
+               const bool any = __any_sync(0xffffffffu, bad);
+               if (lane == 0) L.notFinite[(n & 7) * kBfSplitWarps + warp] = any;
+            }
             tc::fenceProxyAsync();
             __syncwarp();
             if (lane == 0) {
@@ -841,6 +894,16 @@ __device__ __forceinline__ void bfPipeline(const BfSmem &L, int nRuns, int *err,
             }
             tc::fenceAfterSync();
             bfDrain(r, L, tmem + (uint32_t) b * 128, b, t, warp - kBfSplitWarps, lane);
+            // tile n + 8 is split after accumulator n + 4 was freed by every drain warp
+            if (LEAD && *(const volatile uint64_t *) (L.notFinite + (n & 7) * kBfSplitWarps)) {
+               const BfRun q = get(i); // not held across the tiles
+               const int first = 32 * (1 - ((warp - kBfSplitWarps) >> 2));
+               const long long j0 = (long long) t * kBfTile + (warp & 3) * (32 * kBfPhases);
+               __syncwarp(); // the warp's outputs are stored
+               if (q.lead)
+                  bfRestoreRows(q.x, q.inLen, q.inShift + j0, q.h, q.T, q.reverse, q.lead, q.y + j0 + first,
+                                (long long) q.outLen - j0 - first, first);
+            }
          }
       }
    }
@@ -898,12 +961,12 @@ __device__ __forceinline__ void bfPipeline(const BfSmem &L, int nRuns, int *err,
 }
 
 // Dense batch: run i = tiles [part * tilesPerRun, ...) of channel i / parts.
-__global__ void __launch_bounds__(kBfCta, 1) fir_bf16x3_tc_kernel(FirLaunch a, int tilesPerRun)
+template <bool LEAD> __global__ void __launch_bounds__(kBfCta, 1) fir_bf16x3_tc_kernel(FirLaunch a, int tilesPerRun)
 {
    extern __shared__ __align__(16) unsigned char smraw[];
    const int nt = (a.outSize + kBfTile - 1) / kBfTile;
    const int parts = (nt + tilesPerRun - 1) / tilesPerRun;
-   bfPipeline(bfSmemLayout(smraw, a.T), a.batch * parts, a.err, [&](int i) {
+   bfPipeline<LEAD>(bfSmemLayout(smraw, a.T), a.batch * parts, a.err, [&](int i) {
       const int l = i / parts, part = i - l * parts;
       BfRun r;
       r.x = (const float *) a.x + (long long) l * a.inPitch;
@@ -929,7 +992,7 @@ __global__ void __launch_bounds__(kBfCta, 1)
                              const float *taps, float *out, int dx, int Tmax, int *err)
 {
    extern __shared__ __align__(16) unsigned char smraw[];
-   bfPipeline(bfSmemLayout(smraw, Tmax), nRuns, err, [&](int i) {
+   bfPipeline<true>(bfSmemLayout(smraw, Tmax), nRuns, err, [&](int i) {
       const int4 it = runs[i];
       const RaggedChan c = chans[it.x];
       BfRun r;
@@ -1270,15 +1333,17 @@ cudaError_t launchFirBf16x3(const FirLaunch &a, cudaStream_t s)
 {
    if (!firBf16x3Supported(a)) return cudaErrorNotSupported;
    const size_t smem = bfSmemBytes(a.T);
+   const bool aligned = ((uintptr_t) a.x & 15) == 0 && (a.batch == 1 || a.inPitch % 4 == 0); // no row has a lead
+   const auto fn = aligned ? fir_bf16x3_tc_kernel<false> : fir_bf16x3_tc_kernel<true>;
    cudaError_t e =
-       cudaFuncSetAttribute(fir_bf16x3_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bfSmemBytes(kBfMaxTaps));
+       cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bfSmemBytes(kBfMaxTaps));
    if (e != cudaSuccess) return e;
    const int nt = (a.outSize + kBfTile - 1) / kBfTile;
    const int tpr = a.tuneTpc > 0 ? (a.tuneTpc < nt ? a.tuneTpc : nt) : bfTilesPerRun(nt, a.batch);
    const long long runs = (long long) a.batch * ((nt + tpr - 1) / tpr);
    if (runs > INT_MAX) return cudaErrorInvalidValue;
    const int sms = deviceSms() > 0 ? deviceSms() : 148;
-   fir_bf16x3_tc_kernel<<<(int) std::min<long long>(runs, sms), kBfCta, smem, s>>>(a, tpr);
+   fn<<<(int) std::min<long long>(runs, sms), kBfCta, smem, s>>>(a, tpr);
    countLaunch();
    return cudaGetLastError();
 }

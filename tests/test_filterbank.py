@@ -466,6 +466,35 @@ def test_adjoint_stage_groups(S):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("v", [np.inf, np.nan])
+def test_bank_not_finite_samples(v):
+    """One sample of x and one of gy that are not finite, in channels without stages at any offset: of y
+    and gx they spoil the rows of 64 whose window holds them (whole groups of 16 samples) and no more."""
+    import torch
+
+    taps = [1, 2, 17, 34, 64, 255, 512, 3, 130]
+    lengths = [9001 + T + k for k, T in enumerate(taps)]
+    bank, x, h, c, gy, (a, _) = _bank_tensors(lengths, taps, [0] * len(taps), 11)
+    place = [0, 63, 64, 64 * 40 - 1, 64 * 128 - 2, 64 * 33 - 3, 700, 8191, 8999]
+    results = []
+    for bad in (False, True):
+        if bad:
+            for o, q in zip(bank.x_off, place):
+                x[o + q] = gy[o + q] = v
+        bank.forward_raw(x, h, c, a[0], a[1])
+        bank.backward_raw(x, h, c, a[1], gy, *a[2:])
+        results.append([t.cpu().numpy().copy() for t in (a[0], a[2])])
+    for k, (T, L, q) in enumerate(zip(taps, lengths, place)):
+        K = (63 + T + 15) // 16 * 16
+        for got, want, n, start in zip(results[1], results[0], (L - T + 1, L), (0, -(T - 1))):
+            got, want = (r[bank.x_off[k]:bank.x_off[k] + n] for r in (got, want))
+            row = np.arange(n) // 64 * 64 + start
+            clean = (q < row) | (q >= row + K)
+            assert clean.any() and np.isfinite(got[clean]).all(), (k, start)
+            assert np.abs(got[clean] - want[clean]).max() <= 1e-5 * np.abs(want).max(), (k, start)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("C,S", [(8, 3), (74, 8), (75, 8), (49, 9), (50, 9)])
 def test_captured_step_beside_and_in_turn(C, S):
     """Captured steps of plans whose tables are made beside the FIR and of plans just too large for that

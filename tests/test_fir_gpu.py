@@ -337,6 +337,40 @@ def _golden_cases():
     return case_keys(d, "f")
 
 
+@pytest.mark.parametrize("v", [np.inf, -np.inf, np.nan, 3.4e38])
+@pytest.mark.parametrize("T", [1, 2, 17, 34, 64, 255, 512])
+def test_bf16x3_not_finite_samples(T, v):
+    """A sample that is not finite, or not in BF16, spoils rows of 64 outputs (their windows are whole groups
+    of 16 samples) and no others, however the channel lies in memory; the rest is as exact as always."""
+    rng = np.random.default_rng(T)
+    B, N = 6, 9000 + T
+    place = [0, 63, 64, 64 * 40 - 1, 64 * 128 - 2, N - 1]
+    out = N - T + 1
+    x = rng.standard_normal((B, N)).astype(np.float32)
+    h = (rng.standard_normal((B, T)) / np.sqrt(T)).astype(np.float32)
+    y64 = oracle.fir_f64(x, h, T, nch=1)
+    for shift in range(4):
+        xv = x.copy()
+        for l, q in enumerate(place):
+            xv[l, q] = v
+        buf = torch.zeros(shift + B * (N + 1), device="cuda")
+        rows = buf[shift:].view(B, N + 1)
+        rows[:, :N] = dev(xv)
+        args, pin, pfilt, pout = D.fir_setup(D.FLOAT32, B, N, T, nch=1, in_pitch=N + 1)
+        hd = D.FirHandle()
+        assert hd.init(args, pin, pfilt, pout) == D.SUCCESS
+        hd.set_precision(D.FIR_BF16X3)
+        yd = torch.zeros((B, out), device="cuda")
+        assert hd.exec(rows, dev(h), yd) == D.SUCCESS
+        y = host(yd)
+        for l, q in enumerate(place):
+            row = np.arange(out) // 64 * 64
+            clean = (q < row) | (q >= row + (63 + T + 15) // 16 * 16)
+            assert clean.any() and np.isfinite(y[l, clean]).all(), (shift, l)
+            err = np.abs(y[l, clean] - y64[l, clean]).max() / np.abs(y64[l]).max()
+            assert err <= 1e-5, (shift, l, err)
+
+
 @pytest.mark.parametrize("key", _golden_cases())
 @pytest.mark.parametrize("style", [D.NATC, D.OPTIMIZED])
 def test_reference_flow_golden(golden_fir, key, style):
