@@ -77,9 +77,9 @@ constexpr int kChainGroup = 32;      // units of one of its groups
 static_assert(kUnit == kBankSpan, "unit size");
 
 // Stage table (floats): [0, 5) b0 b1 b2 a1 a2; [8 + 4k, 12 + 4k) P[k] = M^(2^k), M = A^16,
-// k = 0..8, row-major.
-constexpr int kTabP = 8;
-static_assert(kTabP + 4 * 9 <= kBankTabFloats && kBankTabFloats % 4 == 0, "stage table layout");
+// row-major: a lane's second chunk, its 32 samples, and 2, 4, 8 and 16 lanes.
+constexpr int kTabP = 8, kPowers = 6;
+static_assert(kTabP + 4 * kPowers <= kBankTabFloats && kBankTabFloats % 4 == 0, "stage table layout");
 
 __device__ __forceinline__ M2f tabP(const float *tb, int k)
 {
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(128) bank_tables_kernel(const float *coefs, in
    const double a1 = cf[3], a2 = cf[4];
    M2 M = {-a1, -a2, 1.0, 0.0};
    for (int r = 1; r < kL; r <<= 1) M = scan::mmul(M, M);
-   for (int k = 0; k <= 8; k++) {
+   for (int k = 0; k < kPowers; k++) {
       const M2f f = scan::toF(M);
       *(float4 *) (tb + kTabP + 4 * k) = make_float4(f.a, f.b, f.c, f.d);
       M = scan::mmul(M, M);

@@ -333,7 +333,7 @@ cudaError_t launchFirBf16x3Ragged(const RaggedChan *chans, const int4 *runs, int
 // powers), per channel the unit transitions of both directions.
 constexpr int kRaggedMaxStages = 64; // deepest cascade of a plan
 constexpr int kBankSpan = 1024;
-constexpr int kBankTabFloats = 44;
+constexpr int kBankTabFloats = 32;
 
 struct BankLaunch {
    const RaggedChan *chans;

@@ -198,7 +198,7 @@ typedef enum {
    DSPLIB_GPU_RAGGED_WORK = 3,    /* floats the forward leaves for the adjoint: the FIR output
                                      (sum_c round16(L_c - T_c + 1) floats), one 2-float state per
                                      1024 samples and stage (the cascade's checkpoints), as much
-                                     for the unit aggregates, and per channel 176 S + 64 S (S + 1)
+                                     for the unit aggregates, and per channel 128 S + 64 S (S + 1)
                                      bytes of stage tables and unit transitions: about 4 bytes
                                      per sample plus 0.016 per sample and stage on long
                                      channels; no stage output is kept */

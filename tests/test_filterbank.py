@@ -375,7 +375,7 @@ def test_plan_sizes(C, L, T, S):
     sizes = RaggedFilterBank([L] * C, [T] * C, [S] * C).sizes
     out = L - T + 1
     units, groups = -(-out // 1024), -(-out // 32768)
-    work = 4 * -(-out // 16) * 16 + 16 * units * S + 176 * S + 64 * S * (S + 1) + 8 * S * groups
+    work = 4 * -(-out // 16) * 16 + 16 * units * S + 128 * S + 64 * S * (S + 1) + 8 * S * groups
     assert 4 * sizes[WORK] <= C * work + 6 * 16
     runs = -(-out // 8192)
     scratch = 4 * L + 36 * units * S + 8 * S * groups + 4 * 512 * runs
