@@ -914,31 +914,40 @@ __global__ void __launch_bounds__(32) bank_adjoint_kernel(AdjArgs a)
    storeUnit(g, a.g + c.gOff, t0, Lu, sStage, lane);
 }
 
-// Coefficient gradients of one channel (one CTA, coefficients spread over its warps): per
-// coefficient, lane l adds the partial sums of units l, l + 32, ... in FP64, in that order,
-// four loads in flight, then a fixed butterfly adds the lanes' sums (bitwise repeatable).
-constexpr int kCoefWarps = 8;
-__global__ void __launch_bounds__(32 * kCoefWarps) bank_coef_kernel(const RaggedChan *chans, const float *part,
-                                                                    float *gcoefs)
+// Coefficient gradients of one channel (one CTA): its threads in groups of one thread a coefficient,
+// group g adds the partial sums of units g, g + G, ... in FP64, four loads in flight, so that the CTA
+// reads consecutive rows whole; then the groups' sums are added in order (bitwise repeatable).  Bound by
+// the latency of the longest channel's loads (lanes along the units, 160 bytes apart for 8 stages, took
+// 23 us on 16 channels of up to 900 thousand samples, now 12.7; 256 of up to 262144 13.0, now 8.0).
+constexpr int kCoefThreads = 512;
+static_assert(5 * kRaggedMaxStages <= kCoefThreads, "a thread a coefficient");
+__global__ void __launch_bounds__(kCoefThreads) bank_coef_kernel(const RaggedChan *chans, const float *part, float *gcoefs)
 {
+   __shared__ double sums[kCoefThreads];
    const RaggedChan c = chans[blockIdx.x];
-   const int S = c.S, units = (c.Lu + kUnit - 1) / kUnit, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-   for (int q = warp; q < 5 * S; q += kCoefWarps) {
-      const float *pq = part + c.ckOff * 5 + q;
-      const long long st = 5LL * S; // one unit's partial sums
+   const int n = 5 * c.S, units = (c.Lu + kUnit - 1) / kUnit;
+   if (n == 0) return;
+   const int G = kCoefThreads / n, g = threadIdx.x / n;
+   const float *p = part + c.ckOff * 5 + threadIdx.x; // unit g's row
+   const long long st = (long long) G * n;
+   if (g < G) {
       double acc = 0.0;
-      int j = lane;
-      for (; j + 96 < units; j += 128) {
-         const float v0 = pq[j * st], v1 = pq[(j + 32) * st], v2 = pq[(j + 64) * st], v3 = pq[(j + 96) * st];
+      int j = g;
+      for (; j + 3 * G < units; j += 4 * G, p += 4 * st) {
+         const float v0 = p[0], v1 = p[st], v2 = p[2 * st], v3 = p[3 * st];
          acc += (double) v0;
          acc += (double) v1;
          acc += (double) v2;
          acc += (double) v3;
       }
-      for (; j < units; j += 32) acc += (double) pq[j * st];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane == 0) gcoefs[c.cOff + q] = (float) acc;
+      for (; j < units; j += G, p += st) acc += (double) *p;
+      sums[threadIdx.x] = acc;
+   }
+   __syncthreads();
+   if (threadIdx.x < n) {
+      double acc = 0.0;
+      for (int k = 0; k < G; k++) acc += sums[k * n + threadIdx.x];
+      gcoefs[c.cOff + threadIdx.x] = (float) acc;
    }
 }
 
@@ -1060,7 +1069,7 @@ cudaError_t launchBankBackward(const BankLaunch &b, cudaStream_t s)
 cudaError_t launchBankCoefGradients(const BankLaunch &b, cudaStream_t s)
 {
    if (b.nUnits <= 0) return cudaSuccess;
-   bank_coef_kernel<<<b.C, 32 * kCoefWarps, 0, s>>>(b.chans, b.part, b.gcoefs);
+   bank_coef_kernel<<<b.C, kCoefThreads, 0, s>>>(b.chans, b.part, b.gcoefs);
    countLaunch();
    return cudaGetLastError();
 }
