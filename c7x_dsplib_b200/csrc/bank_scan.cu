@@ -44,8 +44,10 @@
 // checkpoints, keeping every stage's internal sequence w_s in shared memory,
 // and accumulates the coefficient gradients
 //     dL/db_i = sum_t g[t] w[t-i],   dL/da_i = -sum_t lambda[t] w[t-i]
-// in FP32 per unit, then in FP64 per channel in a fixed order (bank_coef_kernel):
+// in FP32 per unit, then in FP64 per channel in a fixed order (bank_sums_kernel):
 // bitwise repeatable.
+#include <algorithm>
+
 #include <cuda_runtime.h>
 
 #include "dsplib_internal.h"
@@ -919,15 +921,13 @@ __global__ void __launch_bounds__(32) bank_adjoint_kernel(AdjArgs a)
 // reads consecutive rows whole; then the groups' sums are added in order (bitwise repeatable).  Bound by
 // the latency of the longest channel's loads (lanes along the units, 160 bytes apart for 8 stages, took
 // 23 us on 16 channels of up to 900 thousand samples, now 12.7; 256 of up to 262144 13.0, now 8.0).
-constexpr int kCoefThreads = 512;
-static_assert(5 * kRaggedMaxStages <= kCoefThreads, "a thread a coefficient");
-__global__ void __launch_bounds__(kCoefThreads) bank_coef_kernel(const RaggedChan *chans, const float *part, float *gcoefs)
+constexpr int kSumThreads = 512;
+__device__ __forceinline__ void coefSums(const RaggedChan &c, const float *part, float *gcoefs)
 {
-   __shared__ double sums[kCoefThreads];
-   const RaggedChan c = chans[blockIdx.x];
+   __shared__ double sums[kSumThreads];
    const int n = 5 * c.S, units = (c.Lu + kUnit - 1) / kUnit;
    if (n == 0) return;
-   const int G = kCoefThreads / n, g = threadIdx.x / n;
+   const int G = blockDim.x / n, g = threadIdx.x / n; // launchBankSums: a thread a coefficient at least
    const float *p = part + c.ckOff * 5 + threadIdx.x; // unit g's row
    const long long st = (long long) G * n;
    if (g < G) {
@@ -949,6 +949,26 @@ __global__ void __launch_bounds__(kCoefThreads) bank_coef_kernel(const RaggedCha
       for (int k = 0; k < G; k++) acc += sums[k * n + threadIdx.x];
       gcoefs[c.cOff + threadIdx.x] = (float) acc;
    }
+}
+
+// Taps gradients of one channel: its runs' sums (512 a run, runs in time order) added in that order in
+// FP64, gtaps[T - 1 - c] = sum_run part[run][c].
+__device__ __forceinline__ void tapSums(const RaggedChan &c, int run0, int run1, const float *part, float *gtaps)
+{
+   for (int k = threadIdx.x; k < c.T; k += blockDim.x) {
+      double s = 0.0;
+      for (int i = run0; i < run1; i++) s += part[(long long) i * kFirBfMaxTaps + k];
+      gtaps[c.hOff + c.T - 1 - k] = (float) s;
+   }
+}
+
+// Both, the last of the adjoint, in one launch.
+__global__ void __launch_bounds__(kSumThreads) bank_sums_kernel(const RaggedChan *chans, const float *part, float *gcoefs,
+                                                                const int *dhStart, const float *dhPart, float *gtaps)
+{
+   const RaggedChan c = chans[blockIdx.x];
+   if (blockIdx.y == 0) coefSums(c, part, gcoefs);
+   else tapSums(c, dhStart[blockIdx.x], dhStart[blockIdx.x + 1], dhPart, gtaps);
 }
 
 } // namespace
@@ -1066,10 +1086,13 @@ cudaError_t launchBankBackward(const BankLaunch &b, cudaStream_t s)
    return cudaGetLastError();
 }
 
-cudaError_t launchBankCoefGradients(const BankLaunch &b, cudaStream_t s)
+cudaError_t launchBankSums(const BankLaunch &b, const int *dhStart, const float *dhPart, float *gtaps, cudaStream_t s)
 {
-   if (b.nUnits <= 0) return cudaSuccess;
-   bank_coef_kernel<<<b.C, kCoefThreads, 0, s>>>(b.chans, b.part, b.gcoefs);
+   static_assert(5 * kRaggedMaxStages <= kSumThreads, "a thread a coefficient");
+   // small CTAs where the channels are short (backward of 4096 channels of 1100 samples, 8 stages: 275 us with
+   // large ones, 250 with small ones)
+   const int least = std::max(128, (5 * b.Smax + 31) / 32 * 32);
+   bank_sums_kernel<<<dim3(b.C, 2), b.nUnits > 16 * b.C ? kSumThreads : least, 0, s>>>(b.chans, b.part, b.gcoefs, dhStart, dhPart, gtaps);
    countLaunch();
    return cudaGetLastError();
 }

@@ -376,8 +376,9 @@ cudaError_t launchBankTables(const BankLaunch &b, const float *coefs, int totalS
                              cudaStream_t s);
 cudaError_t launchBankForward(const BankLaunch &b, cudaStream_t s);
 cudaError_t launchBankBackward(const BankLaunch &b, cudaStream_t s);
-// The coefficient gradients from the partial sums that the backward pass leaves.
-cudaError_t launchBankCoefGradients(const BankLaunch &b, cudaStream_t s);
+// The coefficient gradients from the partial sums that the backward pass leaves, and the taps gradients
+// from those of the runs (channel c's: slots dhStart[c] .. dhStart[c + 1]).
+cudaError_t launchBankSums(const BankLaunch &b, const int *dhStart, const float *dhPart, float *gtaps, cudaStream_t s);
 
 struct BiquadLaunch {
    const float *x;

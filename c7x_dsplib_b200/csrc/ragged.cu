@@ -12,7 +12,7 @@
 //                          as split-BF16x3 tcgen05 contractions over runs of
 //                          8192-output tiles, one run per CTA.
 //   bank_tables_kernel, bank_transition_kernel, bank_unit_kernel, bank_chain_kernel,
-//   bank_adjoint_kernel, bank_coef_kernel (bank_scan.cu)
+//   bank_adjoint_kernel, bank_sums_kernel (bank_scan.cu)
 //                          the cascade split along time into 1024-sample units
 //                          (one warp each) chained per channel through the
 //                          cascade's 2S-dimensional state: unit aggregates, the
@@ -20,7 +20,7 @@
 //                          outputs; the adjoint the same in reverse time, with
 //                          each unit's forward recomputed from the checkpoints
 //                          (no stage output is stored).
-//   fir_dh_bf16x3_kernel (fir_tc.cu) / fir_dh_reduce_kernel  taps gradient
+//   fir_dh_bf16x3_kernel (fir_tc.cu), bank_sums_kernel  taps gradient
 //                          dh[T-1-c] = sum_j gu[j] x[j+c] as split-BF16x3
 //                          tcgen05 contractions over runs of 8192-sample tiles,
 //                          partial sums per run added in run order (deterministic).
@@ -115,17 +115,6 @@ constexpr int kDhMaxT = 512;
 // staged before any MMA and a diagonal-sum epilogue, so runs span up to 16 tiles
 // (131072 samples summed in FP32 in TMEM; runs added in FP64).
 constexpr int kDhRunTiles = 16;
-
-__global__ void __launch_bounds__(256) fir_dh_reduce_kernel(const RaggedChan *chans, const int *start,
-                                                             const float *part, float *gtaps)
-{
-   const RaggedChan c = chans[blockIdx.x];
-   for (int cc = threadIdx.x; cc < c.T; cc += 256) {
-      double s = 0.0;
-      for (int i = start[blockIdx.x]; i < start[blockIdx.x + 1]; i++) s += part[(long long) i * kDhMaxT + cc];
-      gtaps[c.hOff + c.T - 1 - cc] = (float) s;
-   }
-}
 
 // Mean squared error over the valid output samples: gy = scale * (y - target)
 // (scale = 2 / n), zero on each channel's T - 1 tail samples; per-item FP64
@@ -644,25 +633,20 @@ static cudaError_t launchFirAndTables(const RaggedPlan *p, const BankLaunch &b, 
    return e != cudaSuccess ? e : j;
 }
 
-// The adjoint behind the output gradient's aggregates: cascade, the coefficient gradients' sums, then
-// the FIR's input and taps gradients.  The sums are not run beside the FIR's kernels: their CTAs
-// either come first by luck or find every SM held, as above (16 channels of 400 to 900 thousand
+// The adjoint behind the output gradient's aggregates: cascade, the FIR's input and taps gradients, then
+// the coefficient and taps gradients' sums.  The coefficients' are not run beside the FIR's kernels: their
+// CTAs either come first by luck or find every SM held, as above (16 channels of 400 to 900 thousand
 // samples: 23 us, or 222; backward 342 us captured, 476 eager).
 static cudaError_t launchAdjoint(const RaggedPlan *p, BankLaunch &b, const float *x, const float *taps, float *gx,
                                  float *gtaps, float *scratch, cudaStream_t s)
 {
    b.nAux = p->bucketS.size() > 1 && auxFree(p, s) ? p->nAux : 0; // one bucket stays on the caller's stream
    cudaError_t e = launchBankBackward(b, s);
-   if (e == cudaSuccess) e = launchBankCoefGradients(b, s);
    float *part = scratch + p->sDh;
    if (e == cudaSuccess)
       e = launchFirBf16x3Ragged(p->dChan, p->dFirDxRuns, p->nFirDxRuns, b.g, taps, gx, true, p->Tmax, p->err, s);
    if (e == cudaSuccess) e = launchFirDhBf16x3Ragged(p->dChan, p->dDhRuns, p->nDhRuns, x, b.g, part, p->err, s);
-   if (e == cudaSuccess) {
-      fir_dh_reduce_kernel<<<p->C, 256, 0, s>>>(p->dChan, p->dDhStart, part, gtaps);
-      countLaunch();
-      e = cudaGetLastError();
-   }
+   if (e == cudaSuccess) e = launchBankSums(b, p->dDhStart, part, gtaps, s);
    return e;
 }
 
