@@ -208,6 +208,28 @@ def test_opt_single_sample_multi_stage(C):
 
 
 @pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("C,full,N", [(161, 192, 9000), (33, 64, 2049), (17, 32, 700), (3201, 3216, 1500)])
+def test_opt_last_group_partly_filled(form, C, full, N):
+    """Channels of a partly filled last group, over several windows, equal those of a full one bit for
+    bit, samples that are not finite in the last channel included."""
+    rng = np.random.default_rng(C)
+    S = 3
+    x = rng.standard_normal((N, full)).astype(np.float32)
+    x[N // 3, C - 1] = np.nan
+    nat = stable_sections(rng, 1, S)
+    opt, _ = D.opt_coefficients(nat, form, 0, full)
+    st = (rng.standard_normal((S * nv(form), full)) * 0.5).astype(np.float32)
+    got = []
+    for n in (full, C):
+        sd = dev(st[:, :n])
+        y = host(D.cascade_biquad(dev(x[:, :n]), dev(opt), sd, form=form, nch=0))
+        got.append((y[:, :C], host(sd)[:, :C]))
+    for a, b in zip(*got):
+        assert np.array_equal(a, b, equal_nan=True)
+    assert np.isfinite(got[1][0][:, :C - 1]).all()
+
+
+@pytest.mark.parametrize("form", FORMS)
 def test_opt_more_than_a_million_channels(form):
     """More groups of 16 channels than a grid's second dimension holds (65535)."""
     N, C, S = 2, 16 * 65535 + 21, 1
