@@ -87,8 +87,9 @@ template <typename T, int P> struct IntShape {
       return n == 1 ? chunks * 16 : ((chunks * 16 + 63) / 128) * 128 + 64;
    }
    __host__ __device__ static int plane(int taps) { return P / 16 * part(taps); }
-   __host__ __device__ static int taps(int t) { return (K(t) + P + 4 + 15) / 16 * 16; }    // bytes of gb, one plane
-   __host__ __device__ static int band(int t) { return (K(t) - 16 + P) * 16; }             // bytes, one plane
+   static constexpr int lead = per - 1; // longest
+   __host__ __device__ static int taps(int t) { return (K(t) + P + lead + 4 + 15) / 16 * 16; } // bytes of gb, one plane
+   __host__ __device__ static int band(int t) { return (K(t) - 16 + P + lead) * 16; }          // bytes, one plane
    __host__ __device__ static size_t smem(int t) { return 16 + (size_t) planes * (taps(t) + band(t) + 2 * plane(t)); }
 };
 
@@ -168,7 +169,8 @@ template <typename T, int P> __host__ __device__ inline int intTiles(const FirLa
    return (int) (((long long) a.outSize + (aligned ? 0 : al - 1) + kRows * P - 1) / (kRows * P));
 }
 
-template <typename T, int QMODE, int P>
+// ONE: shared taps and channels of one tile each.
+template <typename T, int QMODE, int P, bool ONE>
 __global__ void __launch_bounds__(kThreads, IntShape<T, P>::perSm(QMODE)) fir_int_tc_kernel(FirLaunch a, uint32_t tilesPerRun)
 {
    using Sh = IntShape<T, P>;
@@ -180,7 +182,7 @@ __global__ void __launch_bounds__(kThreads, IntShape<T, P>::perSm(QMODE)) fir_in
    uint64_t *mbar = (uint64_t *) sm;
    uint32_t *tslot = (uint32_t *) (sm + 8);
    // Reversed taps g[c] = h[T-1-c] as bytes (int16: high and low byte planes) at byte
-   // P - 1 + lead + c of gb0 / gb1, zero elsewhere: one 32-bit word per thread to build.
+   // P - 1 + bandLead + c of gb0 / gb1, zero elsewhere: one 32-bit word per thread to build.
    uint32_t *gb0 = (uint32_t *) (sm + 16);
    uint32_t *gb1 = (uint32_t *) (sm + 16 + Sh::taps(T_));
    unsigned char *B0 = sm + 16 + Sh::planes * Sh::taps(T_);
@@ -198,7 +200,11 @@ __global__ void __launch_bounds__(kThreads, IntShape<T, P>::perSm(QMODE)) fir_in
 
    const int inExtent = a.outSize + T_ - 1;
    // Runs of tilesPerRun consecutive tiles (of all channels in turn); CTAs stride over the runs.
-   // The band is built anew when the channel's taps or its lead are others than the last tile's.
+   // The band is built anew when the channel's taps or its lead are others than the last tile's; shared
+   // taps of channels of one tile each are built for the longest lead, and the shorter ones read the
+   // band from a later start (anew for each lead, 3000 channels x 3347 int16 samples x 2048 taps took 131 us
+   // instead of 109; but a start off the 128-byte boundary slows the MMAs' reads: 4096 channels x 16384 int8
+   // samples x 128 taps, five tiles a channel, 43.3 us so, 41.7 built anew).
    const uint32_t nt = (uint32_t) intTiles<T, P>(a);
    const uint32_t nTiles = (uint32_t) a.batch * nt; // with the grid below 2^32: memory bounds it
    auto rowOf = [&](int l) {
@@ -268,14 +274,14 @@ __global__ void __launch_bounds__(kThreads, IntShape<T, P>::perSm(QMODE)) fir_in
             }
          }
       }
-      if (bandOf < 0 || (a.filtPitch != 0 && bandOf != r.l) || bandLead != r.lead) {
+      if (ONE ? bandOf < 0 : bandOf < 0 || (a.filtPitch != 0 && bandOf != r.l) || bandLead != r.lead) {
          const T *h = (const T *) a.h + (long long) r.l * a.filtPitch;
          // the previous band's last MMAs are complete (waited); its words were read before that
          for (int wd = tid; wd < Sh::taps(T_) / 4; wd += kThreads) {
             uint32_t w0 = 0, w1 = 0;
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-               const int c = 4 * wd + j - (P - 1) - r.lead;
+               const int c = 4 * wd + j - (P - 1) - (ONE ? Sh::lead : r.lead);
                const int g = (c >= 0 && c < T_) ? (int) h[T_ - 1 - c] : 0;
                if (SPLIT) {
                   w0 |= (uint32_t) ((g >> 8) & 0xFF) << (8 * j);
@@ -290,10 +296,10 @@ __global__ void __launch_bounds__(kThreads, IntShape<T, P>::perSm(QMODE)) fir_in
          }
          __syncthreads();
          // Taps band, K-major no-swizzle, phases in reverse (column n = phase P-1-n): element
-         // (m, n) = g[m + n - (P-1) - lead] = byte m + n of gb, so the 16-byte chunk of m = 16q,
-         // column n depends on 16q + n alone and is held once, at 16 (16q + n); gathered from
-         // five words with funnel shifts.
-         for (int ch = tid; ch < Kt - 16 + P; ch += kThreads) {
+         // (m, n) = g[m + n - (P-1) - lead] = byte m + n + bandLead - lead of gb, so the 16-byte chunk of
+         // m = 16q, column n depends on 16q + n alone and is held once, at 16 (16q + n + bandLead - lead);
+         // gathered from five words with funnel shifts.
+         for (int ch = tid; ch < Kt - 16 + P + (ONE ? Sh::lead : 0); ch += kThreads) {
             const int w = ch >> 2, sh = (ch & 3) * 8;
 #pragma unroll
             for (int pl = 0; pl < Sh::planes; pl++) {
@@ -308,7 +314,7 @@ __global__ void __launch_bounds__(kThreads, IntShape<T, P>::perSm(QMODE)) fir_in
             }
          }
          bandOf = r.l;
-         bandLead = r.lead;
+         bandLead = ONE ? Sh::lead : r.lead;
       }
       if (!SPLIT) cpAsyncWaitAll();
       tc::fenceProxyAsync();
@@ -322,7 +328,9 @@ __global__ void __launch_bounds__(kThreads, IntShape<T, P>::perSm(QMODE)) fir_in
          const uint32_t lbo = al ? al : (uint32_t) part;
          const uint64_t dA0 = tc::descNoSwizzle(tc::smemAddr(A(buf, 0)), lbo, 128);
          const uint64_t dA1 = tc::descNoSwizzle(tc::smemAddr(A(buf, 1)), lbo, 128);
-         uint64_t dB0 = tc::descNoSwizzle(tc::smemAddr(B0), 256, 128), dB1 = tc::descNoSwizzle(tc::smemAddr(B1), 256, 128);
+         const uint32_t skip = ONE ? 16 * (Sh::lead - r.lead) : 0;
+         uint64_t dB0 = tc::descNoSwizzle(tc::smemAddr(B0) + skip, 256, 128);
+         uint64_t dB1 = tc::descNoSwizzle(tc::smemAddr(B1) + skip, 256, 128);
          // 32 taps a step: two chunks of the segment, 512 bytes of the band (descriptor addresses count 16)
          for (int kk = 0; kk < Kt / 32; kk++, dB0 += 32, dB1 += 32) {
             const uint32_t off = (2 * kk % kParts) * (part / 16) + 2 * kk / kParts;
@@ -437,7 +445,8 @@ template <typename T, int QMODE, int P> static cudaError_t launchIntTcP(const Fi
 {
    using Sh = IntShape<T, P>;
    const size_t smem = Sh::smem(a.T);
-   auto fn = fir_int_tc_kernel<T, QMODE, P>;
+   const auto fn = a.filtPitch == 0 && intTiles<T, P>(a) == 1 ? fir_int_tc_kernel<T, QMODE, P, true>
+                                                              : fir_int_tc_kernel<T, QMODE, P, false>;
    // the same limit for every call: calls on several threads do not lower each other's
    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) Sh::smem(kMaxTapsTc));
    if (e != cudaSuccess) return e;

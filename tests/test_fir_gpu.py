@@ -189,6 +189,26 @@ def _relerr(y, y64):
     return np.max(np.abs(y.astype(np.float64) - y64), axis=1) / np.maximum(np.max(np.abs(y64), axis=1), 1e-30)
 
 
+@pytest.mark.parametrize("dt,qmode", [(np.int8, 0), (np.int8, 1), (np.int16, 0), (np.int16, 1)])
+@pytest.mark.parametrize("out,T,gap", [(1, 1, 0), (37, 200, 0), (37, 201, 1), (1300, 64, 5), (2033, 33, 3), (9, 2048, 7)])
+def test_int_tensor_core_shared_taps_short_channels(dt, qmode, out, T, gap):
+    """Channels of one tile with shared taps and rows on every alignment: one band for all leads, more
+    channels than CTAs where they are short."""
+    B, N = 2500 if out < 100 and T < 1000 else 300, out + T - 1
+    rng = np.random.default_rng(out + T)
+    x = rand(dt, (B, N + gap), rng)
+    h = rand(dt, (1, T), rng)
+    args, pin, pfilt, pout = D.fir_setup(_NP_CODE[dt], B, N, T, nch=0, shift=6 if qmode else 0, in_pitch=N + gap)
+    hd = D.FirHandle()
+    assert hd.init(args, pin, pfilt, pout) == D.SUCCESS
+    hd.set_qmode(bool(qmode))
+    yd = dev(np.zeros((B, out), dt))
+    assert hd.exec(dev(x), dev(h), yd) == D.SUCCESS, hd.last_error()
+    xs = np.ascontiguousarray(x[:, :N])
+    want = oracle.fir_q(xs, h, T, 6, nch=0) if qmode else oracle.fir(xs, h, T, nch=0)
+    assert np.array_equal(host(yd), want)
+
+
 @pytest.mark.parametrize("nch", [0, 1])
 def test_simt_float_accuracy(nch):
     rng = np.random.default_rng(9)
