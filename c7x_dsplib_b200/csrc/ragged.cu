@@ -10,7 +10,7 @@
 //   fir_bf16x3_ragged_kernel (fir_tc.cu)  FIR forward (valid correlation) and
 //                          input gradient (full convolution with the same taps)
 //                          as split-BF16x3 tcgen05 contractions over runs of
-//                          8192-output tiles, one run per CTA.
+//                          8192-output tiles, one persistent CTA an SM.
 //   bank_tables_kernel, bank_transition_kernel, bank_unit_kernel, bank_chain_kernel,
 //   bank_adjoint_kernel, bank_sums_kernel (bank_scan.cu)
 //                          the cascade split along time into 1024-sample units
@@ -344,8 +344,8 @@ static DSPLIB_STATUS raggedPlanBuild(DSPLIB_gpu_raggedPlan *plan, int32_t numCha
    p->nFirFwdRuns = (int) firFwd.size();
    p->nFirDxRuns = (int) firDx.size();
    // deepest cascades first, one bucket per stage count: the adjoint's last pass sizes its
-   // shared memory per bucket (stage sequences of S - 1 stages), so shallow cascades pack
-   // more warps per SM
+   // shared memory per bucket (its stage tables and the sequences of a group of stages), so
+   // shallow cascades pack more warps per SM
    std::stable_sort(units.begin(), units.end(),
                     [&](const int2 &a, const int2 &b) { return stages[a.x] > stages[b.x]; });
    for (size_t i = 0; i < units.size(); i++)
@@ -609,10 +609,10 @@ static cudaError_t sideJoin(const RaggedPlan *p, cudaStream_t s)
 // FIR forward and the stage tables and unit transitions, which depend on the coefficients alone:
 // side by side where the FIR's CTAs (one an SM) leave SMs free for the transitions' two CTAs a
 // channel, one to an SM or, single warps, two; else in turn.  CTAs that find every SM held by the
-// FIR are all placed on the first SMs that it leaves, and share them: 512 channels of at
-// most 4096 samples, 8 stages, captured, forward 105 us side by side and 63 in turn, 50 channels
-// of 60000 and 32 stages 427 and 354, 256 of at most 262144 143 and 133, 2048 521 and 525; with
-// SMs free 20 channels of at most 20000 32 and 40, 70 of at most 5169 46 and 51.
+// FIR are all placed on the first SMs that it leaves, and share them.  Captured forward, side by side and
+// in turn, us: 512 channels of at most 4096 samples, 8 stages 81 and 53; 140 of at most 3000 69 and
+// 41; 100 of 60000, 24 stages 457 and 298; 256 of at most 262144 132 and 127, 2048 506 and 511; with SMs
+// free 20 channels of at most 20000 27 and 34, 70 of at most 5169 35 and 41, 30 of at most 100000 41 and 51.
 static bool tablesBeside(const RaggedPlan *p, cudaStream_t s)
 {
    const int sms = deviceSms() > 0 ? deviceSms() : 148;
@@ -636,7 +636,7 @@ static cudaError_t launchFirAndTables(const RaggedPlan *p, const BankLaunch &b, 
 // The adjoint behind the output gradient's aggregates: cascade, the FIR's input and taps gradients, then
 // the coefficient and taps gradients' sums.  The coefficients' are not run beside the FIR's kernels: their
 // CTAs either come first by luck or find every SM held, as above (16 channels of 400 to 900 thousand
-// samples: 23 us, or 222; backward 342 us captured, 476 eager).
+// samples, lanes along the units: 23 us, or 222; backward 342 us captured, 476 eager).
 static cudaError_t launchAdjoint(const RaggedPlan *p, BankLaunch &b, const float *x, const float *taps, float *gx,
                                  float *gtaps, float *scratch, cudaStream_t s)
 {

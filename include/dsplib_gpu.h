@@ -162,7 +162,7 @@ DSPLIB_STATUS DSPLIB_gpu_firStreamReset(DSPLIB_gpu_firStream stream);
 DSPLIB_STATUS DSPLIB_gpu_firStreamDestroy(DSPLIB_gpu_firStream stream);
 
 /** Adjoint of DSPLIB_fir (FLOAT32, FP32 CUDA-core kernels) over dense device rows, queued on the
- *  given cudaStream_t: from gy [batch, dataSize - filterSize + 1], x [batch, dataSize] and stored
+ *  given cudaStream_t of the current device, whose memory the rows are in: from gy [batch, dataSize - filterSize + 1], x [batch, dataSize] and stored
  *  taps h [tapRows, filterSize] (1 row shared by all channels, or batch) the gradients
  *  gx [batch, dataSize] and gh [batch, filterSize] (per channel also for shared taps: their sum
  *  over the channels is the caller's).  Either may be NULL.  scratch:
