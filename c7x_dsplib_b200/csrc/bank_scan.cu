@@ -25,7 +25,7 @@
 //   pass 1 (bank_agg_kernel): e of every unit but the channel's last, by filtering it from a
 //           zero state.  (As dot products with the impulse responses from the cascade's
 //           input to each stage's internal sequence, two multiply-adds a sample and stage
-//           instead of seven: 1603 us a step against 1604 on 2048 channels of up to 262144
+//           instead of seven: 1603 us a step against 1587 on 2048 channels of up to 262144
 //           samples, the adjoint 4 % faster on a thousand channels of 20000 samples and 12 to 24
 //           stages, the forward up to 17 % slower on channels of 1100 to 6000 samples; and the
 //           responses take 8 KB of work buffer a channel and stage, 138 MB instead of 70 for
@@ -518,7 +518,8 @@ __device__ __forceinline__ void zeroStateEndRev(const P2 (&g)[kL], const StageCo
 // Initial states (w1, w2) of this lane's chunks, packed, from the zero-state end states.  Forward
 // time: the lane's end state is M e_A + e_B; the first lane's takes the unit's entry before
 // the scan over the lanes (maps of 32 samples: powers of M^2 = P[1]), which then carries it on.
-__device__ __forceinline__ void chunkStateUp(P2 e1, P2 e2, float2 entry, const float *tb, int lane, P2 &w1, P2 &w2)
+// Returns the state at the lane's end.
+__device__ __forceinline__ float2 chunkStateUp(P2 e1, P2 e2, float2 entry, const float *tb, int lane, P2 &w1, P2 &w2)
 {
    const float2 x = up(e1), y = up(e2);
    const float2 eA = make_float2(x.x, y.x), eB = make_float2(x.y, y.y);
@@ -535,10 +536,11 @@ __device__ __forceinline__ void chunkStateUp(P2 e1, P2 e2, float2 entry, const f
    const float2 b = scan::affine(M, a, eA);
    w1 = pk(a.x, b.x);
    w2 = pk(a.y, b.y);
+   return val;
 }
 
 // Reverse time: chunk B comes before A, lane 31 first.
-__device__ __forceinline__ void chunkStateDown(P2 e1, P2 e2, float2 entry, const float *tb, int lane, P2 &v1, P2 &v2)
+__device__ __forceinline__ float2 chunkStateDown(P2 e1, P2 e2, float2 entry, const float *tb, int lane, P2 &v1, P2 &v2)
 {
    const float2 x = up(e1), y = up(e2);
    const float2 eA = make_float2(x.x, y.x), eB = make_float2(x.y, y.y);
@@ -555,6 +557,7 @@ __device__ __forceinline__ void chunkStateDown(P2 e1, P2 e2, float2 entry, const
    const float2 a = scan::affine(M, b, eB);
    v1 = pk(a.x, b.x);
    v2 = pk(a.y, b.y);
+   return val;
 }
 
 // One stage of the forward cascade over a unit, in place; keep(i, w) takes its internal sequence.
@@ -573,24 +576,6 @@ __device__ __forceinline__ void forwardStage(P2 (&v)[kL], float2 entry, const fl
       q2 = q1;
       q1 = w;
    }
-}
-
-// One stage of the reverse cascade over a unit that starts (at its end in time) from a zero state,
-// in place; lane 0 returns the state at the unit's beginning in time.
-__device__ __forceinline__ float2 reverseStageZero(P2 (&g)[kL], const float *tb, int lane)
-{
-   const StageCoef c = stageCoef(tb);
-   P2 n1, n2;
-   zeroStateEndRev(g, c, n1, n2);
-   chunkStateDown(n1, n2, make_float2(0.0f, 0.0f), tb, lane, n1, n2);
-#pragma unroll
-   for (int i = kL - 1; i >= 0; i--) {
-      const P2 v = fma2(c.na1, n1, fma2(c.na2, n2, g[i]));
-      g[i] = fma2(c.b0, v, fma2(c.b1, n1, mul2(c.b2, n2)));
-      n2 = n1;
-      n1 = v;
-   }
-   return make_float2(up(n1).x, up(n2).x);
 }
 
 // A unit's per-stage states, read once: lane l holds stage l in lo and stage l + 32 in hi
@@ -647,23 +632,28 @@ __device__ __forceinline__ void loadTables(float *dst, const float *tables, cons
    __syncwarp();
 }
 
-// Aggregates of a unit (held by the warp, overwritten): its stages' end states from a zero state.
+// Aggregates of a unit (held by the warp, overwritten): its stages' end states from a zero state,
+// as the scans over the lanes give them; the last stage is not run again for its output.
 template <bool ADJ>
 __device__ __forceinline__ void unitAggregates(P2 (&v)[kL], const float *sTab, int S, float2 *agg, int lane)
 {
+   const float2 zero = make_float2(0.0f, 0.0f);
    for (int p = 0; p < S; p++) {
       const float *tb = sTab + stageAt(p, S, ADJ) * kBankTabFloats;
-      if (ADJ) {
-         const float2 e = reverseStageZero(v, tb, lane);
-         if (lane == 0) agg[p] = e;
-      }
-      else {
-         P2 w1, w2;
-         forwardStage(v, make_float2(0.0f, 0.0f), tb, lane, [&](int i, P2 w) {
-            if (i == kL - 1) w1 = w;
-            if (i == kL - 2) w2 = w;
-         });
-         if (lane == 31) agg[p] = make_float2(up(w1).y, up(w2).y);
+      const StageCoef c = stageCoef(tb);
+      P2 q1, q2;
+      if (ADJ) zeroStateEndRev(v, c, q1, q2);
+      else zeroStateEnd(v, c, q1, q2);
+      const float2 end = ADJ ? chunkStateDown(q1, q2, zero, tb, lane, q1, q2) : chunkStateUp(q1, q2, zero, tb, lane, q1, q2);
+      if (lane == (ADJ ? 0 : 31)) agg[p] = end;
+      if (p + 1 == S) break;
+#pragma unroll
+      for (int k = 0; k < kL; k++) {
+         const int i = ADJ ? kL - 1 - k : k;
+         const P2 w = fma2(c.na1, q1, fma2(c.na2, q2, v[i]));
+         v[i] = fma2(c.b0, w, fma2(c.b1, q1, mul2(c.b2, q2)));
+         q2 = q1;
+         q1 = w;
       }
    }
 }
