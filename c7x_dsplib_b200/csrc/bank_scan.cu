@@ -6,7 +6,7 @@
 // as packed pairs (A_i, B_i): every FP32 operation on samples is a packed one (fma.rn.f32x2,
 // each half rounded as fmaf).  The FMA pipe's rate is the same, but a packed instruction takes
 // half the issue slots, and one warp scan serves 1024 samples instead of 512.  These passes wait
-// on latency: issue slots 31 to 55 % used, the FMA pipe 22 to 57 %, 10 to 38 % of the warps resident.  Per
+// on latency: issue slots 30 to 55 % used, the FMA pipe 22 to 52 %, 10 to 43 % of the warps resident.  Per
 // stage the chunks are run from a zero state for their end states, a lane's two
 // end states combine, the lanes' end states are combined by a warp scan of the affine maps
 // s -> M s + e (M = A^16 and its powers, A the stage's 2x2 companion matrix,
