@@ -470,6 +470,7 @@ DSPLIB_STATUS DSPLIB_cascadeBiquad_exec(DSPLIB_kernelHandle handle,
    a.varPitch = p->varPitch;
    a.coefPitch = coefPitch;
    a.prefetch = (!rin.onHost || rin.staged) ? 1 : 0; // not for mapped host memory
+   a.mapped = (rin.onHost && !rin.staged) || (rout.onHost && !rout.staged);
    if (!natc) a.tuneChoice = bqChoice(p, bqShape(p));
    auto launch = [&](const BiquadLaunch &l, cudaStream_t st) {
       return natc ? launchBiquadSequential(l, st) : launchBiquadScan(l, st);

@@ -1093,7 +1093,9 @@ template <int FORM> cudaError_t launchChanForm(const BiquadLaunch &a, cudaStream
 //    scanning along time;
 //  * below 2048 samples, half rows of 16 channels: twice the CTAs, without the cluster barriers
 //    that would pay only from four windows on (512 channels x 300: 8.4 against 10.5; x 1024: 10.5
-//    against 12.5 in clusters of two; 203 x 1500: 18.6 against 24.9);
+//    against 12.5 in clusters of two; 203 x 1500: 18.6 against 24.9); but whole rows of 32 of more than 64
+//    channels in host memory used in place, which crosses the bus in pieces of a row (1000 x 1000: 190
+//    against 223), in the same windows of 512, so that the results are those of device memory bit for bit;
 //  * DF2 and TIF: 64-sample chunks in clusters, the largest power of two that its windows fill:
 //    16 for up to 7 groups of 32 channels (no more are co-resident), 8 or fewer with at most
 //    384 CTAs, two an SM (32 x 8192: 12.5 against 14.6 in 32-sample chunks; 1024 x 8192: 36
@@ -1119,8 +1121,10 @@ template <int FORM> cudaError_t launchScanForm(const BiquadLaunch &a, cudaStream
    const int groups = (a.C + 31) / 32;
    constexpr bool packed = FORM == DSPLIB_BIQUAD_DF2 || FORM == DSPLIB_BIQUAD_TIF;
    const int windows = a.N / 512;
-   if (windows < 4) return launchScanShape<FORM, 8, kShortChunk, 2>(a, 1, s);
    int K = 1, KL = 1;
+   if (windows < 4)
+      return a.mapped && groups > 2 ? launchScanShape<FORM, 16, kShortChunk>(a, 1, s)
+                                    : launchScanShape<FORM, 8, kShortChunk, 2>(a, 1, s);
    while (K < 16 && K * 2 <= windows && groups * K * 2 <= 112) K *= 2;
    while (KL < 8 && KL * 2 <= windows && groups * KL * 2 <= (packed ? 384 : 256)) KL *= 2;
    if (packed) {

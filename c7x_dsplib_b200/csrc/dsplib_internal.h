@@ -391,6 +391,7 @@ struct BiquadLaunch {
    int N, C, S;
    long long inPitch, outPitch, varPitch, coefPitch; // elements
    int prefetch = 0; // x is device memory: the scan kernel may fetch the next window early (cp.async)
+   int mapped = 0;   // x or y is host memory used in place
    int tuneChoice = -1; // scan shape from the autotuner: 100 * warps per CTA (32, 33: half rows, 64: long chunks)
                         // + CTAs per cluster, or 1 for the per-channel kernel (-1: the rule)
 };

@@ -416,6 +416,24 @@ def test_opt_pinned_host_buffers_read_in_place(form):
 
 
 @pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("N,C", [(1, 40), (300, 33), (511, 64), (1000, 100), (2047, 49), (2048, 100)])
+def test_opt_short_pinned_signals_equal_device_ones(form, N, C):
+    """Below 2048 samples more than 64 channels in host memory used in place are read in whole rows, device
+    memory in half rows: the results are the same bit for bit."""
+    rng = np.random.default_rng(N + C)
+    S = 3
+    x = rng.standard_normal((N, C)).astype(np.float32)
+    opt, _ = D.opt_coefficients(stable_sections(rng, 1, S), form, 0, C)
+    st0 = (rng.standard_normal((S * nv(form), C)) * 0.1).astype(np.float32)
+    sd = dev(st0)
+    want = host(D.cascade_biquad(dev(x), dev(opt), sd, form=form, nch=0))
+    hs, hy = torch.from_numpy(st0.copy()).pin_memory(), torch.zeros(N, C).pin_memory()
+    D.cascade_biquad(torch.from_numpy(x).pin_memory(), torch.from_numpy(opt).pin_memory(), hs, form=form, nch=0, out=hy)
+    assert np.array_equal(hy.numpy(), want)
+    assert np.array_equal(hs.numpy(), host(sd))
+
+
+@pytest.mark.parametrize("form", FORMS)
 @pytest.mark.parametrize("C,pinned,in_place", [(40, True, False), (16, True, False), (40, True, True),
                                                (40, False, False)])
 def test_opt_large_host_signals(form, C, pinned, in_place):
