@@ -303,9 +303,12 @@ __device__ __forceinline__ void loadRows(float *rows, const double *P, int n2, i
    }
 }
 
-// z' = row . z + e (lane r: component r), z broadcast from lanes 0 .. n2 - 1.
+// z' = row . z + e (lane r: component r), z broadcast from lanes 0 .. n2 - 1.  A zero state stays out of
+// the products: the transition of an unstable cascade may exceed FP32 (1024 samples of a pole at 1.09, or
+// 32 units of one at 1.003), which is nothing to a signal that has not begun.
 __device__ __forceinline__ float chainStep(const float *row, float z, float e, int n2)
 {
+   if (!__any_sync(0xffffffffu, z != 0.0f)) return e;
    float a0 = e, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
 #pragma unroll
    for (int q = 0; q < 2 * kChainFastStages; q += 4) {

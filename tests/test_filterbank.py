@@ -550,6 +550,37 @@ def test_plan_in_two_captures_at_once():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("L,radius,start", [(3000, 1.1, 2600), (2100, 1.12, 1700), (100_000, 1.003, 85_000)])
+def test_bank_unstable_cascades_before_the_signal_begins(L, radius, start):
+    """Poles outside the unit circle and a signal (for the adjoint: a gradient) of zeros but for its last
+    (first) samples: finite and as exact as ever, although the response over a unit, or over 32 of them,
+    is beyond FP32."""
+    import torch
+
+    from c7x_dsplib_b200.filterbank import RaggedFilterBank
+
+    rng = np.random.default_rng(L)
+    S, th = 2, 0.7
+    bank = RaggedFilterBank([L], [1], [S])
+    c = np.array([[1.0, 0.3, 0.2, -2 * radius * np.cos(th), radius * radius], [0.8, -0.1, 0.1, -0.9, 0.4]], np.float32)
+    x, gy = np.zeros(L, np.float32), np.zeros(L, np.float32)
+    x[start:] = rng.standard_normal(L - start)
+    gy[:L - start] = rng.standard_normal(L - start)
+    d = [torch.tensor(a, device="cuda") for a in (x, np.ones(1, np.float32), c.reshape(-1), gy)]
+    y, work = torch.empty(L, device="cuda"), torch.empty(bank.sizes[3], device="cuda")
+    gx, gh, gc = (torch.empty_like(t) for t in d[:3])
+    bank.forward_raw(*d[:3], y, work)
+    bank.backward_raw(*d[:3], work, d[3], gx, gh, gc, torch.empty(bank.sizes[4], device="cuda"))
+    h64 = np.ones(1)
+    y64 = bank_forward([L], [1], [S], x.astype(np.float64), h64, c.astype(np.float64).reshape(-1))
+    gx64 = bank_adjoint([L], [1], [S], x.astype(np.float64), h64, c.astype(np.float64).reshape(-1), gy.astype(np.float64))[0]
+    for got, want in ((y, y64), (gx, gx64)):
+        got = got.cpu().numpy().astype(np.float64)
+        assert np.isfinite(want).all() and np.isfinite(got).all()
+        assert np.abs(got - want).max() <= Y_TOL * np.abs(want).max()
+
+
+@pytest.mark.gpu
 def test_bank_deep_cascades_beyond_shared_memory():
     """24 and 22 stages beside shallow ones: the unit transitions of deep cascades
     (48 x 48 state) and the adjoint's per-stage sequences in shared memory."""
